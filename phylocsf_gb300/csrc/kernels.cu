@@ -156,12 +156,13 @@ cudaError_t launch_jacobi(const double *A, double *U, double *lam, int *status, 
 // Output is E^T: Pbuf[(r*nbr + b)*K2 + j*K + i] = E[i][j].
 
 constexpr int PF_THREADS = 256;
-constexpr int PF_BRANCHES = 4;   // branches per CTA (the eigenvectors are staged once)
+constexpr int PF_BRANCHES = 4;   // most branches per CTA (the eigenvectors are staged once)
+constexpr int PF_SPREAD = 2 * 4 * 152;   // FP32 matrices of a launch up to which each gets its own CTA
 
 template <typename T>
 __global__ void __launch_bounds__(PF_THREADS) k_pform(const PSet *ps, const double *branch, int nbr,
                                                        DevModels m, T *Pbuf, int32_t *status_key, int raw,
-                                                       float *Bop, int bop_nl, float *dlo)
+                                                       float *Bop, int bop_nl, float *dlo, int per_cta)
 {
     extern __shared__ __align__(16) unsigned char psm[];
     T *UT = reinterpret_cast<T *>(psm);     // [K][K]   UT[m][j] = U[j][m]
@@ -195,8 +196,8 @@ __global__ void __launch_bounds__(PF_THREADS) k_pform(const PSet *ps, const doub
     const int ty = tid / 16, tx = tid % 16;
     // per branch of this CTA, in parallel (one thread each; FP64 is a narrow pipe here):
     // 0: direct eigen formula (FP64);  1: t == 0;  2: Taylor below the grid;  3: grid correction
-    if (tid < PF_BRANCHES) {
-        const int b = blockIdx.x * PF_BRANCHES + tid;
+    if (tid < per_cta) {
+        const int b = blockIdx.x * per_cta + tid;
         int mode = 0, g = 0;
         if (b < nbr && fp32 && m.grid_n > 0) {
             const double t = rq.rho * branch[b];
@@ -214,8 +215,8 @@ __global__ void __launch_bounds__(PF_THREADS) k_pform(const PSet *ps, const doub
         mode_s[tid] = mode;
         grid_s[tid] = g;
     }
-    for (int bi = 0; bi < PF_BRANCHES; bi++) {
-        const int b = blockIdx.x * PF_BRANCHES + bi;
+    for (int bi = 0; bi < per_cta; bi++) {
+        const int b = blockIdx.x * per_cta + bi;
         if (b >= nbr) break;                       // uniform across the block
         const double t = rq.rho * branch[b];
         __syncthreads();                           // UT and the branch table ready / previous branch done with smem
@@ -346,13 +347,19 @@ cudaError_t launch_pform(bool fp64, const PSet *req, int nreq, const double *bra
                          void *Pbuf, int32_t *status_key, cudaStream_t s, bool raw, float *bop, int bop_nl, float *dlo)
 {
     if (nreq <= 0) return cudaSuccess;
-    dim3 grid((nbr + PF_BRANCHES - 1) / PF_BRANCHES, nreq);
+    // Four branches per CTA share the staged eigenvectors.  One per CTA where that staging is
+    // nothing beside the product (FP64 runs at 1/64 of the FP32 rate: ~70 us per branch) and
+    // for short FP32 launches, which four would leave on a part of the SMs.  Measured: FP64,
+    // 24 P sets of 29 leaves 0.95 -> 0.69 ms, six of 12 leaves 0.36 -> 0.13 ms; FP32, two P
+    // sets of 12 leaves 39 -> 17 us.
+    const int per_cta = (fp64 || (int64_t)nreq * nbr <= PF_SPREAD) ? 1 : PF_BRANCHES;
+    dim3 grid((nbr + per_cta - 1) / per_cta, nreq);
     if (fp64) {
         size_t smem = sizeof(double) * (2 * K2 + K * (K + 1) + 4 * K);
         cudaError_t e = cudaFuncSetAttribute(k_pform<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         k_pform<double><<<grid, PF_THREADS, smem, s>>>(req, branch, nbr, m, (double *)Pbuf, status_key, raw ? 1 : 0,
-                                                       nullptr, 0, nullptr);
+                                                       nullptr, 0, nullptr, per_cta);
     } else {
         size_t smem = sizeof(float) * (2 * K2 + K * (K + 1) + 2 * K);
         smem = (smem + 15) & ~size_t(15);
@@ -360,7 +367,7 @@ cudaError_t launch_pform(bool fp64, const PSet *req, int nreq, const double *bra
         cudaError_t e = cudaFuncSetAttribute(k_pform<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         k_pform<float><<<grid, PF_THREADS, smem, s>>>(req, branch, nbr, m, (float *)Pbuf, status_key, raw ? 1 : 0,
-                                                      bop, bop_nl, raw ? nullptr : dlo);
+                                                      bop, bop_nl, raw ? nullptr : dlo, per_cta);
     }
     return cudaGetLastError();
 }

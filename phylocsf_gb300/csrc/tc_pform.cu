@@ -16,12 +16,14 @@
 // leaves (row gathers) and the pre-split B operand for the branches above
 // internal nodes.
 //
-// One CTA (128 threads) per P set walks its branch pairs.  A_hi sits in tensor
+// One CTA (128 threads) walks the branch pairs of one P set, or a part of them when the
+// launch has few P sets (launch_pform_tc).  A_hi sits in tensor
 // memory (columns 64..127, lane r = row r) and only A_lo in shared memory, so a CTA
 // takes 64 KB of shared memory and 128 tensor-memory columns and three CTAs share an
 // SM (the kernel is bound by the latency of its per-pair chain).  mbarrier waits are bounded as in the pruning
 // kernel; on timeout the CTA records an error, waits (bounded) for its MMAs,
 // frees its tensor memory and stops.
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 
@@ -37,10 +39,11 @@ constexpr uint32_t PFT_A = 32768;      // [128 x 64]  A_lo, 32 KB
 constexpr uint32_t PFT_SMEM = 65536;
 constexpr uint32_t PFT_TMEM_COLS = 128;   // D in 0..63, A_hi in 64..127
 constexpr int PFT_MAX_BRANCHES = 320;
+constexpr int PFT_TARGET = 4 * 3 * 152;   // CTAs of a launch: four waves of three per SM
 
 __global__ void __launch_bounds__(PFT_THREADS) k_pform_tc(const PSet *ps, const double *branch, int nbr, int nl,
                                                           DevModels m, const float *Bpf, float *Pbuf, float *Bop,
-                                                          int32_t *status_key, int *err)
+                                                          int32_t *status_key, int *err, int per_cta)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
     __shared__ uint32_t tbase_s;
@@ -53,6 +56,7 @@ __global__ void __launch_bounds__(PFT_THREADS) k_pform_tc(const PSet *ps, const 
 
     const int tid = threadIdx.x;
     const int r = blockIdx.x;           // P set (chunk-local)
+    const int bb0 = blockIdx.y * per_cta, bb1 = min(nbr, bb0 + per_cta);   // this CTA's branches (bb0 even)
     const PSet rq = ps[r];
     const int md = rq.model;
     const uint32_t barM = smem_addr(&bar_mma), barB = smem_addr(&bar_b);
@@ -87,7 +91,7 @@ __global__ void __launch_bounds__(PFT_THREADS) k_pform_tc(const PSet *ps, const 
     bool pending = false;               // an MMA group was issued and its completion not seen
     const float isq_i = (float)m.isq[md * K + i];
     // per branch: 0 t = 0, 1 below the grid (Taylor), 2 grid correction at point g
-    for (int b = tid; b < nbr; b += PFT_THREADS) {
+    for (int b = bb0 + tid; b < bb1; b += PFT_THREADS) {
         const double t = rq.rho * branch[b];
         int mode = 0, g = 0;
         if (t == 0.0) mode = 0;
@@ -116,11 +120,11 @@ __global__ void __launch_bounds__(PFT_THREADS) k_pform_tc(const PSet *ps, const 
     }
     const float ntol = -(float)m.tol, dtol = (float)(-1.0 - m.tol);
 
-    for (int b0 = 0; b0 < nbr; b0 += 2) {
+    for (int b0 = bb0; b0 < bb1; b0 += 2) {
         const int b = b0 + bsel;                      // this thread's branch
         if (__syncthreads_or(!ok)) break;             // per-branch table ready / previous pair done
-        const int mode = (b < nbr) ? (mode_g[b] & 3) : 0, g = (b < nbr) ? (mode_g[b] >> 2) : 0;
-        const float t = (b < nbr) ? t_b[b] : 0.0f;
+        const int mode = (b < bb1) ? (mode_g[b] & 3) : 0, g = (b < bb1) ? (mode_g[b] >> 2) : 0;
+        const float t = (b < bb1) ? t_b[b] : 0.0f;
         {
             float cf = 0.0f;
             if (mode == 2) cf = m.grid_eg[((size_t)md * m.grid_n + g) * K + i] * expm1f(lam_i * h_b[b]);
@@ -186,7 +190,7 @@ __global__ void __launch_bounds__(PFT_THREADS) k_pform_tc(const PSet *ps, const 
             }
         }
         tc_fence_before();
-        if (b < nbr && done) {
+        if (b < bb1 && done) {
             // branch-free in j: i differs per lane, and a branch on j == i would split the
             // warp into single-lane paths for everything that follows
             bool neg = false;
@@ -242,7 +246,16 @@ cudaError_t launch_pform_tc(const PSet *ps, int nps, const double *branch, int n
                                          (int)cudaSharedmemCarveoutMaxShared);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_pform_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PFT_SMEM);
     if (e != cudaSuccess) return e;
-    k_pform_tc<<<nps, PFT_THREADS, PFT_SMEM, s>>>(ps, branch, nbr, nl, m, Bpf, Pbuf, Bop, status_key, err);
+    // Branch pairs per CTA: all of a P set's when there are enough P sets to fill the GPU
+    // several times over, fewer for a short list (one exon's search round asks for two to six
+    // P sets): about PFT_TARGET CTAs in all, at the price of one 32 KB fetch of B per CTA.
+    // Measured, P(t) of one mle call on 58 leaves: 1 region (2-6 P sets a round) 5.1 -> 0.28 ms,
+    // 384 regions (~800 P sets a round: 1.7 waves before, three CTAs per P set now) 20.0 -> 14.6 ms.
+    const int pairs = (nbr + 1) / 2;
+    const int want = std::min(pairs, std::max(1, (PFT_TARGET + nps - 1) / nps));
+    const int per_cta = 2 * ((pairs + want - 1) / want);
+    const dim3 grid(nps, (nbr + per_cta - 1) / per_cta);
+    k_pform_tc<<<grid, PFT_THREADS, PFT_SMEM, s>>>(ps, branch, nbr, nl, m, Bpf, Pbuf, Bop, status_key, err, per_cta);
     return cudaGetLastError();
 }
 

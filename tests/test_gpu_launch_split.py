@@ -1,0 +1,38 @@
+"""Values do not depend on how a launch is split over the GPU: a region alone, in a short list
+and in a list long enough for the unsplit forms gives the same bits (every split keeps the
+arithmetic of each matrix and column, so the tolerance is zero)."""
+import numpy as np
+import pytest
+
+import phylocsf_gb300 as P
+from phylocsf_gb300 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _regions(name, lengths, seed=5):
+    ps = synth.load_params(name)
+    rng = np.random.default_rng(seed)
+    gf = synth.gap_fractions(rng, len(lengths), ps.tree.nl, 0.05, 0.4, 0.2)
+    offs, leaves = synth.simulate(ps, np.asarray(lengths), (np.arange(len(lengths)) % 2).astype(np.int32), gf, seed)
+    return ps, offs, leaves
+
+
+# 12 leaves: 22 branches = 11 pairs, a multiple of neither the pairs nor the branches of a CTA;
+# 2,000 P sets are past the unsplit bounds, 1 / 28 / 300 on both sides of the split ones
+@pytest.mark.parametrize("prec", ["tf32x3_direct", "fp32b", "fp64"])
+@pytest.mark.parametrize("name,counts", [("12flies", (1, 28, 300, 2000)), ("29mammals", (1, 33))])
+def test_p_sets_split_over_ctas(name, counts, prec):
+    ps, offs, leaves = _regions(name, [33])
+    eng = P.Engine(ps.tree, ps.S_c, ps.pi_c, ps.S_n, ps.pi_n, precision=prec)
+    rho = np.exp(np.random.default_rng(1).uniform(np.log(0.02), np.log(9.0), size=max(counts)))
+    got = {}
+    for n in counts:
+        if prec == "fp64" and n > 300:
+            continue
+        b = eng.batch(np.arange(n + 1) * 33, np.tile(leaves, (n, 1)))
+        got[n] = eng.lpr(b, 1, rho[:n])
+        assert (got[n][2] == 0).all()
+    for n, (lpr, elpr, _) in got.items():
+        big = got[max(got)]
+        assert np.array_equal(lpr, big[0][:n]) and np.array_equal(elpr, big[1][:n]), n
