@@ -11,15 +11,29 @@
 #include <cmath>
 #include <cstdio>
 
+#include <cooperative_groups.h>
+
 #include "pcsf_internal.h"
 #include "prune_common.cuh"
 
 namespace pcsf {
 
 // ---------------------------------------------------------------------------
-// Eigensolver: one CTA per symmetric 64x64 matrix, 256 threads.  Each Jacobi
-// sweep visits all 2016 pairs as 63 rounds of 32 disjoint rotations (round-robin
+// Eigensolver: parallel cyclic Jacobi, C CTAs (one cluster) per symmetric 64x64 matrix.
+// Each sweep visits all 2016 pairs as 63 rounds of 32 disjoint rotations (round-robin
 // "circle" ordering), which are applied simultaneously.
+//
+// What bounds it: a round is 24,576 FP64 instructions (A <- J^T A J as 1024 blocks of 2x2,
+// V <- V J), and an SM issues two FP64 lanes per clock: ~12,300 clocks a round on one SM, 500
+// to 600 rounds.  The matrices of a call are few (two models, or one per region of an
+// OmegaModel round), so the rows of A and V are spread over a cluster: a block of pair k's
+// rows and pair k' 's columns is read from and written to the owners' shared memory, A is
+// double-buffered so that a round needs one cluster barrier, and V, whose rows are local, is
+// updated between arriving at that barrier and waiting for it.  Every element goes through
+// the same operations in the same order for every C: the results do not depend on it.
+// Measured, OmegaModel scores of six 12-leaf alignments (130 rounds of up to 8 matrices):
+// 514 ms with one CTA per matrix, 243 ms with clusters of 16.  What bounds a round now is the
+// chain of three divisions and two square roots of its rotations (459 and 705 clocks each).
 
 constexpr int JAC_THREADS = 256;
 constexpr int JAC_LD = K + 1;
@@ -33,30 +47,49 @@ __device__ inline void jac_pair(int r, int i, int &p, int &q)
     q = a < b ? b : a;
 }
 
+template <int C>
 __global__ void __launch_bounds__(JAC_THREADS) k_jacobi(const double *A_in, double *U_out, double *lam_out,
                                                          int *status)
 {
+    constexpr int ROWS = K / C;                        // rows of A and V per CTA
     extern __shared__ __align__(16) unsigned char jsm[];
-    double *A = reinterpret_cast<double *>(jsm);      // [K][JAC_LD]
-    double *V = A + K * JAC_LD;                        // [K][JAC_LD]
-    double *red = V + K * JAC_LD;                      // [JAC_THREADS]
-    double *cs = red + JAC_THREADS;                    // [32]
-    double *sn = cs + 32;                              // [32]
-    int *pp = reinterpret_cast<int *>(sn + 32);        // [32]
-    int *qq = pp + 32;                                 // [32]
+    double *A = reinterpret_cast<double *>(jsm);      // [2][ROWS][JAC_LD]
+    double *V = A + 2 * ROWS * JAC_LD;                 // [ROWS][JAC_LD]
+    double *red = V + ROWS * JAC_LD;                   // [JAC_THREADS]
+    double *csb = red + JAC_THREADS;                   // [2][32]
+    double *snb = csb + 64;                            // [2][32]
+    int *ppb = reinterpret_cast<int *>(snb + 64);      // [2][32]
+    int *qqb = ppb + 64;                               // [2][32]
     const int tid = threadIdx.x;
-    const double *Ain = A_in + (size_t)blockIdx.x * K2;
+    const int rank = blockIdx.x % C, row0 = rank * ROWS;
+    const double *Ain = A_in + (size_t)(blockIdx.x / C) * K2;
 
-    for (int f = tid; f < K2; f += JAC_THREADS) {
-        int i = f / K, j = f % K;
-        A[i * JAC_LD + j] = Ain[f];
-        V[i * JAC_LD + j] = (i == j) ? 1.0 : 0.0;
+    auto cluster_arrive = [&]() {
+        if constexpr (C > 1) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    };
+    auto cluster_wait = [&]() {
+        if constexpr (C > 1) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+        else __syncthreads();
+    };
+    // element (row, col) of buffer buf, wherever it lives in the cluster
+    auto at = [&](int buf, int row, int col) -> double * {
+        double *p = A + ((size_t)buf * ROWS + row % ROWS) * JAC_LD + col;
+        if constexpr (C > 1) p = cooperative_groups::this_cluster().map_shared_rank(p, row / ROWS);
+        return p;
+    };
+
+    for (int f = tid; f < ROWS * K; f += JAC_THREADS) {
+        const int i = f / K, j = f % K;
+        A[i * JAC_LD + j] = Ain[(row0 + i) * K + j];
+        V[i * JAC_LD + j] = (row0 + i == j) ? 1.0 : 0.0;
     }
     __syncthreads();
+    cluster_arrive();
+    cluster_wait();
     // ||A||_F^2 (fixed-order tree reduction)
     double part = 0.0;
     for (int f = tid; f < K2; f += JAC_THREADS) {
-        double x = A[(f / K) * JAC_LD + f % K];
+        double x = Ain[f];
         part += x * x;
     }
     red[tid] = part;
@@ -68,12 +101,12 @@ __global__ void __launch_bounds__(JAC_THREADS) k_jacobi(const double *A_in, doub
     const double norm2 = red[0];
     __syncthreads();
 
-    int converged = 0;
+    int converged = 0, cur = 0;
     for (int sweep = 0; sweep < 60; sweep++) {
         part = 0.0;
         for (int f = tid; f < K2; f += JAC_THREADS) {
             int i = f / K, j = f % K;
-            if (i < j) { double x = A[i * JAC_LD + j]; part += x * x; }
+            if (i < j) { double x = *at(cur, i, j); part += x * x; }
         }
         red[tid] = part;
         __syncthreads();
@@ -83,15 +116,17 @@ __global__ void __launch_bounds__(JAC_THREADS) k_jacobi(const double *A_in, doub
         }
         double off = red[0];
         __syncthreads();
-        if (off <= 1e-32 * norm2) { converged = 1; break; }
+        if (off <= 1e-32 * norm2) { converged = 1; break; }     // the same in every CTA of the cluster
         for (int r = 0; r < K - 1; r++) {
-            if (tid < 32) {
+            double *cs = csb + 32 * (cur & 1), *sn = snb + 32 * (cur & 1);
+            int *pp = ppb + 32 * (cur & 1), *qq = qqb + 32 * (cur & 1);
+            if (tid < 32) {                                     // every CTA forms all 32 rotations
                 int p, q;
                 jac_pair(r, tid, p, q);
-                double apq = A[p * JAC_LD + q];
+                const double apq = *at(cur, p, q), aqq = *at(cur, q, q), app = *at(cur, p, p);
                 double c = 1.0, s = 0.0;
                 if (apq != 0.0) {
-                    double theta = (A[q * JAC_LD + q] - A[p * JAC_LD + p]) / (2.0 * apq);
+                    double theta = (aqq - app) / (2.0 * apq);
                     double t = (fabs(theta) > 1e150) ? 0.5 / theta
                                : (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
                     c = 1.0 / sqrt(t * t + 1.0);
@@ -100,47 +135,74 @@ __global__ void __launch_bounds__(JAC_THREADS) k_jacobi(const double *A_in, doub
                 cs[tid] = c; sn[tid] = s; pp[tid] = p; qq[tid] = q;
             }
             __syncthreads();
-            for (int f = tid; f < K * 32; f += JAC_THREADS) {       // columns: A <- A J, V <- V J
-                int row = f >> 5, k = f & 31;
-                int p = pp[k], q = qq[k];
-                double c = cs[k], s = sn[k];
-                double a = A[row * JAC_LD + p], b = A[row * JAC_LD + q];
-                A[row * JAC_LD + p] = c * a - s * b;
-                A[row * JAC_LD + q] = s * a + c * b;
-                double va = V[row * JAC_LD + p], vb = V[row * JAC_LD + q];
+            for (int f = tid; f < (32 / C) * 32; f += JAC_THREADS) {   // 2x2 blocks: columns A <- A J, then rows A <- J^T A
+                const int k = rank * (32 / C) + (f >> 5), kc = f & 31;
+                const int p = pp[k], q = qq[k], pc = pp[kc], qc = qq[kc];
+                const double cc = cs[kc], sc = sn[kc], cr = cs[k], sr = sn[k];
+                const double app = *at(cur, p, pc), apq = *at(cur, p, qc), aqp = *at(cur, q, pc), aqq = *at(cur, q, qc);
+                const double bpp = cc * app - sc * apq, bpq = sc * app + cc * apq;
+                const double bqp = cc * aqp - sc * aqq, bqq = sc * aqp + cc * aqq;
+                const bool diag = k == kc;                      // the pivots become exact zeros
+                *at(cur ^ 1, p, pc) = cr * bpp - sr * bqp;
+                *at(cur ^ 1, q, pc) = diag ? 0.0 : sr * bpp + cr * bqp;
+                *at(cur ^ 1, p, qc) = diag ? 0.0 : cr * bpq - sr * bqq;
+                *at(cur ^ 1, q, qc) = sr * bpq + cr * bqq;
+            }
+            cluster_arrive();
+            for (int f = tid; f < ROWS * 32; f += JAC_THREADS) {       // V <- V J
+                const int row = f >> 5, k = f & 31;
+                const int p = pp[k], q = qq[k];
+                const double c = cs[k], s = sn[k];
+                const double va = V[row * JAC_LD + p], vb = V[row * JAC_LD + q];
                 V[row * JAC_LD + p] = c * va - s * vb;
                 V[row * JAC_LD + q] = s * va + c * vb;
             }
-            __syncthreads();
-            for (int f = tid; f < K * 32; f += JAC_THREADS) {       // rows: A <- J^T A
-                int col = f >> 5, k = f & 31;
-                int p = pp[k], q = qq[k];
-                double c = cs[k], s = sn[k];
-                double a = A[p * JAC_LD + col], b = A[q * JAC_LD + col];
-                A[p * JAC_LD + col] = c * a - s * b;
-                A[q * JAC_LD + col] = s * a + c * b;
-            }
-            __syncthreads();
-            if (tid < 32) {
-                A[pp[tid] * JAC_LD + qq[tid]] = 0.0;
-                A[qq[tid] * JAC_LD + pp[tid]] = 0.0;
-            }
-            __syncthreads();
+            cluster_wait();
+            cur ^= 1;
         }
     }
-    double *Uo = U_out + (size_t)blockIdx.x * K2;
-    for (int f = tid; f < K2; f += JAC_THREADS) Uo[f] = V[(f / K) * JAC_LD + f % K];
-    if (tid < K) lam_out[(size_t)blockIdx.x * K + tid] = A[tid * JAC_LD + tid];
-    if (tid == 0) status[blockIdx.x] = converged ? 0 : 1;
+    __syncthreads();
+    double *Uo = U_out + (size_t)(blockIdx.x / C) * K2;
+    for (int f = tid; f < ROWS * K; f += JAC_THREADS) Uo[row0 * K + f] = V[(f / K) * JAC_LD + f % K];
+    if (tid < ROWS) lam_out[(size_t)(blockIdx.x / C) * K + row0 + tid] = A[(cur * ROWS + tid) * JAC_LD + row0 + tid];
+    if (rank == 0 && tid == 0) status[blockIdx.x / C] = converged ? 0 : 1;
+    if (C > 1) {                       // no CTA leaves while another may still read its rows
+        cluster_arrive();
+        cluster_wait();
+    }
+}
+
+template <int C>
+static cudaError_t launch_jacobi_c(const double *A, double *U, double *lam, int *status, int nmat, cudaStream_t s)
+{
+    const size_t smem = sizeof(double) * (3 * (K / C) * JAC_LD + JAC_THREADS + 128) + sizeof(int) * 128;
+    cudaError_t err = cudaFuncSetAttribute(k_jacobi<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (err == cudaSuccess && C > 8)
+        err = cudaFuncSetAttribute(k_jacobi<C>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (err != cudaSuccess) return err;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(nmat * C);
+    cfg.blockDim = dim3(JAC_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = C;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = C > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, k_jacobi<C>, A, U, lam, status);
 }
 
 cudaError_t launch_jacobi(const double *A, double *U, double *lam, int *status, int nmat, cudaStream_t s)
 {
-    size_t smem = sizeof(double) * (2 * K * JAC_LD + JAC_THREADS + 64) + sizeof(int) * 64;
-    cudaError_t err = cudaFuncSetAttribute(k_jacobi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err != cudaSuccess) return err;
-    k_jacobi<<<nmat, JAC_THREADS, smem, s>>>(A, U, lam, status);
-    return cudaGetLastError();
+    if (nmat <= 0) return cudaSuccess;
+    // the largest cluster whose CTAs still have an SM each
+    if (nmat <= 8) return launch_jacobi_c<16>(A, U, lam, status, nmat, s);
+    if (nmat <= 18) return launch_jacobi_c<8>(A, U, lam, status, nmat, s);
+    if (nmat <= 38) return launch_jacobi_c<4>(A, U, lam, status, nmat, s);
+    if (nmat <= 76) return launch_jacobi_c<2>(A, U, lam, status, nmat, s);
+    return launch_jacobi_c<1>(A, U, lam, status, nmat, s);
 }
 
 // ---------------------------------------------------------------------------

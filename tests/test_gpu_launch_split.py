@@ -36,3 +36,20 @@ def test_p_sets_split_over_ctas(name, counts, prec):
     for n, (lpr, elpr, _) in got.items():
         big = got[max(got)]
         assert np.array_equal(lpr, big[0][:n]) and np.array_equal(elpr, big[1][:n]), n
+
+
+# eigensolver clusters of 16, 8, 4, 2 and 1 CTAs per matrix (1 / 10 / 20 / 50 / 90 rate matrices)
+@pytest.mark.parametrize("prec", ["fp64", "fp32b"])
+def test_rate_matrices_split_over_clusters(prec):
+    ps, offs, leaves = _regions("12flies", [41])
+    eng = P.Engine.for_tree(ps.tree, precision=prec)
+    rng = np.random.default_rng(2)
+    kappa, omega, rho = rng.uniform(1.2, 6, 90), rng.uniform(0.05, 2, 90), rng.uniform(0.3, 3, 90)
+    got = {}
+    for n in (1, 10, 20, 50, 90):
+        b = eng.batch(np.arange(n + 1) * 41, np.tile(leaves, (n, 1)))
+        got[n] = eng.omega_grad(b, kappa[:n], omega[:n], rho[:n])
+        assert (got[n]["status"] == 0).all()
+    for n in got:
+        for k in ("lpr", "d_branch", "d_rho", "d_kappa", "d_omega"):
+            assert np.array_equal(got[n][k], got[90][k][:n]), (n, k)
