@@ -171,6 +171,8 @@ struct pcsf_engine {
     int simt_tile = 0;             // SIMT column tile (0: the default rule; set by pcsf_engine_autotune)
     int smem_sm = 0;               // shared memory per SM, for the grid of a tile
     int ff_grid = 0;               // CTAs of the float-float kernel (0: the tree does not fit it)
+    int ff_depth = 0;              // partials that wait at once in its schedule
+    DevBuf<float> ff_stack;        // where they wait, per CTA (made with the engine: pcsf_lpr_noalloc uses it too)
     // returned values (and the accurate search decisions) of a region come from the
     // float-float kernel when columns x (n_leaves - 2) reaches this; FP32 and tensor-core
     // engines only (the FP64 engine is exact already)
@@ -628,8 +630,18 @@ static int engine_init_common(pcsf_engine *e, const pcsf_tree *tree, int32_t fla
     int gper = std::max(1, std::min(4, (int)(prop.sharedMemPerMultiprocessor / (gsmem + 1024))));
     e->grad_grid = prop.multiProcessorCount * gper;
     if (e->prec != PCSF_PREC_FP64 &&
-        prune_ff_smem_bytes(e->nslots, e->nl, (int)e->sched.size()) <= (size_t)prop.sharedMemPerBlockOptin)
-        e->ff_grid = prop.multiProcessorCount * std::max(1, prune_ff_ctas_per_sm(e->nslots, e->nl, (int)e->sched.size()));
+        prune_ff_smem_bytes(e->nl, (int)e->sched.size()) <= (size_t)prop.sharedMemPerBlockOptin) {
+        // a node's partial waits when the next node of the schedule is not its parent
+        int waiting = 0;
+        for (size_t k = 0; k < e->sched.size(); k++) {
+            const SchedNode &sn = e->sched[k];
+            if (sn.lslot >= 0 && sn.rslot >= 0) waiting--;
+            if (k + 1 < e->sched.size() && e->sched[k + 1].lc != sn.node && e->sched[k + 1].rc != sn.node) waiting++;
+            e->ff_depth = std::max(e->ff_depth, waiting);
+        }
+        e->ff_grid = prop.multiProcessorCount;
+        CK(e->ff_stack.reserve(ff_stack_floats(e->ff_grid, e->ff_depth)), "cudaMalloc float-float stack");
+    }
     // P(t) buffer: up to 16 GiB, at most a quarter of free memory.  A round of the
     // search forms one P set per active fit (20,000 fits x 3.6 MB for 58 leaves), so
     // the chunk size sets how many launch pairs (P(t), pruning) a round takes and how
@@ -691,8 +703,8 @@ static int evaluate(pcsf_engine *e, pcsf_batch *b, const std::vector<Request> &r
                                                                                               : e->comp_mode();
 
     const int kind = drho ? 3 : grad ? 2 : tc ? 1 : ff ? 4 : 0;
-    // a float-float P set (8 B per entry) and its FP64 staging take four times an FP32 one
-    const size_t chunk_psets = ff ? std::max<size_t>(1, e->pbuf_psets / 4) : e->pbuf_psets;
+    // a float-float P set (8-12 B per entry) and its FP64 staging take at most five times an FP32 one
+    const size_t chunk_psets = ff ? std::max<size_t>(1, e->pbuf_psets / 5) : e->pbuf_psets;
     int64_t kind_cols = 0;
     // work items, P-set dedup and chunking (at most pbuf_psets distinct P sets per chunk)
     std::vector<Request> reqs(reqs_in);
@@ -773,7 +785,7 @@ static int evaluate(pcsf_engine *e, pcsf_batch *b, const std::vector<Request> &r
         CK(e->ddrho.reserve(nreq), "cudaMalloc");
         CK(e->ddscr.reserve(nreq), "cudaMalloc");
     }
-    size_t pset_bytes = (size_t)e->nbr * K2 * (e->prec == PCSF_PREC_FP64 || ff ? 8 : 4);
+    size_t pset_bytes = ff ? ff_pset_bytes(e->nl, e->nbr) : (size_t)e->nbr * K2 * (e->prec == PCSF_PREC_FP64 ? 8 : 4);
     size_t max_chunk_ps = 0;
     for (size_t c = 0; c + 1 < chunk_ps_begin.size(); c++)
         max_chunk_ps = std::max<size_t>(max_chunk_ps, chunk_ps_begin[c + 1] - chunk_ps_begin[c]);
@@ -819,11 +831,10 @@ static int evaluate(pcsf_engine *e, pcsf_batch *b, const std::vector<Request> &r
         int r0 = chunk_req_begin[c], r1 = chunk_req_begin[c + 1];
         int p0 = chunk_ps_begin[c], p1 = chunk_ps_begin[c + 1];
         CK(cudaEventRecord(e->ev[0], s), "event");
-        if (ff) {   // FP64 formation, split into hi / lo floats
+        if (ff) {   // FP64 formation, split into the float-float kernel's operands
             CK(launch_pform(true, e->dps.p + p0, p1 - p0, e->dbranch.p, e->nbr, dmv, e->Pbuf64.p, e->dstatus.p + p0, s),
                "P(t) formation launch");
-            CK(launch_split_ff(e->Pbuf64.p, reinterpret_cast<float *>(e->Pbuf.p), (size_t)(p1 - p0) * e->nbr, s),
-               "P(t) split launch");
+            CK(launch_split_ff(e->Pbuf64.p, e->Pbuf.p, p1 - p0, e->nbr, e->nl, s), "P(t) split launch");
             e->stats.kernel_launches += 1;
         } else if (stage64) {
             CK(launch_pform(true, e->dps.p + p0, p1 - p0, e->dbranch.p, e->nbr, dmv, e->Pbuf64.p, e->dstatus.p + p0, s),
@@ -860,6 +871,7 @@ static int evaluate(pcsf_engine *e, pcsf_batch *b, const std::vector<Request> &r
         pa.dlo = dlo;
         pa.tile = e->simt_tile;
         pa.tc_shape = e->tc_shape;
+        pa.ff_depth = e->ff_depth;
         if (grad) {
             GradArgs ga{};
             ga.wi = pa.wi;
@@ -895,7 +907,7 @@ static int evaluate(pcsf_engine *e, pcsf_batch *b, const std::vector<Request> &r
                "tensor-core tangent launch");
         } else if (ff) {
             int grid = std::min(e->ff_grid, std::max(pa.nwi, 1));
-            CK(launch_prune_ff(pa, s, grid), "float-float pruning launch");
+            CK(launch_prune_ff(pa, e->ff_stack.p, e->derr.p, s, grid), "float-float pruning launch");
         } else if (tc) {
             int grid = std::min(e->tc_grid, std::max(pa.nwi, 1));
             if (e->prec == PCSF_PREC_BF16X3)
@@ -1756,6 +1768,8 @@ int pcsf_internal_noalloc_ctx(pcsf_engine *e, NoallocCtx *c)
     c->prune_grid = e->prune_grid;
     c->simt_tile = e->simt_tile;
     c->ff_grid = e->prec != PCSF_PREC_FP64 ? e->ff_grid : 0;
+    c->ff_depth = e->ff_depth;
+    c->ff_stack = e->ff_stack.p;
     c->exact_min_units = e->exact_min_units;
     c->derr = e->derr.p;
     return PCSF_OK;

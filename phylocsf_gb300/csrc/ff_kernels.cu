@@ -1,341 +1,654 @@
-// Float-float SIMT pruning: returned likelihoods that agree with the FP64 path
-// to about 1e-12 relative, at FP32 instruction rates.
+// Float-float pruning on the tensor cores: returned likelihoods that agree with the
+// FP64 path to about 1e-12 relative.
 //
 // The FP32 kernels round every stored partial and every contraction to 24 bits.
 // Over a long region those errors add up partly coherently (columns that share
 // sub-patterns repeat them), and the model's P(t) stored in FP32 is itself a fixed
 // perturbation that every column sees; together they grow linearly with the
 // region's length, past 1e-3 dB at a few thousand codons on trees of ~100 leaves.
-// This kernel instead carries every quantity as an unevaluated sum of two floats
-// (hi + lo, ~48 bits):
-//   - E^T = (P - I)^T comes from the FP64 P(t) formation (the FP64 engine's own
-//     matrices, row rule of Q.ml:226-247 applied in FP64), split once per P set into
-//     hi / lo floats (k_split_ff) and staged into shared memory asynchronously, one
-//     node ahead;
-//   - a leaf child's partial P[a][s] = delta_as + E[a][s] is formed from the split
-//     entries with an error-free sum (PhyloLik.ml:87-88 with a one-hot leaf);
-//   - an internal child's v = alpha + sum_j E[a][j] alpha[j] (PhyloLik.ml:89-92)
-//     is a compensated dot product: each hi x hi product is split exactly
-//     (TwoProduct by FMA), its hi part is added with TwoSum, and the product
-//     errors with the TwoSum errors, and the two hi x lo cross terms, are summed in
-//     three separate low accumulators (short dependency chains), added at the end;
+// This kernel instead carries every partial as an unevaluated sum of two floats
+// (hi + lo, ~48 bits) and contracts it exactly:
+//   - E = P - I comes from the FP64 P(t) formation (the FP64 engine's own matrices, row
+//     rule of Q.ml:226-247 applied in FP64).  Once per P set (k_split_ff) each row of a
+//     branch above an internal node is written as its diagonal in hi / lo floats and its
+//     off-diagonal entries as 2^ea sum_l e_l 2^(-8-9l), six signed 9-bit digits (an error
+//     below 2^-54 of the largest of them, the order of the FP64 formation's own), and each
+//     branch above a leaf as P in hi / lo floats;
+//   - a partial alpha, normalised per column to [0.5, 1), becomes sum_k A_k 2^(-8-9k), six
+//     signed 9-bit digits (an error below 2^-54 of the column's largest entry);
+//   - sum_{j != a} E[a][j] alpha[j] = 2^(ea-16) sum_g 2^(-9g) G_g with G_g = sum_{k+l=g} sum_j
+//     e_l[a][j] A_k[j], kept for g <= 6 (26 of the 36 digit products; the rest are below
+//     2^-58).  Digits are FP16 operands of tcgen05.mma kind::f16 (at most 9 bits + sign of
+//     FP16's 11); the products of a group share one FP32 accumulator in tensor memory and
+//     are integers whose sums stay below 2^24 for g <= 3 (64 x 2^16 x 4 pairs) and, in any
+//     case, round by 2^-52 or less beyond, so the accumulation is exact: it does not
+//     matter in which order or with which rounding the tensor cores add;
+//   - the groups are summed, and alpha and the diagonal's term added (v = alpha + E alpha,
+//     PhyloLik.ml:89-92), with error-free transforms; a leaf child's partial is a gathered row of P
+//     (PhyloLik.ml:87-88 with a one-hot leaf);
 //   - node products alpha = v_l * v_r are float-float products;
 //   - each column is rescaled by an exact power of two after every node;
 //   - the root dot with the prior, the log and the tile sums are FP64.
-// The error-free steps use __fadd_rn / __fmul_rn, which the compiler never fuses
-// into an FMA (a fused form would break the exactness the transforms rely on).  The
-// kernel has no FP64 arithmetic outside the root stage: FP64 runs at 1/64 of the FP32
-// rate on this part, and splitting the staged doubles in every tile had cost more
-// than the contractions themselves.
+// Splitting an operand into digits whose products a low-precision unit adds without
+// error is Ozaki's scheme (Ozaki, Ogita, Oishi, Rump 2012).  The error-free steps use
+// explicitly rounded add / sub / mul / fma on pairs (f32x2: the same lanes per clock as
+// scalar FP32 at half the issue slots), which the compiler never contracts.
+//
+// Shape: one CTA of 512 threads per SM and 128-column tile; thread t owns column t % 128
+// (its TMEM lane) and states 16 (t / 128) .. + 15.  A_k (6 x 16 KB) and the e_l of one
+// branch (48 KB, one bulk copy, fetched while the previous contraction is combined) sit in
+// shared memory.  B's rows are ordered [digit l][state], so one MMA of A_k against the
+// first digits of B adds into consecutive groups: D column 32 g + state for half of the
+// states at a time, so the first half is combined while the second half's MMAs run.
+// The node evaluated just before its parent is handed over in registers; the other
+// internal child (a first child whose sibling is internal) waits on a per-thread stack in
+// global memory (L2).
+// What bounds it: the chain of a contraction's phases, 13,900 clocks on 120 leaves: digits
+// 1,900, staging barrier 1,100, first half's MMAs 2,700 (with the sibling leaf's gather), its
+// combination beside the second half's MMAs 2,300, the second half's 2,000, the maximum and
+// rescale 500, and per node 3,200 of leaf gathers and stack traffic; a third of the issue slots
+// are used.  The MMAs need 3,400 clocks, and a float-float dot product on the FP32 units (64 x
+// 12 instructions per state and column instead of about 75) took 75,000.  Measured per column
+// and evaluation: 120 leaves 238 -> 43 ns, 100 leaves 210 -> 39, 58 leaves (launches of a few
+// regions, which leave SMs idle) 133 -> 43.  Against the FP64 engine on the same P(t), lpr is
+// within 6e-16 relative at rho >= 1 and 5e-14 at rho = 0.01, where two independent FP64
+// evaluations differ by 2e-12.
 #include <algorithm>
+
+#include <cuda_fp16.h>
 
 #include "pcsf_internal.h"
 #include "prune_common.cuh"
+#include "tc_common.cuh"
 
 namespace pcsf {
 
 namespace {
 
-constexpr int FF_THREADS = 256;
-constexpr int FF_TC = 16;            // columns per tile (1 per thread): ~98 KB of shared memory, two CTAs per SM
-constexpr int FF_CPT = FF_TC / 16;
+constexpr int FF_THREADS = 512;
+constexpr int FF_TC = 128;           // columns per tile
+constexpr int FF_DIG = 6;            // 9-bit digits per operand
+constexpr int FF_GRP = 7;            // digit groups k + l = 0 .. 6
+constexpr int FF_SPT = 16;           // states per thread
+constexpr size_t FF_LEAF_BYTES = 2 * K2 * sizeof(float);            // P of a leaf branch, [s][hi 64 | lo 64]
+constexpr uint32_t FF_HALF_BYTES = FF_DIG * 32 * K * 2;             // e_l of 32 states: 192 rows x 64, FP16
+constexpr size_t FF_INNER_BYTES = 2 * FF_HALF_BYTES;
+constexpr uint32_t FF_ROW_BYTES = 3 * K * 4;                        // per row: scale 2^(ea - 16), E_aa hi, E_aa lo
 
-__device__ __forceinline__ void two_sum(float a, float b, float &s, float &e)
+// dynamic shared memory (bytes)
+constexpr uint32_t FS_A = 0;                                        // [digit][128 x 64] FP16
+constexpr uint32_t FS_ADIG = 128 * K * 2;
+constexpr uint32_t FS_B = FS_A + FF_DIG * FS_ADIG;                  // [half][192 x 64] FP16
+constexpr uint32_t FS_SC = FS_B + 2 * FF_HALF_BYTES;                // [2][3][64] row scales and diagonals
+constexpr uint32_t FS_CM = FS_SC + 2 * FF_ROW_BYTES;                       // [2][4][128] column maxima
+constexpr uint32_t FS_LV = FS_CM + 2 * 4 * FF_TC * 4;               // [nl][128] leaf states, schedule, order
+
+// byte offset of (leaf l, site c): words XOR-swizzled per leaf, so that the fill (consecutive
+// threads on consecutive leaves) and the reads (on consecutive sites) are free of conflicts
+__device__ __forceinline__ int ff_lv(int l, int c) { return l * FF_TC + (c ^ ((l & 31) << 2)); }
+
+size_t ff_smem(int nl, int nint)
 {
-    s = __fadd_rn(a, b);
-    const float bb = __fsub_rn(s, a);
-    e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+    return FS_LV + (((size_t)nl * FF_TC + 15) & ~size_t(15)) + (size_t)nint * (sizeof(SchedNode) + 2) + 16;
 }
 
-// |a| >= |b| (or a == 0)
-__device__ __forceinline__ void fast_two_sum(float a, float b, float &s, float &e)
+// ---- pairs of floats (one 64-bit register pair), elementwise round-to-nearest
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pk(float x, float y) { f2 d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y)); return d; }
+__device__ __forceinline__ void upk(f2 a, float &x, float &y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a)); }
+__device__ __forceinline__ f2 add2(f2 a, f2 b) { f2 d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ f2 sub2(f2 a, f2 b) { f2 d; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) { f2 d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) { f2 d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
+__device__ __forceinline__ f2 neg2(f2 a) { return a ^ 0x8000000080000000ull; }
+// s + e = a + b exactly (Knuth)
+__device__ __forceinline__ void two_sum2(f2 a, f2 b, f2 &s, f2 &e)
 {
-    s = __fadd_rn(a, b);
-    e = __fsub_rn(b, __fsub_rn(s, a));
+    s = add2(a, b);
+    const f2 bb = sub2(s, a);
+    e = add2(sub2(a, sub2(s, bb)), sub2(b, bb));
+}
+// the same when |a| >= |b| (or a == 0) (Dekker)
+__device__ __forceinline__ void fast_two_sum2(f2 a, f2 b, f2 &s, f2 &e)
+{
+    s = add2(a, b);
+    e = sub2(b, sub2(s, a));
+}
+// two FP16 values from a pair of floats that hold small integers (exact)
+__device__ __forceinline__ uint32_t half2_of(f2 a)
+{
+    float x, y;
+    upk(a, x, y);
+    uint32_t r;
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(y), "f"(x));
+    return r;
 }
 
-struct FFSmem {
-    static size_t bytes(int nslots, int nl, int nint)
-    {
-        size_t b = sizeof(float) * (4 * (size_t)K2 + 2 * (size_t)nslots * K * FF_TC);   // E^T hi/lo x 2 sides, slots hi/lo
-        b += sizeof(int) * 2 * FF_TC;                                                   // column maxima (as int bits)
-        b += sizeof(int) * FF_TC;                                                       // column exponents
-        b += sizeof(SchedNode) * nint;
-        b = (b + 15) & ~size_t(15);
-        b += (size_t)nl * FF_TC;
-        return (b + 15) & ~size_t(15);
+// float-float product of (ah, al) and (bh, bl)
+__device__ __forceinline__ void ff_mul2(f2 ah, f2 al, f2 bh, f2 bl, f2 &h, f2 &l)
+{
+    const f2 p = mul2(ah, bh);
+    f2 lo = fma2(ah, bh, neg2(p));
+    lo = fma2(ah, bl, lo);
+    lo = fma2(al, bh, lo);
+    fast_two_sum2(p, lo, h, l);
+}
+
+// Six signed 9-bit digits of a pair x = h + l in [0, 1): x = sum_k d_k 2^(-8-9k).  Rounding to
+// an integer by adding 1.5 x 2^23; the residual r is kept negated, so that each digit comes out
+// as magic - t without a sign flip.  l joins before digit 2 (error-free: its sum's error e joins
+// the residual of digit 3).
+__device__ __forceinline__ void ff_digits(f2 h, f2 l, uint32_t d[FF_DIG])
+{
+    const f2 M = pk(12582912.0f, 12582912.0f), S = pk(512.0f, 512.0f);
+    const f2 x = mul2(h, pk(-256.0f, -256.0f));
+    f2 nd = sub2(M, add2(x, M));
+    d[0] = half2_of(nd);
+    f2 r = add2(x, nd);
+    nd = sub2(M, fma2(r, S, M));
+    d[1] = half2_of(nd);
+    r = fma2(r, S, nd);
+    f2 s, e;
+    two_sum2(r, mul2(l, pk(-131072.0f, -131072.0f)), s, e);      // units 2^-17
+    nd = sub2(M, fma2(s, S, M));
+    d[2] = half2_of(nd);
+    r = fma2(s, S, nd);
+    nd = sub2(M, fma2(r, S, M));
+    d[3] = half2_of(nd);
+    r = fma2(r, S, nd);
+    r = fma2(e, pk(262144.0f, 262144.0f), r);
+    nd = sub2(M, fma2(r, S, M));
+    d[4] = half2_of(nd);
+    r = fma2(r, S, nd);
+    d[5] = half2_of(sub2(M, fma2(r, S, M)));
+}
+
+__device__ __forceinline__ void mma_f16(uint32_t dt, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t acc)
+{
+    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                 " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+                 :: "r"(dt), "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
+}
+
+// four columns of each of the seven groups (32 columns apart), and the wait, in one asm block
+__device__ __forceinline__ void tmem_ld_groups(uint32_t ta, float g[FF_GRP][4])
+{
+    uint32_t r[FF_GRP * 4];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%28];\n"
+                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%4,%5,%6,%7}, [%29];\n"
+                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%8,%9,%10,%11}, [%30];\n"
+                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%12,%13,%14,%15}, [%31];\n"
+                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%16,%17,%18,%19}, [%32];\n"
+                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%20,%21,%22,%23}, [%33];\n"
+                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%24,%25,%26,%27}, [%34];\n"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+                   "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+                   "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27])
+                 : "r"(ta), "r"(ta + 32), "r"(ta + 64), "r"(ta + 96), "r"(ta + 128), "r"(ta + 160), "r"(ta + 192)
+                 : "memory");
+#pragma unroll
+    for (int k = 0; k < FF_GRP; k++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) g[k][j] = __uint_as_float(r[4 * k + j]);
+}
+
+// Split of FP64 E^T sets [nps][nbr][K2] into the operands of k_prune_ff, one CTA per matrix.
+// Per P set: the leaf branches' P, the inner branches' digits, the inner branches' row scales
+// (ff_pset_bytes).  FP64 instructions are the scarce ones (two lanes per clock): two per entry.
+__global__ void __launch_bounds__(256) k_split_ff(const double *in, unsigned char *out, int nbr, int nl, size_t pset_bytes)
+{
+    __shared__ int emax[4][K];
+    const int tid = threadIdx.x, a = tid & (K - 1), qd = tid >> 6;      // row a, columns 16 qd ..
+    const int b = blockIdx.x % nbr;
+    const double *src = in + (size_t)blockIdx.x * K2;
+    unsigned char *base = out + (size_t)(blockIdx.x / nbr) * pset_bytes;
+    double x[16];
+#pragma unroll
+    for (int j = 0; j < 16; j++) x[j] = src[(16 * qd + j) * K + a];     // E[a][16 qd + j]
+    if (b < nl) {
+        float *dst = reinterpret_cast<float *>(base + (size_t)b * FF_LEAF_BYTES);
+#pragma unroll
+        for (int j = 0; j < 16; j++) {
+            const int s = 16 * qd + j;
+            const double p = x[j] + (a == s ? 1.0 : 0.0);
+            const float h = (float)p;
+            dst[(size_t)s * 2 * K + a] = h;
+            dst[(size_t)s * 2 * K + K + a] = (float)(p - (double)h);
+        }
+        return;
     }
-};
-
-// FP64 E^T sets [nmat][K2] -> float-float [nmat][hi K2 | lo K2]: hi = the nearest float,
-// lo = the nearest float to the remainder (together ~48 bits).
-__global__ void k_split_ff(const double *in, float *out, size_t nmat)
-{
-    const size_t n = nmat * K2;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const double x = in[i];
-        const float h = (float)x;
-        const size_t m = i / K2, k = i - m * K2;
-        out[m * 2 * K2 + k] = h;
-        out[m * 2 * K2 + K2 + k] = (float)(x - (double)h);
+    float *row = reinterpret_cast<float *>(base + (size_t)nl * FF_LEAF_BYTES + (size_t)(nbr - nl) * FF_INNER_BYTES +
+                                           (size_t)(b - nl) * FF_ROW_BYTES);
+    // ea: every off-diagonal |E[a][j]| < 2^ea (at least 2^-110, so that the scale stays a normal
+    // float); the diagonal, hundreds of times the entries that matter beside it, is kept apart
+    int hi = 0;
+#pragma unroll
+    for (int j = 0; j < 16; j++) {
+        if (16 * qd + j == a) {
+            const float d = (float)x[j];
+            row[K + a] = d;
+            row[2 * K + a] = (float)(x[j] - (double)d);
+            x[j] = 0.0;
+        }
+        hi = max(hi, __double2hiint(x[j]) & 0x7fffffff);
     }
+    emax[qd][a] = hi;
+    __syncthreads();
+    hi = max(max(emax[0][a], emax[1][a]), max(emax[2][a], emax[3][a]));
+    const int ea = max((hi >> 20) - 1022, -110);
+    const double up = __hiloint2double((1023 + 53 - ea) << 20, 0);
+    const int half = (a >> 3) & 1, n0 = (a >> 4) * 8 + (a & 7);         // state 16 q + 8 half + i -> row 8 q + i
+    unsigned char *dst = base + (size_t)nl * FF_LEAF_BYTES + (size_t)(b - nl) * FF_INNER_BYTES + half * FF_HALF_BYTES;
+#pragma unroll
+    for (int c = 0; c < 2; c++) {                                       // 8 columns: one core-matrix row of 16 bytes
+        uint32_t w[FF_DIG][4];
+#pragma unroll
+        for (int j2 = 0; j2 < 4; j2++) {
+            long long v[2];
+#pragma unroll
+            for (int u = 0; u < 2; u++) v[u] = __double2ll_rn(x[8 * c + 2 * j2 + u] * up);
+#pragma unroll
+            for (int l = FF_DIG - 1; l >= 0; l--) {
+                uint32_t hb = 0;
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    const int d = l ? (int)((v[u] + 256) & 511) - 256 : (int)v[u];
+                    v[u] = (v[u] - d) >> 9;
+                    hb |= (uint32_t)__half_as_ushort(__int2half_rn(d)) << (16 * u);
+                }
+                w[l][j2] = hb;
+            }
+        }
+#pragma unroll
+        for (int l = 0; l < FF_DIG; l++) {
+            const int n = 32 * l + n0;
+            *reinterpret_cast<uint4 *>(dst + (((2 * qd + c) * 24 + (n >> 3)) << 7) + ((n & 7) << 4)) =
+                make_uint4(w[l][0], w[l][1], w[l][2], w[l][3]);
+        }
+    }
+    if (qd == 0) row[a] = __int_as_float((127 + ea - 16) << 23);
 }
 
-__global__ void __launch_bounds__(FF_THREADS) k_prune_ff(PruneArgs a)
+__global__ void __launch_bounds__(FF_THREADS, 1) k_prune_ff(PruneArgs a, size_t pset_bytes, float *stack, int *err)
 {
-    extern __shared__ __align__(16) unsigned char ssm[];
-    float *Et = reinterpret_cast<float *>(ssm);              // [2 sides][hi K2 | lo K2]
-    float *slH = Et + 4 * K2;                                // [nslots][K][TC]
-    float *slL = slH + (size_t)a.nslots * K * FF_TC;         // [nslots][K][TC]
-    int *colmax = reinterpret_cast<int *>(slL + (size_t)a.nslots * K * FF_TC);   // [2][TC]
-    int *cscale = colmax + 2 * FF_TC;                                            // [TC]
-    SchedNode *sched = reinterpret_cast<SchedNode *>(cscale + FF_TC);
-    size_t off = (reinterpret_cast<unsigned char *>(sched + a.n_internal) - ssm + 15) & ~size_t(15);
-    uint8_t *lvT = ssm + off;                                                     // [nl][TC]
+    extern __shared__ __align__(1024) unsigned char sm[];
+    __shared__ uint32_t tbase_s;
+    __shared__ __align__(8) uint64_t bar_h0, bar_h1, bar_b;
+    __shared__ double prd[K], wld[K];
+    __shared__ double red_l[4], red_e[4];
+    __shared__ int nbseq_s;
 
-    const int tid = threadIdx.x;
-    const int ty = tid / 16, tx = tid % 16;
-    const int a0 = 4 * ty, c0 = FF_CPT * tx;
-    const int nl = a.nl;
-    __shared__ double red_l[FF_THREADS / 32], red_e[FF_THREADS / 32];
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int site = tid & (FF_TC - 1);          // tile column = TMEM lane
+    const int h = tid >> 7, s0 = FF_SPT * h;      // states s0 .. s0 + 15
+    const int nl = a.nl, nin = a.n_internal;
+    uint8_t *lvT = sm + FS_LV;
+    SchedNode *sched = reinterpret_cast<SchedNode *>(sm + FS_LV + ((nl * FF_TC + 15) & ~15));
+    int16_t *bseq = reinterpret_cast<int16_t *>(sched + nin);        // internal child of each contraction, in order
+    const uint32_t bar0 = smem_addr(&bar_h0), bar1 = smem_addr(&bar_h1), barB = smem_addr(&bar_b);
+    const uint32_t sA = smem_addr(sm + FS_A), sB = smem_addr(sm + FS_B);
+    float *stk = stack + (size_t)blockIdx.x * a.ff_depth * (2 * FF_SPT * FF_THREADS) + tid;
 
-    for (int f = tid; f < a.n_internal; f += FF_THREADS) sched[f] = a.sched[f];
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                     :: "r"(smem_addr(&tbase_s)), "r"(512));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    if (tid == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bar0), "r"(1));
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bar1), "r"(1));
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(barB), "r"(1));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        // contraction order: the child evaluated just before its parent (handed over in
+        // registers), then the child that waits on the stack
+        int k = 0;
+        for (int f = 0; f < nin; f++) {
+            const SchedNode sn = a.sched[f];
+            const int prev = f ? a.sched[f - 1].node : -1;
+            const bool li = sn.lslot >= 0, ri = sn.rslot >= 0;
+            if (li && ri) {
+                bseq[k++] = prev == sn.lc ? sn.lc : sn.rc;
+                bseq[k++] = prev == sn.lc ? sn.rc : sn.lc;
+            } else if (li || ri) {
+                bseq[k++] = li ? sn.lc : sn.rc;
+            }
+        }
+        nbseq_s = k;
+    }
+    for (int f = tid; f < nin; f += FF_THREADS) sched[f] = a.sched[f];
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tbase = tbase_s;
+    const int nbseq = nbseq_s;
+    const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
+    uint32_t ph_d = 0, ph_b = 0;        // parities: both D halves complete once per contraction
+    int ld_w = blockIdx.x, ld_k = 0, ld_n = 0;   // next B load: work item, index into bseq, loads issued
+    int b_inflight = 0;
+    int cn = 0;                          // contractions so far (parity: the row-scale buffer)
+    bool ok = true;
+    const size_t inner0 = (size_t)nl * FF_LEAF_BYTES, scale0 = inner0 + (size_t)(a.nbr - nl) * FF_INNER_BYTES;
 
-    for (int w = blockIdx.x; w < a.nwi; w += gridDim.x) {
+    auto issue_next_b = [&]() {          // thread 0: the B buffer is free
+        while (ld_w < a.nwi && ld_k >= nbseq) { ld_w += gridDim.x; ld_k = 0; }
+        if (ld_w >= a.nwi || nbseq == 0) return;
+        const unsigned char *ps = static_cast<const unsigned char *>(a.Pbuf) +
+                                  (size_t)a.req[a.wi[ld_w].request].pset * pset_bytes;
+        const int c = bseq[ld_k++] - nl;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+                     :: "r"(barB), "r"((uint32_t)FF_INNER_BYTES + FF_ROW_BYTES) : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                     :: "r"(sB), "l"(ps + inner0 + (size_t)c * FF_INNER_BYTES), "r"((uint32_t)FF_INNER_BYTES), "r"(barB)
+                     : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                     :: "r"(smem_addr(sm + FS_SC) + (uint32_t)(ld_n & 1) * FF_ROW_BYTES), "l"(ps + scale0 + (size_t)c * FF_ROW_BYTES),
+                        "r"(FF_ROW_BYTES), "r"(barB)
+                     : "memory");
+        ld_n++;
+        b_inflight++;
+    };
+    if (tid == 0) issue_next_b();
+
+    // thread 0, after the staging barrier: the digit products of one contraction.  Operand
+    // layouts: K-major core matrices (8 rows x 16 bytes); A_k 128 rows: 2048 B between core
+    // matrices along K, B 192 rows: 3072 B; a K step (16 values) is two of them.
+    auto issue_mma = [&]() {
+        const uint64_t dA = sdesc(sA, 2048, 128), dB = sdesc(sB, 3072, 128);
+        const uint32_t id0 = (1u << 4) | ((128u >> 4) << 24);     // f32 += f16 x f16, M = 128
+#pragma unroll 1
+        for (int hf = 0; hf < 2; hf++) {
+            const uint32_t dt = tbase + 224 * hf;
+            const uint64_t dBh = dB + (FF_HALF_BYTES >> 4) * hf;
+            // the first K step starts every group: groups 1-6 by A_1 x e_0..5, group 0 by A_0 x e_0
+            mma_f16(dt + 32, dA + (FS_ADIG >> 4), dBh, id0 | ((192u >> 3) << 17), 0);
+            mma_f16(dt, dA, dBh, id0 | ((32u >> 3) << 17), 0);
+            mma_f16(dt + 32, dA, dBh + (32 * 16 >> 4), id0 | ((160u >> 3) << 17), 1);
+#pragma unroll
+            for (int ks = 0; ks < 4; ks++) {
+#pragma unroll
+                for (int k = 0; k < FF_DIG; k++) {
+                    if (ks == 0 && k < 2) continue;
+                    const uint32_t n = 32u * (k == 0 ? 6 : 7 - k);
+                    mma_f16(dt + 32 * k, dA + (FS_ADIG >> 4) * k + 256 * ks, dBh + 384 * ks, id0 | ((n >> 3) << 17), 1);
+                }
+            }
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                         :: "r"(hf ? bar1 : bar0) : "memory");
+        }
+    };
+    // this thread's 16 states of a leaf branch's P: v (or v *=) P[.][s], 1 where marginalised
+    auto leaf_rows = [&](const unsigned char *P, int s, float *xh, float *xl) {
+        const float *row = reinterpret_cast<const float *>(P) + (size_t)(s < K ? s : 0) * 2 * K + s0;
+        ldg8(row, xh);
+        ldg8(row + 8, xh + 8);
+        ldg8(row + K, xl);
+        ldg8(row + K + 8, xl + 8);
+#pragma unroll
+        for (int j = 0; j < FF_SPT; j++) {
+            xh[j] = (s < K) ? xh[j] : 1.0f;
+            xl[j] = (s < K) ? xl[j] : 0.0f;
+        }
+    };
+
+    for (int w = blockIdx.x; w < a.nwi && ok; w += gridDim.x) {
         const WorkItem wi = a.wi[w];
         const Request rq = a.req[wi.request];
         const int md = rq.model;
-        const float *Pbase = reinterpret_cast<const float *>(a.Pbuf) + (size_t)rq.pset * a.nbr * 2 * K2;
+        const unsigned char *Pbase = static_cast<const unsigned char *>(a.Pbuf) + (size_t)rq.pset * pset_bytes;
         const int ncols = wi.ncols;
         const uint8_t *lg = a.leaves + (size_t)wi.col0 * nl;
-        // the split E^T (hi and lo blocks, 32 KB) of a node's internal children into shared
-        // memory, copied asynchronously one node ahead; leaf children read their rows from
-        // global memory instead
-        auto copy_inner = [&](const SchedNode &nx) {
-            constexpr int NV = 2 * K2 * sizeof(float) / 16;
-#pragma unroll
-            for (int side = 0; side < 2; side++) {
-                if ((side ? nx.rslot : nx.lslot) < 0) continue;
-                const char *src = reinterpret_cast<const char *>(Pbase + (size_t)(side ? nx.rc : nx.lc) * 2 * K2);
-                const uint32_t dst = (uint32_t)__cvta_generic_to_shared(Et + side * 2 * K2);
-                for (int f = tid; f < NV; f += FF_THREADS)
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst + 16 * f), "l"(src + 16 * f)
-                                 : "memory");
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        };
-        __syncthreads();   // previous work item finished with shared memory
+        __syncthreads();
         for (int f = tid; f < FF_TC * nl; f += FF_THREADS) {
             const int c = f / nl, l = f - c * nl;
-            lvT[l * FF_TC + c] = (c < ncols) ? lg[f] : (uint8_t)K;
+            lvT[ff_lv(l, c)] = (c < ncols) ? lg[f] : (uint8_t)K;
         }
-        for (int f = tid; f < 2 * FF_TC; f += FF_THREADS) colmax[f] = 0;
-        for (int f = tid; f < FF_TC; f += FF_THREADS) cscale[f] = 0;
+        if (tid < K) {
+            prd[tid] = a.m.prior[md * K + tid];
+            wld[tid] = a.m.wlog[md * K + tid];
+        }
+        __syncthreads();
+        int escale = 0;          // this column's sum of rescale exponents
+        int sp = 0;              // stack entries in use
+        bool bad = false;        // a timed-out wait not yet agreed on
+        f2 ah[FF_SPT / 2], al[FF_SPT / 2];      // the last node's partial
 
-        copy_inner(sched[0]);
-        for (int ni = 0; ni < a.n_internal; ni++) {
+        for (int ni = 0; ni < nin && ok; ni++) {
             const SchedNode sn = sched[ni];
-            asm volatile("cp.async.wait_all;" ::: "memory");
-            __syncthreads();   // this node's E^T staged, the previous node's slots written
-            float vh[2][4][FF_CPT], vl[2][4][FF_CPT];
+            const int nint = (sn.lslot >= 0) + (sn.rslot >= 0);
+            f2 vh[FF_SPT / 2], vl[FF_SPT / 2];
+            bool have = false;
+            if (nint == 0) {
+                float xh[FF_SPT], xl[FF_SPT], yh[FF_SPT], yl[FF_SPT];
+                leaf_rows(Pbase + (size_t)sn.lc * FF_LEAF_BYTES, lvT[ff_lv(sn.lc, site)], xh, xl);
+                leaf_rows(Pbase + (size_t)sn.rc * FF_LEAF_BYTES, lvT[ff_lv(sn.rc, site)], yh, yl);
 #pragma unroll
-            for (int side = 0; side < 2; side++) {
-                const int slot = side ? sn.rslot : sn.lslot;
-                const int child = side ? sn.rc : sn.lc;
-                if (slot < 0) {
-                    // leaf: P[a][s] = delta_as + E[a][s] from the split entries; 1 for a marginalised leaf
-                    const float *Eg = Pbase + (size_t)child * 2 * K2;
+                for (int i = 0; i < FF_SPT / 2; i++)
+                    ff_mul2(pk(xh[2 * i], xh[2 * i + 1]), pk(xl[2 * i], xl[2 * i + 1]), pk(yh[2 * i], yh[2 * i + 1]),
+                            pk(yl[2 * i], yl[2 * i + 1]), vh[i], vl[i]);
+            }
+            for (int c = 0; c < nint; c++) {
+                if (c == 1) {                   // the waiting child, back from the stack
+                    sp--;
+                    const float *st = stk + (size_t)sp * (2 * FF_SPT * FF_THREADS);
 #pragma unroll
-                    for (int cc = 0; cc < FF_CPT; cc++) {
-                        const int s = lvT[child * FF_TC + c0 + cc];
-                        const int sr = s < K ? s : 0;
-                        const float4 h4 = __ldg(reinterpret_cast<const float4 *>(Eg + sr * K + a0));
-                        const float4 l4 = __ldg(reinterpret_cast<const float4 *>(Eg + K2 + sr * K + a0));
-                        const float hv[4] = {h4.x, h4.y, h4.z, h4.w}, lv[4] = {l4.x, l4.y, l4.z, l4.w};
+                    for (int i = 0; i < FF_SPT / 2; i++) {
+                        ah[i] = pk(st[(2 * i) * FF_THREADS], st[(2 * i + 1) * FF_THREADS]);
+                        al[i] = pk(st[(FF_SPT + 2 * i) * FF_THREADS], st[(FF_SPT + 2 * i + 1) * FF_THREADS]);
+                    }
+                }
+                // ---- digits of alpha: the A operand (free: the last contraction's MMAs completed)
 #pragma unroll
-                        for (int i = 0; i < 4; i++) {
-                            float h = hv[i], l = lv[i];
-                            if (a0 + i == s) {   // 1 + E_ss: exact sum, then the low part folded in
-                                float t, e;
-                                two_sum(1.0f, h, t, e);
-                                fast_two_sum(t, __fadd_rn(e, l), h, l);
-                            }
-                            vh[side][i][cc] = (s >= K) ? 1.0f : h;
-                            vl[side][i][cc] = (s >= K) ? 0.0f : l;
+                for (int q = 0; q < 2; q++) {
+                    uint32_t d[4][FF_DIG];
+#pragma unroll
+                    for (int i = 0; i < 4; i++) ff_digits(ah[4 * q + i], al[4 * q + i], d[i]);
+                    const uint32_t o = (uint32_t)((((s0 >> 3) + q) * 16 + (site >> 3)) << 7) + ((site & 7) << 4);
+#pragma unroll
+                    for (int k = 0; k < FF_DIG; k++)
+                        *reinterpret_cast<uint4 *>(sm + FS_A + FS_ADIG * k + o) = make_uint4(d[0][k], d[1][k], d[2][k], d[3][k]);
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                if (tid == 0) {
+                    if (mbar_wait(barB, ph_b)) b_inflight--;
+                    else bad = true;
+                }
+                tc_fence_before();
+                if (__syncthreads_or(bad)) { ok = false; break; }
+                tc_fence_after();
+                ph_b ^= 1u;
+                if (tid == 0) issue_mma();
+                if (nint == 1) {                // the leaf beside it, gathered while the MMAs run
+                    const int lc = (sn.lslot < 0) ? sn.lc : sn.rc;
+                    float xh[FF_SPT], xl[FF_SPT];
+                    leaf_rows(Pbase + (size_t)lc * FF_LEAF_BYTES, lvT[ff_lv(lc, site)], xh, xl);
+#pragma unroll
+                    for (int i = 0; i < FF_SPT / 2; i++) {
+                        vh[i] = pk(xh[2 * i], xh[2 * i + 1]);
+                        vl[i] = pk(xl[2 * i], xl[2 * i + 1]);
+                    }
+                    have = true;
+                }
+                // ---- v (or v *=) alpha + E alpha, half of the states at a time
+                const float *sc = reinterpret_cast<const float *>(sm + FS_SC) + (cn & 1) * 3 * K + s0;
+#pragma unroll
+                for (int hf = 0; hf < 2; hf++) {
+                    if (!mbar_wait(hf ? bar1 : bar0, ph_d)) bad = true;
+                    tc_fence_after();
+                    if (hf == 1 && tid == 0 && !bad) issue_next_b();     // every MMA of B has completed
+#pragma unroll
+                    for (int q = 0; q < 2; q++) {
+                        float g[FF_GRP][4];
+                        tmem_ld_groups(tbase + lane_off + 224 * hf + 8 * h + 4 * q, g);
+#pragma unroll
+                        for (int i = 0; i < 2; i++) {
+                            const int x = 4 * hf + 2 * q + i;            // pair of states s0 + 2 x, s0 + 2 x + 1
+                            f2 G[FF_GRP];
+#pragma unroll
+                            for (int k = 0; k < FF_GRP; k++) G[k] = pk(g[k][2 * i], g[k][2 * i + 1]);
+                            const f2 c9 = pk(0x1p-9f, 0x1p-9f);
+                            f2 s1, e1, s2, e2, s3, e3;
+                            two_sum2(G[0], mul2(G[1], c9), s1, e1);
+                            two_sum2(s1, mul2(G[2], pk(0x1p-18f, 0x1p-18f)), s2, e2);
+                            two_sum2(s2, mul2(G[3], pk(0x1p-27f, 0x1p-27f)), s3, e3);
+                            const f2 L = fma2(fma2(G[6], c9, G[5]), c9, G[4]);
+                            const f2 lo = add2(add2(e1, e2), fma2(L, pk(0x1p-36f, 0x1p-36f), e3));
+                            const f2 scale = *reinterpret_cast<const f2 *>(sc + 2 * x);
+                            // + (alpha + E_aa alpha), the largest terms: three float-float numbers
+                            const f2 dh = *reinterpret_cast<const f2 *>(sc + K + 2 * x);
+                            const f2 dl = *reinterpret_cast<const f2 *>(sc + 2 * K + 2 * x);
+                            const f2 p = mul2(dh, ah[x]);
+                            f2 pl = fma2(dh, ah[x], neg2(p));
+                            pl = fma2(dh, al[x], pl);
+                            pl = fma2(dl, ah[x], pl);
+                            f2 t, e, u, f, uh, ul;
+                            two_sum2(ah[x], p, t, e);
+                            two_sum2(t, mul2(s3, scale), u, f);
+                            fast_two_sum2(u, add2(add2(al[x], pl), add2(e, fma2(lo, scale, f))), uh, ul);
+                            if (have) ff_mul2(vh[x], vl[x], uh, ul, vh[x], vl[x]);
+                            else { vh[x] = uh; vl[x] = ul; }
                         }
                     }
-                } else {
-                    // internal: v = alpha + sum_j E[a][j] alpha[j], compensated
-                    const float *Eh = Et + side * 2 * K2, *El = Eh + K2;
-                    const float *xH = slH + (size_t)slot * K * FF_TC, *xL = slL + (size_t)slot * K * FF_TC;
-                    float sh[4][FF_CPT], sa[4][FF_CPT], sb[4][FF_CPT], se[4][FF_CPT];
-#pragma unroll
-                    for (int i = 0; i < 4; i++)
-#pragma unroll
-                        for (int cc = 0; cc < FF_CPT; cc++) sh[i][cc] = sa[i][cc] = sb[i][cc] = se[i][cc] = 0.f;
-#pragma unroll 2
-                    for (int j = 0; j < K; j++) {
-                        const float4 eh = *reinterpret_cast<const float4 *>(Eh + j * K + a0);
-                        const float4 el = *reinterpret_cast<const float4 *>(El + j * K + a0);
-                        float xhv[FF_CPT], xlv[FF_CPT];
-                        if constexpr (FF_CPT == 2) {
-                            const float2 xh = *reinterpret_cast<const float2 *>(xH + j * FF_TC + c0);
-                            const float2 xl = *reinterpret_cast<const float2 *>(xL + j * FF_TC + c0);
-                            xhv[0] = xh.x; xhv[FF_CPT - 1] = xh.y; xlv[0] = xl.x; xlv[FF_CPT - 1] = xl.y;
-                        } else {
-                            xhv[0] = xH[j * FF_TC + c0];
-                            xlv[0] = xL[j * FF_TC + c0];
-                        }
-                        const float ehv[4] = {eh.x, eh.y, eh.z, eh.w}, elv[4] = {el.x, el.y, el.z, el.w};
-#pragma unroll
-                        for (int i = 0; i < 4; i++)
-#pragma unroll
-                            for (int cc = 0; cc < FF_CPT; cc++) {
-                                const float p = __fmul_rn(ehv[i], xhv[cc]);
-                                const float pe = fmaf(ehv[i], xhv[cc], -p);   // exact product error
-                                float s, e;
-                                two_sum(sh[i][cc], p, s, e);
-                                sh[i][cc] = s;
-                                sa[i][cc] = fmaf(ehv[i], xlv[cc], sa[i][cc]);
-                                sb[i][cc] = fmaf(elv[i], xhv[cc], sb[i][cc]);
-                                se[i][cc] = se[i][cc] + (pe + e);
-                            }
-                    }
-#pragma unroll
-                    for (int i = 0; i < 4; i++)
-#pragma unroll
-                        for (int cc = 0; cc < FF_CPT; cc++) {
-                            const float ah = xH[(a0 + i) * FF_TC + c0 + cc], al = xL[(a0 + i) * FF_TC + c0 + cc];
-                            float s, e;
-                            two_sum(ah, sh[i][cc], s, e);
-                            const float lo = __fadd_rn(__fadd_rn(al, (sa[i][cc] + sb[i][cc]) + se[i][cc]), e);
-                            fast_two_sum(s, lo, vh[side][i][cc], vl[side][i][cc]);
-                        }
                 }
+                ph_d ^= 1u;
+                cn++;
+                have = true;
             }
-            __syncthreads();   // every thread is past its reads of the E^T buffers and the child slots
-            if (ni + 1 < a.n_internal) copy_inner(sched[ni + 1]);   // E^T buffers are free again
-            // alpha = v_l * v_r (float-float product), column maxima of the hi parts
-            int *cm = colmax + (ni & 1) * FF_TC;
-            int *cm_next = colmax + ((ni + 1) & 1) * FF_TC;
-            if (tid < FF_TC) cm_next[tid] = 0;
+            if (!ok) break;
+            // ---- column maximum over the four threads of a column, rescale by an exact power of two
+            float mx = 0.0f;
 #pragma unroll
-            for (int cc = 0; cc < FF_CPT; cc++) {
-                float mx = 0.f;
+            for (int i = 0; i < FF_SPT / 2; i++) {
+                float x, y;
+                upk(vh[i], x, y);
+                mx = fmaxf(mx, fmaxf(x, y));
+            }
+            float *cm = reinterpret_cast<float *>(sm + FS_CM) + (ni & 1) * 4 * FF_TC;
+            cm[h * FF_TC + site] = mx;
+            // the four warps that share these columns: a named barrier (1-4) of those 128 threads
+            asm volatile("bar.sync %0, 128;" :: "r"(1 + (warp & 3)) : "memory");
+            mx = fmaxf(fmaxf(cm[site], cm[FF_TC + site]), fmaxf(cm[2 * FF_TC + site], cm[3 * FF_TC + site]));
+            const int e = (mx > 0.0f) ? exp_of(mx) : 0;
+            escale += e;
+            const int ehalf = (-e) >> 1;                     // 2^-e as two factors, as scale2
+            const float f1 = __int_as_float((ehalf + 127) << 23), f2s = __int_as_float((-e - ehalf + 127) << 23);
+            const f2 p1 = pk(f1, f1), p2 = pk(f2s, f2s);
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const float xh = vh[0][i][cc], xl = vl[0][i][cc], yh = vh[1][i][cc], yl = vl[1][i][cc];
-                    const float p = __fmul_rn(xh, yh);
-                    float lo = fmaf(xh, yh, -p);
-                    lo = fmaf(xh, yl, lo);
-                    lo = fmaf(xl, yh, lo);
-                    float h, l;
-                    fast_two_sum(p, lo, h, l);
-                    vh[0][i][cc] = h;
-                    vl[0][i][cc] = l;
-                    mx = h > mx ? h : mx;
+            for (int i = 0; i < FF_SPT / 2; i++) {
+                ah[i] = mul2(mul2(vh[i], p1), p2);
+                al[i] = mul2(mul2(vl[i], p1), p2);
+            }
+            // not a child of the next node: it waits on the stack
+            if (ni + 1 < nin && sched[ni + 1].lc != sn.node && sched[ni + 1].rc != sn.node) {
+                float *st = stk + (size_t)sp * (2 * FF_SPT * FF_THREADS);
+#pragma unroll
+                for (int i = 0; i < FF_SPT / 2; i++) {
+                    float x, y;
+                    upk(ah[i], x, y);
+                    st[(2 * i) * FF_THREADS] = x;
+                    st[(2 * i + 1) * FF_THREADS] = y;
+                    upk(al[i], x, y);
+                    st[(FF_SPT + 2 * i) * FF_THREADS] = x;
+                    st[(FF_SPT + 2 * i + 1) * FF_THREADS] = y;
                 }
-                atomicMax(cm + c0 + cc, __float_as_int(mx));   // non-negative floats order as ints
-            }
-            __syncthreads();   // column maxima complete
-            float *oH = slH + (size_t)sn.oslot * K * FF_TC, *oL = slL + (size_t)sn.oslot * K * FF_TC;
-            int ecol[FF_CPT];
-#pragma unroll
-            for (int cc = 0; cc < FF_CPT; cc++) {
-                const float mx = __int_as_float(cm[c0 + cc]);
-                ecol[cc] = (mx > 0.f) ? exp_of(mx) : 0;
-                if (ty == 0) cscale[c0 + cc] += ecol[cc];
-            }
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                float yh[FF_CPT], yl[FF_CPT];
-#pragma unroll
-                for (int cc = 0; cc < FF_CPT; cc++) {
-                    yh[cc] = scale2(vh[0][i][cc], -ecol[cc]);
-                    yl[cc] = scale2(vl[0][i][cc], -ecol[cc]);
-                }
-                ColStore<float, FF_CPT>::store(oH + (a0 + i) * FF_TC + c0, yh);
-                ColStore<float, FF_CPT>::store(oL + (a0 + i) * FF_TC + c0, yl);
+                sp++;
             }
         }
-        __syncthreads();   // the root's slot written
-        // root: z = alpha_root . prior ; elpr term = (alpha_root . prior*log prior) / z, in FP64
-        double tl = 0.0, te = 0.0;
-        if (tid < FF_TC && tid < ncols) {
-            const int os = sched[a.n_internal - 1].oslot;
-            const float *rH = slH + (size_t)os * K * FF_TC, *rL = slL + (size_t)os * K * FF_TC;
-            const double *pr = a.m.prior + md * K;
-            const double *wl = a.m.wlog + md * K;
+        if (!ok) break;
+        if (__syncthreads_or(bad)) { ok = false; break; }
+        // ---- root: z = alpha_root . prior ; elpr term = (alpha_root . prior*log prior) / z, in
+        // FP64 (the A operand is idle: partial sums [z, wz][4][128])
+        double *zp = reinterpret_cast<double *>(sm + FS_A);
+        {
             double z = 0.0, wz = 0.0;
-            for (int s = 0; s < K; s++) {
-                const double x = (double)rH[s * FF_TC + tid] + (double)rL[s * FF_TC + tid];
-                z += x * pr[s];
-                wz += x * wl[s];
-            }
-            if (z > 0.0) {
-                tl = log(z) + (double)cscale[tid] * 0.69314718055994530942;
-                te = wz / z;
-            } else {
-                tl = -INFINITY;
-                te = 0.0;
-            }
-        }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            tl += __shfl_down_sync(0xffffffffu, tl, o);
-            te += __shfl_down_sync(0xffffffffu, te, o);
+            for (int i = 0; i < FF_SPT / 2; i++) {
+                float xh[2], xl[2];
+                upk(ah[i], xh[0], xh[1]);
+                upk(al[i], xl[0], xl[1]);
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    const double x = (double)xh[u] + (double)xl[u];
+                    z += x * prd[s0 + 2 * i + u];
+                    wz += x * wld[s0 + 2 * i + u];
+                }
+            }
+            zp[h * FF_TC + site] = z;
+            zp[(4 + h) * FF_TC + site] = wz;
         }
-        if ((tid & 31) == 0) {
-            red_l[tid >> 5] = tl;
-            red_e[tid >> 5] = te;
+        __syncthreads();
+        if (h == 0) {
+            double tl = 0.0, te = 0.0;
+            if (site < ncols) {
+                const double z = (zp[site] + zp[FF_TC + site]) + (zp[2 * FF_TC + site] + zp[3 * FF_TC + site]);
+                const double wz = (zp[4 * FF_TC + site] + zp[5 * FF_TC + site]) + (zp[6 * FF_TC + site] + zp[7 * FF_TC + site]);
+                if (z > 0.0) {
+                    tl = log(z) + (double)escale * 0.69314718055994530942;
+                    te = wz / z;
+                } else {
+                    tl = -INFINITY;
+                }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                tl += __shfl_down_sync(0xffffffffu, tl, o);
+                te += __shfl_down_sync(0xffffffffu, te, o);
+            }
+            if ((tid & 31) == 0) {
+                red_l[warp] = tl;
+                red_e[warp] = te;
+            }
         }
         __syncthreads();
         if (tid == 0) {
-            double sl = 0.0, se = 0.0;
-            for (int k = 0; k < (FF_TC + 31) / 32; k++) {
-                sl += red_l[k];
-                se += red_e[k];
-            }
-            a.partials[2 * (size_t)w] = sl;
-            a.partials[2 * (size_t)w + 1] = se;
+            a.partials[2 * (size_t)w] = ((red_l[0] + red_l[1]) + red_l[2]) + red_l[3];
+            a.partials[2 * (size_t)w + 1] = ((red_e[0] + red_e[1]) + red_e[2]) + red_e[3];
         }
     }
+    if (!ok && tid == 0) atomicExch(err, 1);
+    // quiesce: a bulk copy may be outstanding (loads run one ahead) and, after a timed-out
+    // wait, MMAs; both waits are bounded
+    if (tid == 0 && b_inflight > 0 && !mbar_wait(barB, ph_b)) atomicExch(err, 1);
+    if (!ok) {
+        mbar_wait(bar0, ph_d);
+        mbar_wait(bar1, ph_d);
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tbase), "r"(512));
 }
 
 }  // namespace
 
 int ff_tile_cols() { return FF_TC; }
 
-cudaError_t launch_split_ff(const double *in, float *out, size_t nmat, cudaStream_t s)
+size_t ff_pset_bytes(int nl, int nbr)
 {
-    if (nmat == 0) return cudaSuccess;
-    const size_t n = nmat * K2;
-    const unsigned blocks = (unsigned)std::min<size_t>((n + 255) / 256, 4096);
-    k_split_ff<<<blocks, 256, 0, s>>>(in, out, nmat);
+    return (size_t)nl * FF_LEAF_BYTES + (size_t)(nbr - nl) * (FF_INNER_BYTES + FF_ROW_BYTES);
+}
+
+size_t ff_stack_floats(int grid, int depth) { return (size_t)grid * std::max(depth, 1) * 2 * FF_SPT * FF_THREADS; }
+
+cudaError_t launch_split_ff(const double *in, void *out, int nps, int nbr, int nl, cudaStream_t s)
+{
+    if (nps <= 0 || nbr <= 0) return cudaSuccess;
+    k_split_ff<<<(unsigned)nps * (unsigned)nbr, 256, 0, s>>>(in, static_cast<unsigned char *>(out), nbr, nl,
+                                                             ff_pset_bytes(nl, nbr));
     return cudaGetLastError();
 }
 
-size_t prune_ff_smem_bytes(int nslots, int nl, int nint) { return FFSmem::bytes(nslots, nl, nint); }
+size_t prune_ff_smem_bytes(int nl, int nint) { return ff_smem(nl, nint); }
 
-int prune_ff_ctas_per_sm(int nslots, int nl, int nint)
-{
-    const size_t smem = FFSmem::bytes(nslots, nl, nint);
-    int n = 0;
-    if (cudaFuncSetAttribute(k_prune_ff, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_prune_ff, FF_THREADS, smem) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    return n;
-}
-
-cudaError_t launch_prune_ff(const PruneArgs &a, cudaStream_t s, int grid)
+cudaError_t launch_prune_ff(const PruneArgs &a, float *stack, int *err, cudaStream_t s, int grid)
 {
     if (a.nwi <= 0) return cudaSuccess;
-    const size_t smem = FFSmem::bytes(a.nslots, a.nl, a.n_internal);
+    const size_t smem = ff_smem(a.nl, a.n_internal);
     cudaError_t e = cudaFuncSetAttribute(k_prune_ff, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_prune_ff<<<grid, FF_THREADS, smem, s>>>(a);
+    k_prune_ff<<<grid, FF_THREADS, smem, s>>>(a, ff_pset_bytes(a.nl, a.nbr), stack, err);
     return cudaGetLastError();
 }
 

@@ -34,6 +34,7 @@ constexpr size_t NOALLOC_BYTES = size_t(24) << 20;
 constexpr int NOALLOC_MAX_REGIONS = 32768;
 constexpr int NOALLOC_MAX_WORK = 131072;
 constexpr int NOALLOC_MAX_DEVICES = 64;
+constexpr int NOALLOC_LONG_TILE = 16;   // a long region counts as tiles of this many columns against the limits
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_BYTES];
 
@@ -114,6 +115,7 @@ extern "C" int pcsf_lpr_noalloc(pcsf_engine *e, int32_t model, double rho, int32
     };
     // requests: the short regions first, then the long ones; work items contiguous per request
     int nreq = 0, nwi = 0, nws = 0;
+    int64_t tiles = 0;     // column tiles as the limits count them
     bool any_short = false, any_long = false;
     for (int pass = 0; pass < 2; pass++) {
         for (int r = 0; r < n_regions; r++) {
@@ -125,9 +127,11 @@ extern "C" int pcsf_lpr_noalloc(pcsf_engine *e, int32_t model, double rho, int32
             h_req[nreq] = Request{r, model, 0, (uint32_t)c0, rho};
             h_out[nreq] = r;
             h_wib[nreq] = nwi;
+            const int tl = pass ? NOALLOC_LONG_TILE : TC;
+            tiles += (c1 - c0 + tl - 1) / tl;
+            if (tiles > NOALLOC_MAX_WORK)
+                return pcsf_internal_fail(e, PCSF_ERANGE, "pcsf_lpr_noalloc: more than 131072 column tiles in one call");
             for (int64_t c = c0; c < c1; c += tc) {
-                if (nwi >= NOALLOC_MAX_WORK)
-                    return pcsf_internal_fail(e, PCSF_ERANGE, "pcsf_lpr_noalloc: more than 131072 column tiles in one call");
                 h_wi[nwi++] = WorkItem{nreq, (int32_t)std::min<int64_t>(tc, c1 - c), c};
             }
             nreq++;
@@ -135,23 +139,29 @@ extern "C" int pcsf_lpr_noalloc(pcsf_engine *e, int32_t model, double rho, int32
         if (pass == 0) nws = nwi;
     }
     h_wib[nreq] = nwi;
-    // scratch map: [status key, invalid-code slot][requests][request -> region][P set][P(t) in the
-    // arithmetic type][diag(E) low parts][FP64 P(t)][float-float P(t)][work items][wi_begin][partials][elpr]
+    // scratch map: [status key, invalid-code slot][requests][request -> region][P set][diag(E) low
+    // parts][FP64 P(t)][P(t) in the arithmetic type, then the float-float operands over it][work
+    // items][wi_begin][partials][elpr].  The limit counts P(t), a float-float P set of 8 bytes per
+    // entry and the tiles above separately; the map itself is smaller.
     const bool stage64 = fp32 && ((cx.pt64 && any_short) || any_long);   // FP64 formation needed
-    const size_t split_bytes = any_long ? up256(nbr * 2 * K2 * sizeof(float)) : 0;   // float-float P set
+    const size_t bytes_P = std::max(any_short ? nbr * K2 * es : 0, any_long ? ff_pset_bytes(cx.nl, cx.nbr) : 0);
     const size_t off_req = 256;
     const size_t off_out = off_req + up256(sizeof(Request) * (size_t)n_regions);
     const size_t off_ps = off_out + up256(sizeof(int32_t) * (size_t)n_regions);
-    const size_t off_P = off_ps + 256;
-    const size_t off_dlo = off_P + up256(nbr * K2 * es);
+    const size_t off_dlo = off_ps + 256;
     const size_t off_stage = off_dlo + (fp32 ? up256(nbr * K * sizeof(float)) : 0);
-    const size_t off_split = off_stage + (stage64 ? up256(nbr * K2 * sizeof(double)) : 0);
-    const size_t off_wi = off_split + split_bytes;
+    const size_t off_P = off_stage + (stage64 ? up256(nbr * K2 * sizeof(double)) : 0);
+    const size_t off_wi = off_P + up256(bytes_P);
     const size_t off_wib = off_wi + up256(sizeof(WorkItem) * (size_t)nwi);
     const size_t off_part = off_wib + up256(sizeof(int32_t) * (size_t)(n_regions + 1));
     const size_t off_elpr = off_part + up256(sizeof(double) * 2 * (size_t)std::max(nwi, 1));
-    const size_t need = off_elpr + (d_elpr ? 0 : sizeof(double) * (size_t)n_regions);
-    if (need > NOALLOC_BYTES)
+    const size_t end = off_elpr + (d_elpr ? 0 : sizeof(double) * (size_t)n_regions);
+    const size_t need = off_dlo + (off_P - off_dlo) + up256(nbr * K2 * es) +
+                        (any_long ? up256(nbr * 2 * K2 * sizeof(float)) : 0) + up256(sizeof(WorkItem) * (size_t)tiles) +
+                        up256(sizeof(int32_t) * (size_t)(n_regions + 1)) +
+                        up256(sizeof(double) * 2 * (size_t)std::max<int64_t>(tiles, 1)) +
+                        (d_elpr ? 0 : sizeof(double) * (size_t)n_regions);
+    if (need > NOALLOC_BYTES || end > NOALLOC_BYTES)
         return pcsf_internal_fail(e, PCSF_ERANGE, "pcsf_lpr_noalloc: batch needs more than the 24 MiB static scratch area");
     unsigned char *sc = nullptr;
     cudaError_t ce = scratch_on(cx.device, &sc);
@@ -165,7 +175,6 @@ extern "C" int pcsf_lpr_noalloc(pcsf_engine *e, int32_t model, double rho, int32
     void *d_P = sc + off_P;
     float *d_dlo = fp32 ? reinterpret_cast<float *>(sc + off_dlo) : nullptr;   // as the allocating path
     double *d_stage = stage64 ? reinterpret_cast<double *>(sc + off_stage) : nullptr;
-    float *d_split = any_long ? reinterpret_cast<float *>(sc + off_split) : nullptr;
     WorkItem *d_wi = reinterpret_cast<WorkItem *>(sc + off_wi);
     int32_t *d_wib = reinterpret_cast<int32_t *>(sc + off_wib);
     double *d_part = reinterpret_cast<double *>(sc + off_part);
@@ -190,7 +199,6 @@ extern "C" int pcsf_lpr_noalloc(pcsf_engine *e, int32_t model, double rho, int32
     if (ce == cudaSuccess && nwi) ce = cudaMemcpyAsync(d_wi, h_wi, sizeof(WorkItem) * nwi, cudaMemcpyHostToDevice, s);
     if (ce == cudaSuccess) ce = cudaMemcpyAsync(d_wib, h_wib, sizeof(int32_t) * (nreq + 1), cudaMemcpyHostToDevice, s);
     if (ce == cudaSuccess && stage64) ce = launch_pform(true, d_ps, 1, cx.branch, cx.nbr, cx.m, d_stage, d_status, s);
-    if (ce == cudaSuccess && any_long) ce = launch_split_ff(d_stage, d_split, nbr, s);
     if (ce == cudaSuccess && any_short) {
         if (fp32 && cx.pt64)   // FP64 formation rounded to FP32, as pcsf_lpr on a PCSF_PT_FP64 engine
             ce = launch_d2f_rows(d_stage, reinterpret_cast<float *>(d_P), nbr, cx.nbr, nullptr, cx.nl, s, d_dlo);
@@ -216,14 +224,16 @@ extern "C" int pcsf_lpr_noalloc(pcsf_engine *e, int32_t model, double rho, int32
         pa.dlo = d_dlo;
         ce = launch_prune(fp32 ? PCSF_PREC_FP32 : PCSF_PREC_FP64, cx.comp, pa, s, std::min(cx.prune_grid, nws));
     }
+    if (ce == cudaSuccess && any_long) ce = launch_split_ff(d_stage, d_P, 1, cx.nbr, cx.nl, s);   // the short regions are done with d_P
     if (ce == cudaSuccess && nwi > nws) {
         pa.wi = d_wi + nws;
         pa.nwi = nwi - nws;
-        pa.Pbuf = d_split;
+        pa.Pbuf = d_P;
         pa.partials = d_part + 2 * (size_t)nws;
         pa.dither = 0;
         pa.dlo = nullptr;
-        ce = launch_prune_ff(pa, s, std::min(cx.ff_grid, nwi - nws));
+        pa.ff_depth = cx.ff_depth;
+        ce = launch_prune_ff(pa, cx.ff_stack, cx.derr, s, std::min(cx.ff_grid, nwi - nws));
     }
     if (ce == cudaSuccess) ce = launch_reduce(d_part, d_wib, nreq, d_lpr, d_elpr_out, s, d_out);
     int32_t key = STATUS_NONE;

@@ -116,6 +116,7 @@ struct PruneArgs {
     int dither;              // SIMT FP32 kernel: per-column dithering of the leaf partials (prune_common.cuh)
     const float *dlo;        // SIMT FP32 kernel, may be null: per chunk-local P set [nbr][K] low parts of diag(E)
     int tile;                // SIMT FP32 kernel: column tile 32 or 64, 0 = the default rule (simt_tile_cols)
+    int ff_depth;            // float-float kernel: partials that wait at once (its stack's entries)
     int tc_shape;            // TF32 tensor-core kernel: 0 alpha kept in registers, 1 read back (identical values)
 };
 // comp: 0 plain FP32 sums, 1 Kahan, 2 blocked Kahan (see prune_common.cuh)
@@ -191,15 +192,17 @@ bool prune_tc_dual_supported(int nslots, int nl);
 cudaError_t launch_reduce(const double *partials, const int32_t *wi_begin, int nreq, double *out_lpr,
                           double *out_elpr, cudaStream_t s, const int32_t *out_index = nullptr);
 
-// Float-float SIMT pruning (ff_kernels.cu): returned values that agree with the FP64
-// path to ~1e-12 relative.  Pbuf holds split E^T sets, per P set [nbr][hi K2 | lo K2]
-// floats, made from the FP64 P(t) formation's output by launch_split_ff; tiles of
-// ff_tile_cols() columns; partials as k_prune.
-cudaError_t launch_prune_ff(const PruneArgs &a, cudaStream_t s, int grid);
-cudaError_t launch_split_ff(const double *in, float *out, size_t nmat, cudaStream_t s);
+// Float-float pruning on the tensor cores (ff_kernels.cu): returned values that agree with
+// the FP64 path to ~1e-12 relative.  Pbuf holds per P set ff_pset_bytes() of operands, made
+// from the FP64 P(t) formation's output by launch_split_ff; tiles of ff_tile_cols() columns,
+// one CTA per SM; stack = ff_stack_floats(grid, PruneArgs.ff_depth) floats; partials as
+// k_prune; err is set if a bounded wait timed out.
+cudaError_t launch_prune_ff(const PruneArgs &a, float *stack, int *err, cudaStream_t s, int grid);
+cudaError_t launch_split_ff(const double *in, void *out, int nps, int nbr, int nl, cudaStream_t s);
 int ff_tile_cols();
-size_t prune_ff_smem_bytes(int nslots, int nl, int nint);
-int prune_ff_ctas_per_sm(int nslots, int nl, int nint);
+size_t ff_pset_bytes(int nl, int nbr);
+size_t ff_stack_floats(int grid, int depth);
+size_t prune_ff_smem_bytes(int nl, int nint);
 
 // Outside-pass products (outside_kernels.cu): per request (one CTA at a time, tiles of
 // outside_tile_cols() columns in order) the log-likelihood, optionally the expected
@@ -244,6 +247,8 @@ struct NoallocCtx {
     int prune_grid;
     int simt_tile;         // SIMT column tile chosen for the engine (0: the default rule)
     int ff_grid;           // CTAs of the float-float kernel (0: not available)
+    int ff_depth;          // its stack: entries per CTA, and the memory
+    float *ff_stack;
     int64_t exact_min_units;   // regions with columns x (nl - 2) >= this use the float-float kernel
     int *derr;             // device error flag of timed-out waits
 };
