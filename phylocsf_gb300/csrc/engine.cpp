@@ -1613,19 +1613,28 @@ static int outside_impl(pcsf_engine *e, pcsf_batch *b, int model, const double *
     const size_t scr = outside_scratch_per_cta(fp64, e->nl);
     const size_t pset_bytes = (size_t)e->nbr * K2 * es;
     const size_t cnt_bytes = counts ? (size_t)e->nbr * K2 * sizeof(double) : 0;
-    // regions per launch: P sets and counts of a chunk within ~2 GiB
+    // regions per launch: P sets and counts of a chunk within ~2 GiB (a region of several parts has
+    // its parts' counts beside its own: one more per region and one per CTA at most)
     const int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)std::max(nreg, 1),
-                                                                (size_t(2) << 30) / (pset_bytes + cnt_bytes)));
-    const int grid = std::max(1, std::min(e->sm_count, chunk));
+                                                                (size_t(2) << 30) / (pset_bytes + 2 * cnt_bytes)));
+    // CTAs of a launch: every SM's worth, at most the tiles of the longest chunk
+    int64_t most_tiles = 1;
+    for (int r0 = 0; r0 < nreg; r0 += chunk) {
+        int64_t t = 0;
+        for (int r = r0; r < std::min(nreg, r0 + chunk); r++) t += (b->offs[r + 1] - b->offs[r] + TC - 1) / TC;
+        most_tiles = std::max(most_tiles, t);
+    }
+    const int grid = (int)std::min<int64_t>(
+        (int64_t)e->sm_count * outside_ctas_per_sm(fp64, comp, e->nslots, e->nl, (int)e->sched.size()), most_tiles);
     DevBuf<unsigned char> dP, dscr;
-    DevBuf<double> dcnt, dlpr, dpost;
+    DevBuf<double> dcnt, dlpr, dlprp, dpost;
+    DevBuf<OutsidePart> dparts;
     DevBuf<PSet> dps;
     DevBuf<Request> dreq;
     DevBuf<WorkItem> dwi;
     DevBuf<int32_t> dwib, dstatus, dsel;
     CK(dP.reserve((size_t)chunk * pset_bytes), "cudaMalloc P(t)");
     CK(dscr.reserve((size_t)grid * scr), "cudaMalloc outside-pass scratch");
-    if (counts) CK(dcnt.reserve((size_t)chunk * e->nbr * K2), "cudaMalloc counts");
     CK(dlpr.reserve(chunk), "cudaMalloc");
     CK(dps.reserve(chunk), "cudaMalloc");
     CK(dreq.reserve(chunk), "cudaMalloc");
@@ -1642,28 +1651,45 @@ static int outside_impl(pcsf_engine *e, pcsf_batch *b, int model, const double *
         std::vector<PSet> ps(nr);
         std::vector<Request> rq(nr);
         std::vector<WorkItem> wis;
-        std::vector<int32_t> wib(nr + 1);
+        std::vector<OutsidePart> parts;
+        std::vector<int32_t> pbeg(nr + 1);
+        // tiles per part: the chunk's tiles over the CTAs (a part's counts stay in its own buffer,
+        // so that shorter parts would only cost memory and the summing)
+        int64_t ntiles = 0;
+        for (int r = r0; r < r1; r++) ntiles += (b->offs[r + 1] - b->offs[r] + TC - 1) / TC;
+        const int tpp = (int)std::max<int64_t>(1, (ntiles + grid - 1) / grid);
+        int nslot = nr;
         for (int r = 0; r < nr; r++) {
             const int reg = r0 + r;
             if (!(rho[reg] > 0.0) || !std::isfinite(rho[reg])) return e->fail(PCSF_EINVAL, "rho[%d] = %g", reg, rho[reg]);
             ps[r] = PSet{model, 0, rho[reg]};
             rq[r] = Request{reg, model, r, (uint32_t)b->offs[reg], rho[reg]};
-            wib[r] = (int)wis.size();
+            pbeg[r] = (int)parts.size();
+            const int w0 = (int)wis.size();
             for (int64_t c = b->offs[reg]; c < b->offs[reg + 1]; c += TC)
                 wis.push_back(WorkItem{r, (int32_t)std::min<int64_t>(TC, b->offs[reg + 1] - c), c});
+            const int w1 = (int)wis.size();
+            for (int w = w0; w < w1; w += tpp)
+                parts.push_back(OutsidePart{r, w, std::min(w + tpp, w1), w1 - w0 <= tpp ? r : nslot++});
         }
-        wib[nr] = (int)wis.size();
+        pbeg[nr] = (int)parts.size();
+        if (counts) CK(dcnt.reserve((size_t)nslot * e->nbr * K2), "cudaMalloc counts");
+        CK(dparts.reserve(parts.size()), "cudaMalloc");
+        CK(dlprp.reserve(parts.size()), "cudaMalloc");
         CK(dwi.reserve(std::max<size_t>(wis.size(), 1)), "cudaMalloc");
         CK(cudaMemcpyAsync(dps.p, ps.data(), sizeof(PSet) * nr, cudaMemcpyHostToDevice, s), "H2D");
         CK(cudaMemcpyAsync(dreq.p, rq.data(), sizeof(Request) * nr, cudaMemcpyHostToDevice, s), "H2D");
         if (!wis.empty()) CK(cudaMemcpyAsync(dwi.p, wis.data(), sizeof(WorkItem) * wis.size(), cudaMemcpyHostToDevice, s), "H2D");
-        CK(cudaMemcpyAsync(dwib.p, wib.data(), sizeof(int32_t) * (nr + 1), cudaMemcpyHostToDevice, s), "H2D");
+        CK(cudaMemcpyAsync(dwib.p, pbeg.data(), sizeof(int32_t) * (nr + 1), cudaMemcpyHostToDevice, s), "H2D");
+        if (!parts.empty())
+            CK(cudaMemcpyAsync(dparts.p, parts.data(), sizeof(OutsidePart) * parts.size(), cudaMemcpyHostToDevice, s), "H2D");
         CK(cudaMemsetAsync(dstatus.p, 0x7f, sizeof(int32_t) * nr, s), "memset");
-        if (counts) CK(cudaMemsetAsync(dcnt.p, 0, sizeof(double) * (size_t)nr * e->nbr * K2, s), "memset");
         CK(launch_pform(fp64, dps.p, nr, e->dbranch.p, e->nbr, e->dm, dP.p, dstatus.p, s), "P(t) formation launch");
         OutsideArgs oa{};
         oa.wi = dwi.p;
-        oa.wi_begin = dwib.p;
+        oa.parts = dparts.p;
+        oa.nparts = (int)parts.size();
+        oa.part_begin = dwib.p;
         oa.nreq = nr;
         oa.req = dreq.p;
         oa.leaves = b->dleaves.p;
@@ -1676,13 +1702,14 @@ static int outside_impl(pcsf_engine *e, pcsf_batch *b, int model, const double *
         oa.m = e->dm;
         oa.scratch = dscr.p;
         oa.scratch_per_cta = scr;
-        oa.lpr = dlpr.p;
+        oa.lpr = dlprp.p;
+        oa.lpr_out = dlpr.p;
         oa.counts = counts ? dcnt.p : nullptr;
         oa.sel = n_sel > 0 ? dsel.p : nullptr;
         oa.post = dpost.p;
         oa.total_cols = b->total_cols;
-        CK(launch_outside(fp64, comp, oa, s, std::min(grid, nr)), "outside-pass launch");
-        e->stats.kernel_launches += 2;
+        CK(launch_outside(fp64, comp, oa, s, grid), "outside-pass launch");
+        e->stats.kernel_launches += 3;
         std::vector<int32_t> keys(nr);
         std::vector<double> hl(nr);
         CK(cudaMemcpyAsync(keys.data(), dstatus.p, sizeof(int32_t) * nr, cudaMemcpyDeviceToHost, s), "D2H");

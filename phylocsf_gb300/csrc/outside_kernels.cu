@@ -12,14 +12,20 @@
 // per tile a 64 x 64 x (tile columns) product, accumulated over the tiles of a region
 // and multiplied by P_c once at the end.
 //
-// One CTA owns one request (region, model, rho) at a time and walks its column tiles
-// in order, so every count is summed in a fixed order (no atomics): the results do
-// not depend on the launch configuration.  The inside pass is the one of k_grad and
+// One CTA owns one part of a request (region, model, rho) at a time, a run of its column
+// tiles, and walks them in order; k_counts sums a request's parts in order and multiplies
+// by P_c (no atomics; the parts depend on the number of tiles and SMs alone).  A CTA per
+// request left a call of 64 regions waiting for the longest one, 47 tiles in a row, and the
+// count products read alpha from global memory with 16 lines per load: 38.4 ms on 29 leaves
+// (27,641 columns), 3.1 ms with parts and the products' operands column by column in shared
+// memory.  What bounds it now is the chain of a side's phases at three CTAs per SM, FP64
+// conversions and sums (two lanes per clock) among them.  The inside pass is the one of k_grad and
 // stores every child partial, the alpha of every internal node and the per-column
 // exponents of the power-of-two rescaling in a per-CTA scratch area; exponent
 // bookkeeping per column as in k_grad:
 //   alpha_i = alpha~_i 2^{e(i)},  beta_c = beta~_c 2^{f(c)},  z = z~ 2^{e(root)}.
 // FP64 on the FP64 engine; FP32 with compensated sums on the others.
+#include <algorithm>
 #include <cmath>
 
 #include "pcsf_internal.h"
@@ -37,7 +43,9 @@ template <typename T>
 struct OutLayout {
     static size_t smem(int nslots, int nl, int nint)
     {
-        size_t b = sizeof(T) * (2 * (size_t)K2 + (size_t)nslots * K * OS_TC + (size_t)K * OS_TC);   // Mat[2], slots, X
+        // Mat[2], slots, X; in the outside pass E^T (rows of LDN) and the two transposed tiles take their place
+        size_t b = sizeof(T) * (std::max<size_t>(2 * (size_t)K2 + (size_t)nslots * K * OS_TC, (size_t)K * LDN + 2 * OS_TC * LDN) +
+                                (size_t)K * OS_TC);
         b += sizeof(typename AtomMax<T>::U) * OS_TC;                                               // column maxima
         b += sizeof(double) * 2 * OS_TC;                                                           // z~, column weights
         b += sizeof(int) * OS_TC;                                                                  // e(root)
@@ -63,7 +71,12 @@ __global__ void __launch_bounds__(OS_THREADS) k_outside(OutsideArgs a)
     extern __shared__ __align__(16) unsigned char osm[];
     T *Mat = reinterpret_cast<T *>(osm);                           // [2][K][K]
     T *slots = Mat + 2 * K2;                                        // [nslots][K][TC]
-    T *X = slots + (size_t)a.nslots * K * TC;                       // [K][TC]
+    // outside pass: E^T of a branch, and inter and alpha column by column (the inside pass's
+    // Mat and slots are idle then)
+    T *Ert = Mat, *XT = Mat + K * LDN, *YT = XT + TC * LDN;         // [K][LDN], [TC][LDN], [TC][LDN]
+    constexpr size_t OUT = (size_t)K * LDN + 2 * TC * LDN;
+    const size_t inw = 2 * (size_t)K2 + (size_t)a.nslots * K * TC;
+    T *X = Mat + (inw > OUT ? inw : OUT);                           // [K][TC]
     MU *colmax = reinterpret_cast<MU *>(X + K * TC);                // [TC]
     double *zt = reinterpret_cast<double *>(colmax + TC);           // [TC]
     double *wcol = zt + TC;                                         // [TC]
@@ -88,15 +101,16 @@ __global__ void __launch_bounds__(OS_THREADS) k_outside(OutsideArgs a)
 
     for (int f = tid; f < a.n_internal; f += OS_THREADS) sched[f] = a.sched[f];
 
-    for (int r = blockIdx.x; r < a.nreq; r += gridDim.x) {
-        const Request rq = a.req[r];
+    for (int pt = blockIdx.x; pt < a.nparts; pt += gridDim.x) {
+        const OutsidePart part = a.parts[pt];
+        const Request rq = a.req[part.request];
         const int md = rq.model;
         const T *Pbase = reinterpret_cast<const T *>(a.Pbuf) + (size_t)rq.pset * a.nbr * K2;
         const double *pr = a.m.prior + md * K;
-        double *cnt = a.counts ? a.counts + (size_t)r * a.nbr * K2 : nullptr;
-        double lpr = 0.0;    // thread 0: the request's log-likelihood, summed tile by tile in order
+        double *cnt = a.counts ? a.counts + (size_t)part.slot * a.nbr * K2 : nullptr;
+        double lpr = 0.0;    // thread 0: the part's log-likelihood, summed tile by tile in order
 
-        for (int w = a.wi_begin[r]; w < a.wi_begin[r + 1]; w++) {
+        for (int w = part.wi0; w < part.wi1; w++) {
             const WorkItem wi = a.wi[w];
             const int ncols = wi.ncols;
             const uint8_t *lg = a.leaves + (size_t)wi.col0 * nl;
@@ -222,11 +236,7 @@ __global__ void __launch_bounds__(OS_THREADS) k_outside(OutsideArgs a)
                     const int s = side ? sn.lc : sn.rc;
                     const bool internal = c >= nl;
                     __syncthreads();   // the previous side is finished with X, Mat[0], colmax, wcol
-                    if (internal) {
-                        // E_c in row-major order (the buffer holds E_c^T)
-                        const T *g = Pbase + (size_t)c * K2;
-                        for (int f = tid; f < K2; f += OS_THREADS) Mat[(f % K) * K + f / K] = g[f];
-                    }
+                    if (internal) stage_rows<T, OS_THREADS>(Ert, Pbase + (size_t)c * K2, tid);
                     for (int f = tid; f < TC; f += OS_THREADS) colmax[f] = 0;
                     const T *Vs = V + (size_t)s * K * TC;
                     for (int f = tid; f < K * TC; f += OS_THREADS) X[f] = Bp[f] * Vs[f];    // inter~
@@ -236,11 +246,12 @@ __global__ void __launch_bounds__(OS_THREADS) k_outside(OutsideArgs a)
                                         ? ldexp(1.0, fS[(size_t)p * TC + tid] + e_of(s, tid) + e_of(c, tid) - eroot[tid]) / z
                                         : 0.0;
                     }
+                    asm volatile("cp.async.wait_all;" ::: "memory");
                     __syncthreads();
                     if (internal) {
                         // beta~_c = P_c^T inter~ = inter~ + E_c^T inter~, rescaled per column
                         T bt[4][CPT];
-                        contract<T, TC, KAHAN>(Mat, X, a0, c0, bt);
+                        contract_rows<T, TC, KAHAN>(Ert, X, a0, c0, bt);
 #pragma unroll
                         for (int cc = 0; cc < CPT; cc++) {
                             T mx = (T)0;
@@ -277,70 +288,88 @@ __global__ void __launch_bounds__(OS_THREADS) k_outside(OutsideArgs a)
                         }
                     }
                     if (cnt) {
-                        __syncthreads();   // the beta contraction is finished with X
-                        for (int f = tid; f < K * TC; f += OS_THREADS) X[f] = (T)((double)X[f] * wcol[f % TC]);
+                        // inter~ w and alpha~_c, column by column (from here a column's 64 states
+                        // are contiguous: one vector load for each of a thread's two sides)
+                        const T *Ac = A + (size_t)(internal ? c - nl : 0) * K * TC;
+                        for (int f = tid; f < K * TC; f += OS_THREADS) {
+                            XT[(f % TC) * LDN + f / TC] = (T)((double)X[f] * wcol[f % TC]);
+                            if (internal) YT[(f % TC) * LDN + f / TC] = Ac[f];
+                        }
                         __syncthreads();
                         // M_c[a][b] += sum_col inter~[a] w alpha~_c[b] for this thread's 4 x 4 block
-                        double m4[4][4];
                         T acc[4][4];
 #pragma unroll
                         for (int i = 0; i < 4; i++)
 #pragma unroll
                             for (int j = 0; j < 4; j++) acc[i][j] = (T)0;
                         if (internal) {
-                            const T *Ac = A + (size_t)(c - nl) * K * TC;
+#pragma unroll 4
                             for (int col = 0; col < TC; col++) {
                                 T xa[4], yb[4];
-#pragma unroll
-                                for (int i = 0; i < 4; i++) xa[i] = X[(a0 + i) * TC + col];
-#pragma unroll
-                                for (int j = 0; j < 4; j++) yb[j] = Ac[(size_t)(b0 + j) * TC + col];
+                                Vec4<T>::load(XT + col * LDN + a0, xa);
+                                Vec4<T>::load(YT + col * LDN + b0, yb);
 #pragma unroll
                                 for (int i = 0; i < 4; i++)
 #pragma unroll
                                     for (int j = 0; j < 4; j++) acc[i][j] += xa[i] * yb[j];
                             }
                         } else {
+#pragma unroll 4
                             for (int col = 0; col < TC; col++) {
                                 const int sl = lvT[c * TC + col];
+                                T xa[4];
+                                Vec4<T>::load(XT + col * LDN + a0, xa);
 #pragma unroll
-                                for (int i = 0; i < 4; i++) {
-                                    const T xa = X[(a0 + i) * TC + col];
+                                for (int j = 0; j < 4; j++) {
+                                    const bool hit = sl >= K || sl == b0 + j;
 #pragma unroll
-                                    for (int j = 0; j < 4; j++)
-                                        if (sl >= K || sl == b0 + j) acc[i][j] += xa;
+                                    for (int i = 0; i < 4; i++) acc[i][j] = hit ? acc[i][j] + xa[i] : acc[i][j];
                                 }
                             }
                         }
                         double *cc4 = cnt + (size_t)c * K2;
+                        const bool first = w == part.wi0;
 #pragma unroll
-                        for (int i = 0; i < 4; i++)
-#pragma unroll
-                            for (int j = 0; j < 4; j++) {
-                                m4[i][j] = cc4[(a0 + i) * K + b0 + j] + (double)acc[i][j];
-                                cc4[(a0 + i) * K + b0 + j] = m4[i][j];
-                            }
+                        for (int i = 0; i < 4; i++) {
+                            double2 *q = reinterpret_cast<double2 *>(cc4 + (a0 + i) * K + b0);
+                            double2 u = first ? make_double2(0.0, 0.0) : q[0], v = first ? make_double2(0.0, 0.0) : q[1];
+                            u.x += (double)acc[i][0];
+                            u.y += (double)acc[i][1];
+                            v.x += (double)acc[i][2];
+                            v.y += (double)acc[i][3];
+                            q[0] = u;
+                            q[1] = v;
+                        }
                     }
                 }
             }
         }
-        // counts = P_c o M_c (each thread its own entries, as accumulated)
-        if (cnt) {
-            for (int c = 0; c < a.nbr; c++) {
-                const T *Et = Pbase + (size_t)c * K2;
-                double *cc4 = cnt + (size_t)c * K2;
-#pragma unroll
-                for (int i = 0; i < 4; i++)
-#pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        const int aa = a0 + i, bb = b0 + j;
-                        const double pab = (double)Et[bb * K + aa] + (aa == bb ? 1.0 : 0.0);
-                        cc4[aa * K + bb] *= pab;
-                    }
-            }
-        }
-        if (tid == 0) a.lpr[r] = lpr;
+        if (tid == 0) a.lpr[pt] = lpr;
         __syncthreads();
+    }
+}
+
+// Request r's parts in order: counts = P_c o sum M_c, and the log-likelihood.  A request of one
+// part has accumulated in its own counts already (slot r); the others' parts hold slots from
+// nreq on.  One CTA per (branch, request).
+template <typename T>
+__global__ void __launch_bounds__(OS_THREADS) k_counts(OutsideArgs a)
+{
+    const int c = blockIdx.y, r = blockIdx.x, tid = threadIdx.x;
+    const int p0 = a.part_begin[r], p1 = a.part_begin[r + 1];
+    if (c == 0 && tid == 0) {
+        double lpr = 0.0;
+        for (int p = p0; p < p1; p++) lpr += a.lpr[p];
+        a.lpr_out[r] = lpr;
+    }
+    if (!a.counts) return;
+    const T *Et = reinterpret_cast<const T *>(a.Pbuf) + ((size_t)a.req[r].pset * a.nbr + c) * K2;
+    double *out = a.counts + ((size_t)r * a.nbr + c) * K2;
+    for (int f = tid; f < K2; f += OS_THREADS) {
+        const int aa = f / K, bb = f % K;
+        double m = 0.0;
+        for (int p = p0; p < p1; p++) m += a.counts[((size_t)a.parts[p].slot * a.nbr + c) * K2 + f];
+        out[f] = m * ((double)Et[bb * K + aa] + (aa == bb ? 1.0 : 0.0));
     }
 }
 
@@ -350,13 +379,35 @@ cudaError_t launch_outside_t(const OutsideArgs &a, cudaStream_t s, int grid)
     const size_t smem = OutLayout<T>::smem(a.nslots, a.nl, a.n_internal);
     cudaError_t e = cudaFuncSetAttribute(k_outside<T, KAHAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_outside<T, KAHAN><<<grid, OS_THREADS, smem, s>>>(a);
+    if (a.nparts > 0) k_outside<T, KAHAN><<<std::min(grid, a.nparts), OS_THREADS, smem, s>>>(a);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    k_counts<T><<<dim3(a.nreq, a.counts ? a.nbr : 1), OS_THREADS, 0, s>>>(a);
     return cudaGetLastError();
+}
+
+template <typename T, int KAHAN>
+int ctas_per_sm_t(int nslots, int nl, int nint)
+{
+    const size_t smem = OutLayout<T>::smem(nslots, nl, nint);
+    int n = 0;
+    if (cudaFuncSetAttribute(k_outside<T, KAHAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_outside<T, KAHAN>, OS_THREADS, smem) != cudaSuccess) {
+        cudaGetLastError();
+        return 1;
+    }
+    return std::max(n, 1);
 }
 
 }  // namespace
 
 int outside_tile_cols() { return OS_TC; }
+
+int outside_ctas_per_sm(bool fp64, int comp, int nslots, int nl, int nint)
+{
+    if (fp64) return ctas_per_sm_t<double, 0>(nslots, nl, nint);
+    return comp == 2 ? ctas_per_sm_t<float, 2>(nslots, nl, nint) : ctas_per_sm_t<float, 1>(nslots, nl, nint);
+}
 
 size_t outside_smem_bytes(bool fp64, int nslots, int nl, int nint)
 {

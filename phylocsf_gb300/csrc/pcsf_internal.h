@@ -204,12 +204,20 @@ size_t ff_pset_bytes(int nl, int nbr);
 size_t ff_stack_floats(int grid, int depth);
 size_t prune_ff_smem_bytes(int nl, int nint);
 
-// Outside-pass products (outside_kernels.cu): per request (one CTA at a time, tiles of
-// outside_tile_cols() columns in order) the log-likelihood, optionally the expected
-// substitution counts of every branch and the posteriors of selected nodes.
+// Outside-pass products (outside_kernels.cu): per request the log-likelihood, optionally the
+// expected substitution counts of every branch and the posteriors of selected nodes.  A part is
+// a run of one request's work items (tiles of outside_tile_cols() columns, in order), worked by
+// one CTA at a time; parts of one request are contiguous.
+struct OutsidePart {
+    int32_t request;             // the request's index
+    int32_t wi0, wi1;            // its work items
+    int32_t slot;                // where its counts accumulate: the request, or nreq + k if it has several parts
+};
 struct OutsideArgs {
-    const WorkItem *wi;          // work items, contiguous per request
-    const int32_t *wi_begin;     // [nreq + 1]
+    const WorkItem *wi;
+    const OutsidePart *parts;
+    int nparts;
+    const int32_t *part_begin;   // [nreq + 1]
     int nreq;
     const Request *req;          // Request.pset indexes Pbuf
     const uint8_t *leaves;       // [total_cols][nl]
@@ -219,14 +227,16 @@ struct OutsideArgs {
     DevModels m;
     void *scratch;               // gridDim.x * scratch_per_cta bytes
     size_t scratch_per_cta;
-    double *lpr;                 // [nreq]
-    double *counts;              // [nreq][nbr][K][K], zeroed by the caller; null: none
+    double *lpr;                 // [nparts]
+    double *lpr_out;             // [nreq]
+    double *counts;              // [nreq + parts of split requests][nbr][K][K]; null: none
     const int32_t *sel;          // [n] output row of each node, -1 if not selected; null: no posteriors
     double *post;                // [n_selected][total_cols][K]
     int64_t total_cols;
 };
 cudaError_t launch_outside(bool fp64, int comp, const OutsideArgs &a, cudaStream_t s, int grid);
 int outside_tile_cols();
+int outside_ctas_per_sm(bool fp64, int comp, int nslots, int nl, int nint);
 size_t outside_smem_bytes(bool fp64, int nslots, int nl, int nint);
 size_t outside_scratch_per_cta(bool fp64, int nl);
 

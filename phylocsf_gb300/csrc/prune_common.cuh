@@ -249,6 +249,94 @@ __device__ inline void contract(const T *M, const T *X, int a0, int c0, T out[4]
     }
 }
 
+// out[i][cc] = sum_j N[a0+i][j] * X[j][c0+cc] with row a of N at N + a * LDN: contract() of the
+// transposed matrix (the same products in the same order, so the same values), for the outside
+// pass, which multiplies by E^T as it is stored.  Four consecutive j of a row come in one load;
+// LDN = K + 4 keeps the two row groups of a warp on different banks.
+constexpr int LDN = K + 4;
+template <typename T, int TC, int COMP>
+__device__ inline void contract_rows(const T *N, const T *X, int a0, int c0, T out[4][TC / 16])
+{
+    constexpr int CPT = TC / 16;
+    T comp[4][CPT];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int cc = 0; cc < CPT; cc++) {
+            out[i][cc] = (T)0;
+            comp[i][cc] = (T)0;
+        }
+    // sum (or, first = true, start) of J products from j0
+    auto products = [&](int j0, T g[4][CPT], bool first) {
+        T e[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) Vec4<T>::load(N + (a0 + i) * LDN + j0, e[i]);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            T x[CPT];
+            ColLoad<T, CPT>::load(X + (j0 + j) * TC + c0, x);
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int cc = 0; cc < CPT; cc++) {
+                    if (COMP == 1) {
+                        const T y = e[i][j] * x[cc] - comp[i][cc];
+                        const T t = g[i][cc] + y;
+                        comp[i][cc] = (t - g[i][cc]) - y;
+                        g[i][cc] = t;
+                    } else if (COMP == 2) {
+                        g[i][cc] = (first && j == 0) ? e[i][j] * x[cc] : fma(e[i][j], x[cc], g[i][cc]);
+                    } else {
+                        g[i][cc] += e[i][j] * x[cc];
+                    }
+                }
+        }
+    };
+    if (COMP == 2) {
+        products(0, out, true);
+        products(4, out, false);
+#pragma unroll 1
+        for (int jb = 8; jb < K; jb += 8) {
+            T g[4][CPT];
+            products(jb, g, true);
+            products(jb + 4, g, false);
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int cc = 0; cc < CPT; cc++) {
+                    T y = g[i][cc] - comp[i][cc];
+                    T t = out[i][cc] + y;
+                    comp[i][cc] = (t - out[i][cc]) - y;
+                    out[i][cc] = t;
+                }
+        }
+    } else {
+#pragma unroll 1
+        for (int jb = 0; jb < K; jb += 4) products(jb, out, false);
+    }
+    if (COMP) {
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int cc = 0; cc < CPT; cc++) out[i][cc] -= comp[i][cc];
+    }
+}
+
+// E^T of a branch [K][K] into shared memory with rows of LDN, asynchronously (the caller commits
+// and waits)
+template <typename T, int THREADS>
+__device__ inline void stage_rows(T *dst, const T *src, int tid)
+{
+    constexpr int V = 16 / sizeof(T);          // entries of one 16-byte copy
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    for (int f = tid; f < K2 / V; f += THREADS) {
+        const int r = f / (K / V), c = (f - r * (K / V)) * V;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + (uint32_t)((r * LDN + c) * sizeof(T))),
+                     "l"(src + (size_t)r * K + c) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
 // Partial of child c at its parent: v[a] = alpha_c[a] + sum_j E_c[a][j] alpha_c[j]
 // (internal child, slot >= 0; Et = E_c^T) or the gather v[a] = P_c[a][s] of a
 // leaf in state s (1 for a marginalised leaf: P rows sum to 1).

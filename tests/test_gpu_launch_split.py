@@ -53,3 +53,29 @@ def test_rate_matrices_split_over_clusters(prec):
     for n in got:
         for k in ("lpr", "d_branch", "d_rho", "d_kappa", "d_omega"):
             assert np.array_equal(got[n][k], got[90][k][:n]), (n, k)
+
+
+# one region in one part (a call of many tiles) and split into parts of one tile each (alone):
+# counts and lpr differ by the FP64 rounding of their sums alone (a few hundred terms), node
+# posteriors not at all
+@pytest.mark.parametrize("prec", ["fp32b", "fp64"])
+def test_outside_parts(prec):
+    ps, offs, leaves = _regions("12flies", [32 * 9 + 5])
+    eng = P.Engine(ps.tree, ps.S_c, ps.pi_c, ps.S_n, ps.pi_n, precision=prec)
+    n = 120 if prec == "fp32b" else 3
+    L = int(offs[-1])
+    one = eng.batch(offs, leaves)
+    many = eng.batch(np.arange(n + 2) * L, np.tile(leaves, (n + 1, 1)))
+    empty = eng.batch([0, 0, L], leaves)
+    c1, l1, st = eng.branch_counts(one, 0, 0.7)
+    assert (st == 0).all()
+    for b in (many, empty):
+        c, l, st = eng.branch_counts(b, 0, 0.7)
+        assert (st == 0).all()
+        if b is empty:
+            assert (c[0] == 0).all() and l[0] == 0
+            c, l = c[1:], l[1:]
+        assert np.abs(c - c1).max() <= 1e-12 * np.abs(c1).max() and np.abs(l - l1).max() <= 1e-12 * np.abs(l1).max()
+    p1, _ = eng.node_posteriors(one, 0, 0.7, [0, ps.tree.nl, ps.tree.n - 1])
+    pm, _ = eng.node_posteriors(many, 0, 0.7, [0, ps.tree.nl, ps.tree.n - 1])
+    assert np.array_equal(p1, pm[:, :L]) and np.array_equal(p1, pm[:, -L:])
