@@ -161,7 +161,7 @@ struct pcsf_engine {
     DevBuf<float> dQrowf;
     DevBuf<double> dQrowd;
     HostBuf<double> hgrad;
-    int grad_grid = 0;
+    int grad_grid[2] = {0, 0};     // CTAs of the adjoint: without, with the rate parameters
     HostBuf<PSet> hps;
     HostBuf<Request> hreq;
     HostBuf<WorkItem> hwi;
@@ -627,8 +627,10 @@ static int engine_init_common(pcsf_engine *e, const pcsf_tree *tree, int32_t fla
     size_t gsmem = grad_smem_bytes(e->prec, e->nslots, e->nl, (int)e->sched.size(), 0);
     if (gsmem > (size_t)prop.sharedMemPerBlockOptin)
         return e->fail(PCSF_EINVAL, "tree needs %zu B shared memory for the gradient", gsmem);
-    int gper = std::max(1, std::min(4, (int)(prop.sharedMemPerMultiprocessor / (gsmem + 1024))));
-    e->grad_grid = prop.multiProcessorCount * gper;
+    for (int k = 0; k < 2; k++)
+        e->grad_grid[k] = prop.multiProcessorCount *
+                          grad_ctas_per_sm(e->prec == PCSF_PREC_FP64 ? PCSF_PREC_FP64 : PCSF_PREC_FP32, e->nslots, e->nl,
+                                           (int)e->sched.size(), 2 * k);
     if (e->prec != PCSF_PREC_FP64 &&
         prune_ff_smem_bytes(e->nl, (int)e->sched.size()) <= (size_t)prop.sharedMemPerBlockOptin) {
         // a node's partial waits when the next node of the schedule is not its parent
@@ -695,8 +697,8 @@ static int evaluate(pcsf_engine *e, pcsf_batch *b, const std::vector<Request> &r
     if (drho && (grad || dyn || accurate || !e->dual_ok))
         return e->fail(PCSF_EINVAL, "d lpr / d rho by the tangent pass needs a tensor-core engine and a tree of <= 4 slots");
     const bool tc = tc_prec(e->prec) && !accurate;
-    // the gradient always runs the SIMT adjoint kernel (64-column tiles in FP32)
-    const int TC = grad ? (e->prec == PCSF_PREC_FP64 ? 32 : 64)
+    // the gradient always runs the SIMT adjoint kernel
+    const int TC = grad ? grad_tile_cols()
                         : ff ? ff_tile_cols() : !tc ? simt_tile_cols(e->prec, e->nslots, e->simt_tile)
                                                     : prune_tile_cols(e->prec);
     const int comp = (accurate && tc_prec(e->prec)) ? e->accurate_comp()
@@ -803,8 +805,8 @@ static int evaluate(pcsf_engine *e, pcsf_batch *b, const std::vector<Request> &r
     size_t gscr = 0;
     if (grad) {
         gscr = grad_scratch_per_cta(e->prec, e->nl, npar, e->grad_recompute);
-        CK(e->gscratch.reserve(gscr * (size_t)e->grad_grid), "cudaMalloc gradient scratch");
-        CK(e->dgpart.reserve((size_t)std::max(nwi, 1) * gstride), "cudaMalloc");
+        CK(e->gscratch.reserve(gscr * (size_t)e->grad_grid[npar ? 1 : 0]), "cudaMalloc gradient scratch");
+        CK(e->dgpart.reserve(grad_part_doubles(std::max(nwi, 1), gstride)), "cudaMalloc");
         CK(e->dgrad.reserve((size_t)nreq * gstride), "cudaMalloc");
         CK(e->hgrad.reserve((size_t)nreq * gstride), "cudaMallocHost");
         if (npar)
@@ -896,8 +898,8 @@ static int evaluate(pcsf_engine *e, pcsf_batch *b, const std::vector<Request> &r
             ga.scratch_per_cta = gscr;
             ga.recompute_leaves = e->grad_recompute ? 1 : 0;
             ga.partials = pa.partials;
-            ga.gpart = e->dgpart.p + (size_t)wib[r0] * gstride;
-            int grid = std::min(e->grad_grid, std::max(pa.nwi, 1));
+            ga.gpart = e->dgpart.p + grad_part_doubles(wib[r0], gstride);
+            int grid = std::min(e->grad_grid[npar ? 1 : 0], std::max(pa.nwi, 1));
             const bool tce = tc_prec(e->prec);
             CK(launch_grad(e->prec == PCSF_PREC_FP64 ? PCSF_PREC_FP64 : PCSF_PREC_FP32,
                            tce ? e->accurate_comp() : e->comp_mode(), ga, s, grid), "gradient launch");

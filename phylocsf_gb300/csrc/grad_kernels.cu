@@ -10,17 +10,28 @@
 // s its sibling:
 //   inter_c = beta_p . v_s,   d log z / d t_c = inter_c^T Q v_c / z,   beta_c = P_c^T inter_c.
 //
-// One CTA (256 threads) owns a tile of TC columns.  The inside pass is the one of
-// k_prune but also stores the partial v_c of every internal child and the per-column
-// exponents of the power-of-two rescaling in a per-CTA global scratch area; the
-// outside pass then walks the schedule in reverse.  A leaf child's partial is one
-// gathered row of E^T plus the identity (P_c[a][s]); with RECOMP the outside pass
-// recomputes it from the leaf state instead of storing it (the scratch then holds
-// nl - 1 partials and nl - 1 betas instead of 2 nl - 2 and nl - 1: a third less, the
-// same values, ~5 % more time for the scattered re-reads of E^T rows).  Exponent bookkeeping per column:
+// One CTA (256 threads) owns a tile of 32 columns, two CTAs share an SM.  The inside pass is
+// the one of k_prune (internal children's E^T copied one node ahead, leaf rows from global
+// memory) but also stores the partial v_c of every child and the per-column exponents of the
+// power-of-two rescaling in a per-CTA global scratch area; the outside pass then walks the
+// schedule in reverse.  A leaf child's partial is one gathered row of E^T plus the identity
+// (P_c[a][s]); with RECOMP the outside pass recomputes it from the leaf state instead of
+// storing it (a third less scratch, the same values, a few percent more time for the
+// scattered re-reads of E^T rows).  Exponent bookkeeping per column:
 // alpha_i = alpha~_i 2^{e(i)} with e(i) = e(l) + e(r) + s_i, beta_c = beta~_c 2^{f(c)}
 // with f(c) = f(p) + e(s) + t_c, and the gradient term carries
 // 2^{f(p) + e(s) + e(c) - e(root)} against the scaled z~.
+//
+// What bounds it: the FP32 contractions (two per internal branch, one per leaf branch, and
+// three or four more with the rate parameters), about half of the time.  The rest was the
+// chain around them: 64-column tiles left one CTA per SM, E^T was transposed into shared
+// memory with 32-way bank conflicts, and each side ended in 16 FP64 additions, an ldexp and
+// a division on two of the eight warps (an SM issues two FP64 lanes per clock).  Now E^T is
+// contracted as stored, a column's weight 2^ex / z~ is formed once ahead by one warp, all
+// eight warps share the FP64 sums of a side, and these run beside the next side's
+// contractions; each warp's sum goes to gpart, which k_reduce_grad adds up.  Measured, per
+// column: 58 leaves 173 -> 101 ns, 100 leaves with two rate parameters 955 -> 525 ns.
+#include <algorithm>
 #include <cmath>
 
 #include "pcsf_internal.h"
@@ -29,31 +40,40 @@
 namespace pcsf {
 
 constexpr int GR_THREADS = 256;
+constexpr int GR_WARPS = GR_THREADS / 32;
+constexpr int GR_TC = 32;            // columns per tile
 
-template <typename T, int TC, bool RECOMP>
+template <typename T, bool RECOMP>
 struct GradLayout {
-    __host__ __device__ static size_t base(int nslots, int nl, int nint)
+    static constexpr int TC = GR_TC;
+    // shared memory: Q, [U], then a region that holds the inside pass's slots and E^T (with the
+    // rate parameters E^T sits where Q and U go afterwards: two CTAs per SM on 100 leaves), and in
+    // the outside pass E^T (rows of LDN), [H_x^T and two tiles,] and X
+    __host__ __device__ static size_t region(int nslots, int npar)
     {
-        size_t b = sizeof(T) * (3 * (size_t)K2 + (size_t)nslots * K * TC + (size_t)K * TC + 16 * TC);
-        b += sizeof(typename AtomMax<T>::U) * TC;
-        b += sizeof(double) * TC + sizeof(int) * 2 * TC;
+        const size_t in = (npar ? 0 : 2 * (size_t)K2) + (size_t)nslots * K * TC;
+        const size_t out = (size_t)K * LDN + (size_t)K * TC + (npar ? (size_t)K2 + 2 * (size_t)K * TC : 0);
+        return in > out ? in : out;
+    }
+    // [2][1 + npar][16][TC] column sums; the root's [2][warps][TC] FP64 sums share the space
+    __host__ __device__ static size_t reds(int npar)
+    {
+        const size_t r = 2 * (size_t)(1 + npar) * 16 * TC, z = 2 * GR_WARPS * TC * sizeof(double) / sizeof(T);
+        return r > z ? r : z;
+    }
+    static size_t smem(int nslots, int nl, int nint, int npar)
+    {
+        size_t b = sizeof(T) * ((size_t)K2 + (npar ? (size_t)K2 + 3 * K : 0) + region(nslots, npar) + reds(npar));
+        b += sizeof(double) * 3 * TC;
+        b += sizeof(typename AtomMax<T>::U) * 2 * TC + sizeof(int) * (4 * TC + (size_t)nslots * TC);
         b += sizeof(SchedNode) * nint;
         b = (b + 15) & ~size_t(15);
         b += (size_t)nl * TC;
         return (b + 15) & ~size_t(15);
     }
-    // parameter derivatives need U (appended) and two [K][TC] tiles, kept in the partial
-    // slots (idle during the outside pass) when there are at least two, else appended
-    // too; H_x^T uses Mat[1], which the outside pass does not touch
-    static size_t extra(int nslots, int npar)
-    {
-        if (!npar) return 0;
-        return sizeof(T) * ((size_t)K2 + (nslots >= 2 ? 0 : 2 * (size_t)K * TC));
-    }
-    static size_t smem(int nslots, int nl, int nint, int npar) { return base(nslots, nl, nint) + extra(nslots, npar); }
     // stored child partials: every child's (n - 1), or with RECOMP the internal children's
     __host__ __device__ static size_t nv(int nl) { return RECOMP ? (size_t)(nl - 1) : (size_t)(2 * nl - 2); }
-    static size_t scratch(int nl, int npar)
+    __host__ __device__ static size_t scratch(int nl, int npar)
     {
         const int n = 2 * nl - 1;
         size_t b = sizeof(T) * (nv(nl) + (nl - 1)) * K * TC;        // child partials, betas
@@ -64,34 +84,35 @@ struct GradLayout {
     }
 };
 
-template <typename T, int TC, int KAHAN, bool RECOMP>
-__global__ void __launch_bounds__(GR_THREADS) k_grad(GradArgs a)
+template <typename T, int KAHAN, bool RECOMP>
+__global__ void __launch_bounds__(GR_THREADS, sizeof(T) == 4 ? 2 : 1) k_grad(GradArgs a)
 {
-    typedef GradLayout<T, TC, RECOMP> Layout;
-    constexpr int CPT = TC / 16;
+    typedef GradLayout<T, RECOMP> Layout;
+    constexpr int TC = GR_TC, CPT = TC / 16;
     typedef typename AtomMax<T>::U MU;
     extern __shared__ __align__(16) unsigned char gsm[];
-    T *Mat = reinterpret_cast<T *>(gsm);                          // [3][K][K]
-    T *slots = Mat + 3 * K2;                                       // [nslots][K][TC]
-    T *X = slots + (size_t)a.nslots * K * TC;                      // [K][TC]
-    T *red = X + K * TC;                                           // [16][TC]
-    MU *colmax = reinterpret_cast<MU *>(red + 16 * TC);            // [TC]
-    double *zt = reinterpret_cast<double *>(colmax + TC);          // [TC]
-    int *eroot = reinterpret_cast<int *>(zt + TC);                 // [TC]
-    int *sexp = eroot + TC;                                        // [TC]
-    SchedNode *sched = reinterpret_cast<SchedNode *>(sexp + TC);   // [n_internal]
+    const int npar = a.npar;
+    T *Qs = reinterpret_cast<T *>(gsm);                            // [K][K] Q row-major
+    T *Us = Qs + K2;                                                // [K][K] U row-major (npar)
+    T *isT = Us + (npar ? K2 : 0), *sqT = isT + (npar ? K : 0), *wmT = sqT + (npar ? K : 0);   // [K] each (npar)
+    T *R = wmT + (npar ? K : 0);
+    T *Mat = npar ? Qs : R, *slots = npar ? R : R + 2 * K2;         // inside: [2][K][K], [nslots][K][TC]
+    T *Er = R, *X = R + K * LDN;                                    // outside: [K][LDN], [K][TC]
+    T *Hb = X + K * TC, *Q1 = Hb + K2, *Q2 = Q1 + K * TC;           // [K][K], [K][TC] x 2 (npar)
+    T *red = R + Layout::region(a.nslots, npar);                    // [2][1 + npar][16][TC]
+    double *zp = reinterpret_cast<double *>(red);                   // root: [2][GR_WARPS][TC]
+    double *zt = reinterpret_cast<double *>(red + Layout::reds(npar));   // [TC] 1 / z~ (0: no gradient)
+    double *wcol = zt + TC;                                         // [2][TC] column weights 2^ex / z~
+    MU *colmax = reinterpret_cast<MU *>(wcol + 2 * TC);             // [2][TC]
+    int *eroot = reinterpret_cast<int *>(colmax + 2 * TC);          // [TC]
+    int *ebase = eroot + TC;                                        // [TC] f(p) + e(s)
+    int *wexp = ebase + TC;                                         // [2][TC] the weight's exponent where 2^ex / z~ may not be normal, else 0
+    int *slexp = wexp + 2 * TC;                                        // [nslots][TC] exponents of the slots' partials
+    SchedNode *sched = reinterpret_cast<SchedNode *>(slexp + a.nslots * TC);   // [n_internal]
     size_t off = (reinterpret_cast<unsigned char *>(sched + a.n_internal) - gsm + 15) & ~size_t(15);
-    uint8_t *lvT = gsm + off;                                      // [nl][TC]
-    // parameter derivatives (outside pass only): U and the eigenbasis images of inter and
-    // alpha_c over the slots (continuing past them into the extra space at the end of the
-    // layout when the slots are fewer), H_x^T in Mat[1]
-    T *Ubuf = reinterpret_cast<T *>(gsm + Layout::base(a.nslots, a.nl, a.n_internal));   // [K][K]
-    T *Pt = (a.nslots >= 2) ? slots : Ubuf + K2;                   // [K][TC]
-    T *Qt = Pt + K * TC;                                           // [K][TC]
-    T *Hbuf = Mat + K2;                                            // [K][K]
-    __shared__ double wsum_l[GR_THREADS / 32], wsum_e[GR_THREADS / 32];
+    uint8_t *lvT = gsm + off;                                       // [nl][TC]
 
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int ty = tid / 16, tx = tid % 16;
     const int a0 = 4 * ty, c0 = CPT * tx;
     const int nl = a.nl, n = 2 * nl - 1;
@@ -104,13 +125,11 @@ __global__ void __launch_bounds__(GR_THREADS) k_grad(GradArgs a)
                                               sizeof(int) * 2 * (size_t)n * TC + 255) & ~size_t(255)));   // [nl-1][K][TC]
     // a child's slab among the stored partials (RECOMP: internal children only)
     auto vslot = [&](int c) -> size_t { return RECOMP ? (size_t)(c - nl) : (size_t)c; };
-    const int gstride = a.nbr + a.npar;
+    const int gstride = a.nbr + npar;
     auto e_of = [&](int node, int col) -> int { return node < nl ? 0 : eS[(size_t)node * TC + col]; };
-    // partial of child c at its parent, state st, tile column col: stored, or (RECOMP, a
-    // leaf) recomputed exactly as the inside pass formed it (child_partial: E^T[s][st] +
-    // delta, in one rounding; 1 for a marginalised leaf)
-    auto vpart = [&](const T *Pbase, int c, int st, int col) -> T {
-        if (!RECOMP || c >= nl) return V[(vslot(c) * K + st) * TC + col];
+    // partial of a RECOMP leaf child c, state st, tile column col: exactly as the inside pass
+    // formed it (E^T[s][st] + delta, in one rounding; 1 for a marginalised leaf)
+    auto leaf_part = [&](const T *Pbase, int c, int st, int col) -> T {
         const int sl = lvT[c * TC + col];
         if (sl >= K) return (T)1;
         return fma(Pbase[(size_t)c * K2 + (size_t)sl * K + st], (T)1, sl == st ? (T)1 : (T)0);
@@ -125,49 +144,45 @@ __global__ void __launch_bounds__(GR_THREADS) k_grad(GradArgs a)
         const T *Pbase = reinterpret_cast<const T *>(a.Pbuf) + (size_t)rq.pset * a.nbr * K2;
         const int ncols = wi.ncols;
         const uint8_t *lg = a.leaves + (size_t)wi.col0 * nl;
-        __syncthreads();
+        double *gout = a.gpart + ((size_t)w * GR_WARPS + warp) * gstride;    // this warp's sums
+        auto copy_inner = [&](const SchedNode &nx) {
+            constexpr int NV = K2 * sizeof(T) / 16;
+#pragma unroll
+            for (int side = 0; side < 2; side++) {
+                if ((side ? nx.rslot : nx.lslot) < 0) continue;
+                const char *src = reinterpret_cast<const char *>(Pbase + (size_t)(side ? nx.rc : nx.lc) * K2);
+                const uint32_t dst = (uint32_t)__cvta_generic_to_shared(Mat + side * K2);
+                for (int f = tid; f < NV; f += GR_THREADS)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst + 16 * f), "l"(src + 16 * f)
+                                 : "memory");
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        __syncthreads();   // previous work item finished with shared memory
         for (int f = tid; f < TC * nl; f += GR_THREADS) {
             int c = f / nl, l = f - c * nl;
             lvT[l * TC + c] = (c < ncols) ? lg[f] : (uint8_t)K;
         }
-        for (int f = tid; f < TC; f += GR_THREADS) colmax[f] = 0;
-        {
-            const T *Qg = reinterpret_cast<const T *>(a.Qrow) + (size_t)md * K2;
-            for (int f = tid; f < K2; f += GR_THREADS) Mat[2 * K2 + f] = Qg[f];
-            if (a.npar) {
-                const T *Ug = reinterpret_cast<const T *>(a.Umat) + (size_t)md * K2;
-                for (int f = tid; f < K2; f += GR_THREADS) Ubuf[f] = Ug[f];
-            }
-        }
-        double pacc[2] = {0.0, 0.0};      // this work item's parameter derivatives (thread 0)
+        for (int f = tid; f < 2 * TC; f += GR_THREADS) colmax[f] = 0;
 
         // ---------------- inside pass, storing the child partials
+        copy_inner(sched[0]);
         for (int ni = 0; ni < a.n_internal; ni++) {
             const SchedNode sn = sched[ni];
-            {
-                const float4 *gl = reinterpret_cast<const float4 *>(Pbase + (size_t)sn.lc * K2);
-                const float4 *gr = reinterpret_cast<const float4 *>(Pbase + (size_t)sn.rc * K2);
-                float4 *sl = reinterpret_cast<float4 *>(Mat);
-                float4 *sr = reinterpret_cast<float4 *>(Mat + K2);
-                constexpr int NV = K2 * sizeof(T) / 16;
-                for (int f = tid; f < NV; f += GR_THREADS) {
-                    sl[f] = __ldg(gl + f);
-                    sr[f] = __ldg(gr + f);
-                }
-            }
+            asm volatile("cp.async.wait_all;" ::: "memory");
             __syncthreads();
             T vl[4][CPT], vr[4][CPT];
-            child_partial<T, TC, KAHAN>(Mat, slots, sn.lslot, sn.lc, lvT, a0, c0, vl);
-            child_partial<T, TC, KAHAN>(Mat + K2, slots, sn.rslot, sn.rc, lvT, a0, c0, vr);
-            T mxc[CPT];
+            child_partial<T, TC, KAHAN>(Mat, slots, sn.lslot, sn.lc, lvT, a0, c0, vl, -1, Pbase + (size_t)sn.lc * K2);
+            child_partial<T, TC, KAHAN>(Mat + K2, slots, sn.rslot, sn.rc, lvT, a0, c0, vr, -1, Pbase + (size_t)sn.rc * K2);
 #pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int cc = 0; cc < CPT; cc++) {
-                    if (!RECOMP || sn.lc >= nl) V[(vslot(sn.lc) * K + a0 + i) * TC + c0 + cc] = vl[i][cc];
-                    if (!RECOMP || sn.rc >= nl) V[(vslot(sn.rc) * K + a0 + i) * TC + c0 + cc] = vr[i][cc];
-                }
-            __syncthreads();   // Mat and slots reads done; colmax zeroed
+            for (int i = 0; i < 4; i++) {
+                if (!RECOMP || sn.lc >= nl) ColStore<T, CPT>::store(V + (vslot(sn.lc) * K + a0 + i) * TC + c0, vl[i]);
+                if (!RECOMP || sn.rc >= nl) ColStore<T, CPT>::store(V + (vslot(sn.rc) * K + a0 + i) * TC + c0, vr[i]);
+            }
+            __syncthreads();   // Mat and slot reads done
+            if (ni + 1 < a.n_internal) copy_inner(sched[ni + 1]);
+            MU *cm = colmax + (ni & 1) * TC, *cm_next = colmax + ((ni + 1) & 1) * TC;
+            if (tid < TC) cm_next[tid] = 0;
 #pragma unroll
             for (int cc = 0; cc < CPT; cc++) {
                 T mx = (T)0;
@@ -176,110 +191,221 @@ __global__ void __launch_bounds__(GR_THREADS) k_grad(GradArgs a)
                     vl[i][cc] *= vr[i][cc];
                     mx = vl[i][cc] > mx ? vl[i][cc] : mx;
                 }
-                mxc[cc] = mx;
-                AtomMax<T>::upd(colmax + c0 + cc, mx);
+                AtomMax<T>::upd(cm + c0 + cc, mx);
             }
             __syncthreads();
             T *out = slots + (size_t)sn.oslot * K * TC;
+            int ecol[CPT];
 #pragma unroll
             for (int cc = 0; cc < CPT; cc++) {
-                T mx = AtomMax<T>::get(colmax + c0 + cc);
-                int e = (mx > (T)0) ? exp_of(mx) : 0;
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const T x = scale2(vl[i][cc], -e);
-                    out[(a0 + i) * TC + c0 + cc] = x;
-                    if (a.npar) Ascr[((size_t)(sn.node - nl) * K + a0 + i) * TC + c0 + cc] = x;
-                }
-                if (ty == 0) {
-                    const int col = c0 + cc;
-                    eS[(size_t)sn.node * TC + col] = e_of(sn.lc, col) + e_of(sn.rc, col) + e;
-                }
+                const T mx = AtomMax<T>::get(cm + c0 + cc);
+                ecol[cc] = (mx > (T)0) ? exp_of(mx) : 0;
             }
-            (void)mxc;
-            __syncthreads();   // colmax reads done
-            for (int f = tid; f < TC; f += GR_THREADS) colmax[f] = 0;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                T y[CPT];
+#pragma unroll
+                for (int cc = 0; cc < CPT; cc++) y[cc] = scale2(vl[i][cc], -ecol[cc]);
+                ColStore<T, CPT>::store(out + (a0 + i) * TC + c0, y);
+                if (npar) ColStore<T, CPT>::store(Ascr + ((size_t)(sn.node - nl) * K + a0 + i) * TC + c0, y);
+            }
+            if (ty == 0)
+#pragma unroll
+                for (int cc = 0; cc < CPT; cc++) {
+                    const int col = c0 + cc;
+                    const int e = (sn.lslot < 0 ? 0 : slexp[sn.lslot * TC + col]) +
+                                  (sn.rslot < 0 ? 0 : slexp[sn.rslot * TC + col]) + ecol[cc];
+                    slexp[sn.oslot * TC + col] = e;
+                    eS[(size_t)sn.node * TC + col] = e;
+                }
         }
         __syncthreads();
-        // ---------------- root: z~, lpr and elpr terms
+        // ---------------- root: z~, lpr and elpr terms (eight states per thread, then per column)
         const int root = n - 1;
-        double tl = 0.0, te = 0.0;
-        if (tid < TC) {
+        {
             const T *ar = slots + (size_t)sched[a.n_internal - 1].oslot * K * TC;
-            const double *pr = a.m.prior + md * K;
-            const double *wl = a.m.wlog + md * K;
+            const double *pr = a.m.prior + md * K, *wl = a.m.wlog + md * K;
             double z = 0.0, wz = 0.0;
-            for (int s = 0; s < K; s++) {
-                double x = (double)ar[s * TC + tid];
+            for (int s = 8 * warp; s < 8 * warp + 8; s++) {
+                const double x = (double)ar[s * TC + lane];
                 z += x * pr[s];
                 wz += x * wl[s];
             }
-            zt[tid] = z;
-            eroot[tid] = eS[(size_t)root * TC + tid];
-            if (tid < ncols) {
+            zp[warp * TC + lane] = z;
+            zp[(GR_WARPS + warp) * TC + lane] = wz;
+            // beta~_root = prior, f(root) = 0
+            T *Br = B + (size_t)(root - nl) * K * TC;
+            for (int f = tid; f < K * TC; f += GR_THREADS) Br[f] = (T)pr[f / TC];
+            for (int f = tid; f < TC; f += GR_THREADS) fS[(size_t)root * TC + f] = 0;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            double z = 0.0, wz = 0.0;
+            for (int q = 0; q < GR_WARPS; q++) {
+                z += zp[q * TC + lane];
+                wz += zp[(GR_WARPS + q) * TC + lane];
+            }
+            const int er = slexp[sched[a.n_internal - 1].oslot * TC + lane];
+            zt[lane] = (lane < ncols && z > 0.0) ? 1.0 / z : 0.0;
+            eroot[lane] = er;
+            double tl = 0.0, te = 0.0;
+            if (lane < ncols) {
                 if (z > 0.0) {
-                    tl = log(z) + (double)eroot[tid] * 0.69314718055994530942;
+                    tl = log(z) + (double)er * 0.69314718055994530942;
                     te = wz / z;
                 } else {
                     tl = -INFINITY;
                 }
             }
-        }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            tl += __shfl_down_sync(0xffffffffu, tl, o);
-            te += __shfl_down_sync(0xffffffffu, te, o);
+            for (int o = 16; o > 0; o >>= 1) {
+                tl += __shfl_down_sync(0xffffffffu, tl, o);
+                te += __shfl_down_sync(0xffffffffu, te, o);
+            }
+            if (lane == 0) {
+                a.partials[2 * (size_t)w] = tl;
+                a.partials[2 * (size_t)w + 1] = te;
+            }
         }
-        if ((tid & 31) == 0) { wsum_l[tid >> 5] = tl; wsum_e[tid >> 5] = te; }
-        // beta~_root = prior, f(root) = 0
+        for (int f = tid; f < 2 * TC; f += GR_THREADS) colmax[f] = 0;
         {
-            T *Br = B + (size_t)(root - nl) * K * TC;
-            const double *pr = a.m.prior + md * K;
-            for (int f = tid; f < K * TC; f += GR_THREADS) Br[f] = (T)pr[f / TC];
-            for (int f = tid; f < TC; f += GR_THREADS) fS[(size_t)root * TC + f] = 0;
-        }
-        __syncthreads();
-        if (tid == 0) {
-            double sl = 0.0, se = 0.0;
-            for (int k = 0; k < (TC + 31) / 32; k++) { sl += wsum_l[k]; se += wsum_e[k]; }
-            a.partials[2 * (size_t)w] = sl;
-            a.partials[2 * (size_t)w + 1] = se;
+            const T *Qg = reinterpret_cast<const T *>(a.Qrow) + (size_t)md * K2;
+            for (int f = tid; f < K2; f += GR_THREADS) Qs[f] = Qg[f];
+            if (npar) {
+                const T *Ug = reinterpret_cast<const T *>(a.Umat) + (size_t)md * K2;
+                for (int f = tid; f < K2; f += GR_THREADS) Us[f] = Ug[f];
+                if (tid < K) {
+                    isT[tid] = (T)a.m.isq[md * K + tid];
+                    sqT[tid] = (T)a.m.sq[md * K + tid];
+                }
+                __syncthreads();
+                // U^T D^1/2 1, the eigenbasis image of a marginalised leaf (the same in every column)
+                for (int f = tid; f < K * TC; f += GR_THREADS) X[f] = sqT[f / TC];
+                __syncthreads();
+                T qv[4][CPT];
+                contract<T, TC, KAHAN>(Us, X, a0, c0, qv);
+                if (tx == 0)
+#pragma unroll
+                    for (int i = 0; i < 4; i++) wmT[a0 + i] = qv[i][0];
+            }
         }
 
         // ---------------- outside pass, parents before children
+        // a side's column sums (FP32, 16 per column) are weighted and added over the columns in
+        // FP64 one side later: pc = the branch that waits in buffer pb
+        int pc = -1, pb = 0;
+        double pacc[2] = {0.0, 0.0};      // this warp's parameter derivatives (lane 0)
+        auto flush = [&]() {
+            if (pc < 0) return;
+            const double wv = wcol[pb * TC + lane];
+            const int we = wexp[pb * TC + lane];
+            for (int x = 0; x <= npar; x++) {
+                const T *rd = red + (size_t)(pb * (1 + npar) + x) * 16 * TC + lane;
+                double g = (double)rd[2 * warp * TC] + (double)rd[(2 * warp + 1) * TC];
+                g = (we ? ldexp(g, we) : g) * wv;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) g += __shfl_down_sync(0xffffffffu, g, o);
+                if (lane == 0) {
+                    if (x == 0) gout[pc] = g;
+                    else pacc[x - 1] += g;
+                }
+            }
+            pc = -1;
+        };
+        int sidx = 0;
         for (int ni = a.n_internal - 1; ni >= 0; ni--) {
             const SchedNode sn = sched[ni];
             const int p = sn.node;
             const T *Bp = B + (size_t)(p - nl) * K * TC;
-            for (int side = 0; side < 2; side++) {
+            __syncthreads();   // the betas of the last node are written, X and E^T are free
+            for (int side = 0; side < 2; side++, sidx++) {
                 const int c = side ? sn.rc : sn.lc;
                 const int s = side ? sn.lc : sn.rc;
                 const bool internal = c >= nl;
-                __syncthreads();   // previous side finished with X, Mat[0], red, colmax, wsum
-                if (internal) {
-                    // E_c in row-major order (the buffer holds E_c^T)
-                    const T *g = Pbase + (size_t)c * K2;
-                    for (int f = tid; f < K2; f += GR_THREADS) {
-                        int b = f / K, aa = f % K;
-                        Mat[aa * K + b] = g[f];
+                const int buf = sidx & 1;
+                if (side && npar) __syncthreads();     // the last side is finished with X, E^T and H
+                if (internal) stage_rows<T, GR_THREADS>(Er, Pbase + (size_t)c * K2, tid);
+                const T *Hg = reinterpret_cast<const T *>(a.Hmat) + ((size_t)rq.pset * a.nbr + c) * npar * K2;
+                constexpr int NV = K2 * sizeof(T) / 16;
+                if (npar) {
+                    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(Hb);
+                    for (int f = tid; f < NV; f += GR_THREADS)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst + 16 * f),
+                                     "l"(reinterpret_cast<const char *>(Hg) + 16 * f) : "memory");
+                    asm volatile("cp.async.commit_group;" ::: "memory");
+                }
+                // inter~ = beta~_p . v_s
+                if (!RECOMP || s >= nl) {
+                    const T *Vs = V + vslot(s) * K * TC;
+                    for (int f = 4 * tid; f < K * TC; f += 4 * GR_THREADS) {
+                        T bq[4], vq[4], x[4];
+                        Vec4<T>::load(Bp + f, bq);
+                        Vec4<T>::load(Vs + f, vq);
+#pragma unroll
+                        for (int i = 0; i < 4; i++) x[i] = bq[i] * vq[i];
+                        ColStore<T, 4>::store(X + f, x);
+                        if (npar) {
+#pragma unroll
+                            for (int i = 0; i < 4; i++) x[i] = x[i] * isT[f / TC];
+                            ColStore<T, 4>::store(Q1 + f, x);
+                        }
+                    }
+                } else {
+                    for (int f = tid; f < K * TC; f += GR_THREADS) {
+                        const T x = Bp[f] * leaf_part(Pbase, s, f / TC, f % TC);
+                        X[f] = x;
+                        if (npar) Q1[f] = x * isT[f / TC];
                     }
                 }
-                for (int f = tid; f < TC; f += GR_THREADS) colmax[f] = 0;
-                for (int f = tid; f < K * TC; f += GR_THREADS) X[f] = Bp[f] * vpart(Pbase, s, f / TC, f % TC);
+                if (npar && internal) {
+                    const T *Ac = Ascr + (size_t)(c - nl) * K * TC;
+                    for (int f = 4 * tid; f < K * TC; f += 4 * GR_THREADS) {
+                        T x[4];
+                        Vec4<T>::load(Ac + f, x);
+#pragma unroll
+                        for (int i = 0; i < 4; i++) x[i] = x[i] * sqT[f / TC];
+                        ColStore<T, 4>::store(Q2 + f, x);
+                    }
+                }
+                if (tid < TC) {
+                    const int eb = fS[(size_t)p * TC + tid] + e_of(s, tid);
+                    ebase[tid] = eb;
+                    const int ex = eb + e_of(c, tid) - eroot[tid];
+                    const bool far = ex <= -900 || ex >= 900;
+                    wcol[buf * TC + tid] = far ? zt[tid] : zt[tid] * __hiloint2double((ex + 1023) << 20, 0);
+                    wexp[buf * TC + tid] = far ? ex : 0;
+                }
+                // the child's own partial, for the gradient
+                T vc[4][CPT];
+                if (!RECOMP || internal) {
+#pragma unroll
+                    for (int i = 0; i < 4; i++) ColLoad<T, CPT>::load(V + (vslot(c) * K + a0 + i) * TC + c0, vc[i]);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+#pragma unroll
+                        for (int cc = 0; cc < CPT; cc++) vc[i][cc] = leaf_part(Pbase, c, a0 + i, c0 + cc);
+                }
+                asm volatile("cp.async.wait_all;" ::: "memory");
                 __syncthreads();
                 // gradient: (Q^T inter) . v_c per column, summed over this thread's 4 states
-                T wq[4][CPT];
-                contract<T, TC, KAHAN>(Mat + 2 * K2, X, a0, c0, wq);
+                T *rd = red + (size_t)buf * (1 + npar) * 16 * TC + ty * TC + c0;
+                {
+                    T wq[4][CPT];
+                    contract<T, TC, KAHAN>(Qs, X, a0, c0, wq);
 #pragma unroll
-                for (int cc = 0; cc < CPT; cc++) {
-                    T acc = (T)0;
+                    for (int cc = 0; cc < CPT; cc++) {
+                        T acc = (T)0;
 #pragma unroll
-                    for (int i = 0; i < 4; i++) acc += wq[i][cc] * vpart(Pbase, c, a0 + i, c0 + cc);
-                    red[ty * TC + c0 + cc] = acc;
+                        for (int i = 0; i < 4; i++) acc += wq[i][cc] * vc[i][cc];
+                        rd[cc] = acc;
+                    }
                 }
+                flush();       // the last side's sums
+                MU *cm = colmax + buf * TC, *cm_next = colmax + (buf ^ 1) * TC;
                 T bt[4][CPT];
                 if (internal) {
-                    contract<T, TC, KAHAN>(Mat, X, a0, c0, bt);
+                    contract_rows<T, TC, KAHAN>(Er, X, a0, c0, bt);
 #pragma unroll
                     for (int cc = 0; cc < CPT; cc++) {
                         T mx = (T)0;
@@ -288,140 +414,145 @@ __global__ void __launch_bounds__(GR_THREADS) k_grad(GradArgs a)
                             bt[i][cc] += X[(a0 + i) * TC + c0 + cc];
                             mx = bt[i][cc] > mx ? bt[i][cc] : mx;
                         }
-                        AtomMax<T>::upd(colmax + c0 + cc, mx);
+                        AtomMax<T>::upd(cm + c0 + cc, mx);
                     }
                 }
-                __syncthreads();
-                if (internal) {
-                    T *Bc = B + (size_t)(c - nl) * K * TC;
-#pragma unroll
-                    for (int cc = 0; cc < CPT; cc++) {
-                        const int col = c0 + cc;
-                        T mx = AtomMax<T>::get(colmax + col);
-                        int e = (mx > (T)0) ? exp_of(mx) : 0;
-#pragma unroll
-                        for (int i = 0; i < 4; i++) Bc[(size_t)(a0 + i) * TC + col] = scale2(bt[i][cc], -e);
-                        if (ty == 0) fS[(size_t)c * TC + col] = fS[(size_t)p * TC + col] + e_of(s, col) + e;
-                    }
-                }
-                double gl = 0.0;
-                if (tid < TC && tid < ncols && zt[tid] > 0.0) {
-                    double sum = 0.0;
-                    for (int k = 0; k < 16; k++) sum += (double)red[k * TC + tid];
-                    const int ex = fS[(size_t)p * TC + tid] + e_of(s, tid) + e_of(c, tid) - eroot[tid];
-                    gl = ldexp(sum, ex) / zt[tid];
-                }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) gl += __shfl_down_sync(0xffffffffu, gl, o);
-                if ((tid & 31) == 0) wsum_l[tid >> 5] = gl;
-                __syncthreads();
-                if (tid == 0) {
-                    double g = 0.0;
-                    for (int k = 0; k < (TC + 31) / 32; k++) g += wsum_l[k];
-                    a.gpart[(size_t)w * gstride + c] = g;
-                }
-                if (a.npar) {
-                    // inter^T (dP_c / dx) alpha_c = p^T H_x q with p = U^T D^-1/2 inter, q = U^T D^1/2 alpha_c
-                    const double *sqd = a.m.sq + md * K, *isqd = a.m.isq + md * K;
-                    __syncthreads();   // wsum_l, red read; X still holds inter
-                    for (int f = tid; f < K * TC; f += GR_THREADS) Qt[f] = X[f] * (T)isqd[f / TC];
-                    __syncthreads();
-                    T pv[4][CPT];
-                    contract<T, TC, KAHAN>(Ubuf, Qt, a0, c0, pv);
-                    __syncthreads();
+                // parameters: inter^T (dP_c / dx) alpha_c = p^T H_x q with p = U^T D^-1/2 inter and
+                // q = U^T D^1/2 alpha_c, for a leaf one row of U (its alpha_c is one-hot)
+                T pv[4][CPT], qv[4][CPT];
+                if (npar) {
+                    contract<T, TC, KAHAN>(Us, Q1, a0, c0, pv);
                     if (internal) {
-                        const T *Ac = Ascr + (size_t)(c - nl) * K * TC;
-                        for (int f = tid; f < K * TC; f += GR_THREADS) Qt[f] = Ac[f] * (T)sqd[f / TC];
+                        contract<T, TC, KAHAN>(Us, Q2, a0, c0, qv);
                     } else {
-                        for (int f = tid; f < K * TC; f += GR_THREADS) {
-                            const int st = f / TC, col = f % TC;
-                            const int sl = lvT[c * TC + col];
-                            Qt[f] = (sl >= K) ? (T)sqd[st] : (sl == st ? (T)sqd[st] : (T)0);
+#pragma unroll
+                        for (int cc = 0; cc < CPT; cc++) {
+                            const int sl = lvT[c * TC + c0 + cc];
+                            T u[4];
+                            Vec4<T>::load(sl < K ? Us + sl * K + a0 : wmT + a0, u);
+#pragma unroll
+                            for (int i = 0; i < 4; i++) qv[i][cc] = sl < K ? u[i] * sqT[sl] : u[i];
                         }
                     }
-                    __syncthreads();
-                    {
-                        T qv[4][CPT];
-                        contract<T, TC, KAHAN>(Ubuf, Qt, a0, c0, qv);
+                }
+                __syncthreads();
+                if (tid < TC) cm_next[tid] = 0;
+                if (internal) {
+                    T *Bc = B + (size_t)(c - nl) * K * TC;
+                    int ecol[CPT];
 #pragma unroll
-                        for (int i = 0; i < 4; i++)
-#pragma unroll
-                            for (int cc = 0; cc < CPT; cc++) Pt[(a0 + i) * TC + c0 + cc] = qv[i][cc];
+                    for (int cc = 0; cc < CPT; cc++) {
+                        const T mx = AtomMax<T>::get(cm + c0 + cc);
+                        ecol[cc] = (mx > (T)0) ? exp_of(mx) : 0;
+                        if (ty == 0) fS[(size_t)c * TC + c0 + cc] = ebase[c0 + cc] + ecol[cc];
                     }
-                    for (int x = 0; x < a.npar; x++) {
-                        const T *Hg = reinterpret_cast<const T *>(a.Hmat) +
-                                      (((size_t)rq.pset * a.nbr + c) * a.npar + x) * K2;
-                        for (int f = tid; f < K2; f += GR_THREADS) Hbuf[f] = Hg[f];
-                        __syncthreads();   // Hbuf and the q tile (Pt) ready
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        T y[CPT];
+#pragma unroll
+                        for (int cc = 0; cc < CPT; cc++) y[cc] = scale2(bt[i][cc], -ecol[cc]);
+                        ColStore<T, CPT>::store(Bc + (size_t)(a0 + i) * TC + c0, y);
+                    }
+                }
+                if (npar) {
+                    // H_1 takes the place of E^T while H_0 is used; q takes that of D^-1/2 inter
+                    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(Er);
+                    for (int f = tid; f < NV; f += GR_THREADS)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst + 16 * f),
+                                     "l"(reinterpret_cast<const char *>(Hg + K2) + 16 * f) : "memory");
+                    asm volatile("cp.async.commit_group;" ::: "memory");
+#pragma unroll
+                    for (int i = 0; i < 4; i++) ColStore<T, CPT>::store(Q1 + (a0 + i) * TC + c0, qv[i]);
+                    for (int x = 0; x < 2; x++) {
+                        if (x) asm volatile("cp.async.wait_all;" ::: "memory");
+                        __syncthreads();
                         T rv[4][CPT];
-                        contract<T, TC, KAHAN>(Hbuf, Pt, a0, c0, rv);
+                        contract<T, TC, KAHAN>(x ? Er : Hb, Q1, a0, c0, rv);
 #pragma unroll
                         for (int cc = 0; cc < CPT; cc++) {
                             T acc = (T)0;
 #pragma unroll
                             for (int i = 0; i < 4; i++) acc += pv[i][cc] * rv[i][cc];
-                            red[ty * TC + c0 + cc] = acc;
+                            rd[(size_t)(1 + x) * 16 * TC + cc] = acc;
                         }
-                        __syncthreads();
-                        double gx = 0.0;
-                        if (tid < TC && tid < ncols && zt[tid] > 0.0) {
-                            double sum = 0.0;
-                            for (int k = 0; k < 16; k++) sum += (double)red[k * TC + tid];
-                            const int ex = fS[(size_t)p * TC + tid] + e_of(s, tid) + e_of(c, tid) - eroot[tid];
-                            gx = ldexp(sum, ex) / zt[tid];
-                        }
-#pragma unroll
-                        for (int o = 16; o > 0; o >>= 1) gx += __shfl_down_sync(0xffffffffu, gx, o);
-                        if ((tid & 31) == 0) wsum_l[tid >> 5] = gx;
-                        __syncthreads();
-                        if (tid == 0)
-                            for (int k = 0; k < (TC + 31) / 32; k++) pacc[x] += wsum_l[k];
-                        __syncthreads();   // Hbuf, red, wsum_l free
                     }
                 }
+                pc = c;
+                pb = buf;
             }
         }
-        if (a.npar && tid == 0)
-            for (int x = 0; x < a.npar; x++) a.gpart[(size_t)w * gstride + a.nbr + x] = pacc[x];
+        __syncthreads();
+        flush();
+        if (npar && lane == 0)
+            for (int x = 0; x < npar; x++) gout[a.nbr + x] = pacc[x];
     }
+}
+
+// The most shared memory a tree may ask for: three matrices, the slots and a tile of 64 (FP64: 32)
+// columns, with the rate parameters U and two tiles more.  The kernel's own layout is smaller; the
+// limit on trees is part of the interface.
+size_t grad_smem_bytes(int prec, int nslots, int nl, int nint, int npar)
+{
+    const size_t es = prec == PCSF_PREC_FP64 ? 8 : 4, tc = prec == PCSF_PREC_FP64 ? 32 : 64;
+    size_t b = es * (3 * (size_t)K2 + (size_t)nslots * K * tc + (size_t)K * tc + 16 * tc) + es * tc + 16 * tc +
+               sizeof(SchedNode) * nint;
+    b = (b + 15) & ~size_t(15);
+    b = (b + (size_t)nl * tc + 15) & ~size_t(15);
+    return b + (npar ? es * ((size_t)K2 + (nslots >= 2 ? 0 : 2 * (size_t)K * tc)) : 0);
+}
+
+int grad_tile_cols() { return GR_TC; }
+size_t grad_part_doubles(int nwi, int gstride) { return (size_t)nwi * GR_WARPS * gstride; }
+
+template <typename T, int KAHAN, bool RECOMP>
+static int ctas_per_sm_r(int nslots, int nl, int nint, int npar)
+{
+    const size_t smem = GradLayout<T, RECOMP>::smem(nslots, nl, nint, npar);
+    int n = 0;
+    if (cudaFuncSetAttribute(k_grad<T, KAHAN, RECOMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_grad<T, KAHAN, RECOMP>, GR_THREADS, smem) != cudaSuccess) {
+        cudaGetLastError();
+        return 1;
+    }
+    return std::max(n, 1);
+}
+
+int grad_ctas_per_sm(int prec, int nslots, int nl, int nint, int npar)
+{
+    if (prec == PCSF_PREC_FP64) return ctas_per_sm_r<double, 0, false>(nslots, nl, nint, npar);
+    return ctas_per_sm_r<float, 2, false>(nslots, nl, nint, npar);
 }
 
 size_t grad_scratch_per_cta(int prec, int nl, int npar, bool recompute_leaves)
 {
     if (prec == PCSF_PREC_FP64)
-        return recompute_leaves ? GradLayout<double, 32, true>::scratch(nl, npar) : GradLayout<double, 32, false>::scratch(nl, npar);
-    return recompute_leaves ? GradLayout<float, 64, true>::scratch(nl, npar) : GradLayout<float, 64, false>::scratch(nl, npar);
+        return recompute_leaves ? GradLayout<double, true>::scratch(nl, npar) : GradLayout<double, false>::scratch(nl, npar);
+    return recompute_leaves ? GradLayout<float, true>::scratch(nl, npar) : GradLayout<float, false>::scratch(nl, npar);
 }
 
-size_t grad_smem_bytes(int prec, int nslots, int nl, int nint, int npar)
-{
-    if (prec == PCSF_PREC_FP64) return GradLayout<double, 32, false>::smem(nslots, nl, nint, npar);
-    return GradLayout<float, 64, false>::smem(nslots, nl, nint, npar);
-}
-
-template <typename T, int TC, int KAHAN, bool RECOMP>
+template <typename T, int KAHAN, bool RECOMP>
 static cudaError_t launch_grad_r(const GradArgs &a, cudaStream_t s, int grid)
 {
-    size_t smem = GradLayout<T, TC, RECOMP>::smem(a.nslots, a.nl, a.n_internal, a.npar);
-    cudaError_t e = cudaFuncSetAttribute(k_grad<T, TC, KAHAN, RECOMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    size_t smem = GradLayout<T, RECOMP>::smem(a.nslots, a.nl, a.n_internal, a.npar);
+    cudaError_t e = cudaFuncSetAttribute(k_grad<T, KAHAN, RECOMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_grad<T, TC, KAHAN, RECOMP><<<grid, GR_THREADS, smem, s>>>(a);
+    k_grad<T, KAHAN, RECOMP><<<grid, GR_THREADS, smem, s>>>(a);
     return cudaGetLastError();
 }
 
-template <typename T, int TC, int KAHAN>
+template <typename T, int KAHAN>
 static cudaError_t launch_grad_t(const GradArgs &a, cudaStream_t s, int grid)
 {
-    return a.recompute_leaves ? launch_grad_r<T, TC, KAHAN, true>(a, s, grid) : launch_grad_r<T, TC, KAHAN, false>(a, s, grid);
+    return a.recompute_leaves ? launch_grad_r<T, KAHAN, true>(a, s, grid) : launch_grad_r<T, KAHAN, false>(a, s, grid);
 }
 
 cudaError_t launch_grad(int prec, int comp, const GradArgs &a, cudaStream_t s, int grid)
 {
     if (a.nwi <= 0) return cudaSuccess;
-    if (prec == PCSF_PREC_FP64) return launch_grad_t<double, 32, 0>(a, s, grid);
-    if (comp == 1) return launch_grad_t<float, 64, 1>(a, s, grid);
-    if (comp == 2) return launch_grad_t<float, 64, 2>(a, s, grid);
-    return launch_grad_t<float, 64, 0>(a, s, grid);
+    if (prec == PCSF_PREC_FP64) return launch_grad_t<double, 0>(a, s, grid);
+    if (comp == 1) return launch_grad_t<float, 1>(a, s, grid);
+    if (comp == 2) return launch_grad_t<float, 2>(a, s, grid);
+    return launch_grad_t<float, 0>(a, s, grid);
 }
 
 // H_x^T = (F(t) o Bdot_x)^T per (P set, branch, parameter).  F_ij = (e^{lam_i t} -
@@ -460,14 +591,14 @@ cudaError_t launch_hform(bool fp64, const PSet *ps, int nps, const double *branc
     return cudaGetLastError();
 }
 
-// grad[r][c] = sum of gpart over request r's work items (fixed order)
+// grad[r][c] = sum of gpart ([work item][warp][branch]) over request r's work items (fixed order)
 __global__ void k_reduce_grad(const double *gpart, const int32_t *wi_begin, int nreq, int nbr, double *grad)
 {
     int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= nreq * nbr) return;
     int r = idx / nbr, c = idx % nbr;
     double g = 0.0;
-    for (int w = wi_begin[r]; w < wi_begin[r + 1]; w++) g += gpart[(size_t)w * nbr + c];
+    for (size_t w = (size_t)wi_begin[r] * GR_WARPS; w < (size_t)wi_begin[r + 1] * GR_WARPS; w++) g += gpart[w * nbr + c];
     grad[idx] = g;
 }
 

@@ -118,3 +118,25 @@ def test_recomputed_leaf_partials_identical(name, prec):
     for x, y in zip(ref, got):
         for u, v in zip(x, y):
             assert u.tobytes() == v.tobytes()
+
+
+@pytest.mark.parametrize("name,prec", [("12flies", "fp32b"), ("12flies", "fp64"), ("58mammals", "fp32c")])
+@pytest.mark.parametrize("lengths", [[1], [31, 32, 33], [0, 65, 7]])
+def test_gradient_tiles(name, prec, lengths):
+    """Regions at the edges of the adjoint's 32-column tiles: the gradient of a region is the sum of
+    its columns' gradients taken one by one (FP64 sums of at most 65 terms that carry the same FP32
+    values: 1e-12 of the largest entry)."""
+    ps = synth.load_params(name)
+    rng = np.random.default_rng(4)
+    gf = synth.gap_fractions(rng, len(lengths), ps.tree.nl, 0.05, 0.4, 0.2)
+    offs, leaves = synth.simulate(ps, np.array(lengths), np.zeros(len(lengths), np.int32), gf, 4)
+    e = P.Engine(ps.tree, ps.S_c, ps.pi_c, ps.S_n, ps.pi_n, precision=prec)
+    _, db, dr, st = e.grad(e.batch(offs, leaves), 0, 0.8)
+    n = int(offs[-1])
+    _, db1, dr1, st1 = e.grad(e.batch(np.arange(n + 1), leaves), 0, 0.8)
+    assert (st == 0).all() and (st1 == 0).all()
+    for r in range(len(lengths)):
+        s = slice(int(offs[r]), int(offs[r + 1]))
+        scale = np.abs(db1).max() * max(lengths)
+        assert np.abs(db[r] - db1[s].sum(0)).max() <= 1e-12 * scale
+        assert abs(dr[r] - dr1[s].sum()) <= 1e-12 * scale * ps.tree.branch[:ps.tree.n - 1].sum()
