@@ -563,6 +563,22 @@ static int simt_grid(const pcsf_engine *e, int tile)
     return e->sm_count * std::min(per_sm, 8);
 }
 
+// Column tile of a SIMT pruning launch over these requests: small tiles while all of them are
+// resident at once (four per SM), the engine's tile beyond.  A launch of a few hundred columns is
+// as long as one CTA's walk down the tree, which takes a third to a half of the time with a
+// column per thread.  Measured with 64 (FP64: 32) against 8 columns: 58 leaves FP32 300 columns
+// 254 / 129 us, 4,800 columns 258 / 159, 9,600 columns 261 / 354; 12 leaves FP32 300 columns 66 /
+// 39; 12 leaves FP64 1,200 columns 404 / 135, 4,800 columns 404 / 301, 9,600 columns 783 / 799.
+static int launch_tile(const pcsf_engine *e, const pcsf_batch *b, const std::vector<Request> &reqs)
+{
+    int64_t tiles = 0;
+    for (const Request &q : reqs) {
+        tiles += (b->offs[q.region + 1] - b->offs[q.region] + PRUNE_SMALL_TILE - 1) / PRUNE_SMALL_TILE;
+        if (tiles > 4 * (int64_t)e->sm_count) return simt_tile_cols(e->prec, e->nslots, e->simt_tile);
+    }
+    return PRUNE_SMALL_TILE;
+}
+
 static int engine_init_common(pcsf_engine *e, const pcsf_tree *tree, int32_t flags)
 {
     int prec = flags & 0xff;
@@ -699,8 +715,8 @@ static int evaluate(pcsf_engine *e, pcsf_batch *b, const std::vector<Request> &r
     const bool tc = tc_prec(e->prec) && !accurate;
     // the gradient always runs the SIMT adjoint kernel
     const int TC = grad ? grad_tile_cols()
-                        : ff ? ff_tile_cols() : !tc ? simt_tile_cols(e->prec, e->nslots, e->simt_tile)
-                                                    : prune_tile_cols(e->prec);
+                        : ff ? ff_tile_cols() : !tc ? launch_tile(e, b, reqs_in) : prune_tile_cols(e->prec);
+    const bool cols = !grad && !ff && !tc && TC == PRUNE_SMALL_TILE;    // small tiles: per-column terms, summed in the long launch's order
     const int comp = (accurate && tc_prec(e->prec)) ? e->accurate_comp()
                                                                                               : e->comp_mode();
 
@@ -779,7 +795,7 @@ static int evaluate(pcsf_engine *e, pcsf_batch *b, const std::vector<Request> &r
     CK(e->dwi.reserve(nwi), "cudaMalloc");
     CK(e->dwib.reserve(nreq + 1), "cudaMalloc");
     CK(e->dstatus.reserve(nps), "cudaMalloc");
-    CK(e->dpart.reserve(2 * (size_t)std::max(nwi, 1)), "cudaMalloc");
+    CK(e->dpart.reserve(2 * (size_t)std::max(nwi, 1) * (cols ? TC : 1)), "cudaMalloc");
     CK(e->dlpr.reserve(nreq), "cudaMalloc");
     CK(e->delpr.reserve(nreq), "cudaMalloc");
     if (drho) {
@@ -871,7 +887,8 @@ static int evaluate(pcsf_engine *e, pcsf_batch *b, const std::vector<Request> &r
         pa.nbop = nbop;
         pa.dither = e->prec != PCSF_PREC_FP64;
         pa.dlo = dlo;
-        pa.tile = e->simt_tile;
+        pa.tile = (!grad && !ff && !tc) ? TC : 0;
+        pa.colv = cols ? e->dpart.p + 2 * (size_t)wib[r0] * TC : nullptr;
         pa.tc_shape = e->tc_shape;
         pa.ff_depth = e->ff_depth;
         if (grad) {
@@ -917,7 +934,7 @@ static int evaluate(pcsf_engine *e, pcsf_batch *b, const std::vector<Request> &r
             else
                 CK(launch_prune_tc(e->prec == PCSF_PREC_TF32X3 ? 3 : 1, pa, e->derr.p, s, grid), "tensor-core pruning launch");
         } else {
-            int grid = std::min(e->prune_grid, std::max(pa.nwi, 1));
+            int grid = std::min(cols ? simt_grid(e, TC) : e->prune_grid, std::max(pa.nwi, 1));
             CK(launch_prune(e->prec == PCSF_PREC_FP64 ? PCSF_PREC_FP64 : PCSF_PREC_FP32, comp, pa, s, grid),
                "pruning launch");
         }
@@ -934,7 +951,11 @@ static int evaluate(pcsf_engine *e, pcsf_batch *b, const std::vector<Request> &r
         pr_ms += t2;
     }
     CK(cudaEventRecord(e->ev[3], s), "event");
-    CK(launch_reduce(e->dpart.p, e->dwib.p, nreq, e->dlpr.p, e->delpr.p, s), "reduce launch");
+    if (cols)
+        CK(launch_reduce_cols(e->dpart.p, e->dwi.p, e->dwib.p, nreq, TC, simt_tile_cols(e->prec, e->nslots, e->simt_tile),
+                              e->dlpr.p, e->delpr.p, s), "reduce launch");
+    else
+        CK(launch_reduce(e->dpart.p, e->dwib.p, nreq, e->dlpr.p, e->delpr.p, s), "reduce launch");
     e->stats.kernel_launches += 1;
     std::vector<double> hdrho;
     if (drho) {

@@ -536,9 +536,11 @@ cudaError_t launch_d2f_rows(const double *in, float *out, size_t nmat, int nbr, 
 
 constexpr int PR_THREADS = 256;
 
+// threads of a tile: 16 groups of 4 states; 4 or 2 columns per thread, or 1 in half a block (8 columns)
+template <int TC> struct PruneThreads { static constexpr int N = TC >= 16 ? PR_THREADS : 16 * TC; };
+
 template <typename T, int TC>
 struct PruneSmem {
-    static constexpr int CPT = TC / 16;
     static size_t bytes(int nslots, int nl, int nint)
     {
         size_t b = sizeof(T) * (2 * K2 + (size_t)nslots * K * TC);
@@ -552,9 +554,9 @@ struct PruneSmem {
 };
 
 template <typename T, int TC, int KAHAN>
-__global__ void __launch_bounds__(PR_THREADS) k_prune(PruneArgs a)
+__global__ void __launch_bounds__(PruneThreads<TC>::N) k_prune(PruneArgs a)
 {
-    constexpr int CPT = TC / 16;
+    constexpr int THREADS = PruneThreads<TC>::N, TXN = THREADS / 16, CPT = TC / TXN;
     typedef typename AtomMax<T>::U MU;
     extern __shared__ __align__(16) unsigned char ssm[];
     T *Et = reinterpret_cast<T *>(ssm);                 // [2][K][K]
@@ -566,17 +568,17 @@ __global__ void __launch_bounds__(PR_THREADS) k_prune(PruneArgs a)
     uint8_t *lvT = ssm + off;                                                  // [nl][TC]
 
     const int tid = threadIdx.x;
-    const int ty = tid / 16, tx = tid % 16;
+    const int ty = tid / TXN, tx = tid % TXN;
     const int a0 = 4 * ty, c0 = CPT * tx;
     const int nl = a.nl;
-    __shared__ double red_l[PR_THREADS / 32], red_e[PR_THREADS / 32];
+    __shared__ double red_l[THREADS / 32], red_e[THREADS / 32];
     __shared__ double ltab[256];           // log(1 + k/256), the dither factors' logs
     __shared__ double dsum[TC];            // per column: sum over leaves of log c
     const bool dith = a.dither && sizeof(T) == 4;
 
-    for (int f = tid; f < a.n_internal; f += PR_THREADS) sched[f] = a.sched[f];
+    for (int f = tid; f < a.n_internal; f += THREADS) sched[f] = a.sched[f];
     if (dith)
-        for (int f = tid; f < 256; f += PR_THREADS) ltab[f] = log1p((double)f / 256.0);
+        for (int f = tid; f < 256; f += THREADS) ltab[f] = log1p((double)f / 256.0);
 
     for (int w = blockIdx.x; w < a.nwi; w += gridDim.x) {
         const WorkItem wi = a.wi[w];
@@ -597,25 +599,25 @@ __global__ void __launch_bounds__(PR_THREADS) k_prune(PruneArgs a)
                 if ((side ? nx.rslot : nx.lslot) < 0) continue;
                 const char *src = reinterpret_cast<const char *>(Pbase + (size_t)(side ? nx.rc : nx.lc) * K2);
                 const uint32_t dst = (uint32_t)__cvta_generic_to_shared(Et + side * K2);
-                for (int f = tid; f < NV; f += PR_THREADS)
+                for (int f = tid; f < NV; f += THREADS)
                     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst + 16 * f), "l"(src + 16 * f)
                                  : "memory");
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
         __syncthreads();   // previous work item finished with shared memory
-        for (int f = tid; f < TC * nl; f += PR_THREADS) {
+        for (int f = tid; f < TC * nl; f += THREADS) {
             int c = f / nl, l = f - c * nl;
             lvT[l * TC + c] = (c < ncols) ? lg[f] : (uint8_t)K;
         }
-        for (int f = tid; f < 2 * TC; f += PR_THREADS) colmax[f] = 0;
-        for (int f = tid; f < TC; f += PR_THREADS) cscale[f] = 0;
+        for (int f = tid; f < 2 * TC; f += THREADS) colmax[f] = 0;
+        for (int f = tid; f < TC; f += THREADS) cscale[f] = 0;
         // dither keys are the column's position within its region, so that results
         // do not depend on where a region sits in the batch
         const int64_t dcol0 = dith ? (int64_t)(uint32_t)((uint32_t)wi.col0 - rq.start) : -1;
         if (dith) {
             __syncthreads();   // ltab ready
-            for (int c = tid; c < TC; c += PR_THREADS) {
+            for (int c = tid; c < TC; c += THREADS) {
                 double sd = 0.0;
                 for (int l = 0; l < nl; l++) sd += ltab[dither_k(dcol0 + c, l)];
                 dsum[c] = sd;
@@ -628,9 +630,9 @@ __global__ void __launch_bounds__(PR_THREADS) k_prune(PruneArgs a)
             asm volatile("cp.async.wait_all;" ::: "memory");
             __syncthreads();
             T vl[4][CPT], vr[4][CPT];
-            child_partial<T, TC, KAHAN>(Et, slots, sn.lslot, sn.lc, lvT, a0, c0, vl, dcol0, Pbase + (size_t)sn.lc * K2,
+            child_partial<T, TC, KAHAN, CPT>(Et, slots, sn.lslot, sn.lc, lvT, a0, c0, vl, dcol0, Pbase + (size_t)sn.lc * K2,
                                         dlo ? dlo + (size_t)sn.lc * K : nullptr);
-            child_partial<T, TC, KAHAN>(Et + K2, slots, sn.rslot, sn.rc, lvT, a0, c0, vr, dcol0,
+            child_partial<T, TC, KAHAN, CPT>(Et + K2, slots, sn.rslot, sn.rc, lvT, a0, c0, vr, dcol0,
                                         Pbase + (size_t)sn.rc * K2, dlo ? dlo + (size_t)sn.rc * K : nullptr);
             __syncthreads();
             if (ni + 1 < a.n_internal) copy_inner(sched[ni + 1]);   // E^T buffers are free again
@@ -687,6 +689,10 @@ __global__ void __launch_bounds__(PR_THREADS) k_prune(PruneArgs a)
                 te = 0.0;
             }
         }
+        if (a.colv) {      // small tiles: the columns' terms, summed by k_reduce_cols
+            if (tid < TC) reinterpret_cast<double2 *>(a.colv)[(size_t)w * TC + tid] = make_double2(tl, te);
+            continue;
+        }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             tl += __shfl_down_sync(0xffffffffu, tl, o);
@@ -709,8 +715,8 @@ int prune_tile_cols(int prec)
     return prec == PCSF_PREC_FP64 ? 32 : 64;
 }
 
-// Column tile of the SIMT pruning kernel.  FP32 uses 64 columns, except for trees of
-// five or more partial slots (the 120-leaf tree): there 64 columns take ~124 KB of
+// Column tile of the SIMT pruning kernel in a long launch.  FP32 uses 64 columns, except for
+// trees of five or more partial slots (the 120-leaf tree): there 64 columns take ~124 KB of
 // shared memory, one CTA per SM, and 32 columns let two CTAs share an SM.
 // tile (32 or 64) overrides this rule for the FP32 kernel (the engine's autotuner sets it).
 int simt_tile_cols(int prec, int nslots, int tile)
@@ -720,11 +726,18 @@ int simt_tile_cols(int prec, int nslots, int tile)
     return nslots >= 5 ? 32 : 64;
 }
 
+template <typename T>
+static size_t prune_smem_t(int tc, int nslots, int nl, int nint)
+{
+    if (tc == PRUNE_SMALL_TILE) return PruneSmem<T, PRUNE_SMALL_TILE>::bytes(nslots, nl, nint);
+    if (tc == 32) return PruneSmem<T, 32>::bytes(nslots, nl, nint);
+    return PruneSmem<T, 64>::bytes(nslots, nl, nint);
+}
+
 size_t prune_smem_bytes(int prec, int nslots, int nl, int nint, int tile)
 {
-    if (prec == PCSF_PREC_FP64) return PruneSmem<double, 32>::bytes(nslots, nl, nint);
-    if (simt_tile_cols(prec, nslots, tile) == 32) return PruneSmem<float, 32>::bytes(nslots, nl, nint);
-    return PruneSmem<float, 64>::bytes(nslots, nl, nint);
+    const int tc = tile == PRUNE_SMALL_TILE ? tile : simt_tile_cols(prec, nslots, tile);
+    return prec == PCSF_PREC_FP64 ? prune_smem_t<double>(tc, nslots, nl, nint) : prune_smem_t<float>(tc, nslots, nl, nint);
 }
 
 template <typename T, int TC, int KAHAN>
@@ -733,22 +746,28 @@ static cudaError_t launch_prune_t(const PruneArgs &a, cudaStream_t s, int grid)
     size_t smem = PruneSmem<T, TC>::bytes(a.nslots, a.nl, a.n_internal);
     cudaError_t e = cudaFuncSetAttribute(k_prune<T, TC, KAHAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_prune<T, TC, KAHAN><<<grid, PR_THREADS, smem, s>>>(a);
+    k_prune<T, TC, KAHAN><<<grid, PruneThreads<TC>::N, smem, s>>>(a);
     return cudaGetLastError();
+}
+
+template <int TC>
+static cudaError_t launch_prune_f(int comp, const PruneArgs &a, cudaStream_t s, int grid)
+{
+    if (comp == 1) return launch_prune_t<float, TC, 1>(a, s, grid);
+    if (comp == 2) return launch_prune_t<float, TC, 2>(a, s, grid);
+    return launch_prune_t<float, TC, 0>(a, s, grid);
 }
 
 cudaError_t launch_prune(int prec, int comp, const PruneArgs &a, cudaStream_t s, int grid)
 {
     if (a.nwi <= 0) return cudaSuccess;
-    if (prec == PCSF_PREC_FP64) return launch_prune_t<double, 32, 0>(a, s, grid);
-    if (simt_tile_cols(prec, a.nslots, a.tile) == 32) {
-        if (comp == 1) return launch_prune_t<float, 32, 1>(a, s, grid);
-        if (comp == 2) return launch_prune_t<float, 32, 2>(a, s, grid);
-        return launch_prune_t<float, 32, 0>(a, s, grid);
+    if (prec == PCSF_PREC_FP64) {
+        if (a.tile == PRUNE_SMALL_TILE) return launch_prune_t<double, PRUNE_SMALL_TILE, 0>(a, s, grid);
+        return launch_prune_t<double, 32, 0>(a, s, grid);
     }
-    if (comp == 1) return launch_prune_t<float, 64, 1>(a, s, grid);
-    if (comp == 2) return launch_prune_t<float, 64, 2>(a, s, grid);
-    return launch_prune_t<float, 64, 0>(a, s, grid);
+    if (a.tile == PRUNE_SMALL_TILE) return launch_prune_f<PRUNE_SMALL_TILE>(comp, a, s, grid);
+    if (simt_tile_cols(prec, a.nslots, a.tile) == 32) return launch_prune_f<32>(comp, a, s, grid);
+    return launch_prune_f<64>(comp, a, s, grid);
 }
 
 // ---------------------------------------------------------------------------
@@ -767,6 +786,49 @@ __global__ void k_reduce(const double *partials, const int32_t *wi_begin, int nr
     const int o = out_index ? out_index[r] : r;
     out_lpr[o] = sl;
     out_elpr[o] = se;
+}
+
+// The same sums from the columns' terms of a launch of small tiles (tc columns, ragged last tile
+// per request): per group of `group` columns (the tile of a long launch) a tree over each 32, the
+// groups in order -- bit for bit what k_prune and k_reduce form with tiles of that size.  One
+// warp per request.
+__global__ void __launch_bounds__(128) k_reduce_cols(const double2 *colv, const WorkItem *wi, const int32_t *wi_begin,
+                                                     int nreq, int tc, int group, double *out_lpr, double *out_elpr)
+{
+    const int r = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (r >= nreq) return;
+    const int w0 = wi_begin[r], w1 = wi_begin[r + 1];
+    const int64_t ncols = w1 > w0 ? (int64_t)(w1 - 1 - w0) * tc + wi[w1 - 1].ncols : 0;
+    const double2 *src = colv + (size_t)w0 * tc;
+    double sl = 0.0, se = 0.0;
+    for (int64_t g = 0; g < ncols; g += group) {
+        double gl = 0.0, ge = 0.0;
+        for (int64_t c = g; c < g + group; c += 32) {
+            double2 t = c + lane < ncols ? src[c + lane] : make_double2(0.0, 0.0);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                t.x += __shfl_down_sync(0xffffffffu, t.x, o);
+                t.y += __shfl_down_sync(0xffffffffu, t.y, o);
+            }
+            gl += t.x;
+            ge += t.y;
+        }
+        sl += gl;
+        se += ge;
+    }
+    if (lane == 0) {
+        out_lpr[r] = sl;
+        out_elpr[r] = se;
+    }
+}
+
+cudaError_t launch_reduce_cols(const double *colv, const WorkItem *wi, const int32_t *wi_begin, int nreq, int tc, int group,
+                               double *out_lpr, double *out_elpr, cudaStream_t s)
+{
+    if (nreq <= 0) return cudaSuccess;
+    k_reduce_cols<<<(nreq + 3) / 4, 128, 0, s>>>(reinterpret_cast<const double2 *>(colv), wi, wi_begin, nreq, tc, group,
+                                                 out_lpr, out_elpr);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_reduce(const double *partials, const int32_t *wi_begin, int nreq, double *out_lpr,

@@ -115,12 +115,14 @@ struct PruneArgs {
     int nbop;                //   of the branches above internal nodes (node nl + k)
     int dither;              // SIMT FP32 kernel: per-column dithering of the leaf partials (prune_common.cuh)
     const float *dlo;        // SIMT FP32 kernel, may be null: per chunk-local P set [nbr][K] low parts of diag(E)
-    int tile;                // SIMT FP32 kernel: column tile 32 or 64, 0 = the default rule (simt_tile_cols)
+    int tile;                // SIMT kernel: column tile PRUNE_SMALL_TILE (short launches), 32 or 64 (FP32), 0 = the default rule
+    double *colv;            // SIMT kernel, small tiles: [nwi][tile][2] the columns' terms instead of partials
     int ff_depth;            // float-float kernel: partials that wait at once (its stack's entries)
     int tc_shape;            // TF32 tensor-core kernel: 0 alpha kept in registers, 1 read back (identical values)
 };
 // comp: 0 plain FP32 sums, 1 Kahan, 2 blocked Kahan (see prune_common.cuh)
 cudaError_t launch_prune(int prec, int comp, const PruneArgs &a, cudaStream_t s, int grid);
+constexpr int PRUNE_SMALL_TILE = 8;   // the SIMT kernel's column tile in a short launch
 int prune_tile_cols(int prec);
 int simt_tile_cols(int prec, int nslots, int tile = 0);   // the SIMT kernel's column tile (k_prune)
 size_t prune_smem_bytes(int prec, int nslots, int nl, int nint, int tile = 0);
@@ -194,6 +196,11 @@ bool prune_tc_dual_supported(int nslots, int nl);
 // out_index (may be null): request r's sums go to out_*[out_index[r]] instead of out_*[r].
 cudaError_t launch_reduce(const double *partials, const int32_t *wi_begin, int nreq, double *out_lpr,
                           double *out_elpr, cudaStream_t s, const int32_t *out_index = nullptr);
+
+// The same from the columns' terms of small tiles (PruneArgs.colv): tc the tile, group the tile
+// of a long launch, whose order of summation is kept.
+cudaError_t launch_reduce_cols(const double *colv, const WorkItem *wi, const int32_t *wi_begin, int nreq, int tc, int group,
+                               double *out_lpr, double *out_elpr, cudaStream_t s);
 
 // Float-float pruning on the tensor cores (ff_kernels.cu): returned values that agree with
 // the FP64 path to ~1e-12 relative.  Pbuf holds per P set ff_pset_bytes() of operands, made

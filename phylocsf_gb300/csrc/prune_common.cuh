@@ -36,6 +36,9 @@ template <> struct AtomMax<double> {
 };
 
 template <typename T, int CPT> struct ColLoad;
+template <typename T> struct ColLoad<T, 1> {
+    static __device__ inline void load(const T *p, T v[1]) { v[0] = p[0]; }
+};
 template <> struct ColLoad<float, 4> {
     static __device__ inline void load(const float *p, float v[4]) { Vec4<float>::load(p, v); }
 };
@@ -61,8 +64,8 @@ template <typename T, int CPT> struct ColStore;
 template <> struct ColStore<float, 4> {
     static __device__ inline void store(float *p, const float v[4]) { *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]); }
 };
-template <> struct ColStore<float, 1> {
-    static __device__ inline void store(float *p, const float v[1]) { *p = v[0]; }
+template <typename T> struct ColStore<T, 1> {
+    static __device__ inline void store(T *p, const T v[1]) { *p = v[0]; }
 };
 template <> struct ColStore<float, 2> {
     static __device__ inline void store(float *p, const float v[2]) { *reinterpret_cast<float2 *>(p) = make_float2(v[0], v[1]); }
@@ -174,10 +177,10 @@ __device__ __forceinline__ double scale2(double x, int e)
 // eight products summed plainly, then each block folded into the running sum
 // with Kahan's correction (about a ninth of the plain bias at 1.5 operations per
 // product instead of 5).
-template <typename T, int TC, int COMP>
-__device__ inline void contract(const T *M, const T *X, int a0, int c0, T out[4][TC / 16])
+// CPT: columns per thread (TC / 16 with 256 threads of 4 states each).
+template <typename T, int TC, int COMP, int CPT = TC / 16>
+__device__ inline void contract(const T *M, const T *X, int a0, int c0, T out[4][CPT])
 {
-    constexpr int CPT = TC / 16;
     T comp[4][CPT];
 #pragma unroll
     for (int i = 0; i < 4; i++)
@@ -340,12 +343,11 @@ __device__ inline void stage_rows(T *dst, const T *src, int tid)
 // Partial of child c at its parent: v[a] = alpha_c[a] + sum_j E_c[a][j] alpha_c[j]
 // (internal child, slot >= 0; Et = E_c^T) or the gather v[a] = P_c[a][s] of a
 // leaf in state s (1 for a marginalised leaf: P rows sum to 1).
-template <typename T, int TC, int KAHAN>
+template <typename T, int TC, int KAHAN, int CPT = TC / 16>
 __device__ inline void child_partial(const T *Et, const T *slots, int slot, int leaf, const uint8_t *lvT, int a0,
-                                     int c0, T v[4][TC / 16], int64_t dither_col0 = -1, const T *leaf_g = nullptr,
+                                     int c0, T v[4][CPT], int64_t dither_col0 = -1, const T *leaf_g = nullptr,
                                      const float *dlo = nullptr)
 {
-    constexpr int CPT = TC / 16;
     // dlo (may be null): the low parts of this branch's diag(E), added to the diagonal
     // term: FP32 storage of E_ii is the one rounding that every column sharing a state
     // at this node repeats identically, so over a long region it adds up coherently
@@ -390,7 +392,7 @@ __device__ inline void child_partial(const T *Et, const T *slots, int slot, int 
         return;
     }
     const T *al = slots + (size_t)slot * K * TC;
-    contract<T, TC, KAHAN>(Et, al, a0, c0, v);
+    contract<T, TC, KAHAN, CPT>(Et, al, a0, c0, v);
     T lo[4] = {(T)0, (T)0, (T)0, (T)0};
     if (dlo) {
         const float4 l4 = *reinterpret_cast<const float4 *>(dlo + a0);

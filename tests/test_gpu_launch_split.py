@@ -79,3 +79,21 @@ def test_outside_parts(prec):
     p1, _ = eng.node_posteriors(one, 0, 0.7, [0, ps.tree.nl, ps.tree.n - 1])
     pm, _ = eng.node_posteriors(many, 0, 0.7, [0, ps.tree.nl, ps.tree.n - 1])
     assert np.array_equal(p1, pm[:, :L]) and np.array_equal(p1, pm[:, -L:])
+
+
+# pruning tiles of 8 columns (a region alone) and of 32 or 64 (in a long launch): the same bits
+@pytest.mark.parametrize("name,prec", [("12flies", "fp32b"), ("12flies", "fp32c"), ("12flies", "fp64"), ("120mammals", "fp32b")])
+def test_small_pruning_tiles(name, prec):
+    lengths = [1, 7, 8, 9, 31, 32, 33, 63, 64, 65, 0, 128, 200]
+    ps, offs, leaves = _regions(name, lengths)
+    eng = P.Engine(ps.tree, ps.S_c, ps.pi_c, ps.S_n, ps.pi_n, precision=prec)
+    n, L = len(lengths), int(offs[-1])
+    reps = 12                                              # 7,700 columns: past the small tiles
+    big = eng.batch(np.concatenate([[0]] + [offs[1:] + k * L for k in range(reps)]), np.tile(leaves, (reps, 1)))
+    few = eng.batch(offs, leaves)
+    for rho in (0.3, 2.0):
+        lpr, elpr, st = eng.lpr(big, 1, rho)
+        one = eng.lpr(few, 1, rho)
+        assert (st == 0).all()
+        assert np.array_equal(one[0], lpr[:n]) and np.array_equal(one[1], elpr[:n])
+        assert np.array_equal(one[0], lpr[-n:])
