@@ -24,6 +24,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <deque>
+#include <memory>
 #include <map>
 #include <unordered_map>
 #include <string>
@@ -90,12 +91,23 @@ inline uint64_t splitmix64(uint64_t &s)
 }
 inline double uniform01(uint64_t &s) { return (double)(splitmix64(s) >> 11) * (1.0 / 9007199254740992.0); }
 
+constexpr size_t ONESHOT_KEEP = size_t(64) << 20;   // most leaf bytes an engine keeps after pcsf_score_batch
+
 constexpr double GOLDEN = 0.3819660;
 constexpr double SQRT_DBL_EPS = 1.4901161193847656e-08;
 
 }  // namespace
 
 void pcsf_internal_set_error(const std::string &msg) { g_static_error = msg; }
+
+struct pcsf_batch {
+    pcsf_engine *e = nullptr;
+    int device = 0;       // the engine's device, for destroying the batch after its engine
+    int nreg = 0;
+    std::vector<int64_t> offs;
+    int64_t total_cols = 0;
+    DevBuf<uint8_t> dleaves;
+};
 
 struct pcsf_engine {
     int device = 0;
@@ -149,11 +161,15 @@ struct pcsf_engine {
     int deriv_mode = 0;
     double tc_shape_ms[PCSF_TC_SHAPES] = {};   // the autotuner's time per pass of each shape (0: untimed)
     size_t pbuf_psets = 0;
-    DevBuf<PSet> dps;
-    DevBuf<Request> dreq;
-    DevBuf<WorkItem> dwi;
-    DevBuf<int32_t> dwib, dstatus;
-    DevBuf<double> dpart, dlpr, delpr;
+    // an evaluation's small arrays in one block each, on the device and page-locked on the host:
+    // one copy up (P sets, requests, work items, their begins, status keys) and one down
+    // (status keys, lpr, elpr)
+    DevBuf<unsigned char> dio;
+    HostBuf<unsigned char> hio;
+    HostBuf<int> herr;             // copy of derr
+    HostBuf<unsigned long long> hbad;
+    DevBuf<double> dpart;
+    std::unique_ptr<pcsf_batch> oneshot;   // pcsf_score_batch's regions; the leaf buffer stays up to ONESHOT_KEEP
     // gradient path
     DevBuf<unsigned char> gscratch;
     bool grad_recompute = false;   // adjoint: recompute leaf children's partials instead of storing them
@@ -162,11 +178,6 @@ struct pcsf_engine {
     DevBuf<double> dQrowd;
     HostBuf<double> hgrad;
     int grad_grid[2] = {0, 0};     // CTAs of the adjoint: without, with the rate parameters
-    HostBuf<PSet> hps;
-    HostBuf<Request> hreq;
-    HostBuf<WorkItem> hwi;
-    HostBuf<int32_t> hwib, hstatus;
-    HostBuf<double> hlpr, helpr;
     int prune_grid = 0;
     int simt_tile = 0;             // SIMT column tile (0: the default rule; set by pcsf_engine_autotune)
     int smem_sm = 0;               // shared memory per SM, for the grid of a tile
@@ -211,15 +222,6 @@ static inline bool tc_prec(int prec)
 {
     return prec == PCSF_PREC_TF32X3 || prec == PCSF_PREC_TF32 || prec == PCSF_PREC_BF16X3;
 }
-
-struct pcsf_batch {
-    pcsf_engine *e = nullptr;
-    int device = 0;       // the engine's device, for destroying the batch after its engine
-    int nreg = 0;
-    std::vector<int64_t> offs;
-    int64_t total_cols = 0;
-    DevBuf<uint8_t> dleaves;
-};
 
 #define CK(call, what)                                      \
     do {                                                    \
@@ -783,21 +785,22 @@ static int evaluate(pcsf_engine *e, pcsf_batch *b, const std::vector<Request> &r
     const int nps = (int)psets.size(), nwi = (int)wis.size();
     e->stats.evaluations += nreq;
 
-    CK(e->hps.reserve(nps), "cudaMallocHost");
-    CK(e->hreq.reserve(nreq), "cudaMallocHost");
-    CK(e->hwi.reserve(nwi), "cudaMallocHost");
-    CK(e->hwib.reserve(nreq + 1), "cudaMallocHost");
-    CK(e->hstatus.reserve(nps), "cudaMallocHost");
-    CK(e->hlpr.reserve(nreq), "cudaMallocHost");
-    CK(e->helpr.reserve(nreq), "cudaMallocHost");
-    CK(e->dps.reserve(nps), "cudaMalloc");
-    CK(e->dreq.reserve(nreq), "cudaMalloc");
-    CK(e->dwi.reserve(nwi), "cudaMalloc");
-    CK(e->dwib.reserve(nreq + 1), "cudaMalloc");
-    CK(e->dstatus.reserve(nps), "cudaMalloc");
+    auto up256 = [](size_t x) { return (x + 255) & ~size_t(255); };
+    const size_t o_ps = 0, o_req = o_ps + up256(sizeof(PSet) * nps), o_wi = o_req + up256(sizeof(Request) * nreq),
+                 o_wib = o_wi + up256(sizeof(WorkItem) * nwi), o_st = o_wib + up256(sizeof(int32_t) * (nreq + 1)),
+                 o_lpr = o_st + up256(sizeof(int32_t) * nps), o_elpr = o_lpr + up256(sizeof(double) * nreq),
+                 o_end = o_elpr + sizeof(double) * nreq;
+    if (o_end > e->dio.n) CK(e->dio.reserve(o_end + o_end / 2), "cudaMalloc");
+    if (o_end > e->hio.n) CK(e->hio.reserve(o_end + o_end / 2), "cudaMallocHost");
+    CK(e->herr.reserve(1), "cudaMallocHost");
+    auto dptr = [&](size_t o) { return e->dio.p + o; };
+    auto hptr = [&](size_t o) { return e->hio.p + o; };
+    PSet *dps = reinterpret_cast<PSet *>(dptr(o_ps));
+    Request *dreq = reinterpret_cast<Request *>(dptr(o_req));
+    WorkItem *dwi = reinterpret_cast<WorkItem *>(dptr(o_wi));
+    int32_t *dwib = reinterpret_cast<int32_t *>(dptr(o_wib)), *dstatus = reinterpret_cast<int32_t *>(dptr(o_st));
+    double *dlpr = reinterpret_cast<double *>(dptr(o_lpr)), *delpr = reinterpret_cast<double *>(dptr(o_elpr));
     CK(e->dpart.reserve(2 * (size_t)std::max(nwi, 1) * (cols ? TC : 1)), "cudaMalloc");
-    CK(e->dlpr.reserve(nreq), "cudaMalloc");
-    CK(e->delpr.reserve(nreq), "cudaMalloc");
     if (drho) {
         CK(e->ddpart.reserve(2 * (size_t)std::max(nwi, 1)), "cudaMalloc");
         CK(e->ddrho.reserve(nreq), "cudaMalloc");
@@ -832,48 +835,52 @@ static int evaluate(pcsf_engine *e, pcsf_batch *b, const std::vector<Request> &r
             return e->fail(PCSF_EINVAL, "parameter derivatives need more shared memory than this device has for this tree");
     }
 
-    std::memcpy(e->hps.p, psets.data(), sizeof(PSet) * nps);
-    std::memcpy(e->hreq.p, reqs.data(), sizeof(Request) * nreq);
-    if (nwi) std::memcpy(e->hwi.p, wis.data(), sizeof(WorkItem) * nwi);
-    std::memcpy(e->hwib.p, wib.data(), sizeof(int32_t) * (nreq + 1));
+    std::memcpy(hptr(o_ps), psets.data(), sizeof(PSet) * nps);
+    std::memcpy(hptr(o_req), reqs.data(), sizeof(Request) * nreq);
+    if (nwi) std::memcpy(hptr(o_wi), wis.data(), sizeof(WorkItem) * nwi);
+    std::memcpy(hptr(o_wib), wib.data(), sizeof(int32_t) * (nreq + 1));
+    std::memset(hptr(o_st), 0x7f, sizeof(int32_t) * nps);
     cudaStream_t s = e->stream;
-    CK(cudaMemcpyAsync(e->dps.p, e->hps.p, sizeof(PSet) * nps, cudaMemcpyHostToDevice, s), "H2D psets");
-    CK(cudaMemcpyAsync(e->dreq.p, e->hreq.p, sizeof(Request) * nreq, cudaMemcpyHostToDevice, s), "H2D requests");
-    if (nwi) CK(cudaMemcpyAsync(e->dwi.p, e->hwi.p, sizeof(WorkItem) * nwi, cudaMemcpyHostToDevice, s), "H2D work");
-    CK(cudaMemcpyAsync(e->dwib.p, e->hwib.p, sizeof(int32_t) * (nreq + 1), cudaMemcpyHostToDevice, s), "H2D wib");
-    CK(cudaMemsetAsync(e->dstatus.p, 0x7f, sizeof(int32_t) * nps, s), "memset status");
+    CK(cudaMemcpyAsync(dptr(0), hptr(0), o_st + sizeof(int32_t) * nps, cudaMemcpyHostToDevice, s), "H2D requests");
 
     float pf_ms = 0.f, pr_ms = 0.f;
     const int nchunks = (int)chunk_req_begin.size() - 1;
+    auto chunk_times = [&]() {
+        float t1 = 0.f, t2 = 0.f;
+        cudaEventElapsedTime(&t1, e->ev[0], e->ev[1]);
+        cudaEventElapsedTime(&t2, e->ev[1], e->ev[2]);
+        pf_ms += t1;
+        pr_ms += t2;
+    };
     for (int c = 0; c < nchunks; c++) {
         int r0 = chunk_req_begin[c], r1 = chunk_req_begin[c + 1];
         int p0 = chunk_ps_begin[c], p1 = chunk_ps_begin[c + 1];
         CK(cudaEventRecord(e->ev[0], s), "event");
         if (ff) {   // FP64 formation, split into the float-float kernel's operands
-            CK(launch_pform(true, e->dps.p + p0, p1 - p0, e->dbranch.p, e->nbr, dmv, e->Pbuf64.p, e->dstatus.p + p0, s),
+            CK(launch_pform(true, dps + p0, p1 - p0, e->dbranch.p, e->nbr, dmv, e->Pbuf64.p, dstatus + p0, s),
                "P(t) formation launch");
             CK(launch_split_ff(e->Pbuf64.p, e->Pbuf.p, p1 - p0, e->nbr, e->nl, s), "P(t) split launch");
             e->stats.kernel_launches += 1;
         } else if (stage64) {
-            CK(launch_pform(true, e->dps.p + p0, p1 - p0, e->dbranch.p, e->nbr, dmv, e->Pbuf64.p, e->dstatus.p + p0, s),
+            CK(launch_pform(true, dps + p0, p1 - p0, e->dbranch.p, e->nbr, dmv, e->Pbuf64.p, dstatus + p0, s),
                "P(t) formation launch");
             CK(launch_d2f_rows(e->Pbuf64.p, reinterpret_cast<float *>(e->Pbuf.p), (size_t)(p1 - p0) * e->nbr, e->nbr,
                                bop, e->nl, s, dlo), "P(t) conversion launch");
             e->stats.kernel_launches += 1;
         } else if (want_bop && !dyn) {
-            CK(launch_pform_tc(e->dps.p + p0, p1 - p0, e->dbranch.p, e->nbr, e->nl, dmv, e->dPfB.p,
-                               reinterpret_cast<float *>(e->Pbuf.p), bop, e->dstatus.p + p0, e->derr.p, s),
+            CK(launch_pform_tc(dps + p0, p1 - p0, e->dbranch.p, e->nbr, e->nl, dmv, e->dPfB.p,
+                               reinterpret_cast<float *>(e->Pbuf.p), bop, dstatus + p0, e->derr.p, s),
                "tensor-core P(t) formation launch");
         } else {
-            CK(launch_pform(e->prec == PCSF_PREC_FP64 || dyn || ff, e->dps.p + p0, p1 - p0, e->dbranch.p, e->nbr, dmv,
-                            e->Pbuf.p, e->dstatus.p + p0, s, false, bop, e->nl, (dyn || ff) ? nullptr : dlo),
+            CK(launch_pform(e->prec == PCSF_PREC_FP64 || dyn || ff, dps + p0, p1 - p0, e->dbranch.p, e->nbr, dmv,
+                            e->Pbuf.p, dstatus + p0, s, false, bop, e->nl, (dyn || ff) ? nullptr : dlo),
                "P(t) formation launch");
         }
         CK(cudaEventRecord(e->ev[1], s), "event");
         PruneArgs pa{};
-        pa.wi = e->dwi.p + wib[r0];
+        pa.wi = dwi + wib[r0];
         pa.nwi = wib[r1] - wib[r0];
-        pa.req = e->dreq.p;
+        pa.req = dreq;
         pa.leaves = b->dleaves.p;
         pa.Pbuf = e->Pbuf.p;
         pa.sched = e->dsched.p;
@@ -909,7 +916,7 @@ static int evaluate(pcsf_engine *e, pcsf_batch *b, const std::vector<Request> &r
             ga.Umat = dg ? dg->Umat : nullptr;
             ga.Hmat = e->dHmat.p;
             if (npar)
-                CK(launch_hform(e->prec == PCSF_PREC_FP64, e->dps.p + p0, p1 - p0, e->dbranch.p, e->nbr, dmv.lam, dg->Bdot,
+                CK(launch_hform(e->prec == PCSF_PREC_FP64, dps + p0, p1 - p0, e->dbranch.p, e->nbr, dmv.lam, dg->Bdot,
                                 e->dHmat.p, s), "derivative matrix launch");
             ga.scratch = e->gscratch.p;
             ga.scratch_per_cta = gscr;
@@ -943,40 +950,38 @@ static int evaluate(pcsf_engine *e, pcsf_batch *b, const std::vector<Request> &r
         e->stats.prune_launches += (pa.nwi > 0);
         e->stats.kind_launches[kind] += (pa.nwi > 0);
         e->stats.kernel_launches += (p1 > p0) + (pa.nwi > 0);
-        CK(cudaEventSynchronize(e->ev[2]), "pruning");
-        float t1 = 0.f, t2 = 0.f;
-        cudaEventElapsedTime(&t1, e->ev[0], e->ev[1]);
-        cudaEventElapsedTime(&t2, e->ev[1], e->ev[2]);
-        pf_ms += t1;
-        pr_ms += t2;
+        if (c + 1 < nchunks) {         // the next chunk records the same events
+            CK(cudaEventSynchronize(e->ev[2]), "pruning");
+            chunk_times();
+        }
     }
     CK(cudaEventRecord(e->ev[3], s), "event");
     if (cols)
-        CK(launch_reduce_cols(e->dpart.p, e->dwi.p, e->dwib.p, nreq, TC, simt_tile_cols(e->prec, e->nslots, e->simt_tile),
-                              e->dlpr.p, e->delpr.p, s), "reduce launch");
+        CK(launch_reduce_cols(e->dpart.p, dwi, dwib, nreq, TC, simt_tile_cols(e->prec, e->nslots, e->simt_tile),
+                              dlpr, delpr, s), "reduce launch");
     else
-        CK(launch_reduce(e->dpart.p, e->dwib.p, nreq, e->dlpr.p, e->delpr.p, s), "reduce launch");
+        CK(launch_reduce(e->dpart.p, dwib, nreq, dlpr, delpr, s), "reduce launch");
     e->stats.kernel_launches += 1;
     std::vector<double> hdrho;
     if (drho) {
-        CK(launch_reduce(e->ddpart.p, e->dwib.p, nreq, e->ddrho.p, e->ddscr.p, s), "reduce launch");
+        CK(launch_reduce(e->ddpart.p, dwib, nreq, e->ddrho.p, e->ddscr.p, s), "reduce launch");
         e->stats.kernel_launches += 1;
         hdrho.resize(nreq);
         CK(cudaMemcpyAsync(hdrho.data(), e->ddrho.p, sizeof(double) * nreq, cudaMemcpyDeviceToHost, s), "D2H drho");
     }
     if (grad) {
-        CK(launch_reduce_grad(e->dgpart.p, e->dwib.p, nreq, gstride, e->dgrad.p, s), "gradient reduce launch");
+        CK(launch_reduce_grad(e->dgpart.p, dwib, nreq, gstride, e->dgrad.p, s), "gradient reduce launch");
         e->stats.kernel_launches += 1;
         CK(cudaMemcpyAsync(e->hgrad.p, e->dgrad.p, sizeof(double) * nreq * gstride, cudaMemcpyDeviceToHost, s), "D2H grad");
     }
     CK(cudaEventRecord(e->ev[4], s), "event");
-    CK(cudaMemcpyAsync(e->hlpr.p, e->dlpr.p, sizeof(double) * nreq, cudaMemcpyDeviceToHost, s), "D2H lpr");
-    CK(cudaMemcpyAsync(e->helpr.p, e->delpr.p, sizeof(double) * nreq, cudaMemcpyDeviceToHost, s), "D2H elpr");
-    CK(cudaMemcpyAsync(e->hstatus.p, e->dstatus.p, sizeof(int32_t) * nps, cudaMemcpyDeviceToHost, s), "D2H status");
-    int herr = 0;
-    CK(cudaMemcpyAsync(&herr, e->derr.p, sizeof(int), cudaMemcpyDeviceToHost, s), "D2H error flag");
+    CK(cudaMemcpyAsync(hptr(o_st), dptr(o_st), o_end - o_st, cudaMemcpyDeviceToHost, s), "D2H results");
+    CK(cudaMemcpyAsync(e->herr.p, e->derr.p, sizeof(int), cudaMemcpyDeviceToHost, s), "D2H error flag");
     CK(cudaStreamSynchronize(s), "evaluation");
-    if (herr) return e->fail(PCSF_ECUDA, "a tensor-core wait timed out; results of this call are invalid");
+    chunk_times();
+    const int32_t *hstatus = reinterpret_cast<const int32_t *>(hptr(o_st));
+    const double *hlpr = reinterpret_cast<const double *>(hptr(o_lpr)), *helpr = reinterpret_cast<const double *>(hptr(o_elpr));
+    if (*e->herr.p) return e->fail(PCSF_ECUDA, "a tensor-core wait timed out; results of this call are invalid");
     float rd_ms = 0.f;
     cudaEventElapsedTime(&rd_ms, e->ev[3], e->ev[4]);
     e->stats.pform_ms += pf_ms;
@@ -985,9 +990,9 @@ static int evaluate(pcsf_engine *e, pcsf_batch *b, const std::vector<Request> &r
     e->stats.kind_columns[kind] += kind_cols;
     e->stats.other_ms += rd_ms;
     for (int r = 0; r < nreq; r++) {
-        int key = e->hstatus.p[req_pset_global[r]];
+        int key = hstatus[req_pset_global[r]];
         int st = (key >= 0 && key < 0x7f000000) ? (key & 15) : PCSF_OK;
-        out[r] = Eval{e->hlpr.p[r], e->helpr.p[r], st};
+        out[r] = Eval{hlpr[r], helpr[r], st};
     }
     if (grad) grad->assign(e->hgrad.p, e->hgrad.p + (size_t)nreq * gstride);
     if (drho) *drho = hdrho;
@@ -1943,9 +1948,10 @@ static double prior_value(int kind, double x)
 struct DynModels {
     std::map<OmegaKey, int> index;                  // key -> cache slot
     std::vector<std::vector<double>> U, lam, eq;    // host cache
-    DevBuf<double> dU, dlam, dsq, disq, dwrow, dprior, dwlog;
-    DevBuf<int16_t> dwlist;
-    DevBuf<float> dUf;
+    DevBuf<unsigned char> dtab;                     // the round's table, and its host image (pageable: page-
+    std::vector<unsigned char> htab;                // locking it would cost a call more than its one copy)
+    DevBuf<double> deig;                            // eigensolver: matrices in, eigenvectors and values out
+    std::vector<double> heig;
     DevModels dm{};
     DevBuf<unsigned char> dQrow, dBdot;             // parameter derivatives (dyn_derivs)
 };
@@ -1971,7 +1977,12 @@ static int dyn_prepare(pcsf_engine *e, DynModels &dmod, const std::vector<OmegaK
     }
     if (!fresh.empty()) {
         const int nf = (int)fresh.size();
-        std::vector<double> A((size_t)nf * K2), Q(K2), pi(K);
+        std::vector<double> Q(K2), pi(K);
+        const size_t nA = (size_t)nf * K2, nst = (size_t)(nf + 1) / 2;   // status words share the block
+        if (2 * nA + (size_t)nf * K + nst > dmod.deig.n) CK(dmod.deig.reserve(3 * nA + 2 * (size_t)nf * K + 2 * nst), "cudaMalloc");
+        dmod.heig.resize(2 * nA + (size_t)nf * K + nst);
+        double *A = dmod.heig.data(), *Uh = A + nA, *lh = Uh + nA;
+        const int *sth = reinterpret_cast<const int *>(lh + (size_t)nf * K);
         for (int f = 0; f < nf; f++) {
             omega_q(keys[fresh[f]], Q.data(), pi.data());
             std::vector<double> &eqv = dmod.eq[slot[fresh[f]]];
@@ -1983,83 +1994,66 @@ static int dyn_prepare(pcsf_engine *e, DynModels &dmod, const std::vector<OmegaK
                     A[(size_t)f * K2 + i * K + j] = 0.5 * (aij + aji);
                 }
         }
-        DevBuf<double> dA, dUo, dlo;
-        DevBuf<int> dst;
-        CK(dA.reserve((size_t)nf * K2), "cudaMalloc");
-        CK(dUo.reserve((size_t)nf * K2), "cudaMalloc");
-        CK(dlo.reserve((size_t)nf * K), "cudaMalloc");
-        CK(dst.reserve(nf), "cudaMalloc");
-        CK(cudaMemcpyAsync(dA.p, A.data(), sizeof(double) * nf * K2, cudaMemcpyHostToDevice, e->stream), "H2D");
-        CK(launch_jacobi(dA.p, dUo.p, dlo.p, dst.p, nf, e->stream), "eigensolver launch");
+        double *dA = dmod.deig.p, *dUo = dA + nA, *dlo = dUo + nA;
+        CK(cudaMemcpyAsync(dA, A, sizeof(double) * nA, cudaMemcpyHostToDevice, e->stream), "H2D");
+        CK(launch_jacobi(dA, dUo, dlo, reinterpret_cast<int *>(dlo + (size_t)nf * K), nf, e->stream), "eigensolver launch");
         e->stats.kernel_launches += 1;
-        std::vector<double> Uh((size_t)nf * K2), lh((size_t)nf * K);
-        std::vector<int> sth(nf);
-        CK(cudaMemcpyAsync(Uh.data(), dUo.p, sizeof(double) * nf * K2, cudaMemcpyDeviceToHost, e->stream), "D2H");
-        CK(cudaMemcpyAsync(lh.data(), dlo.p, sizeof(double) * nf * K, cudaMemcpyDeviceToHost, e->stream), "D2H");
-        CK(cudaMemcpyAsync(sth.data(), dst.p, sizeof(int) * nf, cudaMemcpyDeviceToHost, e->stream), "D2H");
+        CK(cudaMemcpyAsync(Uh, dUo, sizeof(double) * (nA + (size_t)nf * K + nst), cudaMemcpyDeviceToHost, e->stream), "D2H");
         CK(cudaStreamSynchronize(e->stream), "eigensolver");
         for (int f = 0; f < nf; f++) {
             if (sth[f]) return e->fail(PCSF_EEIG, "eigensolver did not converge for an OmegaModel rate matrix");
-            std::copy(Uh.begin() + (size_t)f * K2, Uh.begin() + (size_t)(f + 1) * K2, dmod.U[slot[fresh[f]]].begin());
-            std::copy(lh.begin() + (size_t)f * K, lh.begin() + (size_t)(f + 1) * K, dmod.lam[slot[fresh[f]]].begin());
+            std::copy(Uh + (size_t)f * K2, Uh + (size_t)(f + 1) * K2, dmod.U[slot[fresh[f]]].begin());
+            std::copy(lh + (size_t)f * K, lh + (size_t)(f + 1) * K, dmod.lam[slot[fresh[f]]].begin());
         }
     }
-    // device table for this round: model m of the round = keys[m]
-    const int M = (int)keys.size();
-    std::vector<double> U((size_t)M * K2), lam((size_t)M * K), sq((size_t)M * K), isq((size_t)M * K),
-        wrow((size_t)M * K), prior((size_t)M * K), wlog((size_t)M * K);
-    std::vector<float> Uf((size_t)M * K2);
-    std::vector<int16_t> wlist((size_t)M * WLIST);
-    for (int m = 0; m < M; m++) {
+    // device table for this round: model m of the round = keys[m]; one block, one copy
+    const size_t M = keys.size();
+    size_t o = 0;
+    auto take = [&](size_t bytes) { const size_t at = o; o = (o + bytes + 255) & ~size_t(255); return at; };
+    const size_t o_U = take(M * K2 * 8), o_lam = take(M * K * 8), o_sq = take(M * K * 8), o_isq = take(M * K * 8),
+                 o_w = take(M * K * 8), o_pr = take(M * K * 8), o_wl = take(M * K * 8), o_Uf = take(M * K2 * 4),
+                 o_list = take(M * WLIST * 2);
+    if (o > dmod.dtab.n) CK(dmod.dtab.reserve(o + o / 2), "cudaMalloc");
+    dmod.htab.resize(o);
+    auto hd = [&](size_t at) { return reinterpret_cast<double *>(dmod.htab.data() + at); };
+    for (size_t m = 0; m < M; m++) {
         const int id = slot[m];
         const std::vector<double> &eqv = dmod.eq[id];
+        double *sq = hd(o_sq) + m * K, *wrow = hd(o_w) + m * K, *prior = hd(o_pr) + m * K;
         double tot = 0.0;
         for (int i = 0; i < K; i++) tot += eqv[i];
         for (int i = 0; i < K; i++) {
-            sq[(size_t)m * K + i] = std::sqrt(eqv[i]);
-            isq[(size_t)m * K + i] = 1.0 / std::sqrt(eqv[i]);
-            prior[(size_t)m * K + i] = eqv[i] / tot;     // the equilibrium, normalised (PhyloModel.ml:25-29)
-            wlog[(size_t)m * K + i] = prior[(size_t)m * K + i] * std::log(prior[(size_t)m * K + i]);
-            lam[(size_t)m * K + i] = dmod.lam[id][i];
+            sq[i] = std::sqrt(eqv[i]);
+            hd(o_isq)[m * K + i] = 1.0 / std::sqrt(eqv[i]);
+            prior[i] = eqv[i] / tot;     // the equilibrium, normalised (PhyloModel.ml:25-29)
+            hd(o_wl)[m * K + i] = prior[i] * std::log(prior[i]);
+            hd(o_lam)[m * K + i] = dmod.lam[id][i];
         }
+        float *Uf = reinterpret_cast<float *>(dmod.htab.data() + o_Uf) + m * K2;
         for (int i = 0; i < K2; i++) {
-            U[(size_t)m * K2 + i] = dmod.U[id][i];
-            Uf[(size_t)m * K2 + i] = (float)dmod.U[id][i];
+            hd(o_U)[m * K2 + i] = dmod.U[id][i];
+            Uf[i] = (float)dmod.U[id][i];
         }
         const double nrm = std::sqrt(tot);
         for (int mm = 0; mm < K; mm++) {
             double w = 0.0;
-            for (int j = 0; j < K; j++) w += dmod.U[id][j * K + mm] * sq[(size_t)m * K + j];
-            wrow[(size_t)m * K + mm] = (std::fabs(w) > 1e-9 * nrm) ? w : 0.0;
+            for (int j = 0; j < K; j++) w += dmod.U[id][j * K + mm] * sq[j];
+            wrow[mm] = (std::fabs(w) > 1e-9 * nrm) ? w : 0.0;
         }
-        make_wlist(&wrow[(size_t)m * K], &wlist[(size_t)m * WLIST]);
+        make_wlist(wrow, reinterpret_cast<int16_t *>(dmod.htab.data() + o_list) + m * WLIST);
     }
-    CK(dmod.dwlist.reserve((size_t)M * WLIST), "cudaMalloc");
-    CK(cudaMemcpyAsync(dmod.dwlist.p, wlist.data(), sizeof(int16_t) * M * WLIST, cudaMemcpyHostToDevice, e->stream),
-       "H2D");
-    CK(dmod.dU.reserve((size_t)M * K2), "cudaMalloc");
-    CK(dmod.dUf.reserve((size_t)M * K2), "cudaMalloc");
-    for (auto *bp : {&dmod.dlam, &dmod.dsq, &dmod.disq, &dmod.dwrow, &dmod.dprior, &dmod.dwlog})
-        CK(bp->reserve((size_t)M * K), "cudaMalloc");
-    CK(cudaMemcpyAsync(dmod.dU.p, U.data(), sizeof(double) * M * K2, cudaMemcpyHostToDevice, e->stream), "H2D");
-    CK(cudaMemcpyAsync(dmod.dUf.p, Uf.data(), sizeof(float) * M * K2, cudaMemcpyHostToDevice, e->stream), "H2D");
-    CK(cudaMemcpyAsync(dmod.dlam.p, lam.data(), sizeof(double) * M * K, cudaMemcpyHostToDevice, e->stream), "H2D");
-    CK(cudaMemcpyAsync(dmod.dsq.p, sq.data(), sizeof(double) * M * K, cudaMemcpyHostToDevice, e->stream), "H2D");
-    CK(cudaMemcpyAsync(dmod.disq.p, isq.data(), sizeof(double) * M * K, cudaMemcpyHostToDevice, e->stream), "H2D");
-    CK(cudaMemcpyAsync(dmod.dwrow.p, wrow.data(), sizeof(double) * M * K, cudaMemcpyHostToDevice, e->stream), "H2D");
-    CK(cudaMemcpyAsync(dmod.dprior.p, prior.data(), sizeof(double) * M * K, cudaMemcpyHostToDevice, e->stream), "H2D");
-    CK(cudaMemcpyAsync(dmod.dwlog.p, wlog.data(), sizeof(double) * M * K, cudaMemcpyHostToDevice, e->stream), "H2D");
-    CK(cudaStreamSynchronize(e->stream), "model upload");
+    CK(cudaMemcpyAsync(dmod.dtab.p, dmod.htab.data(), o, cudaMemcpyHostToDevice, e->stream), "H2D");
+    auto dd = [&](size_t at) { return reinterpret_cast<const double *>(dmod.dtab.p + at); };
     dmod.dm = DevModels{};
-    dmod.dm.U = dmod.dU.p;
-    dmod.dm.Uf = dmod.dUf.p;
-    dmod.dm.lam = dmod.dlam.p;
-    dmod.dm.sq = dmod.dsq.p;
-    dmod.dm.isq = dmod.disq.p;
-    dmod.dm.wrow = dmod.dwrow.p;
-    dmod.dm.wlist = dmod.dwlist.p;
-    dmod.dm.prior = dmod.dprior.p;
-    dmod.dm.wlog = dmod.dwlog.p;
+    dmod.dm.U = dd(o_U);
+    dmod.dm.Uf = reinterpret_cast<const float *>(dmod.dtab.p + o_Uf);
+    dmod.dm.lam = dd(o_lam);
+    dmod.dm.sq = dd(o_sq);
+    dmod.dm.isq = dd(o_isq);
+    dmod.dm.wrow = dd(o_w);
+    dmod.dm.wlist = reinterpret_cast<const int16_t *>(dmod.dtab.p + o_list);
+    dmod.dm.prior = dd(o_pr);
+    dmod.dm.wlog = dd(o_wl);
     dmod.dm.tol = e->tol;
     dmod.dm.grid_n = 0;
     return PCSF_OK;
@@ -2310,6 +2304,50 @@ static int omega_impl(pcsf_engine *e, pcsf_batch *b, double omega_h1, double sig
         o.evals = R.evals;
     }
     return PCSF_OK;
+}
+
+// ---------------------------------------------------------------------------
+// Regions on the device.  The codes are checked there after the upload (a host loop over a
+// multi-GB batch would cost more than scoring it): batch_upload queues the copy and the check,
+// batch_codes reads the check's result once the stream has been waited for.  Until then no code
+// can lead out of bounds: every kernel treats one above 63 as a marginalised leaf.
+
+static int batch_upload(pcsf_engine *e, pcsf_batch *b, int32_t n_regions, const int64_t *col_offsets, const uint8_t *leaves)
+{
+    if (n_regions < 0 || (n_regions > 0 && !col_offsets)) return e->fail(PCSF_EINVAL, "pcsf_batch_create: bad regions");
+    b->e = e;
+    b->device = e->device;
+    b->nreg = n_regions;
+    b->offs.assign(n_regions + 1, 0);
+    if (n_regions > 0) {
+        if (col_offsets[0] != 0) return e->fail(PCSF_EINVAL, "pcsf_batch_create: col_offsets[0] must be 0");
+        for (int r = 0; r <= n_regions; r++) {
+            b->offs[r] = col_offsets[r];
+            if (r > 0 && col_offsets[r] < col_offsets[r - 1])
+                return e->fail(PCSF_EINVAL, "pcsf_batch_create: col_offsets not non-decreasing at %d", r);
+        }
+    }
+    b->total_cols = b->offs[n_regions];
+    if (b->total_cols > 0 && !leaves) return e->fail(PCSF_EINVAL, "pcsf_batch_create: leaves is NULL");
+    const size_t nbytes = (size_t)b->total_cols * e->nl;
+    cudaError_t ce = b->dleaves.reserve(nbytes + 16);
+    if (ce == cudaSuccess) ce = e->dbadcode.reserve(1);
+    if (ce == cudaSuccess) ce = e->hbad.reserve(1);
+    if (ce == cudaSuccess) ce = cudaMemsetAsync(e->dbadcode.p, 0xff, sizeof(unsigned long long), e->stream);
+    if (ce == cudaSuccess && nbytes)
+        ce = cudaMemcpyAsync(b->dleaves.p, leaves, nbytes, cudaMemcpyHostToDevice, e->stream);
+    if (ce == cudaSuccess) ce = launch_check_codes(b->dleaves.p, nbytes, e->dbadcode.p, e->stream);
+    if (ce == cudaSuccess)
+        ce = cudaMemcpyAsync(e->hbad.p, e->dbadcode.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost, e->stream);
+    return ce == cudaSuccess ? PCSF_OK : e->cuda_fail(ce, "batch upload");
+}
+
+static int batch_codes(pcsf_engine *e, const uint8_t *leaves)
+{
+    const unsigned long long bad = *e->hbad.p;
+    if (bad == ~0ull) return PCSF_OK;
+    return e->fail(PCSF_EINVAL, "pcsf_batch_create: leaf code %d at column %zu leaf %d (max %d)", leaves[bad],
+                   (size_t)(bad / (unsigned long long)e->nl), (int)(bad % (unsigned long long)e->nl), PCSF_MARGINALIZE);
 }
 
 // ---------------------------------------------------------------------------
@@ -2740,57 +2778,15 @@ int pcsf_batch_create(pcsf_engine *e, int32_t n_regions, const int64_t *col_offs
     CK(cudaSetDevice(e->device), "cudaSetDevice");
     if (!out) return e->fail(PCSF_EINVAL, "pcsf_batch_create: out is NULL");
     *out = nullptr;
-    if (n_regions < 0 || (n_regions > 0 && !col_offsets)) return e->fail(PCSF_EINVAL, "pcsf_batch_create: bad regions");
-    pcsf_batch *b = new (std::nothrow) pcsf_batch();
+    std::unique_ptr<pcsf_batch> b(new (std::nothrow) pcsf_batch());
     if (!b) return e->fail(PCSF_ENOMEM, "out of host memory");
-    b->e = e;
-    b->device = e->device;
-    b->nreg = n_regions;
-    b->offs.assign(n_regions + 1, 0);
-    if (n_regions > 0) {
-        if (col_offsets[0] != 0) {
-            delete b;
-            return e->fail(PCSF_EINVAL, "pcsf_batch_create: col_offsets[0] must be 0");
-        }
-        for (int r = 0; r <= n_regions; r++) {
-            b->offs[r] = col_offsets[r];
-            if (r > 0 && col_offsets[r] < col_offsets[r - 1]) {
-                delete b;
-                return e->fail(PCSF_EINVAL, "pcsf_batch_create: col_offsets not non-decreasing at %d", r);
-            }
-        }
+    int rc = batch_upload(e, b.get(), n_regions, col_offsets, leaves);
+    if (rc == PCSF_OK) {
+        CK(cudaStreamSynchronize(e->stream), "batch upload");
+        rc = batch_codes(e, leaves);
     }
-    b->total_cols = b->offs[n_regions];
-    if (b->total_cols > 0 && !leaves) {
-        delete b;
-        return e->fail(PCSF_EINVAL, "pcsf_batch_create: leaves is NULL");
-    }
-    const size_t nbytes = (size_t)b->total_cols * e->nl;
-    // the codes are checked on the device after the upload (a host loop over a
-    // multi-GB batch would cost more than scoring it)
-    unsigned long long bad = ~0ull;
-    cudaError_t ce = b->dleaves.reserve(nbytes + 16);
-    if (ce == cudaSuccess) ce = e->dbadcode.reserve(1);
-    if (ce == cudaSuccess) ce = cudaMemcpyAsync(e->dbadcode.p, &bad, sizeof(bad), cudaMemcpyHostToDevice, e->stream);
-    if (ce == cudaSuccess && nbytes)
-        ce = cudaMemcpyAsync(b->dleaves.p, leaves, nbytes, cudaMemcpyHostToDevice, e->stream);
-    if (ce == cudaSuccess) ce = launch_check_codes(b->dleaves.p, nbytes, e->dbadcode.p, e->stream);
-    if (ce == cudaSuccess) ce = cudaMemcpyAsync(&bad, e->dbadcode.p, sizeof(bad), cudaMemcpyDeviceToHost, e->stream);
-    if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->stream);
-    if (ce != cudaSuccess) {
-        delete b;
-        return e->cuda_fail(ce, "batch upload");
-    }
-    if (bad != ~0ull) {
-        const size_t col = (size_t)(bad / (unsigned long long)e->nl);
-        const int lf = (int)(bad % (unsigned long long)e->nl);
-        const int code = leaves[bad];
-        delete b;
-        return e->fail(PCSF_EINVAL, "pcsf_batch_create: leaf code %d at column %zu leaf %d (max %d)", code, col, lf,
-                       PCSF_MARGINALIZE);
-    }
-    *out = b;
-    return PCSF_OK;
+    if (rc == PCSF_OK) *out = b.release();
+    return rc;
 }
 
 void pcsf_batch_destroy(pcsf_batch *b)
@@ -2813,11 +2809,25 @@ int pcsf_score(pcsf_engine *e, pcsf_batch *b, int32_t strategy, pcsf_result *out
 int pcsf_score_batch(pcsf_engine *e, int32_t n_regions, const int64_t *col_offsets, const uint8_t *leaves,
                      int32_t strategy, pcsf_result *out)
 {
-    pcsf_batch *b = nullptr;
-    int rc = pcsf_batch_create(e, n_regions, col_offsets, leaves, &b);
-    if (rc) return rc;
-    rc = pcsf_score(e, b, strategy, out);
-    pcsf_batch_destroy(b);
+    if (!e) return PCSF_EINVAL;
+    CK(cudaSetDevice(e->device), "cudaSetDevice");
+    // the regions of a one-shot call live in the engine's own batch, whose leaf buffer is kept for
+    // the next call unless it is large; the codes' check is read after the scoring, which waits for
+    // the stream in any case, and nothing is written to out before
+    if (!e->oneshot) e->oneshot.reset(new (std::nothrow) pcsf_batch());
+    if (!e->oneshot) return e->fail(PCSF_ENOMEM, "out of host memory");
+    pcsf_batch *b = e->oneshot.get();
+    int rc = batch_upload(e, b, n_regions, col_offsets, leaves);
+    if (rc == PCSF_OK) {
+        std::vector<pcsf_result> res(n_regions);
+        int rs = pcsf_score(e, b, strategy, n_regions > 0 && !out ? nullptr : res.data());
+        const std::string why = e->err;
+        CK(cudaStreamSynchronize(e->stream), "batch upload");
+        rc = batch_codes(e, leaves);
+        if (rc == PCSF_OK && rs != PCSF_OK) rc = e->fail(rs, "%s", why.c_str());
+        if (rc == PCSF_OK && n_regions > 0) std::memcpy(out, res.data(), sizeof(pcsf_result) * n_regions);
+    }
+    if (b->dleaves.n > ONESHOT_KEEP) b->dleaves.release();
     return rc;
 }
 
