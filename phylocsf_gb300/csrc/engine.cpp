@@ -17,7 +17,6 @@
 // performs and which give bit-identical results) are not recomputed.
 #include <algorithm>
 #include <array>
-#include <thread>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -1882,49 +1881,6 @@ static void omega_q(const OmegaKey &q, double *Q, double *pi)
     for (int i = 0; i < K2; i++) Q[i] = Q[i] / scale;
 }
 
-// dQ/dx of the scaled OmegaModel rate matrix for x = kappa (0) or omega (1): with
-// R the unscaled matrix (R_ij = pi_j kappa^[transition] omega^[nonsynonymous]) and
-// s = -sum_i pi_i R_ii, Q = R / s and dQ/dx = R'/s - R s'/s^2 (pi does not depend on
-// kappa or omega).
-static void omega_dq(const OmegaKey &q, int x, double *dQ)
-{
-    std::vector<double> Q(K2), pi(K), R(K2), dR(K2);
-    omega_q(q, Q.data(), pi.data());
-    static const char *aa = "KNKNTTTTRSRSIIMIQHQHPPPPRRRRLLLLEDEDAAAAGGGGVVVV*Y*YSSSS*CWCLFLF";
-    auto nuc = [](int i, int pos) { return pos == 0 ? i / 16 : pos == 1 ? (i / 4) % 4 : i % 4; };
-    auto is_stop = [](int i) { return i == 48 || i == 50 || i == 56; };
-    for (int i = 0; i < K; i++) {
-        double tot = 0.0, dtot = 0.0;
-        for (int j = 0; j < K; j++) {
-            double v = 0.0, dv = 0.0;
-            if (i != j) {
-                int nd = 0, a = 0, bb = 0;
-                for (int pos = 0; pos < 3; pos++)
-                    if (nuc(i, pos) != nuc(j, pos)) { nd++; a = nuc(i, pos); bb = nuc(j, pos); }
-                if (nd == 1) {
-                    const bool transition = (a + bb == 2 && a != 1 && bb != 1) || (a + bb == 4 && a != 2 && bb != 2);
-                    const bool nonsyn = !is_stop(i) && !is_stop(j) && aa[i] != aa[j];
-                    v = pi[j] * ((transition ? q[0] : 1.0) * (nonsyn ? q[1] : 1.0));
-                    if (x == 0 && transition) dv = v / q[0];
-                    if (x == 1 && nonsyn) dv = v / q[1];
-                }
-            }
-            R[i * K + j] = v;
-            dR[i * K + j] = dv;
-            tot += v;
-            dtot += dv;
-        }
-        R[i * K + i] = -tot;
-        dR[i * K + i] = -dtot;
-    }
-    double sc = 0.0, dsc = 0.0;
-    for (int i = 0; i < K; i++) {
-        sc -= pi[i] * R[i * K + i];
-        dsc -= pi[i] * dR[i * K + i];
-    }
-    for (int i = 0; i < K2; i++) dQ[i] = dR[i] / sc - R[i] * dsc / (sc * sc);
-}
-
 // half_cauchy_lpdf ~mode:1 ~scale:0.5 (OmegaModel.ml:148-156) and the Gamma(7, 0.25)
 // density of kappa - 1 (OmegaModel.ml:157; GSL gamma_pdf with shape a, scale b).
 static double prior_value(int kind, double x)
@@ -1954,6 +1910,7 @@ struct DynModels {
     std::vector<double> heig;
     DevModels dm{};
     DevBuf<unsigned char> dQrow, dBdot;             // parameter derivatives (dyn_derivs)
+    DevBuf<double> dkeys;
 };
 
 static int dyn_prepare(pcsf_engine *e, DynModels &dmod, const std::vector<OmegaKey> &keys, std::vector<int> &slot)
@@ -2062,57 +2019,19 @@ static int dyn_prepare(pcsf_engine *e, DynModels &dmod, const std::vector<OmegaK
 // For the round's models (as laid out by dyn_prepare): Q row-major and
 // Bdot_x = U^T D^1/2 (dQ/dx) D^-1/2 U for x = kappa, omega, in the engine's
 // arithmetic type, on the device; dg points at them and at the round's U.
-static int dyn_derivs(pcsf_engine *e, DynModels &dmod, const std::vector<OmegaKey> &keys, const std::vector<int> &slot,
-                      DynGrad &dg)
+static int dyn_derivs(pcsf_engine *e, DynModels &dmod, const std::vector<OmegaKey> &keys, DynGrad &dg)
 {
     const int M = (int)keys.size();
     const bool fp64 = e->prec == PCSF_PREC_FP64;
-    std::vector<double> Qall((size_t)M * K2), Ball((size_t)M * 2 * K2);
-    auto work = [&](int m0, int m1) {
-        std::vector<double> Q(K2), pi(K), dQ(K2), A(K2), T1(K2);
-        for (int m = m0; m < m1; m++) {
-            omega_q(keys[m], Q.data(), pi.data());
-            std::copy(Q.begin(), Q.end(), Qall.begin() + (size_t)m * K2);
-            const std::vector<double> &U = dmod.U[slot[m]];
-            const std::vector<double> &eq = dmod.eq[slot[m]];
-            for (int x = 0; x < 2; x++) {
-                omega_dq(keys[m], x, dQ.data());
-                for (int i = 0; i < K; i++)
-                    for (int j = 0; j < K; j++) A[i * K + j] = std::sqrt(eq[i]) * dQ[i * K + j] / std::sqrt(eq[j]);
-                // T1 = A U, Bdot = U^T T1
-                for (int i = 0; i < K; i++)
-                    for (int j = 0; j < K; j++) {
-                        double acc = 0.0;
-                        for (int k = 0; k < K; k++) acc += A[i * K + k] * U[k * K + j];
-                        T1[i * K + j] = acc;
-                    }
-                double *Bd = &Ball[((size_t)m * 2 + x) * K2];
-                for (int i = 0; i < K; i++)
-                    for (int j = 0; j < K; j++) {
-                        double acc = 0.0;
-                        for (int k = 0; k < K; k++) acc += U[k * K + i] * T1[k * K + j];
-                        Bd[i * K + j] = acc;
-                    }
-            }
-        }
-    };
-    const int nth = std::max(1, std::min<int>(16, (int)std::thread::hardware_concurrency()));
-    std::vector<std::thread> th;
-    for (int t = 0; t < nth; t++) th.emplace_back(work, (int)((int64_t)M * t / nth), (int)((int64_t)M * (t + 1) / nth));
-    for (auto &t : th) t.join();
     const size_t es = fp64 ? 8 : 4;
+    static_assert(sizeof(OmegaKey) == 12 * sizeof(double), "OmegaKey is uploaded as 12 doubles");
+    CK(dmod.dkeys.reserve(12 * (size_t)M), "cudaMalloc");
     CK(dmod.dQrow.reserve((size_t)M * K2 * es), "cudaMalloc");
     CK(dmod.dBdot.reserve((size_t)M * 2 * K2 * es), "cudaMalloc");
-    if (fp64) {
-        CK(cudaMemcpyAsync(dmod.dQrow.p, Qall.data(), sizeof(double) * Qall.size(), cudaMemcpyHostToDevice, e->stream), "H2D");
-        CK(cudaMemcpyAsync(dmod.dBdot.p, Ball.data(), sizeof(double) * Ball.size(), cudaMemcpyHostToDevice, e->stream), "H2D");
-        CK(cudaStreamSynchronize(e->stream), "derivative upload");
-    } else {
-        std::vector<float> qf(Qall.begin(), Qall.end()), bf(Ball.begin(), Ball.end());
-        CK(cudaMemcpyAsync(dmod.dQrow.p, qf.data(), sizeof(float) * qf.size(), cudaMemcpyHostToDevice, e->stream), "H2D");
-        CK(cudaMemcpyAsync(dmod.dBdot.p, bf.data(), sizeof(float) * bf.size(), cudaMemcpyHostToDevice, e->stream), "H2D");
-        CK(cudaStreamSynchronize(e->stream), "derivative upload");
-    }
+    CK(cudaMemcpyAsync(dmod.dkeys.p, keys.data(), sizeof(OmegaKey) * M, cudaMemcpyHostToDevice, e->stream), "H2D");
+    CK(launch_omega_deriv(fp64, dmod.dkeys.p, dmod.dm.U, dmod.dm.sq, dmod.dm.isq, M, dmod.dQrow.p, dmod.dBdot.p, e->stream),
+       "rate matrix derivatives launch");
+    e->stats.kernel_launches += 1;
     dg.Qrow = dmod.dQrow.p;
     dg.Bdot = dmod.dBdot.p;
     dg.Umat = fp64 ? (const void *)dmod.dm.U : (const void *)dmod.dm.Uf;
@@ -2155,18 +2074,26 @@ struct OmegaRegion {
 static int region_f3x4(pcsf_engine *e, pcsf_batch *b, std::vector<std::array<double, 9>> &out)
 {
     out.assign(b->nreg, {});
-    std::vector<uint8_t> lv((size_t)b->total_cols * e->nl);
-    if (!lv.empty()) CK(cudaMemcpy(lv.data(), b->dleaves.p, lv.size(), cudaMemcpyDeviceToHost), "D2H leaves");
+    if (b->nreg == 0) return PCSF_OK;
+    DevBuf<int64_t> doffs;
+    DevBuf<unsigned long long> dhist;
+    std::vector<unsigned long long> hist((size_t)b->nreg * K);
+    CK(doffs.reserve(b->nreg + 1), "cudaMalloc");
+    CK(dhist.reserve(hist.size()), "cudaMalloc");
+    CK(cudaMemcpyAsync(doffs.p, b->offs.data(), sizeof(int64_t) * (b->nreg + 1), cudaMemcpyHostToDevice, e->stream), "H2D");
+    CK(launch_codon_hist(b->dleaves.p, doffs.p, b->nreg, e->nl, dhist.p, e->stream), "codon counts launch");
+    e->stats.kernel_launches += 1;
+    CK(cudaMemcpyAsync(hist.data(), dhist.p, sizeof(hist[0]) * hist.size(), cudaMemcpyDeviceToHost, e->stream), "D2H");
+    CK(cudaStreamSynchronize(e->stream), "codon counts");
     for (int r = 0; r < b->nreg; r++) {
         double counts[3][4];
         for (auto &row : counts)
             for (double &c : row) c = 1.0;
-        for (size_t i = (size_t)b->offs[r] * e->nl; i < (size_t)b->offs[r + 1] * e->nl; i++) {
-            const int c = lv[i];
-            if (c >= K) continue;
-            counts[0][c / 16] += 1.0;
-            counts[1][(c / 4) % 4] += 1.0;
-            counts[2][c % 4] += 1.0;
+        for (int c = 0; c < K; c++) {
+            const double n = (double)hist[(size_t)r * K + c];
+            counts[0][c / 16] += n;
+            counts[1][(c / 4) % 4] += n;
+            counts[2][c % 4] += n;
         }
         for (int pos = 0; pos < 3; pos++)
             for (int n = 0; n < 3; n++) out[r][3 * pos + n] = counts[pos][n] / counts[pos][3];
@@ -2474,7 +2401,7 @@ int pcsf_omega_grad(pcsf_engine *e, pcsf_batch *b, const double *kappa, const do
     rc = dyn_prepare(e, dmod, keys, slot);
     if (rc) return rc;
     DynGrad dg{};
-    rc = dyn_derivs(e, dmod, keys, slot, dg);
+    rc = dyn_derivs(e, dmod, keys, dg);
     if (rc) return rc;
     std::vector<Eval> res;
     std::vector<double> g;

@@ -611,4 +611,154 @@ cudaError_t launch_reduce_grad(const double *gpart, const int32_t *wi_begin, int
     return cudaGetLastError();
 }
 
+// OmegaModel rate matrices and their derivatives in the eigenbasis, per model (its parameters
+// key[m] = kappa, omega, sigma, F3x4) and parameter x = kappa, omega: Q (lib OmegaModel.ml:21-80,
+// scaled to mean rate 1) and Bdot_x = U^T D^1/2 (dQ/dx) D^-1/2 U.  With R the unscaled matrix and
+// s = -sum_i pi_i R_ii, Q = R / s and dQ/dx = R'/s - R s'/s^2 (pi does not depend on kappa or omega).
+// One CTA per (model, x); two 64^3 products in FP64 (two lanes per clock on an SM: 120 us) are
+// what bounds it.  On 16 host threads the matrices of 40 models took ~5 ms of a call.
+constexpr int OD_THREADS = 256;
+
+__device__ __forceinline__ int codon_nuc(int i, int pos) { return (i >> (4 - 2 * pos)) & 3; }
+
+template <typename T>
+__global__ void __launch_bounds__(OD_THREADS) k_omega_deriv(const double *keys, const double *U_all, const double *sq_all,
+                                                            const double *isq_all, T *Qout, T *Bout)
+{
+    extern __shared__ __align__(16) unsigned char odsm[];
+    double *A = reinterpret_cast<double *>(odsm);      // [K][K] D^1/2 dQ D^-1/2
+    double *Us = A + K2;                                // [K][K]
+    double *T1 = Us + K2;                               // [K][K] A U
+    __shared__ double pi[K], rs[K], drs[K];
+    __shared__ double tot_s[2];
+    const int m = blockIdx.x, x = blockIdx.y, tid = threadIdx.x;
+    const double *q = keys + 12 * (size_t)m;
+    const double *U = U_all + (size_t)m * K2, *sq = sq_all + (size_t)m * K, *isq = isq_all + (size_t)m * K;
+    auto sc = [&](int i) {
+        double out = 1.0;
+        for (int pos = 0; pos < 3; pos++) {
+            const int n = codon_nuc(i, pos), base = 3 + 3 * pos;
+            out *= ((n == 3) ? 1.0 : q[base + n]) / (q[base] + (q[base + 1] + (q[base + 2] + 1.0)));
+        }
+        return out;
+    };
+    if (tid < K) pi[tid] = sc(tid) / (1.0 - (1.0 - q[2]) * (sc(48) + (sc(50) + sc(56))));
+    for (int f = tid; f < K2; f += OD_THREADS) Us[f] = U[f];
+    __syncthreads();
+    // R_ij and dR_ij / dx (i != j)
+    const char *aa = "KNKNTTTTRSRSIIMIQHQHPPPPRRRRLLLLEDEDAAAAGGGGVVVV*Y*YSSSS*CWCLFLF";
+    auto rate = [&](int i, int j, double &v, double &dv) {
+        v = dv = 0.0;
+        int nd = 0, a = 0, b = 0;
+        for (int pos = 0; pos < 3; pos++)
+            if (codon_nuc(i, pos) != codon_nuc(j, pos)) { nd++; a = codon_nuc(i, pos); b = codon_nuc(j, pos); }
+        if (nd != 1) return;
+        const bool transition = a + b == 2 ? a != 1 : a + b == 4 && a != 2;
+        const bool nonsyn = aa[i] != '*' && aa[j] != '*' && aa[i] != aa[j];
+        v = pi[j] * ((transition ? q[0] : 1.0) * (nonsyn ? q[1] : 1.0));
+        if (x == 0 ? transition : nonsyn) dv = v / q[x];
+    };
+    if (tid < K) {
+        double t = 0.0, dt = 0.0;
+        for (int j = 0; j < K; j++) {
+            double v, dv;
+            rate(tid, j, v, dv);
+            t += v;
+            dt += dv;
+        }
+        rs[tid] = t;
+        drs[tid] = dt;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        double s = 0.0, ds = 0.0;
+        for (int i = 0; i < K; i++) {
+            s += pi[i] * rs[i];
+            ds += pi[i] * drs[i];
+        }
+        tot_s[0] = s;
+        tot_s[1] = ds;
+    }
+    __syncthreads();
+    const double s = tot_s[0], ds = tot_s[1];
+    for (int f = tid; f < K2; f += OD_THREADS) {
+        const int i = f / K, j = f % K;
+        double v, dv;
+        rate(i, j, v, dv);
+        if (i == j) {
+            v = -rs[i];
+            dv = -drs[i];
+        }
+        if (x == 0) Qout[(size_t)m * K2 + f] = (T)(v / s);
+        A[f] = sq[i] * (dv / s - v * ds / (s * s)) * isq[j];
+    }
+    __syncthreads();
+    // T1 = A U, Bdot = U^T T1: four rows and four columns per thread
+    const int r0 = 4 * (tid / 16), c0 = 4 * (tid % 16);
+    for (int pass = 0; pass < 2; pass++) {
+        const double *L = pass ? Us : A, *M = pass ? T1 : Us;
+        double acc[4][4] = {};
+        for (int k = 0; k < K; k++) {
+            double l[4], c[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) l[i] = pass ? L[k * K + r0 + i] : L[(r0 + i) * K + k];
+            Vec4<double>::load(M + k * K + c0, c);
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) acc[i][j] = fma(l[i], c[j], acc[i][j]);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                if (pass) Bout[((size_t)m * 2 + x) * K2 + (r0 + i) * K + c0 + j] = (T)acc[i][j];
+                else T1[(r0 + i) * K + c0 + j] = acc[i][j];
+            }
+        __syncthreads();
+    }
+}
+
+cudaError_t launch_omega_deriv(bool fp64, const double *keys, const double *U, const double *sq, const double *isq, int nmodels,
+                               void *Q, void *Bdot, cudaStream_t s)
+{
+    if (nmodels <= 0) return cudaSuccess;
+    const size_t smem = sizeof(double) * 3 * K2;
+    const dim3 grid(nmodels, 2);
+    cudaError_t e = fp64 ? cudaFuncSetAttribute(k_omega_deriv<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+                         : cudaFuncSetAttribute(k_omega_deriv<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    if (fp64) k_omega_deriv<double><<<grid, OD_THREADS, smem, s>>>(keys, U, sq, isq, (double *)Q, (double *)Bdot);
+    else k_omega_deriv<float><<<grid, OD_THREADS, smem, s>>>(keys, U, sq, isq, (float *)Q, (float *)Bdot);
+    return cudaGetLastError();
+}
+
+// Codons of each region's leaves, counted (codes above 63 are not): hist [nreg][64].  One CTA per
+// region, a histogram per warp.
+__global__ void __launch_bounds__(256) k_codon_hist(const uint8_t *codes, const int64_t *offs, int nl, unsigned long long *hist)
+{
+    __shared__ uint32_t h[8][K];
+    const int r = blockIdx.x, tid = threadIdx.x;
+    for (int f = tid; f < 8 * K; f += 256) h[f / K][f % K] = 0;
+    __syncthreads();
+    const size_t b1 = (size_t)offs[r + 1] * nl;
+    for (size_t b = (size_t)offs[r] * nl + tid; b < b1; b += 256) {
+        const int c = codes[b];
+        if (c < K) atomicAdd(&h[tid >> 5][c], 1u);
+    }
+    __syncthreads();
+    if (tid < K) {
+        unsigned long long n = 0;
+        for (int w = 0; w < 8; w++) n += h[w][tid];
+        hist[(size_t)r * K + tid] = n;
+    }
+}
+
+cudaError_t launch_codon_hist(const uint8_t *codes, const int64_t *offs, int nreg, int nl, unsigned long long *hist, cudaStream_t s)
+{
+    if (nreg <= 0) return cudaSuccess;
+    k_codon_hist<<<nreg, 256, 0, s>>>(codes, offs, nl, hist);
+    return cudaGetLastError();
+}
+
 }  // namespace pcsf

@@ -163,6 +163,12 @@ int grad_ctas_per_sm(int prec, int nslots, int nl, int nint, int npar);
 // (lam_i - lam_j), t e^{lam_i t} on the diagonal (Frechet derivative of exp in the eigenbasis)
 cudaError_t launch_hform(bool fp64, const PSet *ps, int nps, const double *branch, int nbr, const double *lam,
                          const void *Bdot, void *H, cudaStream_t s);
+// OmegaModel models keys [nmodels][12] with eigenvectors U and sqrt(pi), 1/sqrt(pi): Q row-major and
+// Bdot_x = U^T D^1/2 (dQ/dx) D^-1/2 U, x = kappa, omega, [nmodels][2], in the arithmetic type
+cudaError_t launch_omega_deriv(bool fp64, const double *keys, const double *U, const double *sq, const double *isq, int nmodels,
+                               void *Q, void *Bdot, cudaStream_t s);
+// codon counts of each region's leaves, hist [nreg][64]; offs [nreg + 1] column offsets
+cudaError_t launch_codon_hist(const uint8_t *codes, const int64_t *offs, int nreg, int nl, unsigned long long *hist, cudaStream_t s);
 cudaError_t launch_reduce_grad(const double *gpart, const int32_t *wi_begin, int nreq, int nbr, double *grad,
                                cudaStream_t s);
 
