@@ -92,15 +92,6 @@ size_t ff_smem(int nl, int nint)
     return FS_LV + (((size_t)nl * FF_TC + 15) & ~size_t(15)) + (size_t)nint * (sizeof(SchedNode) + 2) + 16;
 }
 
-// ---- pairs of floats (one 64-bit register pair), elementwise round-to-nearest
-typedef unsigned long long f2;
-__device__ __forceinline__ f2 pk(float x, float y) { f2 d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y)); return d; }
-__device__ __forceinline__ void upk(f2 a, float &x, float &y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a)); }
-__device__ __forceinline__ f2 add2(f2 a, f2 b) { f2 d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-__device__ __forceinline__ f2 sub2(f2 a, f2 b) { f2 d; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) { f2 d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) { f2 d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
-__device__ __forceinline__ f2 neg2(f2 a) { return a ^ 0x8000000080000000ull; }
 // s + e = a + b exactly (Knuth)
 __device__ __forceinline__ void two_sum2(f2 a, f2 b, f2 &s, f2 &e)
 {

@@ -11,8 +11,7 @@
 //   inter_c = beta_p . v_s,   d log z / d t_c = inter_c^T Q v_c / z,   beta_c = P_c^T inter_c.
 //
 // One CTA (256 threads) owns a tile of 32 columns, two CTAs share an SM.  The inside pass is
-// the one of k_prune (internal children's E^T copied one node ahead, leaf rows from global
-// memory) but also stores the partial v_c of every child and the per-column exponents of the
+// the one of k_prune (a node's operands copied one node ahead) but also stores the partial v_c of every child and the per-column exponents of the
 // power-of-two rescaling in a per-CTA global scratch area; the outside pass then walks the
 // schedule in reverse.  A leaf child's partial is one gathered row of E^T plus the identity
 // (P_c[a][s]); with RECOMP the outside pass recomputes it from the leaf state instead of
@@ -145,19 +144,6 @@ __global__ void __launch_bounds__(GR_THREADS, sizeof(T) == 4 ? 2 : 1) k_grad(Gra
         const int ncols = wi.ncols;
         const uint8_t *lg = a.leaves + (size_t)wi.col0 * nl;
         double *gout = a.gpart + ((size_t)w * GR_WARPS + warp) * gstride;    // this warp's sums
-        auto copy_inner = [&](const SchedNode &nx) {
-            constexpr int NV = K2 * sizeof(T) / 16;
-#pragma unroll
-            for (int side = 0; side < 2; side++) {
-                if ((side ? nx.rslot : nx.lslot) < 0) continue;
-                const char *src = reinterpret_cast<const char *>(Pbase + (size_t)(side ? nx.rc : nx.lc) * K2);
-                const uint32_t dst = (uint32_t)__cvta_generic_to_shared(Mat + side * K2);
-                for (int f = tid; f < NV; f += GR_THREADS)
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst + 16 * f), "l"(src + 16 * f)
-                                 : "memory");
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        };
         __syncthreads();   // previous work item finished with shared memory
         for (int f = tid; f < TC * nl; f += GR_THREADS) {
             int c = f / nl, l = f - c * nl;
@@ -166,21 +152,22 @@ __global__ void __launch_bounds__(GR_THREADS, sizeof(T) == 4 ? 2 : 1) k_grad(Gra
         for (int f = tid; f < 2 * TC; f += GR_THREADS) colmax[f] = 0;
 
         // ---------------- inside pass, storing the child partials
-        copy_inner(sched[0]);
+        __syncthreads();       // leaf states ready
+        stage_children<T, TC, CPT, GR_THREADS>(Mat, Pbase, sched[0], lvT, tid);
         for (int ni = 0; ni < a.n_internal; ni++) {
             const SchedNode sn = sched[ni];
             asm volatile("cp.async.wait_all;" ::: "memory");
             __syncthreads();
             T vl[4][CPT], vr[4][CPT];
-            child_partial<T, TC, KAHAN>(Mat, slots, sn.lslot, sn.lc, lvT, a0, c0, vl, -1, Pbase + (size_t)sn.lc * K2);
-            child_partial<T, TC, KAHAN>(Mat + K2, slots, sn.rslot, sn.rc, lvT, a0, c0, vr, -1, Pbase + (size_t)sn.rc * K2);
+            child_partial<T, TC, KAHAN>(Mat, slots, sn.lslot, sn.lc, lvT, a0, c0, vl, -1, true);
+            child_partial<T, TC, KAHAN>(Mat + K2, slots, sn.rslot, sn.rc, lvT, a0, c0, vr, -1, true);
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 if (!RECOMP || sn.lc >= nl) ColStore<T, CPT>::store(V + (vslot(sn.lc) * K + a0 + i) * TC + c0, vl[i]);
                 if (!RECOMP || sn.rc >= nl) ColStore<T, CPT>::store(V + (vslot(sn.rc) * K + a0 + i) * TC + c0, vr[i]);
             }
             __syncthreads();   // Mat and slot reads done
-            if (ni + 1 < a.n_internal) copy_inner(sched[ni + 1]);
+            if (ni + 1 < a.n_internal) stage_children<T, TC, CPT, GR_THREADS>(Mat, Pbase, sched[ni + 1], lvT, tid);
             MU *cm = colmax + (ni & 1) * TC, *cm_next = colmax + ((ni + 1) & 1) * TC;
             if (tid < TC) cm_next[tid] = 0;
 #pragma unroll

@@ -589,22 +589,6 @@ __global__ void __launch_bounds__(PruneThreads<TC>::N) k_prune(PruneArgs a)
         const float *dlo = (sizeof(T) == 4 && a.dlo) ? a.dlo + (size_t)rq.pset * a.nbr * K : nullptr;
         const int ncols = wi.ncols;
         const uint8_t *lg = a.leaves + (size_t)wi.col0 * nl;
-        // E^T of a node's internal children into shared memory, copied asynchronously one
-        // node ahead (issued once the previous node's contraction has released the
-        // buffers); leaf children read their rows from global memory instead
-        auto copy_inner = [&](const SchedNode &nx) {
-            constexpr int NV = K2 * sizeof(T) / 16;
-#pragma unroll
-            for (int side = 0; side < 2; side++) {
-                if ((side ? nx.rslot : nx.lslot) < 0) continue;
-                const char *src = reinterpret_cast<const char *>(Pbase + (size_t)(side ? nx.rc : nx.lc) * K2);
-                const uint32_t dst = (uint32_t)__cvta_generic_to_shared(Et + side * K2);
-                for (int f = tid; f < NV; f += THREADS)
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst + 16 * f), "l"(src + 16 * f)
-                                 : "memory");
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        };
         __syncthreads();   // previous work item finished with shared memory
         for (int f = tid; f < TC * nl; f += THREADS) {
             int c = f / nl, l = f - c * nl;
@@ -615,8 +599,11 @@ __global__ void __launch_bounds__(PruneThreads<TC>::N) k_prune(PruneArgs a)
         // dither keys are the column's position within its region, so that results
         // do not depend on where a region sits in the batch
         const int64_t dcol0 = dith ? (int64_t)(uint32_t)((uint32_t)wi.col0 - rq.start) : -1;
+        __syncthreads();       // leaf states (and ltab) ready
+        // a node's operands are copied one node ahead (issued once the previous node's contraction
+        // has released the buffers)
+        stage_children<T, TC, CPT, THREADS>(Et, Pbase, sched[0], lvT, tid);
         if (dith) {
-            __syncthreads();   // ltab ready
             for (int c = tid; c < TC; c += THREADS) {
                 double sd = 0.0;
                 for (int l = 0; l < nl; l++) sd += ltab[dither_k(dcol0 + c, l)];
@@ -624,18 +611,17 @@ __global__ void __launch_bounds__(PruneThreads<TC>::N) k_prune(PruneArgs a)
             }
         }
 
-        copy_inner(sched[0]);
         for (int ni = 0; ni < a.n_internal; ni++) {
             const SchedNode sn = sched[ni];
             asm volatile("cp.async.wait_all;" ::: "memory");
             __syncthreads();
             T vl[4][CPT], vr[4][CPT];
-            child_partial<T, TC, KAHAN, CPT>(Et, slots, sn.lslot, sn.lc, lvT, a0, c0, vl, dcol0, Pbase + (size_t)sn.lc * K2,
+            child_partial<T, TC, KAHAN, CPT>(Et, slots, sn.lslot, sn.lc, lvT, a0, c0, vl, dcol0, true,
                                         dlo ? dlo + (size_t)sn.lc * K : nullptr);
-            child_partial<T, TC, KAHAN, CPT>(Et + K2, slots, sn.rslot, sn.rc, lvT, a0, c0, vr, dcol0,
-                                        Pbase + (size_t)sn.rc * K2, dlo ? dlo + (size_t)sn.rc * K : nullptr);
+            child_partial<T, TC, KAHAN, CPT>(Et + K2, slots, sn.rslot, sn.rc, lvT, a0, c0, vr, dcol0, true,
+                                        dlo ? dlo + (size_t)sn.rc * K : nullptr);
             __syncthreads();
-            if (ni + 1 < a.n_internal) copy_inner(sched[ni + 1]);   // E^T buffers are free again
+            if (ni + 1 < a.n_internal) stage_children<T, TC, CPT, THREADS>(Et, Pbase, sched[ni + 1], lvT, tid);   // buffers free again
             MU *cm = colmax + (ni & 1) * TC;
             MU *cm_next = colmax + ((ni + 1) & 1) * TC;
             if (tid < TC) cm_next[tid] = 0;

@@ -122,23 +122,15 @@ __global__ void __launch_bounds__(OS_THREADS) k_outside(OutsideArgs a)
             for (int f = tid; f < TC; f += OS_THREADS) colmax[f] = 0;
 
             // ---------------- inside pass, storing the child partials and the node alphas
+            __syncthreads();   // leaf states ready
+            stage_children<T, TC, CPT, OS_THREADS>(Mat, Pbase, sched[0], lvT, tid);
             for (int ni = 0; ni < a.n_internal; ni++) {
                 const SchedNode sn = sched[ni];
-                {
-                    const float4 *gl = reinterpret_cast<const float4 *>(Pbase + (size_t)sn.lc * K2);
-                    const float4 *gr = reinterpret_cast<const float4 *>(Pbase + (size_t)sn.rc * K2);
-                    float4 *sl = reinterpret_cast<float4 *>(Mat);
-                    float4 *sr = reinterpret_cast<float4 *>(Mat + K2);
-                    constexpr int NV = K2 * sizeof(T) / 16;
-                    for (int f = tid; f < NV; f += OS_THREADS) {
-                        sl[f] = __ldg(gl + f);
-                        sr[f] = __ldg(gr + f);
-                    }
-                }
+                asm volatile("cp.async.wait_all;" ::: "memory");
                 __syncthreads();
                 T vl[4][CPT], vr[4][CPT];
-                child_partial<T, TC, KAHAN>(Mat, slots, sn.lslot, sn.lc, lvT, a0, c0, vl);
-                child_partial<T, TC, KAHAN>(Mat + K2, slots, sn.rslot, sn.rc, lvT, a0, c0, vr);
+                child_partial<T, TC, KAHAN>(Mat, slots, sn.lslot, sn.lc, lvT, a0, c0, vl, -1, true);
+                child_partial<T, TC, KAHAN>(Mat + K2, slots, sn.rslot, sn.rc, lvT, a0, c0, vr, -1, true);
 #pragma unroll
                 for (int i = 0; i < 4; i++)
 #pragma unroll
@@ -147,6 +139,7 @@ __global__ void __launch_bounds__(OS_THREADS) k_outside(OutsideArgs a)
                         V[((size_t)sn.rc * K + a0 + i) * TC + c0 + cc] = vr[i][cc];
                     }
                 __syncthreads();   // Mat and slot reads done
+                if (ni + 1 < a.n_internal) stage_children<T, TC, CPT, OS_THREADS>(Mat, Pbase, sched[ni + 1], lvT, tid);
 #pragma unroll
                 for (int cc = 0; cc < CPT; cc++) {
                     T mx = (T)0;

@@ -6,6 +6,17 @@
 
 namespace pcsf {
 
+// Pairs of floats (one 64-bit register pair), elementwise round-to-nearest: two lanes' work in one
+// issue slot at the scalar rate (measured 127 lanes per clock and SM either way).
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pk(float x, float y) { f2 d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y)); return d; }
+__device__ __forceinline__ void upk(f2 a, float &x, float &y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a)); }
+__device__ __forceinline__ f2 add2(f2 a, f2 b) { f2 d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ f2 sub2(f2 a, f2 b) { f2 d; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) { f2 d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) { f2 d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
+__device__ __forceinline__ f2 neg2(f2 a) { return a ^ 0x8000000080000000ull; }
+
 template <typename T> struct Vec4;
 template <> struct Vec4<float> {
     static __device__ inline void load(const float *p, float v[4])
@@ -178,8 +189,9 @@ __device__ __forceinline__ double scale2(double x, int e)
 // with Kahan's correction (about a ninth of the plain bias at 1.5 operations per
 // product instead of 5).
 // CPT: columns per thread (TC / 16 with 256 threads of 4 states each).
+// FP32 with two or four columns per thread works on pairs of columns (contract_pairs).
 template <typename T, int TC, int COMP, int CPT = TC / 16>
-__device__ inline void contract(const T *M, const T *X, int a0, int c0, T out[4][CPT])
+__device__ inline void contract_scalar(const T *M, const T *X, int a0, int c0, T out[4][CPT])
 {
     T comp[4][CPT];
 #pragma unroll
@@ -252,6 +264,98 @@ __device__ inline void contract(const T *M, const T *X, int a0, int c0, T out[4]
     }
 }
 
+// The same sums on pairs of columns: bit for bit the scalar values (each lane rounds as the scalar
+// operation), with half of the issue slots for products and corrections.  The loop is issue-bound:
+// 208 instructions per 8 products of a 4 x 4 block before, 64 + 32 paired ones, 16 loads and the
+// duplication of E's entries now.  The correction is kept negated (a + (-c) rounds as a - c).
+// Measured with the staged leaf rows, blocked compensation, 58 leaves, 141,741 columns: 3.12 ->
+// 2.68 ms; what bounds it now is the mix of FP32 issue, load latency and three barriers a node.
+// entry(j, e): E's four entries of step j.
+template <int TC, int COMP, int CPT, typename Entry>
+__device__ inline void contract_pairs(Entry entry, const float *X, int c0, float out[4][CPT])
+{
+    constexpr int NP = CPT / 2;
+    f2 s[4][NP], nc[4][NP];
+    auto load_x = [&](int j, f2 x[NP]) {
+        float v[CPT];
+        ColLoad<float, CPT>::load(X + j * TC + c0, v);
+#pragma unroll
+        for (int k = 0; k < NP; k++) x[k] = pk(v[2 * k], v[2 * k + 1]);
+    };
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int k = 0; k < NP; k++) s[i][k] = nc[i][k] = 0ull;
+    if (COMP == 2) {
+        auto block = [&](int jb, f2 g[4][NP]) {
+#pragma unroll
+            for (int j = jb; j < jb + 8; j++) {
+                float e[4];
+                f2 x[NP];
+                entry(j, e);
+                load_x(j, x);
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const f2 ee = pk(e[i], e[i]);
+#pragma unroll
+                    for (int k = 0; k < NP; k++) g[i][k] = (j == jb) ? mul2(ee, x[k]) : fma2(ee, x[k], g[i][k]);
+                }
+            }
+        };
+        block(0, s);
+#pragma unroll        // (rolled, each block began with its loads' latency: 2.94 -> 2.68 ms)
+        for (int jb = 8; jb < K; jb += 8) {
+            f2 g[4][NP];
+            block(jb, g);
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int k = 0; k < NP; k++) {
+                    const f2 y = add2(g[i][k], nc[i][k]);
+                    const f2 t = add2(s[i][k], y);
+                    nc[i][k] = sub2(y, sub2(t, s[i][k]));
+                    s[i][k] = t;
+                }
+        }
+    } else {
+#pragma unroll 4
+        for (int j = 0; j < K; j++) {
+            float e[4];
+            f2 x[NP];
+            entry(j, e);
+            load_x(j, x);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const f2 ee = pk(e[i], e[i]);
+#pragma unroll
+                for (int k = 0; k < NP; k++) {
+                    if (COMP == 1) {
+                        const f2 y = fma2(ee, x[k], nc[i][k]);
+                        const f2 t = add2(s[i][k], y);
+                        nc[i][k] = sub2(y, sub2(t, s[i][k]));
+                        s[i][k] = t;
+                    } else {
+                        s[i][k] = fma2(ee, x[k], s[i][k]);
+                    }
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int k = 0; k < NP; k++) upk(COMP ? add2(s[i][k], nc[i][k]) : s[i][k], out[i][2 * k], out[i][2 * k + 1]);
+}
+
+template <typename T, int TC, int COMP, int CPT = TC / 16>
+__device__ inline void contract(const T *M, const T *X, int a0, int c0, T out[4][CPT])
+{
+    if constexpr (sizeof(T) == 4 && CPT % 2 == 0)
+        contract_pairs<TC, COMP, CPT>([&](int j, float e[4]) { Vec4<float>::load(M + j * K + a0, e); }, X, c0, out);
+    else
+        contract_scalar<T, TC, COMP, CPT>(M, X, a0, c0, out);
+}
+
 // out[i][cc] = sum_j N[a0+i][j] * X[j][c0+cc] with row a of N at N + a * LDN: contract() of the
 // transposed matrix (the same products in the same order, so the same values), for the outside
 // pass, which multiplies by E^T as it is stored.  Four consecutive j of a row come in one load;
@@ -261,6 +365,20 @@ template <typename T, int TC, int COMP>
 __device__ inline void contract_rows(const T *N, const T *X, int a0, int c0, T out[4][TC / 16])
 {
     constexpr int CPT = TC / 16;
+    if constexpr (sizeof(T) == 4 && CPT % 2 == 0) {
+        float r[4][4];       // four steps of the thread's four rows
+        contract_pairs<TC, COMP, CPT>(
+            [&](int j, float e[4]) {
+                if (j % 4 == 0) {
+#pragma unroll
+                    for (int i = 0; i < 4; i++) Vec4<float>::load(N + (a0 + i) * LDN + j, r[i]);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; i++) e[i] = r[i][j % 4];
+            },
+            X, c0, out);
+        return;
+    }
     T comp[4][CPT];
 #pragma unroll
     for (int i = 0; i < 4; i++)
@@ -340,12 +458,44 @@ __device__ inline void stage_rows(T *dst, const T *src, int tid)
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
+// What the children of a node need, into the two buffers at Et (K2 entries each), asynchronously
+// (committed; the caller waits): an internal child's E^T as it is, and for a leaf child the row of
+// its E^T that each tile column selects, one row of 64 states per column (the column's row read in
+// one piece; a thread that gathers its four states from global memory touches a line per column:
+// two thirds of the kernel's L1 wavefronts).  The 16-byte chunks of a row are permuted by XOR with
+// the number of the thread column that reads it, so that those reads are free of conflicts.
+template <typename T, int TC, int CPT, int THREADS>
+__device__ inline void stage_children(T *Et, const T *Pbase, const SchedNode &nx, const uint8_t *lvT, int tid)
+{
+    constexpr int V = 16 / sizeof(T), NC = K / V;
+#pragma unroll
+    for (int side = 0; side < 2; side++) {
+        const int child = side ? nx.rc : nx.lc;
+        const T *src = Pbase + (size_t)child * K2;
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(Et + side * K2);
+        if ((side ? nx.rslot : nx.lslot) < 0) {
+            for (int f = tid; f < TC * NC; f += THREADS) {
+                const int col = f / NC, ch = f % NC;
+                const int s = lvT[child * TC + col];
+                if (s < K)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
+                                 :: "r"(dst + (uint32_t)(col * NC + (ch ^ (4 / V * ((col / CPT) & 15)))) * 16),
+                                    "l"(src + s * K + ch * V) : "memory");
+            }
+        } else {
+            for (int f = tid; f < K * NC; f += THREADS)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst + 16 * f), "l"(src + f * V) : "memory");
+        }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
 // Partial of child c at its parent: v[a] = alpha_c[a] + sum_j E_c[a][j] alpha_c[j]
 // (internal child, slot >= 0; Et = E_c^T) or the gather v[a] = P_c[a][s] of a
 // leaf in state s (1 for a marginalised leaf: P rows sum to 1).
 template <typename T, int TC, int KAHAN, int CPT = TC / 16>
 __device__ inline void child_partial(const T *Et, const T *slots, int slot, int leaf, const uint8_t *lvT, int a0,
-                                     int c0, T v[4][CPT], int64_t dither_col0 = -1, const T *leaf_g = nullptr,
+                                     int c0, T v[4][CPT], int64_t dither_col0 = -1, bool staged = false,
                                      const float *dlo = nullptr)
 {
     // dlo (may be null): the low parts of this branch's diag(E), added to the diagonal
@@ -353,15 +503,18 @@ __device__ inline void child_partial(const T *Et, const T *slots, int slot, int 
     // at this node repeats identically, so over a long region it adds up coherently
     // (2-3e-3 dB over 10,000 codons at rho = 3 without it)
     if (slot < 0) {
-        if (leaf_g) {   // the leaf's E^T rows straight from global memory (4 states per column)
+        if (staged) {   // the columns' rows of the leaf's E^T, as stage_children placed them
+            constexpr int V = 16 / sizeof(T);
+            const int ch = (a0 / V) ^ (4 / V * ((c0 / CPT) & 15));
 #pragma unroll
             for (int cc = 0; cc < CPT; cc++) {
                 const int s = lvT[leaf * TC + c0 + cc];
                 const T c = (dither_col0 >= 0) ? (T)(1.0f + (float)dither_k(dither_col0 + c0 + cc, leaf) * (1.0f / 256.0f))
                                                : (T)1;
                 T e[4];
-                Vec4<T>::load(leaf_g + (size_t)(s < K ? s : 0) * K + a0, e);
-                const T lo_s = dlo ? (T)dlo[s < K ? s : 0] : (T)0;
+                Vec4<T>::load(Et + (c0 + cc) * K + ch * V, e);
+                // only the thread that holds state s needs the diagonal's low part
+                const T lo_s = (dlo && s >= a0 && s < a0 + 4 && s < K) ? (T)dlo[s] : (T)0;
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
                     const int a = a0 + i;
