@@ -88,7 +88,7 @@ def test_small_pruning_tiles(name, prec):
     ps, offs, leaves = _regions(name, lengths)
     eng = P.Engine(ps.tree, ps.S_c, ps.pi_c, ps.S_n, ps.pi_n, precision=prec)
     n, L = len(lengths), int(offs[-1])
-    reps = 12                                              # 7,700 columns: past the small tiles
+    reps = 40                                              # 25,600 columns: past the small tiles (FP64: 19,456)
     big = eng.batch(np.concatenate([[0]] + [offs[1:] + k * L for k in range(reps)]), np.tile(leaves, (reps, 1)))
     few = eng.batch(offs, leaves)
     for rho in (0.3, 2.0):
