@@ -218,23 +218,40 @@ cudaError_t launch_jacobi(const double *A, double *U, double *lam, int *status, 
 // Output is E^T: Pbuf[(r*nbr + b)*K2 + j*K + i] = E[i][j].
 
 constexpr int PF_THREADS = 256;
-constexpr int PF_BRANCHES = 4;   // most branches per CTA (the eigenvectors are staged once)
+constexpr int PF_BRANCHES = 2;   // most branches per CTA (the eigenvectors are staged once)
 constexpr int PF_SPREAD = 2 * 4 * 152;   // FP32 matrices of a launch up to which each gets its own CTA
 
+// shared memory (dynamic): U^T, with FP64 U^T times the coefficients, per branch E^T and the coefficients
+template <typename T> __host__ __device__ constexpr size_t pform_smem(int per_cta)
+{
+    return sizeof(T) * ((size_t)(sizeof(T) == 8 ? 2 : 1) * K2 + 2 * K + (size_t)per_cta * (K2 + K)) +
+           sizeof(double) * (size_t)per_cta * K;
+}
+
+// The branches of a CTA go through each phase together: coefficients (a thread per branch and
+// eigenvalue), products (the whole CTA, branch after branch), the row rule (a thread per branch and
+// row: its compensated sum is a chain of 64 dependent steps, which one branch at a time left on two
+// of the eight warps) and the stores.  U^T is stored with the 16-byte chunks of row m permuted by
+// XOR with m mod 16, so that neither the transposing stores nor the loads of a product step
+// conflict by more than 4.  What bounds the FP32 form is the load/store pipe (64 % of its
+// wavefronts at four branches per CTA) and FP32 issue: E^T stays in the layout of the grid and of
+// the output from the asynchronous copy of E(t_g) to the store, and lanes run along its rows.
+// Measured, 301 P sets of 58 leaves: 0.95 ms with E row-major and one branch at a time, 0.82 with
+// this, 0.75 with two branches per CTA (four CTAs per SM) instead of four.
 template <typename T>
 __global__ void __launch_bounds__(PF_THREADS) k_pform(const PSet *ps, const double *branch, int nbr,
                                                        DevModels m, T *Pbuf, int32_t *status_key, int raw,
                                                        float *Bop, int bop_nl, float *dlo, int per_cta)
 {
+    constexpr bool fp32 = sizeof(T) == 4;
     extern __shared__ __align__(16) unsigned char psm[];
-    T *UT = reinterpret_cast<T *>(psm);     // [K][K]   UT[m][j] = U[j][m]
-    T *UeT = UT + K2;                         // [K][K]   UeT[m][i] = U[i][m] * coef_m
-    T *Es = UeT + K2;                         // [K][K+1] E[i][j]
-    T *sqT = Es + K * (K + 1);                // [K]
+    T *UT = reinterpret_cast<T *>(psm);     // [K][K]   UT[m][j] = U[j][m] (chunks permuted)
+    T *UeT = UT + K2;                         // [K][K]   FP64: UeT[m][i] = U[i][m] * coef_m
+    T *sqT = UT + (fp32 ? 1 : 2) * K2;        // [K]
     T *isqT = sqT + K;                        // [K]
-    double *ex = reinterpret_cast<double *>(isqT + K);   // [K] expm1(lam t): row-sum identity
-    double *cf = ex + K;                                 // [K] GEMM coefficients
-    __shared__ T cfT[K];                                 // the same in the storage type
+    T *cfT = isqT + K;                        // [per_cta][K] product coefficients
+    double *ex = reinterpret_cast<double *>(cfT + per_cta * K);   // [per_cta][K] expm1(lam t): row-sum identity
+    T *Eall = reinterpret_cast<T *>(ex + per_cta * K);            // [per_cta][K][K] E^T: element (j, i) = E[i][j]
     __shared__ int mode_s[PF_BRANCHES], grid_s[PF_BRANCHES];
     const int tid = threadIdx.x;
     const int r = blockIdx.y;
@@ -245,24 +262,24 @@ __global__ void __launch_bounds__(PF_THREADS) k_pform(const PSet *ps, const doub
     const double *lam = m.lam + md * K;
     const double *isq = m.isq + md * K;
     const double *wrow = m.wrow + md * K;
-    const bool fp32 = sizeof(T) == 4;
+    const int b0 = blockIdx.x * per_cta, nb = min(per_cta, nbr - b0);
+    auto chunk = [](int c, int mm) { return 4 * (c ^ (mm & 15)); };   // first entry of chunk c (4 entries) of row mm
 
     for (int f = tid; f < K2; f += PF_THREADS) {
         int j = f / K, mm = f % K;   // U[j][mm]
-        UT[mm * K + j] = fp32 ? (T)Uf[f] : (T)U[f];
+        UT[mm * K + chunk(j >> 2, mm) + (j & 3)] = fp32 ? (T)Uf[f] : (T)U[f];
     }
     if (tid < K) {
         sqT[tid] = (T)m.sq[md * K + tid];
         isqT[tid] = (T)isq[tid];
     }
-    const int ty = tid / 16, tx = tid % 16;
+    const int ty = tid % 16, tx = tid / 16;     // rows 4 ty .. (lanes), columns 4 tx .. of E
     // per branch of this CTA, in parallel (one thread each; FP64 is a narrow pipe here):
     // 0: direct eigen formula (FP64);  1: t == 0;  2: Taylor below the grid;  3: grid correction
-    if (tid < per_cta) {
-        const int b = blockIdx.x * per_cta + tid;
+    if (tid < nb) {
         int mode = 0, g = 0;
-        if (b < nbr && fp32 && m.grid_n > 0) {
-            const double t = rq.rho * branch[b];
+        if (fp32 && m.grid_n > 0) {
+            const double t = rq.rho * branch[b0 + tid];
             if (t == 0.0) mode = 1;
             else if (t < m.grid_t[0]) mode = 2;
             else {
@@ -277,100 +294,136 @@ __global__ void __launch_bounds__(PF_THREADS) k_pform(const PSet *ps, const doub
         mode_s[tid] = mode;
         grid_s[tid] = g;
     }
-    for (int bi = 0; bi < per_cta; bi++) {
-        const int b = blockIdx.x * per_cta + bi;
-        if (b >= nbr) break;                       // uniform across the block
-        const double t = rq.rho * branch[b];
-        __syncthreads();                           // UT and the branch table ready / previous branch done with smem
-        const int mode = mode_s[bi];
-        if (tid < K) {
-            // ex feeds the row-sum check, which needs it only where w_m != 0
-            // (the stationary direction); the FP32 modes therefore spend one
-            // FP64 expm1 per branch instead of 64 (FP64 is a narrow pipe here).
-            if (mode == 0) {
-                ex[tid] = expm1(lam[tid] * t);
-                cf[tid] = ex[tid];
-                cfT[tid] = (T)cf[tid];
-            } else {
-                ex[tid] = (wrow[tid] != 0.0) ? (double)expm1f((float)(lam[tid] * t)) : 0.0;   // row-sum check only
-                if (mode == 3) {
-                    // e^{lam t_g} (tabulated) * expm1(lam (t - t_g)) in FP32: the
-                    // coefficient is rounded to FP32 for the GEMM in any case
-                    const double h = t - m.grid_t[grid_s[bi]];
-                    const float eg = m.grid_eg[((size_t)md * m.grid_n + grid_s[bi]) * K + tid];
-                    cf[tid] = (double)(eg * expm1f((float)(lam[tid] * h)));
-                    cfT[tid] = (T)cf[tid];
-                }
+    __syncthreads();
+    // E(t_g), as it is stored, into the place of E^T
+    for (int bi = 0; bi < nb; bi++)
+        if (mode_s[bi] == 3) {
+            const float *base = m.gridT + ((size_t)md * m.grid_n + grid_s[bi]) * K2;
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(Eall + (size_t)bi * K2);
+            for (int f = tid; f < K2 / 4; f += PF_THREADS)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst + 16 * f), "l"(base + 4 * f) : "memory");
+        }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    for (int f = tid; f < nb * K; f += PF_THREADS) {
+        const int bi = f / K, mm = f % K, mode = mode_s[bi];
+        const double t = rq.rho * branch[b0 + bi];
+        // ex feeds the row-sum check, which needs it only where w_m != 0
+        // (the stationary direction); the FP32 modes therefore spend one
+        // FP64 expm1 per branch instead of 64 (FP64 is a narrow pipe here).
+        if (mode == 0) {
+            ex[f] = expm1(lam[mm] * t);
+            cfT[f] = (T)ex[f];
+        } else {
+            ex[f] = (wrow[mm] != 0.0) ? (double)expm1f((float)(lam[mm] * t)) : 0.0;   // row-sum check only
+            if (mode == 3) {
+                // e^{lam t_g} (tabulated) * expm1(lam (t - t_g)) in FP32: the
+                // coefficient is rounded to FP32 for the GEMM in any case
+                const double h = t - m.grid_t[grid_s[bi]];
+                const float eg = m.grid_eg[((size_t)md * m.grid_n + grid_s[bi]) * K + mm];
+                cfT[f] = (T)(eg * expm1f((float)(lam[mm] * h)));
             }
         }
-        __syncthreads();
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    for (int bi = 0; bi < nb; bi++) {
+        T *Es = Eall + (size_t)bi * K2;
+        const int mode = mode_s[bi];
+        const double t = rq.rho * branch[b0 + bi];
         if (mode == 0 || mode == 3) {
-            for (int f = tid; f < K2; f += PF_THREADS) {
-                int mm = f / K;
-                UeT[f] = UT[f] * cfT[mm];
-            }
-            __syncthreads();
-            // E(t_g) (stored transposed) for this thread's 4 x 4 block, loaded before the
-            // GEMM: one 16-byte load per column jj (rows 4 ty .. 4 ty + 3)
-            float gb[4][4];
-            if (mode == 3) {
-                const float *base = m.gridT + ((size_t)md * m.grid_n + grid_s[bi]) * K2;
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const float4 q = __ldg(reinterpret_cast<const float4 *>(base + (size_t)(4 * tx + j) * K + 4 * ty));
-                    gb[j][0] = q.x; gb[j][1] = q.y; gb[j][2] = q.z; gb[j][3] = q.w;
-                }
+            const T *cf = cfT + bi * K;
+            if (!fp32) {
+                if (bi) __syncthreads();
+                for (int f = tid; f < K2; f += PF_THREADS) UeT[f] = UT[f] * cf[f / K];
+                __syncthreads();
             }
             T acc[4][4];
+            if constexpr (fp32) {
+                f2 s2[4][2];
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+                for (int i = 0; i < 4; i++) s2[i][0] = s2[i][1] = 0ull;
+#pragma unroll 4
+                for (int mm = 0; mm < K; mm++) {
+                    float a[4], bb[4];
+                    const float c = cf[mm];
+                    Vec4<float>::load(UT + mm * K + chunk(ty, mm), a);
+                    Vec4<float>::load(UT + mm * K + chunk(tx, mm), bb);
+                    const f2 b01 = pk(bb[0], bb[1]), b23 = pk(bb[2], bb[3]);
 #pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = (T)0;
-            for (int mm = 0; mm < K; mm++) {
-                T a[4], bb[4];
-                Vec4<T>::load(UeT + mm * K + 4 * ty, a);
-                Vec4<T>::load(UT + mm * K + 4 * tx, bb);
+                    for (int i = 0; i < 4; i++) {
+                        const float x = __fmul_rn(a[i], c);
+                        const f2 xx = pk(x, x);
+                        s2[i][0] = fma2(xx, b01, s2[i][0]);
+                        s2[i][1] = fma2(xx, b23, s2[i][1]);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    upk(s2[i][0], acc[i][0], acc[i][1]);
+                    upk(s2[i][1], acc[i][2], acc[i][3]);
+                }
+            } else {
 #pragma unroll
                 for (int i = 0; i < 4; i++)
 #pragma unroll
-                    for (int j = 0; j < 4; j++) acc[i][j] += a[i] * bb[j];
+                    for (int j = 0; j < 4; j++) acc[i][j] = (T)0;
+                for (int mm = 0; mm < K; mm++) {
+                    T a[4], bb[4];
+                    Vec4<T>::load(UeT + mm * K + chunk(ty, mm), a);
+                    Vec4<T>::load(UT + mm * K + chunk(tx, mm), bb);
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+#pragma unroll
+                        for (int j = 0; j < 4; j++) acc[i][j] += a[i] * bb[j];
+                }
             }
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int j = 0; j < 4; j++) {
+                const int jj = 4 * tx + j;
+                T *e = Es + jj * K + 4 * ty, g[4], v[4];
+                if (mode == 3) Vec4<T>::load(e, g);
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    int ii = 4 * ty + i, jj = 4 * tx + j;
-                    T v = acc[i][j] * sqT[jj] * isqT[ii];
-                    if (mode == 3) v += (T)gb[j][i];
-                    Es[ii * (K + 1) + jj] = v;
+                for (int i = 0; i < 4; i++) {
+                    v[i] = acc[i][j] * sqT[jj] * isqT[4 * ty + i];
+                    if (mode == 3) v[i] += g[i];
                 }
+                ColStore<T, 4>::store(e, v);
+            }
         } else {
             const float *Qf = m.Qf + (size_t)md * K2, *Q2f = m.Q2f + (size_t)md * K2;
             const T tt = (T)t, h = (T)(0.5 * t * t);
             for (int f = tid; f < K2; f += PF_THREADS) {
                 int i = f / K, j = f % K;
-                Es[i * (K + 1) + j] = (mode == 1) ? (T)0 : tt * (T)Qf[f] + h * (T)Q2f[f];
+                Es[j * K + i] = (mode == 1) ? (T)0 : tt * (T)Qf[f] + h * (T)Q2f[f];
             }
         }
-        __syncthreads();
-        if (tid < K && !raw) {
-            const int i = tid;
-            // raw row sum - 1, in FP64 through the eigensystem
-            const double rs = rowsum_minus_one(m, md, i, ex);
-            // the diagonal is the compensated sum of the stored (rounded)
-            // off-diagonal entries, so every stored row of P = I + E sums to 1
-            // to within one rounding of the diagonal; a plain FP32 sum here
-            // biases lpr by ~1e-4 nats per 3000 codons at rho = 1.  Branch-free in
-            // j: i differs per lane, and a branch on j == i would split the warp.
-            bool neg = false;
-            T diag = (T)0, dc = (T)0;
-            const T ntol = (T)(-m.tol), dtol = (T)(-1.0 - m.tol);
-            for (int j = 0; j < K; j++) {
+    }
+    __syncthreads();
+    if (tid < nb * K && !raw) {
+        const int bi = tid / K, i = tid % K, b = b0 + bi;
+        T *row = Eall + (size_t)bi * K2 + i;      // entry j at row[j * K]
+        // raw row sum - 1, in FP64 through the eigensystem
+        const double rs = rowsum_minus_one(m, md, i, ex + bi * K);
+        // the diagonal is the compensated sum of the stored (rounded)
+        // off-diagonal entries, so every stored row of P = I + E sums to 1
+        // to within one rounding of the diagonal; a plain FP32 sum here
+        // biases lpr by ~1e-4 nats per 3000 codons at rho = 1.  Branch-free in
+        // j: i differs per lane, and a branch on j == i would split the warp.
+        bool neg = false;
+        T diag = (T)0, dc = (T)0;
+        const T ntol = (T)(-m.tol), dtol = (T)(-1.0 - m.tol);
+        for (int j0 = 0; j0 < K; j0 += 8) {
+            T x8[8];           // loaded ahead of the stores below
+#pragma unroll
+            for (int k = 0; k < 8; k++) x8[k] = row[(j0 + k) * K];
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const int j = j0 + k;
                 const bool dj = (j == i);
-                const T x0 = Es[i * (K + 1) + j];
+                const T x0 = x8[k];
                 neg |= dj ? (x0 < dtol) : (x0 < ntol);   // diagonal: x + 1 < -tol
                 const T x = (x0 < (T)0) ? (T)0 : x0;      // an off-diagonal negative within tol becomes 0
-                if (!dj && x != x0) Es[i * (K + 1) + j] = x;
+                if (!dj && x != x0) row[j * K] = x;
                 if (fp32) {           // Kahan: diag -= x
                     const T y = -x - dc;
                     const T tt = diag + y;
@@ -381,25 +434,27 @@ __global__ void __launch_bounds__(PF_THREADS) k_pform(const PSet *ps, const doub
                     diag = dj ? diag : diag - x;
                 }
             }
-            if (neg) status_min(status_key + r, b, i, PCSF_ENEGP);
-            else if (fabs(rs) > m.tol) status_min(status_key + r, b, i, PCSF_EROWSUM);
-            else if (!(diag > (T)-1)) status_min(status_key + r, b, i, PCSF_EDIAG);
-            // the sum is diag - dc to second order: its low part for the pruning kernel
-            if (fp32 && dlo) dlo[((size_t)r * nbr + b) * K + i] = (float)(-dc);
-            Es[i * (K + 1) + i] = diag;
         }
-        __syncthreads();
+        if (neg) status_min(status_key + r, b, i, PCSF_ENEGP);
+        else if (fabs(rs) > m.tol) status_min(status_key + r, b, i, PCSF_EROWSUM);
+        else if (!(diag > (T)-1)) status_min(status_key + r, b, i, PCSF_EDIAG);
+        // the sum is diag - dc to second order: its low part for the pruning kernel
+        if (fp32 && dlo) dlo[((size_t)r * nbr + b) * K + i] = (float)(-dc);
+        row[i * K] = diag;
+    }
+    __syncthreads();
+    for (int bi = 0; bi < nb; bi++) {
+        const int b = b0 + bi;
+        const T *Es = Eall + (size_t)bi * K2;
         T *out = Pbuf + ((size_t)r * nbr + b) * K2;
-        for (int f = tid; f < K2; f += PF_THREADS) {
-            int j = f / K, i = f % K;
-            out[f] = Es[i * (K + 1) + j];
-        }
+        for (int f = tid; f < (int)(K2 * sizeof(T) / 16); f += PF_THREADS)
+            reinterpret_cast<uint4 *>(out)[f] = reinterpret_cast<const uint4 *>(Es)[f];
         if (fp32 && Bop && b >= bop_nl) {      // branch above an internal node: tensor-core operand too
             float *dst = Bop + ((size_t)r * (nbr - bop_nl) + (b - bop_nl)) * 2 * K2;
             for (int f = tid; f < K2 / 4; f += PF_THREADS) {
                 const int a = f & (K - 1), q = f >> 6;
-                const T *row = Es + a * (K + 1) + 4 * q;
-                bop_store(dst, a, q, make_float4((float)row[0], (float)row[1], (float)row[2], (float)row[3]));
+                const T *col = Es + 4 * q * K + a;
+                bop_store(dst, a, q, make_float4((float)col[0], (float)col[K], (float)col[2 * K], (float)col[3 * K]));
             }
         }
     }
@@ -409,23 +464,21 @@ cudaError_t launch_pform(bool fp64, const PSet *req, int nreq, const double *bra
                          void *Pbuf, int32_t *status_key, cudaStream_t s, bool raw, float *bop, int bop_nl, float *dlo)
 {
     if (nreq <= 0) return cudaSuccess;
-    // Four branches per CTA share the staged eigenvectors.  One per CTA where that staging is
+    // Two branches per CTA share the staged eigenvectors.  One per CTA where that staging is
     // nothing beside the product (FP64 runs at 1/64 of the FP32 rate: ~70 us per branch) and
-    // for short FP32 launches, which four would leave on a part of the SMs.  Measured: FP64,
+    // for short FP32 launches, which more would leave on a part of the SMs.  Measured: FP64,
     // 24 P sets of 29 leaves 0.95 -> 0.69 ms, six of 12 leaves 0.36 -> 0.13 ms; FP32, two P
     // sets of 12 leaves 39 -> 17 us.
     const int per_cta = (fp64 || (int64_t)nreq * nbr <= PF_SPREAD) ? 1 : PF_BRANCHES;
     dim3 grid((nbr + per_cta - 1) / per_cta, nreq);
     if (fp64) {
-        size_t smem = sizeof(double) * (2 * K2 + K * (K + 1) + 4 * K);
+        const size_t smem = pform_smem<double>(per_cta);
         cudaError_t e = cudaFuncSetAttribute(k_pform<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         k_pform<double><<<grid, PF_THREADS, smem, s>>>(req, branch, nbr, m, (double *)Pbuf, status_key, raw ? 1 : 0,
                                                        nullptr, 0, nullptr, per_cta);
     } else {
-        size_t smem = sizeof(float) * (2 * K2 + K * (K + 1) + 2 * K);
-        smem = (smem + 15) & ~size_t(15);
-        smem += sizeof(double) * 2 * K;
+        const size_t smem = pform_smem<float>(per_cta);
         cudaError_t e = cudaFuncSetAttribute(k_pform<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         k_pform<float><<<grid, PF_THREADS, smem, s>>>(req, branch, nbr, m, (float *)Pbuf, status_key, raw ? 1 : 0,
