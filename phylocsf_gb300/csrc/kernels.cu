@@ -669,9 +669,9 @@ __global__ void __launch_bounds__(PruneThreads<TC>::N) k_prune(PruneArgs a)
             asm volatile("cp.async.wait_all;" ::: "memory");
             __syncthreads();
             T vl[4][CPT], vr[4][CPT];
-            child_partial<T, TC, KAHAN, CPT>(Et, slots, sn.lslot, sn.lc, lvT, a0, c0, vl, dcol0, true,
+            child_partial<T, TC, KAHAN, CPT, 7>(Et, slots, sn.lslot, sn.lc, lvT, a0, c0, vl, dcol0, true,
                                         dlo ? dlo + (size_t)sn.lc * K : nullptr);
-            child_partial<T, TC, KAHAN, CPT>(Et + K2, slots, sn.rslot, sn.rc, lvT, a0, c0, vr, dcol0, true,
+            child_partial<T, TC, KAHAN, CPT, 7>(Et + K2, slots, sn.rslot, sn.rc, lvT, a0, c0, vr, dcol0, true,
                                         dlo ? dlo + (size_t)sn.rc * K : nullptr);
             __syncthreads();
             if (ni + 1 < a.n_internal) stage_children<T, TC, CPT, THREADS>(Et, Pbase, sched[ni + 1], lvT, tid);   // buffers free again

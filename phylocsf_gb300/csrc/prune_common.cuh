@@ -271,7 +271,10 @@ __device__ inline void contract_scalar(const T *M, const T *X, int a0, int c0, T
 // Measured with the staged leaf rows, blocked compensation, 58 leaves, 141,741 columns: 3.12 ->
 // 2.68 ms; what bounds it now is the mix of FP32 issue, load latency and three barriers a node.
 // entry(j, e): E's four entries of step j.
-template <int TC, int COMP, int CPT, typename Entry>
+// UNROLL: blocks of the compensated sum in a row (7: all of them).  Rolled, each block begins with
+// its loads' latency (k_prune 2.94 ms against 2.68); unrolled, a kernel with many contractions
+// outgrows the instruction cache (k_grad with rate parameters 15.6 ms against 12.8).
+template <int TC, int COMP, int CPT, int UNROLL, typename Entry>
 __device__ inline void contract_pairs(Entry entry, const float *X, int c0, float out[4][CPT])
 {
     constexpr int NP = CPT / 2;
@@ -303,7 +306,7 @@ __device__ inline void contract_pairs(Entry entry, const float *X, int c0, float
             }
         };
         block(0, s);
-#pragma unroll        // (rolled, each block began with its loads' latency: 2.94 -> 2.68 ms)
+#pragma unroll UNROLL
         for (int jb = 8; jb < K; jb += 8) {
             f2 g[4][NP];
             block(jb, g);
@@ -347,11 +350,11 @@ __device__ inline void contract_pairs(Entry entry, const float *X, int c0, float
         for (int k = 0; k < NP; k++) upk(COMP ? add2(s[i][k], nc[i][k]) : s[i][k], out[i][2 * k], out[i][2 * k + 1]);
 }
 
-template <typename T, int TC, int COMP, int CPT = TC / 16>
+template <typename T, int TC, int COMP, int CPT = TC / 16, int UNROLL = 1>
 __device__ inline void contract(const T *M, const T *X, int a0, int c0, T out[4][CPT])
 {
     if constexpr (sizeof(T) == 4 && CPT % 2 == 0)
-        contract_pairs<TC, COMP, CPT>([&](int j, float e[4]) { Vec4<float>::load(M + j * K + a0, e); }, X, c0, out);
+        contract_pairs<TC, COMP, CPT, UNROLL>([&](int j, float e[4]) { Vec4<float>::load(M + j * K + a0, e); }, X, c0, out);
     else
         contract_scalar<T, TC, COMP, CPT>(M, X, a0, c0, out);
 }
@@ -367,7 +370,7 @@ __device__ inline void contract_rows(const T *N, const T *X, int a0, int c0, T o
     constexpr int CPT = TC / 16;
     if constexpr (sizeof(T) == 4 && CPT % 2 == 0) {
         float r[4][4];       // four steps of the thread's four rows
-        contract_pairs<TC, COMP, CPT>(
+        contract_pairs<TC, COMP, CPT, 1>(
             [&](int j, float e[4]) {
                 if (j % 4 == 0) {
 #pragma unroll
@@ -493,7 +496,7 @@ __device__ inline void stage_children(T *Et, const T *Pbase, const SchedNode &nx
 // Partial of child c at its parent: v[a] = alpha_c[a] + sum_j E_c[a][j] alpha_c[j]
 // (internal child, slot >= 0; Et = E_c^T) or the gather v[a] = P_c[a][s] of a
 // leaf in state s (1 for a marginalised leaf: P rows sum to 1).
-template <typename T, int TC, int KAHAN, int CPT = TC / 16>
+template <typename T, int TC, int KAHAN, int CPT = TC / 16, int UNROLL = 1>
 __device__ inline void child_partial(const T *Et, const T *slots, int slot, int leaf, const uint8_t *lvT, int a0,
                                      int c0, T v[4][CPT], int64_t dither_col0 = -1, bool staged = false,
                                      const float *dlo = nullptr)
@@ -545,7 +548,7 @@ __device__ inline void child_partial(const T *Et, const T *slots, int slot, int 
         return;
     }
     const T *al = slots + (size_t)slot * K * TC;
-    contract<T, TC, KAHAN, CPT>(Et, al, a0, c0, v);
+    contract<T, TC, KAHAN, CPT, UNROLL>(Et, al, a0, c0, v);
     T lo[4] = {(T)0, (T)0, (T)0, (T)0};
     if (dlo) {
         const float4 l4 = *reinterpret_cast<const float4 *>(dlo + a0);
