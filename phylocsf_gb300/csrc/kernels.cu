@@ -31,9 +31,11 @@ namespace pcsf {
 // double-buffered so that a round needs one cluster barrier, and V, whose rows are local, is
 // updated between arriving at that barrier and waiting for it.  Every element goes through
 // the same operations in the same order for every C: the results do not depend on it.
-// Measured, OmegaModel scores of six 12-leaf alignments (130 rounds of up to 8 matrices):
-// 514 ms with one CTA per matrix, 243 ms with clusters of 16.  What bounds a round now is the
-// chain of three divisions and two square roots of its rotations (459 and 705 clocks each).
+// Measured, OmegaModel scores of six 12-leaf alignments (130 rounds of up to 8 matrices): 514 ms
+// with one CTA per matrix, 243 ms with clusters of 16, 207 ms with small pruning tiles, 181 ms with
+// half blocks per thread, their loads ahead of the rotations, and jac_rotation's short chain.  A
+// round is ~4,300 clocks now: about 1,500 of rotations and 500 of updates, the rest distributed
+// shared-memory latency and the barrier.
 
 constexpr int JAC_THREADS = 256;
 constexpr int JAC_LD = K + 1;
@@ -47,11 +49,85 @@ __device__ inline void jac_pair(int r, int i, int &p, int &q)
     q = a < b ? b : a;
 }
 
+// Reciprocal and reciprocal square root of a normal d > 0 (exponent well inside the range) to about
+// 2^-44: the leading 24 bits by the FP32 approximation, the rest by one Newton step on two floats,
+// put together as integers.  FP64 instructions take 69 clocks each in a chain on this part, FP32 and
+// integer ones four.
+__device__ __forceinline__ double seed_bits(float y0, float y1, int e)
+{
+    // (double)y0 + y1 for y0 in [0.5, 1], |y1| < 2^-22, times 2^-e
+    const int k = __float_as_int(fmaf(y1, 0x1p44f, 12582912.0f)) - 0x4B400000;             // y1 in units of 2^-44
+    return __longlong_as_double(((long long)__float_as_int(y0) << 29) + ((long long)(896 - e) << 52) + ((long long)k << 9));
+}
+__device__ __forceinline__ double recip_seed(double d)
+{
+    const long long b = __double_as_longlong(d);
+    const float mh = __int_as_float(0x3F800000 | ((int)(b >> 29) & 0x7FFFFF));              // mantissa in [1, 2): 24 bits
+    const float ml = (__int_as_float(0x4B000000 | ((int)(b >> 6) & 0x7FFFFF)) - 8388608.0f) * 0x1p-46f;
+    float y0;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(y0) : "f"(mh));
+    const float r = fmaf(-ml, y0, fmaf(-mh, y0, 1.0f));
+    return seed_bits(y0, y0 * r, (int)(b >> 52) - 1023);
+}
+__device__ __forceinline__ double rsqrt_seed(double d)
+{
+    const long long b = __double_as_longlong(d);
+    const int e = (int)(b >> 52) - 1023, odd = e & 1;
+    const float mh = __int_as_float((0x3F800000 + (odd << 23)) | ((int)(b >> 29) & 0x7FFFFF));   // [1, 4)
+    const float ml = (__int_as_float(0x4B000000 | ((int)(b >> 6) & 0x7FFFFF)) - 8388608.0f) * (odd ? 0x1p-45f : 0x1p-46f);
+    float y0;
+    asm("rsqrt.approx.f32 %0, %1;" : "=f"(y0) : "f"(mh));
+    const float p = y0 * y0, pl = fmaf(y0, y0, -p);
+    const float r = fmaf(-ml, p, fmaf(-mh, pl, fmaf(-mh, p, 1.0f)));
+    return seed_bits(y0, 0.5f * y0 * r, (e - odd) / 2);
+}
+
+// The rotation (c, s) that annihilates apq != 0: theta = (aqq - app) / (2 apq), t = sign(theta) /
+// (|theta| + sqrt(theta^2 + 1)), c = 1 / sqrt(t^2 + 1), s = t c, each operation rounded to nearest.
+// Quotients and roots are seeds (above) with one residual correction in FP64 (Markstein, IBM J. Res.
+// Dev. 34 (1990) 111): an error of ~2^-88 before the final rounding, so that they round as the
+// library's do (it would take about 2^35 operations to meet one that does not), in 5 x 69 + 90
+// clocks for a root and its reciprocal instead of 705 + 459.  Operands far from 1, and |theta|
+// beyond 2^300, take the library's operations.
+__device__ __forceinline__ void jac_rotation(double app, double aqq, double apq, double &c, double &s)
+{
+    const double num = aqq - app, den = 2.0 * apq, ad = fabs(den);
+    const int en = (__double2hiint(num) >> 20) & 0x7FF, ed = __double2hiint(ad) >> 20;
+    double theta;
+    if ((num == 0.0 || (en > 223 && en < 1823)) && ed > 223 && ed < 1823) {
+        const double y = recip_seed(ad), q = num * y;
+        theta = __fma_rn(__fma_rn(-q, ad, num), y, q);
+        if (den < 0.0) theta = -theta;
+    } else {
+        theta = num / den;
+    }
+    double t;
+    if (fabs(theta) < 0x1p300) {
+        const double x = __fma_rn(theta, theta, 1.0);
+        double y = rsqrt_seed(x);
+        const double g = x * y;
+        const double d = fabs(theta) + __fma_rn(__fma_rn(-g, g, x), 0.5 * y, g);
+        y = recip_seed(d);
+        t = __fma_rn(y, __fma_rn(-d, y, 1.0), y);
+        if (!(theta >= 0.0)) t = -t;
+    } else {
+        t = (fabs(theta) > 1e150) ? 0.5 / theta
+            : (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(__fma_rn(theta, theta, 1.0)));
+    }
+    const double u = __fma_rn(t, t, 1.0);          // in [1, 2]
+    const double y = rsqrt_seed(u), g = u * y;
+    const double v = __fma_rn(__fma_rn(-g, g, u), 0.5 * y, g);
+    c = __fma_rn(y, __fma_rn(-v, y, 1.0), y);
+    s = t * c;
+}
+
 template <int C>
 __global__ void __launch_bounds__(JAC_THREADS) k_jacobi(const double *A_in, double *U_out, double *lam_out,
                                                          int *status)
 {
     constexpr int ROWS = K / C;                        // rows of A and V per CTA
+    constexpr int HALVES = (32 / C) * 64;              // half blocks of a CTA: two per pair of pairs
+    constexpr bool HALF = HALVES <= JAC_THREADS;       // one per thread (C >= 8)
     extern __shared__ __align__(16) unsigned char jsm[];
     double *A = reinterpret_cast<double *>(jsm);      // [2][ROWS][JAC_LD]
     double *V = A + 2 * ROWS * JAC_LD;                 // [ROWS][JAC_LD]
@@ -71,6 +147,10 @@ __global__ void __launch_bounds__(JAC_THREADS) k_jacobi(const double *A_in, doub
         if constexpr (C > 1) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
         else __syncthreads();
     };
+    // a x - b y and a x + b y, the second product rounded (fixed here so that every form of the
+    // update rounds alike)
+    auto diff = [](double a, double x, double b, double y) { return __fma_rn(a, x, -__dmul_rn(b, y)); };
+    auto sum = [](double a, double x, double b, double y) { return __fma_rn(a, x, __dmul_rn(b, y)); };
     // element (row, col) of buffer buf, wherever it lives in the cluster
     auto at = [&](int buf, int row, int col) -> double * {
         double *p = A + ((size_t)buf * ROWS + row % ROWS) * JAC_LD + col;
@@ -120,33 +200,57 @@ __global__ void __launch_bounds__(JAC_THREADS) k_jacobi(const double *A_in, doub
         for (int r = 0; r < K - 1; r++) {
             double *cs = csb + 32 * (cur & 1), *sn = snb + 32 * (cur & 1);
             int *pp = ppb + 32 * (cur & 1), *qq = qqb + 32 * (cur & 1);
+            // HALF: a thread's half block, one of the two columns of pair kc in the rows of pair k, is
+            // on its way while the rotations are formed
+            double x[4];
+            if (HALF && tid < HALVES) {
+                int p, q, pc, qc;
+                jac_pair(r, rank * (32 / C) + (tid >> 6), p, q);
+                jac_pair(r, tid & 31, pc, qc);
+                x[0] = *at(cur, p, pc);
+                x[1] = *at(cur, p, qc);
+                x[2] = *at(cur, q, pc);
+                x[3] = *at(cur, q, qc);
+            }
             if (tid < 32) {                                     // every CTA forms all 32 rotations
                 int p, q;
                 jac_pair(r, tid, p, q);
                 const double apq = *at(cur, p, q), aqq = *at(cur, q, q), app = *at(cur, p, p);
                 double c = 1.0, s = 0.0;
-                if (apq != 0.0) {
-                    double theta = (aqq - app) / (2.0 * apq);
-                    double t = (fabs(theta) > 1e150) ? 0.5 / theta
-                               : (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-                    c = 1.0 / sqrt(t * t + 1.0);
-                    s = t * c;
-                }
+                if (apq != 0.0) jac_rotation(app, aqq, apq, c, s);
                 cs[tid] = c; sn[tid] = s; pp[tid] = p; qq[tid] = q;
             }
             __syncthreads();
-            for (int f = tid; f < (32 / C) * 32; f += JAC_THREADS) {   // 2x2 blocks: columns A <- A J, then rows A <- J^T A
-                const int k = rank * (32 / C) + (f >> 5), kc = f & 31;
-                const int p = pp[k], q = qq[k], pc = pp[kc], qc = qq[kc];
+            // 2x2 blocks: columns A <- A J, then rows A <- J^T A (16 FP64 instructions a block); the
+            // pivots become exact zeros
+            auto column = [&](int k, int kc, bool second) {
+                const int p = pp[k], q = qq[k];
                 const double cc = cs[kc], sc = sn[kc], cr = cs[k], sr = sn[k];
-                const double app = *at(cur, p, pc), apq = *at(cur, p, qc), aqp = *at(cur, q, pc), aqq = *at(cur, q, qc);
-                const double bpp = cc * app - sc * apq, bpq = sc * app + cc * apq;
-                const double bqp = cc * aqp - sc * aqq, bqq = sc * aqp + cc * aqq;
-                const bool diag = k == kc;                      // the pivots become exact zeros
-                *at(cur ^ 1, p, pc) = cr * bpp - sr * bqp;
-                *at(cur ^ 1, q, pc) = diag ? 0.0 : sr * bpp + cr * bqp;
-                *at(cur ^ 1, p, qc) = diag ? 0.0 : cr * bpq - sr * bqq;
-                *at(cur ^ 1, q, qc) = sr * bpq + cr * bqq;
+                if (!second) {
+                    const int pc = pp[kc];
+                    const double bp = diff(cc, x[0], sc, x[1]), bq = diff(cc, x[2], sc, x[3]);
+                    *at(cur ^ 1, p, pc) = diff(cr, bp, sr, bq);
+                    *at(cur ^ 1, q, pc) = k == kc ? 0.0 : sum(sr, bp, cr, bq);
+                } else {
+                    const int qc = qq[kc];
+                    const double bp = sum(sc, x[0], cc, x[1]), bq = sum(sc, x[2], cc, x[3]);
+                    *at(cur ^ 1, p, qc) = k == kc ? 0.0 : diff(cr, bp, sr, bq);
+                    *at(cur ^ 1, q, qc) = sum(sr, bp, cr, bq);
+                }
+            };
+            if (HALF) {
+                if (tid < HALVES) column(rank * (32 / C) + (tid >> 6), tid & 31, (tid & 32) != 0);
+            } else {
+                for (int f = tid; f < HALVES / 2; f += JAC_THREADS) {
+                    const int k = rank * (32 / C) + (f >> 5), kc = f & 31;
+                    const int p = pp[k], q = qq[k], pc = pp[kc], qc = qq[kc];
+                    x[0] = *at(cur, p, pc);
+                    x[1] = *at(cur, p, qc);
+                    x[2] = *at(cur, q, pc);
+                    x[3] = *at(cur, q, qc);
+                    column(k, kc, false);
+                    column(k, kc, true);
+                }
             }
             cluster_arrive();
             for (int f = tid; f < ROWS * 32; f += JAC_THREADS) {       // V <- V J
@@ -154,8 +258,8 @@ __global__ void __launch_bounds__(JAC_THREADS) k_jacobi(const double *A_in, doub
                 const int p = pp[k], q = qq[k];
                 const double c = cs[k], s = sn[k];
                 const double va = V[row * JAC_LD + p], vb = V[row * JAC_LD + q];
-                V[row * JAC_LD + p] = c * va - s * vb;
-                V[row * JAC_LD + q] = s * va + c * vb;
+                V[row * JAC_LD + p] = diff(c, va, s, vb);
+                V[row * JAC_LD + q] = sum(s, va, c, vb);
             }
             cluster_wait();
             cur ^= 1;

@@ -97,3 +97,20 @@ def test_small_pruning_tiles(name, prec):
         assert (st == 0).all()
         assert np.array_equal(one[0], lpr[:n]) and np.array_equal(one[1], elpr[:n])
         assert np.array_equal(one[0], lpr[-n:])
+
+
+# the eigensolver's rotations come from corrected approximations of quotients and roots: an
+# eigensystem (branch lengths put P(t) at both ends of its range) against numpy's in FP64.  The sums
+# behind P(t) have 64 terms of at most 1 in size with a few ulp each: 1e-13
+def test_eigensystem_against_numpy():
+    for name in ("12flies", "29mammals"):
+        ps = synth.load_params(name)
+        eng = P.Engine(ps.tree, ps.S_c, ps.pi_c, ps.S_n, ps.pi_n, precision="fp64")
+        for m, (S, pi) in enumerate(((ps.S_c, ps.pi_c), (ps.S_n, ps.pi_n))):
+            U, lam = eng.eigensystem(m)
+            Q = synth.q_matrix(S, pi)
+            A = np.sqrt(pi)[:, None] * Q / np.sqrt(pi)[None, :]
+            A = 0.5 * (A + A.T)
+            assert np.abs((U * lam) @ U.T - A).max() <= 1e-13 * np.abs(A).max() * 64
+            assert np.abs(U.T @ U - np.eye(64)).max() <= 1e-13
+            assert np.abs(np.sort(lam) - np.linalg.eigvalsh(A)).max() <= 1e-13 * np.abs(lam).max() * 64
