@@ -187,9 +187,8 @@ int pcsf_engine_exact_available(const pcsf_engine *e);
  * on the tree (partial slots and leaves) and the precision.  The FP64 engine has one
  * tile (32) and keeps it.  TF32 tensor-core engines also time the search kernel's
  * shapes on the same sample and keep the faster (pcsf_stats.tc_shape):
- *   0: each column's partial (alpha) kept in registers from the operand staging to the
- *      epilogue;  1: alpha read back from the MMA operands in the epilogue.
- * Both issue the same MMAs on the same operands: the values are identical.
+ *   0: every CTA that fits an SM (two);  1: one CTA per SM.
+ * Both run the same kernel on the same tiles: the values are identical.
  * No reference counterpart (the reference has no device). */
 int pcsf_engine_autotune(pcsf_engine *e, pcsf_batch *b, int32_t *tile);
 

@@ -181,8 +181,9 @@ struct pcsf_engine {
     int simt_tile = 0;             // SIMT column tile (0: the default rule; set by pcsf_engine_autotune)
     int smem_sm = 0;               // shared memory per SM, for the grid of a tile
     int ff_grid = 0;               // CTAs of the float-float kernel (0: the tree does not fit it)
-    int ff_depth = 0;              // partials that wait at once in its schedule
+    int depth = 0;                 // partials that wait at once in the schedule (tensor-core kernels)
     DevBuf<float> ff_stack;        // where they wait, per CTA (made with the engine: pcsf_lpr_noalloc uses it too)
+    DevBuf<float> tc_stack;        // the same of the search kernel
     // returned values (and the accurate search decisions) of a region come from the
     // float-float kernel when columns x (n_leaves - 2) reaches this; FP32 and tensor-core
     // engines only (the FP64 engine is exact already)
@@ -616,6 +617,13 @@ static int engine_init_common(pcsf_engine *e, const pcsf_tree *tree, int32_t fla
     CK(cudaMemcpyAsync(e->dbranch.p, e->branch.data(), sizeof(double) * e->nbr, cudaMemcpyHostToDevice, e->stream), "H2D");
     CK(cudaMemcpyAsync(e->dsched.p, e->sched.data(), sizeof(SchedNode) * e->sched.size(), cudaMemcpyHostToDevice,
                        e->stream), "H2D");
+    // a node's partial waits when the next node of the schedule is not its parent
+    for (size_t k = 0, waiting = 0; k < e->sched.size(); k++) {
+        const SchedNode &sn = e->sched[k];
+        if (sn.lslot >= 0 && sn.rslot >= 0) waiting--;
+        if (k + 1 < e->sched.size() && e->sched[k + 1].lc != sn.node && e->sched[k + 1].rc != sn.node) waiting++;
+        e->depth = std::max(e->depth, (int)waiting);
+    }
     e->sm_count = prop.multiProcessorCount;
     e->smem_optin = prop.sharedMemPerBlockOptin;
     CK(e->derr.reserve(1), "cudaMalloc");
@@ -637,7 +645,7 @@ static int engine_init_common(pcsf_engine *e, const pcsf_tree *tree, int32_t fla
         return e->fail(PCSF_EINVAL, "tensor-core path needs %zu B shared memory",
                        prune_tc_smem_bytes(e->nl, (int)e->sched.size()));
     if (tc)
-        e->tc_grid = prop.multiProcessorCount * prune_tc_ctas_per_sm(e->nslots, e->nl, (int)e->sched.size(), e->tc_shape);
+        e->tc_grid = prop.multiProcessorCount * prune_tc_ctas_per_sm(e->nl, (int)e->sched.size(), e->tc_shape);
     size_t smem = prune_smem_bytes(e->prec, e->nslots, e->nl, (int)e->sched.size());
     if (smem > (size_t)prop.sharedMemPerBlockOptin)
         return e->fail(PCSF_EINVAL, "tree needs %d partial slots (%zu B shared memory > %zu)", e->nslots, smem,
@@ -653,16 +661,8 @@ static int engine_init_common(pcsf_engine *e, const pcsf_tree *tree, int32_t fla
                                            (int)e->sched.size(), 2 * k);
     if (e->prec != PCSF_PREC_FP64 &&
         prune_ff_smem_bytes(e->nl, (int)e->sched.size()) <= (size_t)prop.sharedMemPerBlockOptin) {
-        // a node's partial waits when the next node of the schedule is not its parent
-        int waiting = 0;
-        for (size_t k = 0; k < e->sched.size(); k++) {
-            const SchedNode &sn = e->sched[k];
-            if (sn.lslot >= 0 && sn.rslot >= 0) waiting--;
-            if (k + 1 < e->sched.size() && e->sched[k + 1].lc != sn.node && e->sched[k + 1].rc != sn.node) waiting++;
-            e->ff_depth = std::max(e->ff_depth, waiting);
-        }
         e->ff_grid = prop.multiProcessorCount;
-        CK(e->ff_stack.reserve(ff_stack_floats(e->ff_grid, e->ff_depth)), "cudaMalloc float-float stack");
+        CK(e->ff_stack.reserve(ff_stack_floats(e->ff_grid, e->depth)), "cudaMalloc float-float stack");
     }
     // P(t) buffer: up to 16 GiB, at most a quarter of free memory.  A round of the
     // search forms one P set per active fit (20,000 fits x 3.6 MB for 58 leaves), so
@@ -821,6 +821,8 @@ static int evaluate(pcsf_engine *e, pcsf_batch *b, const std::vector<Request> &r
     if (stage64 || ff) CK(e->Pbuf64.reserve(max_chunk_ps * (size_t)e->nbr * K2), "cudaMalloc P(t) staging buffer");
     const int nbop = e->nbr - e->nl;
     const bool want_bop = tc && !grad && e->prec != PCSF_PREC_BF16X3;   // the BF16 kernel splits E^T itself
+    const bool leaf_rows = want_bop && !drho;    // k_prune_tc's own layout of the leaf branches
+    if (leaf_rows) CK(e->tc_stack.reserve(prune_tc_stack_floats(e->tc_grid, e->depth)), "cudaMalloc tensor-core stack");
     if (want_bop) CK(e->Bop.reserve(max_chunk_ps * (size_t)nbop * 2 * K2), "cudaMalloc tensor-core operand buffer");
     float *bop = want_bop ? e->Bop.p : nullptr;
     size_t gscr = 0;
@@ -867,11 +869,11 @@ static int evaluate(pcsf_engine *e, pcsf_batch *b, const std::vector<Request> &r
             CK(launch_pform(true, dps + p0, p1 - p0, e->dbranch.p, e->nbr, dmv, e->Pbuf64.p, dstatus + p0, s),
                "P(t) formation launch");
             CK(launch_d2f_rows(e->Pbuf64.p, reinterpret_cast<float *>(e->Pbuf.p), (size_t)(p1 - p0) * e->nbr, e->nbr,
-                               bop, e->nl, s, dlo), "P(t) conversion launch");
+                               bop, e->nl, s, dlo, leaf_rows), "P(t) conversion launch");
             e->stats.kernel_launches += 1;
         } else if (want_bop && !dyn) {
             CK(launch_pform_tc(dps + p0, p1 - p0, e->dbranch.p, e->nbr, e->nl, dmv, e->dPfB.p,
-                               reinterpret_cast<float *>(e->Pbuf.p), bop, dstatus + p0, e->derr.p, s),
+                               reinterpret_cast<float *>(e->Pbuf.p), bop, dstatus + p0, e->derr.p, s, leaf_rows),
                "tensor-core P(t) formation launch");
         } else {
             CK(launch_pform(e->prec == PCSF_PREC_FP64 || dyn || ff, dps + p0, p1 - p0, e->dbranch.p, e->nbr, dmv,
@@ -898,8 +900,7 @@ static int evaluate(pcsf_engine *e, pcsf_batch *b, const std::vector<Request> &r
         pa.dlo = dlo;
         pa.tile = (!grad && !ff && !tc) ? TC : 0;
         pa.colv = cols ? e->dpart.p + 2 * (size_t)wib[r0] * TC : nullptr;
-        pa.tc_shape = e->tc_shape;
-        pa.ff_depth = e->ff_depth;
+        pa.depth = e->depth;
         if (grad) {
             GradArgs ga{};
             ga.wi = pa.wi;
@@ -941,7 +942,8 @@ static int evaluate(pcsf_engine *e, pcsf_batch *b, const std::vector<Request> &r
             if (e->prec == PCSF_PREC_BF16X3)
                 CK(launch_prune_bf16(pa, e->derr.p, s, grid), "BF16 tensor-core pruning launch");
             else
-                CK(launch_prune_tc(e->prec == PCSF_PREC_TF32X3 ? 3 : 1, pa, e->derr.p, s, grid), "tensor-core pruning launch");
+                CK(launch_prune_tc(e->prec == PCSF_PREC_TF32X3 ? 3 : 1, pa, e->tc_stack.p, e->derr.p, s, grid),
+                   "tensor-core pruning launch");
         } else {
             int grid = std::min(cols ? simt_grid(e, TC) : e->prune_grid, std::max(pa.nwi, 1));
             CK(launch_prune(e->prec == PCSF_PREC_FP64 ? PCSF_PREC_FP64 : PCSF_PREC_FP32, comp, pa, s, grid),
@@ -1825,7 +1827,7 @@ int pcsf_internal_noalloc_ctx(pcsf_engine *e, NoallocCtx *c)
     c->prune_grid = e->prune_grid;
     c->simt_tile = e->simt_tile;
     c->ff_grid = e->prec != PCSF_PREC_FP64 ? e->ff_grid : 0;
-    c->ff_depth = e->ff_depth;
+    c->depth = e->depth;
     c->ff_stack = e->ff_stack.p;
     c->exact_min_units = e->exact_min_units;
     c->derr = e->derr.p;
@@ -2510,7 +2512,7 @@ int pcsf_engine_autotune(pcsf_engine *e, pcsf_batch *b, int32_t *tile)
         double best_s_ms = 1e300;
         for (int cand = 0; cand < PCSF_TC_SHAPES; cand++) {
             e->tc_shape = cand;
-            e->tc_grid = e->sm_count * prune_tc_ctas_per_sm(e->nslots, e->nl, (int)e->sched.size(), cand);
+            e->tc_grid = e->sm_count * prune_tc_ctas_per_sm(e->nl, (int)e->sched.size(), cand);
             double ms = 0.0;
             std::vector<Eval> res;
             for (int it = 0; it < 3 && rc == PCSF_OK; it++) {
@@ -2532,7 +2534,7 @@ int pcsf_engine_autotune(pcsf_engine *e, pcsf_batch *b, int32_t *tile)
             return rc != PCSF_OK ? rc : e->fail(PCSF_EINVAL, "pcsf_engine_autotune: no tensor-core shape fits");
         }
         e->tc_shape = best_s;
-        e->tc_grid = e->sm_count * prune_tc_ctas_per_sm(e->nslots, e->nl, (int)e->sched.size(), best_s);
+        e->tc_grid = e->sm_count * prune_tc_ctas_per_sm(e->nl, (int)e->sched.size(), best_s);
     }
     return PCSF_OK;
 }
@@ -2546,7 +2548,7 @@ int pcsf_engine_set_tc_shape(pcsf_engine *e, int32_t shape)
         return e->fail(PCSF_EINVAL, "pcsf_engine_set_tc_shape: shape must be 0..%d", PCSF_TC_SHAPES - 1);
     CK(cudaSetDevice(e->device), "cudaSetDevice");
     e->tc_shape = shape;
-    e->tc_grid = e->sm_count * prune_tc_ctas_per_sm(e->nslots, e->nl, (int)e->sched.size(), shape);
+    e->tc_grid = e->sm_count * prune_tc_ctas_per_sm(e->nl, (int)e->sched.size(), shape);
     return PCSF_OK;
 }
 

@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(FF_THREADS, 1) k_prune_ff(PruneArgs a, size_t 
     int16_t *bseq = reinterpret_cast<int16_t *>(sched + nin);        // internal child of each contraction, in order
     const uint32_t bar0 = smem_addr(&bar_h0), bar1 = smem_addr(&bar_h1), barB = smem_addr(&bar_b);
     const uint32_t sA = smem_addr(sm + FS_A), sB = smem_addr(sm + FS_B);
-    float *stk = stack + (size_t)blockIdx.x * a.ff_depth * (2 * FF_SPT * FF_THREADS) + tid;
+    float *stk = stack + (size_t)blockIdx.x * a.depth * (2 * FF_SPT * FF_THREADS) + tid;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"

@@ -609,23 +609,25 @@ cudaError_t launch_d2f(const double *in, float *out, size_t n, cudaStream_t s)
 // Matrices are [set][nbr]; with bop, the branches b >= bop_nl also get their
 // tensor-core B operand (see bop_store).
 __global__ void __launch_bounds__(256) k_d2f_rows(const double *in, float *out, size_t nmat, int nbr, float *bop,
-                                                  int bop_nl, float *dlo)
+                                                  int bop_nl, float *dlo, int leaf_rows)
 {
     const size_t mat = blockIdx.x * (size_t)4 + threadIdx.x / K;
     const int i = threadIdx.x % K;
     if (mat >= nmat) return;
     const double *src = in + mat * K2;
     float *dst = out + mat * K2;
+    const int b = (int)(mat % (size_t)nbr);
+    const bool lr = leaf_rows && b < bop_nl;
+    const int pos = lr ? leaf_pos(i) : i;
     double d = 0.0;
     for (int j = 0; j < K; j++) {
         if (j == i) continue;
         const float x = (float)src[j * K + i];
-        dst[j * K + i] = x;
+        dst[j * K + pos] = x;
         d -= (double)x;
     }
-    dst[i * K + i] = (float)d;
+    dst[i * K + pos] = lr ? (float)d + 1.0f : (float)d;
     if (dlo) dlo[mat * K + i] = (float)(d - (double)(float)d);   // low part of the diagonal
-    const int b = (int)(mat % (size_t)nbr);
     if (bop && b >= bop_nl) {
         float *bd = bop + ((mat / nbr) * (size_t)(nbr - bop_nl) + (b - bop_nl)) * 2 * K2;
         for (int q = 0; q < K / 4; q++)
@@ -669,10 +671,10 @@ cudaError_t launch_check_codes(const uint8_t *codes, size_t n, unsigned long lon
 }
 
 cudaError_t launch_d2f_rows(const double *in, float *out, size_t nmat, int nbr, float *bop, int bop_nl, cudaStream_t s,
-                            float *dlo)
+                            float *dlo, bool leaf_rows)
 {
     if (nmat == 0) return cudaSuccess;
-    k_d2f_rows<<<(unsigned)((nmat + 3) / 4), 256, 0, s>>>(in, out, nmat, nbr, bop, bop_nl, dlo);
+    k_d2f_rows<<<(unsigned)((nmat + 3) / 4), 256, 0, s>>>(in, out, nmat, nbr, bop, bop_nl, dlo, leaf_rows ? 1 : 0);
     return cudaGetLastError();
 }
 

@@ -232,7 +232,7 @@ extern "C" int pcsf_lpr_noalloc(pcsf_engine *e, int32_t model, double rho, int32
         pa.partials = d_part + 2 * (size_t)nws;
         pa.dither = 0;
         pa.dlo = nullptr;
-        pa.ff_depth = cx.ff_depth;
+        pa.depth = cx.depth;
         ce = launch_prune_ff(pa, cx.ff_stack, cx.derr, s, std::min(cx.ff_grid, nwi - nws));
     }
     if (ce == cudaSuccess) ce = launch_reduce(d_part, d_wib, nreq, d_lpr, d_elpr_out, s, d_out);

@@ -92,7 +92,7 @@ cudaError_t launch_pform(bool fp64, const PSet *ps, int nps, const double *branc
                          float *bop = nullptr, int bop_nl = 0, float *dlo = nullptr);
 cudaError_t launch_d2f(const double *in, float *out, size_t n, cudaStream_t s);
 cudaError_t launch_d2f_rows(const double *in, float *out, size_t nmat, int nbr, float *bop, int bop_nl, cudaStream_t s,
-                            float *dlo = nullptr);
+                            float *dlo = nullptr, bool leaf_rows = false);
 // Leaf codes of an uploaded batch: *first_bad = the smallest index of a byte > 64
 // (PCSF_MARGINALIZE), left unchanged when every code is valid.
 cudaError_t launch_check_codes(const uint8_t *codes, size_t n, unsigned long long *first_bad, cudaStream_t s);
@@ -117,8 +117,7 @@ struct PruneArgs {
     const float *dlo;        // SIMT FP32 kernel, may be null: per chunk-local P set [nbr][K] low parts of diag(E)
     int tile;                // SIMT kernel: column tile PRUNE_SMALL_TILE (short launches), 32 or 64 (FP32), 0 = the default rule
     double *colv;            // SIMT kernel, small tiles: [nwi][tile][2] the columns' terms instead of partials
-    int ff_depth;            // float-float kernel: partials that wait at once (its stack's entries)
-    int tc_shape;            // TF32 tensor-core kernel: 0 alpha kept in registers, 1 read back (identical values)
+    int depth;               // tensor-core kernels: partials that wait at once (entries of a CTA's stack)
 };
 // comp: 0 plain FP32 sums, 1 Kahan, 2 blocked Kahan (see prune_common.cuh)
 cudaError_t launch_prune(int prec, int comp, const PruneArgs &a, cudaStream_t s, int grid);
@@ -173,11 +172,13 @@ cudaError_t launch_reduce_grad(const double *gpart, const int32_t *wi_begin, int
                                cudaStream_t s);
 
 // Tensor-core pruning (tc_kernels.cu): nprod 3 = TF32 hi/lo split, 1 = single TF32.
-cudaError_t launch_prune_tc(int nprod, const PruneArgs &a, int *err, cudaStream_t s, int grid);
+// stack = prune_tc_stack_floats(grid, depth) floats.
+cudaError_t launch_prune_tc(int nprod, const PruneArgs &a, float *stack, int *err, cudaStream_t s, int grid);
 size_t prune_tc_smem_bytes(int nl, int nint);
+size_t prune_tc_stack_floats(int grid, int depth);
 bool prune_tc_supported(int nslots, int nl);
-constexpr int PCSF_TC_SHAPES = 2;
-int prune_tc_ctas_per_sm(int nslots, int nl, int nint, int shape);
+constexpr int PCSF_TC_SHAPES = 2;      // 0 every CTA that fits an SM (two), 1 one per SM (identical values)
+int prune_tc_ctas_per_sm(int nl, int nint, int shape);
 bool prune_tc_shape_ok(int shape);
 // Tensor-core pruning with BF16 split products (tc_bf16.cu): x = h + m + l, six
 // products on tcgen05 kind::f16, FP32 accumulation; E^T of every branch in Pbuf (FP32).
@@ -187,9 +188,12 @@ bool prune_bf16_supported(int nslots, int nl);
 int prune_bf16_ctas_per_sm(int nslots, int nl, int nint);
 // tensor-core P(t) formation for the search evaluations (tc_pform.cu): E^T of the
 // branches above leaves into Pbuf, B operands of the branches above internal
-// nodes into Bop; Bpf = per model the pre-split B = U^T D^1/2 [2][hi, lo][64 x 64]
+// nodes into Bop (leaf_rows, here and in launch_d2f_rows: for the branches above leaves
+// P^T = E^T + I instead, in the order that k_prune_tc gathers, leaf_pos); Bpf = per model
+// the pre-split B = U^T D^1/2 [2][hi, lo][64 x 64]
 cudaError_t launch_pform_tc(const PSet *ps, int nps, const double *branch, int nbr, int nl, DevModels m,
-                            const float *Bpf, float *Pbuf, float *Bop, int32_t *status_key, int *err, cudaStream_t s);
+                            const float *Bpf, float *Pbuf, float *Bop, int32_t *status_key, int *err, cudaStream_t s,
+                            bool leaf_rows = false);
 // tensor-core tangent pass (tc_dual.cu): lpr / elpr partials as k_prune_tc plus
 // d lpr / d rho partials dpart [nwi][2] (second entry 0); Qop = per model the
 // pre-split B operand of Q [2][hi, lo][64 x 64]; branch = the tree's lengths
@@ -211,7 +215,7 @@ cudaError_t launch_reduce_cols(const double *colv, const WorkItem *wi, const int
 // Float-float pruning on the tensor cores (ff_kernels.cu): returned values that agree with
 // the FP64 path to ~1e-12 relative.  Pbuf holds per P set ff_pset_bytes() of operands, made
 // from the FP64 P(t) formation's output by launch_split_ff; tiles of ff_tile_cols() columns,
-// one CTA per SM; stack = ff_stack_floats(grid, PruneArgs.ff_depth) floats; partials as
+// one CTA per SM; stack = ff_stack_floats(grid, PruneArgs.depth) floats; partials as
 // k_prune; err is set if a bounded wait timed out.
 cudaError_t launch_prune_ff(const PruneArgs &a, float *stack, int *err, cudaStream_t s, int grid);
 cudaError_t launch_split_ff(const double *in, void *out, int nps, int nbr, int nl, cudaStream_t s);
@@ -273,7 +277,7 @@ struct NoallocCtx {
     int prune_grid;
     int simt_tile;         // SIMT column tile chosen for the engine (0: the default rule)
     int ff_grid;           // CTAs of the float-float kernel (0: not available)
-    int ff_depth;          // its stack: entries per CTA, and the memory
+    int depth;             // its stack: entries per CTA, and the memory
     float *ff_stack;
     int64_t exact_min_units;   // regions with columns x (nl - 2) >= this use the float-float kernel
     int *derr;             // device error flag of timed-out waits

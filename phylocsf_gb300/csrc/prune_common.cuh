@@ -148,6 +148,10 @@ __device__ __forceinline__ int dither_k(int64_t col, int leaf)
     return (int)(h & 255u);
 }
 
+// Where k_prune_tc's leaf rows keep state a (its own inverse): within each 32 states, the four
+// pairs a thread of the row fragment holds are consecutive, 32 bytes.
+__device__ __forceinline__ int leaf_pos(int a) { return (a & 33) | ((a >> 2) & 6) | ((a << 2) & 24); }
+
 // exp_of(x): the e of frexp (x = m 2^e, m in [0.5, 1)) read from the exponent
 // field for normal x; frexp itself for zero, subnormals and non-finite x.
 __device__ __forceinline__ int exp_of(float x)

@@ -115,6 +115,36 @@ __device__ __forceinline__ void tmem_ld16x2(uint32_t ta, uint32_t tb, float *va,
     }
 }
 
+// Row fragments (shape 16x256b): of the 16 lanes from the address and 32 columns, thread l of the
+// warp holds in f[2 i + k] the pair of columns 8 i + 2 (l % 4), + 1 of lane l / 4 + 8 k.  The load
+// waits in the same asm block.
+__device__ __forceinline__ void tmem_ld_rows(uint32_t taddr, f2 *f)
+{
+    uint32_t r[16];
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                    "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
+                    "=r"(r[15])
+                 : "r"(taddr)
+                 : "memory");
+#pragma unroll
+    for (int j = 0; j < 8; j++) f[j] = pk(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+}
+__device__ __forceinline__ void tmem_st_rows(uint32_t taddr, const f2 *f)
+{
+    uint32_t r[16];
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        r[2 * j] = (uint32_t)f[j];
+        r[2 * j + 1] = (uint32_t)(f[j] >> 32);
+    }
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+                 :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+                    "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+                 : "memory");
+}
+
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const float *v)
 {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"

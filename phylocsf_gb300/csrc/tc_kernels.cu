@@ -13,38 +13,39 @@
 // identity part, v_c = alpha_c + D_c (E = P - I), so rounding in D only touches
 // the off-diagonal mass of P.
 //
-// Layout: 256 threads; thread t owns tile column (site) t % 128, i.e. TMEM lane
-// t % 128, and states 32*(t/128) .. +31 (warp w reaches lanes 32*(w%4)..).
-// Tensor memory holds the partial slots as regions of 64 columns (at least four:
-// 256 columns, so two CTAs share an SM).  A contraction has two forms:
-//  - region form (a tensor-memory region holds no live partial): the hi part of
-//    alpha_c is written back over the child's own slot and is the MMA's A operand
-//    there, the lo part goes to shared memory, and D goes to the free region;
-//  - shared form (every region is live, e.g. 6 of the 56 contractions of the
-//    58-leaf tree): hi and lo both go to the shared-memory A operand and D is
-//    written over the child's own slot.
-// The region form moves 80 KB of shared-memory operand reads per contraction
-// instead of 144 KB, and 64 KB of thread traffic instead of 128 KB.  Both forms issue
-// the same MMAs in the same order on the same values, so their results are
-// identical.  The epilogue reads alpha_c = hi + lo back from where the staging put
-// them.  What bounds the kernel is the latency of the per-node chain (MMA issue and
-// completion, the epilogue, the leaf gathers, the barriers), which the two CTAs on an
-// SM overlap: the MMA descriptors are precomputed, the leaf rows are gathered with
-// 256-bit loads, and while a node's MMAs run its threads prefetch into L1 the leaf
-// rows of the next node.
+// Layout: 256 threads, eight warps of 16 tile columns; four threads share a column.  A
+// thread holds 16 states of two columns, as the 16x256b tensor-memory accesses hand them
+// out (pairs of states 8 i + 2 (lane % 4), + 1), so a column's maximum is two shuffles away
+// and no warp waits for another between a contraction and the next staging.  A node's
+// normalised partial stays in those registers: the schedule evaluates a node's last
+// internal child just before the node, so its partial goes from there into the
+// contraction's operands (hi and lo, both in tensor memory) and is still there when D
+// arrives.  Only the first of two internal children waits, on a stack whose top entry is in
+// tensor memory (A hi, A lo, D, top: 256 columns) and the rest in global memory (L2).  With
+// 66 KB of shared memory and 128 registers a thread two CTAs share an SM.
+// B operands are pre-split by the P(t) kernel into the operand layout; one thread fetches
+// each with a 32 KB bulk copy (cp.async.bulk, completion on an mbarrier), two contractions
+// ahead.  One thread issues the MMAs when the eight warps have arrived on an mbarrier.
+// Leaf children are gathers of P^T rows from L2 while the MMAs run: the P(t) kernel writes
+// a leaf branch's rows with the identity added and the states permuted (leaf_pos) so that
+// the four threads of a column read a row with 32-byte loads, each row's 256 bytes in two
+// instructions of eight rows.  The root stage forms z = pi . alpha as an FP32 compensated
+// dot product and log z = log m + e ln 2 (m in [0.5, 1)), with FP64 only for the per-column
+// log and the tile sums.
 //
-// Shared memory (about 106 KB for 58 leaves, 112 KB for 100, so that two CTAs share an
-// SM): one A operand (128 x 64, hi + lo), one B operand (64 x 64, hi + lo), the tile's
-// leaf states and the schedule.
-// The two children of a node are contracted one after the other through the
-// same operand buffers.  B operands are pre-split by the P(t) kernel into this
-// exact layout, so one elected thread fetches each with a single 32 KB bulk copy
-// (cp.async.bulk, completion on an mbarrier), issued as soon as the previous
-// contraction has released the buffer.  Leaf children are gathers of E^T rows
-// from L2 while the MMAs run.  The per-column rescale exponent is the maximum
-// over the two threads of a column.  The root stage forms z = pi . alpha as an FP32
-// compensated dot product and log z = log m + e ln 2 (m in [0.5, 1)), with FP64
-// only for the per-column log and the tile sums.
+// What bounds it: the latency of the per-node chain, about 5,000 clocks a node beside one
+// other CTA: 24 MMAs of 60 clocks (N = 64 fills half of the tensor pipe's width, and a wider
+// N would need the two halves of B in one MMA, another order of the sums), the staging
+// and arrival before them (1,000) and the epilogue (800); a node with two leaves waits
+// 1,700 for its rows.  Tensor pipe and issue slots are each about half used.  Registers
+// decide: one more 32-byte array per thread spills, and spilling variants measured 10 to
+// 40 % slower, so the rows are not fetched a node ahead.
+// Measured, all search launches of a call: 384 regions on 58 leaves 46.5 -> 32.0 ms, 256
+// regions on 100 leaves 30.4 -> 21.0 ms, one region on 58 leaves (3 tiles a launch) 159 ->
+// 119 us a launch.  Before, two threads owned a column (32 states each): every child's
+// partial was stored and loaded again, a lane gathered its row alone (32 lines an
+// instruction, a third of the LSU's wavefronts were leaf reads), and the maximum crossed
+// warps through shared memory.
 //
 // Accuracy: the tensor cores' FP32 accumulation is not round-to-nearest: it
 // rounds toward minus infinity (a measured mean of -5.7 ulp of the result over
@@ -56,6 +57,7 @@
 // Every mbarrier wait is bounded; on timeout the kernel records an error, waits
 // (again bounded) for its outstanding copies and tensor-core work, releases its
 // tensor memory and exits.
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 
@@ -65,428 +67,413 @@
 
 namespace pcsf {
 
-constexpr int TCP_THREADS = 256;     // two threads per tile column
+constexpr int TCP_THREADS = 256;     // eight warps of 16 tile columns
 constexpr int TCP_M = 128;
-constexpr int TCP_MAX_SLOTS = 8;     // 8 x 64 = all 512 tensor-memory columns
+constexpr int TCP_MAX_SLOTS = 8;
 constexpr int TCP_MAX_LEAVES = 160;
+// tensor memory: A hi, A lo, D, and the top of the stack, 64 columns each
+constexpr uint32_t TCP_TMEM_COLS = 256, TM_HI = 0, TM_LO = 64, TM_D = 128, TM_S = 192;
 
 // dynamic shared-memory map (bytes)
-constexpr uint32_t SM_A = 0;            // [hi, lo][128 x 64 fp32] = 2 x 32 KB
-constexpr uint32_t SM_B = 65536;        // [hi, lo][64 x 64 fp32]  = 2 x 16 KB
-constexpr uint32_t SM_LV = 98304;       // [nl][LV_STRIDE] leaf states, then the schedule
-constexpr uint32_t A_BYTES = 32768, B_BYTES = 16384;
-// leaf-state rows padded by 4 bytes: the tile fill writes one byte per (site, leaf)
-// with consecutive threads on consecutive leaves, which would otherwise all hit one bank
+constexpr uint32_t SM_B = 0;            // two B operands, [hi, lo][64 x 64 fp32] = 2 x 16 KB each
+constexpr uint32_t SM_SCHED = 65536;    // the schedule, contraction order, leaf states
+constexpr uint32_t B_BYTES = 16384;
 constexpr int LV_STRIDE = TCP_M;     // leaf-state rows: [leaf][site] bytes, words XOR-swizzled per row
 // byte offset of (leaf l, site c): row l's 4-byte words are permuted by XOR with l mod 32,
 // so that the fill (consecutive threads on consecutive leaves of one site) and the reads
 // (consecutive threads on consecutive sites of one leaf) are both free of bank conflicts
-// without padding the rows (whose bytes decide whether two CTAs fit an SM on 100 leaves)
 __device__ __forceinline__ int lv_off(int l, int c) { return l * LV_STRIDE + (c ^ ((l & 31) << 2)); }
 
+// the schedule as the kernel walks it: children (the leaf, if one is), what to do with them
+struct TcNode {
+    int16_t lc, rc;
+    int32_t flags;
+};
+constexpr int TN_LEAVES = 1, TN_LEAF = 2;    // two leaves; one leaf (lc)
+constexpr int TN_PUSH = 4;                   // the next node does not take the partial: it waits on the stack
+constexpr int TN_PAIR = 8;                   // the next node has two leaves
+static __host__ __device__ size_t tc_sched_bytes(int nint) { return ((size_t)nint * (sizeof(TcNode) + 2) + 15) & ~(size_t)15; }
 
-// alpha = hi + lo of this thread's 32 states, read back from the A operand
-__device__ __forceinline__ void load_alpha(const unsigned char *sm, int site, int s0, int q, float *x)
+__device__ const __align__(32) float ones_row[K] = {
+    1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1,
+    1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1};
+
+// four pairs of floats in one 256-bit load, pinned where it stands (before the wait that hides it)
+__device__ __forceinline__ void ldg4(const float *p, f2 &a, f2 &b, f2 &c, f2 &d)
 {
-#pragma unroll
-    for (int j4 = 0; j4 < 4; j4++) {
-        const uint32_t o = core_off(site, s0 + 16 * q + 4 * j4, 16);
-        const float4 h = *reinterpret_cast<const float4 *>(sm + SM_A + o);
-        const float4 l = *reinterpret_cast<const float4 *>(sm + SM_A + A_BYTES + o);
-        x[4 * j4 + 0] = h.x + l.x;
-        x[4 * j4 + 1] = h.y + l.y;
-        x[4 * j4 + 2] = h.z + l.z;
-        x[4 * j4 + 3] = h.w + l.w;
-    }
+    float r[8];
+    asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]) : "l"(p));
+    a = pk(r[0], r[1]); b = pk(r[2], r[3]); c = pk(r[4], r[5]); d = pk(r[6], r[7]);
 }
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bar), "r"(count));
+}
+// one arrival for the warp: what its lanes did before is visible to those that wait
+__device__ __forceinline__ void warp_arrive(uint32_t bar, int lane)
+{
+    __syncwarp();
+    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(bar) : "memory");
+}
+// stack entries below the one in tensor memory
+static __host__ __device__ int prune_tc_levels(int depth) { return depth > 2 ? depth - 1 : 1; }
 
-// KEEP: each column's partial (alpha) stays in registers from the operand staging to
-// the epilogue, which then reads only D (else the epilogue reads alpha back from the
-// operands, and the second child's staging waits for a barrier that frees them).  Both
-// shapes issue the same MMAs on the same operands and produce identical values; the
-// engine's autotuner times them.
-template <int NPROD, bool KEEP>
-__global__ void __launch_bounds__(TCP_THREADS, 2) k_prune_tc(PruneArgs a, uint32_t tmem_cols, int *err)
+template <int NPROD>
+__global__ void __launch_bounds__(TCP_THREADS, 2) k_prune_tc(PruneArgs a, float *stack, int *err)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
     __shared__ uint32_t tbase_s;
-    __shared__ __align__(8) uint64_t bar_mma, bar_b;
-    __shared__ float cmax[2][2][TCP_M];
-    __shared__ double red_l[TCP_THREADS / 32], red_e[TCP_THREADS / 32];
-    __shared__ int nbseq_s;
+    __shared__ __align__(8) uint64_t bar_a, bar_mma, bar_b[2];
+    __shared__ float zpart[2][2][TCP_M], prf[K], wlf[K];
+    __shared__ int esc[TCP_M];
+    __shared__ double red_l[TCP_M / 32], red_e[TCP_M / 32];
+    __shared__ int nbseq_s, late_s;
+    __shared__ struct { int w, k, ps, n, done; } ld;   // B loads: see load_next_b (kept by thread 32)
 
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int site = tid & (TCP_M - 1);          // tile column = TMEM lane
-    const int half = tid >> 7;                    // states 32*half .. 32*half+31
-    const int s0 = 32 * half;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int nl = a.nl;
-    uint8_t *lvT = sm + SM_LV;
-    SchedNode *sched = reinterpret_cast<SchedNode *>(sm + SM_LV + ((nl * LV_STRIDE + 15) & ~15));
-    // per contraction (fewer than n_internal): the internal child, in order, and the free
-    // tensor-memory region for D or -1
-    int16_t *bseq = reinterpret_cast<int16_t *>(sched + a.n_internal);
-    int8_t *dreg = reinterpret_cast<int8_t *>(bseq + a.n_internal);
-    const uint32_t barM = smem_addr(&bar_mma), barB = smem_addr(&bar_b);
-    const uint32_t sA = smem_addr(sm + SM_A), sB = smem_addr(sm + SM_B);
-    // kind::tf32, D f32, A/B tf32, both K-major, N = 64, M = 128
-    const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
-    const float *Bop = reinterpret_cast<const float *>(a.Bop);
+    TcNode *sched = reinterpret_cast<TcNode *>(sm + SM_SCHED);
+    int16_t *bseq = reinterpret_cast<int16_t *>(sched + a.n_internal);   // internal child of each contraction, in order
+    uint8_t *lvs = sm + SM_SCHED + tc_sched_bytes(a.n_internal);
+    // operands staged (A), contraction done (M), B operand fetched (B)
+    const uint32_t barA = smem_addr(&bar_a), barM = smem_addr(&bar_mma), barB = smem_addr(bar_b);
+    const uint32_t sB = smem_addr(sm + SM_B);
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     :: "r"(smem_addr(&tbase_s)), "r"(tmem_cols));
+                     :: "r"(smem_addr(&tbase_s)), "r"(TCP_TMEM_COLS));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(barM), "r"(1));
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(barB), "r"(1));
+        mbar_init(barA, TCP_THREADS / 32);
+        mbar_init(barM, 1);
+        mbar_init(barB, 1);
+        mbar_init(barB + 8, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        // replay the schedule's slot occupancy: a contraction takes the region form
-        // when some region holds no live partial (the contracted child's slot stays
-        // live until its epilogue has read it)
-        const uint32_t all = (tmem_cols >= 512) ? 0xFFu : ((1u << (tmem_cols / 64)) - 1u);
-        uint32_t occ = 0;
-        int k = 0;
+    }
+    for (int f = tid; f < a.n_internal; f += TCP_THREADS) {
+        const SchedNode sn = a.sched[f], nx = a.sched[min(f + 1, a.n_internal - 1)];
+        const bool ll = sn.lslot < 0, rl = sn.rslot < 0;
+        TcNode t;
+        t.lc = ll || !rl ? sn.lc : sn.rc;
+        t.rc = ll || !rl ? sn.rc : sn.lc;
+        t.flags = (ll && rl ? TN_LEAVES : ll || rl ? TN_LEAF : 0);
+        if (f + 1 < a.n_internal) {
+            if (nx.lc != sn.node && nx.rc != sn.node) t.flags |= TN_PUSH;
+            if (nx.lslot < 0 && nx.rslot < 0) t.flags |= TN_PAIR;
+        }
+        sched[f] = t;
+    }
+    if (tid == 0) {
+        // contraction order: the child evaluated just before its parent, then the one that waits
+        int k = 0, prev = -1;
         for (int f = 0; f < a.n_internal; f++) {
             const SchedNode sn = a.sched[f];
-            for (int side = 0; side < 2; side++) {
-                const int s = side ? sn.rslot : sn.lslot;
-                if (s < 0) continue;
-                const uint32_t fr = all & ~occ;
-                bseq[k] = side ? sn.rc : sn.lc;
-                dreg[k++] = fr ? (int8_t)(__ffs(fr) - 1) : (int8_t)-1;
-                occ &= ~(1u << s);
+            const bool li = sn.lslot >= 0, ri = sn.rslot >= 0;
+            if (li && ri) {
+                bseq[k++] = prev == sn.lc ? sn.lc : sn.rc;
+                bseq[k++] = prev == sn.lc ? sn.rc : sn.lc;
+            } else if (li || ri) {
+                bseq[k++] = li ? sn.lc : sn.rc;
             }
-            occ |= 1u << sn.oslot;
+            prev = sn.node;
         }
         nbseq_s = k;
     }
-    for (int f = tid; f < a.n_internal; f += TCP_THREADS) sched[f] = a.sched[f];
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tbase = tbase_s;
-    const int nbseq = nbseq_s;
-    const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;   // warp w reaches lanes 32*(w%4)..
-    uint32_t ph_mma = 0, ph_b = 0;      // mbarrier parities (every thread tracks both)
-    // B loads: (work item, index into bseq) of the next load to issue; thread 0 only
-    int ld_w = blockIdx.x, ld_k = 0;
-    int b_inflight = 0;                 // loads issued and not yet waited for (thread 0)
-    bool ok = true;
+    bool bad = false;       // a wait ran out: later waits are skipped, nothing more is issued
+    int n = 0;              // contractions so far
 
-    auto issue_next_b = [&]() {         // thread 0: the buffer is free
-        while (ld_w < a.nwi && ld_k >= nbseq) { ld_w += gridDim.x; ld_k = 0; }
-        if (ld_w >= a.nwi || nbseq == 0) return;
-        const int ps = a.req[a.wi[ld_w].request].pset;
-        const int c = bseq[ld_k++];
-        bulk_load(sB, Bop + ((size_t)ps * a.nbop + (c - nl)) * 2 * K2, 2 * B_BYTES, barB);
-        b_inflight++;
+    // B operands, two contractions ahead (thread 32).  ld: the next load's work item, index into bseq
+    // and P set; loads issued, contractions done.
+    auto load_next_b = [&]() {          // buffer ld.n % 2 is free
+        const int nbseq = nbseq_s;
+        if (ld.w >= a.nwi || nbseq == 0) return;
+        const int c = bseq[ld.k], i = ld.n & 1;
+        bulk_load(sB + i * 2 * B_BYTES, reinterpret_cast<const float *>(a.Bop) + ((size_t)ld.ps * a.nbop + (c - nl)) * 2 * K2,
+                  2 * B_BYTES, barB + 8 * i);
+        ld.n++;
+        if (++ld.k == nbseq) {
+            ld.k = 0;
+            ld.w += gridDim.x;
+            if (ld.w < a.nwi) ld.ps = a.req[a.wi[ld.w].request].pset;
+        }
     };
-    if (tid == 0) issue_next_b();
+    if (tid == 0) late_s = -1;
+    if (tid == 32) {
+        ld.w = blockIdx.x;
+        ld.k = ld.n = ld.done = 0;
+        ld.ps = (int)blockIdx.x < a.nwi ? a.req[a.wi[blockIdx.x].request].pset : 0;
+        load_next_b();
+        load_next_b();
+    }
 
-    // stage alpha of slot s (this thread's 32 states) as the A operand: lo to shared
-    // memory; hi to shared memory (shared form) or back over slot s (region form); with
-    // KEEP, alpha itself stays in al for the epilogue
-    // (the output stores of earlier nodes are waited for here, before the first read)
-    auto stage_a = [&](int s, bool region, float *al) {
-        const uint32_t ts = tbase + lane_off + 64 * s + s0;
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-        if constexpr (KEEP) {
-            tmem_ld16x2(ts, ts + 16, al, al + 16);
-#pragma unroll
-            for (int q = 0; q < 2; q++) {
-                float h[16];
-#pragma unroll
-                for (int j4 = 0; j4 < 4; j4++) {
-                    const float *y = al + 16 * q + 4 * j4;
-                    const float4 hv = make_float4(tf32_hi(y[0]), tf32_hi(y[1]), tf32_hi(y[2]), tf32_hi(y[3]));
-                    const float4 lv = make_float4(y[0] - hv.x, y[1] - hv.y, y[2] - hv.z, y[3] - hv.w);
-                    const uint32_t o = core_off(site, s0 + 16 * q + 4 * j4, 16);
-                    if (!region) *reinterpret_cast<float4 *>(sm + SM_A + o) = hv;
-                    *reinterpret_cast<float4 *>(sm + SM_A + A_BYTES + o) = lv;
-                    h[4 * j4] = hv.x; h[4 * j4 + 1] = hv.y; h[4 * j4 + 2] = hv.z; h[4 * j4 + 3] = hv.w;
-                }
-                if (region) tmem_st16(ts + 16 * q, h);
-            }
-            if (region) asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    // D = A_lo B_hi + A_hi B_lo + A_hi B_hi, once every warp has staged (warp 0, lane 0).
+    // kind::tf32, D f32, A/B tf32, both K-major, N = 64, M = 128.  Descriptors advance in 16-byte
+    // units: K-step 2048 B, lo half 16 KB, buffer 32 KB.
+    const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
+    const uint64_t dB = sdesc(sB, 1024, 128);
+    auto contract = [&]() {
+        if (bad || !mbar_wait(barB + 8 * (n & 1), (n >> 1) & 1) || !mbar_wait(barA, n & 1)) {
+            bad = true;
             return;
         }
-        float x[32];
-        tmem_ld16x2(ts, ts + 16, x, x + 16);
+        tc_fence_after();
+        const uint64_t dBhi = dB + (uint64_t)(n & 1) * (2 * B_BYTES / 16), dBlo = dBhi + B_BYTES / 16;
+        if (NPROD == 3) {
 #pragma unroll
-        for (int j4 = 0; j4 < 8; j4++) {
-            const float4 hv = make_float4(tf32_hi(x[4 * j4]), tf32_hi(x[4 * j4 + 1]), tf32_hi(x[4 * j4 + 2]),
-                                          tf32_hi(x[4 * j4 + 3]));
-            const float4 lv = make_float4(x[4 * j4] - hv.x, x[4 * j4 + 1] - hv.y, x[4 * j4 + 2] - hv.z,
-                                          x[4 * j4 + 3] - hv.w);
-            const uint32_t o = core_off(site, s0 + 4 * j4, 16);
-            if (!region) *reinterpret_cast<float4 *>(sm + SM_A + o) = hv;
-            *reinterpret_cast<float4 *>(sm + SM_A + A_BYTES + o) = lv;
-            x[4 * j4] = hv.x; x[4 * j4 + 1] = hv.y; x[4 * j4 + 2] = hv.z; x[4 * j4 + 3] = hv.w;
-        }
-        if (region) {
-            tmem_st16(ts, x);
-            tmem_st16(ts + 16, x + 16);
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    };
-    // thread 0: wait for the B operand
-    auto wait_b = [&]() -> bool {
-        if (!mbar_wait(barB, ph_b)) return false;
-        ph_b ^= 1u;
-        b_inflight--;
-        return true;
-    };
-    // thread 0, after the staging barrier: D = A B into region r (region form: A hi in
-    // slot s) or over slot s (shared form, r < 0); the same MMA sequence either way
-    // Descriptors of K-step k are the step-0 descriptors plus k times the step in
-    // 16-byte units (A 4096 B, B 2048 B), so the issuing loop is adds only.
-    const uint64_t dAhi = sdesc(sA, 2048, 128), dAlo = sdesc(sA + A_BYTES, 2048, 128);
-    const uint64_t dBhi = sdesc(sB, 1024, 128), dBlo = sdesc(sB + B_BYTES, 1024, 128);
-    auto issue_mma = [&](int s, int r) {
-        const uint32_t dt = tbase + 64 * (r >= 0 ? r : s);
-        const uint32_t ta = tbase + 64 * s;
-        if (r >= 0) {
-            if (NPROD == 3) {
-#pragma unroll
-                for (int k = 0; k < 8; k++) {
-                    mma_tf32(dt, dAlo + 256 * k, dBhi + 128 * k, idesc, k > 0);
-                    mma_tf32_ta(dt, ta + 8 * k, dBlo + 128 * k, idesc, 1);
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < 8; k++) mma_tf32_ta(dt, ta + 8 * k, dBhi + 128 * k, idesc, NPROD == 3 || k > 0);
-        } else {
-            if (NPROD == 3) {
-#pragma unroll
-                for (int k = 0; k < 8; k++) {
-                    mma_tf32(dt, dAlo + 256 * k, dBhi + 128 * k, idesc, k > 0);
-                    mma_tf32(dt, dAhi + 256 * k, dBlo + 128 * k, idesc, 1);
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < 8; k++) mma_tf32(dt, dAhi + 256 * k, dBhi + 128 * k, idesc, NPROD == 3 || k > 0);
-        }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                     :: "r"(barM) : "memory");
-    };
-    // v (or v *=) alpha + D for the internal child in slot s, alpha from the registers
-    // the staging filled (KEEP) or hi + lo from where the staging put them
-    auto child_value = [&](int s, int r, const float *al, float *v, bool mul) {
-        const uint32_t tD = tbase + lane_off + 64 * (r >= 0 ? r : s) + s0;
-        const uint32_t tH = tbase + lane_off + 64 * s + s0;
-#pragma unroll
-        for (int q = 0; q < 2; q++) {
-            float d[16], x[16];
-            if constexpr (KEEP) {
-                tmem_ld16(tD + 16 * q, d);
-#pragma unroll
-                for (int j = 0; j < 16; j++) x[j] = al[16 * q + j];
-            } else if (r >= 0) {
-                tmem_ld16x2(tD + 16 * q, tH + 16 * q, d, x);
-#pragma unroll
-                for (int j4 = 0; j4 < 4; j4++) {
-                    const float4 l = *reinterpret_cast<const float4 *>(
-                        sm + SM_A + A_BYTES + core_off(site, s0 + 16 * q + 4 * j4, 16));
-                    x[4 * j4 + 0] += l.x;
-                    x[4 * j4 + 1] += l.y;
-                    x[4 * j4 + 2] += l.z;
-                    x[4 * j4 + 3] += l.w;
-                }
-            } else {
-                tmem_ld16(tD + 16 * q, d);
-                load_alpha(sm, site, s0, q, x);
-            }
-#pragma unroll
-            for (int j = 0; j < 16; j++) {
-                const float u = x[j] + d[j];
-                v[16 * q + j] = mul ? v[16 * q + j] * u : u;
+            for (int j = 0; j < 8; j++) {
+                mma_tf32_ta(tbase + TM_D, tbase + TM_LO + 8 * j, dBhi + 128 * j, idesc, j > 0);
+                mma_tf32_ta(tbase + TM_D, tbase + TM_HI + 8 * j, dBlo + 128 * j, idesc, 1);
             }
         }
-    };
-    // leaf child: v (or v *=) P_c[a][s] = E^T[s][a] + (a == s), 1 if marginalised
-    auto leaf_value = [&](const float *Pc, int s, float *v, bool mul) {
-        const float *row = Pc + (size_t)(s < K ? s : 0) * K + s0;
 #pragma unroll
-        for (int j8 = 0; j8 < 4; j8++) {
-            float x[8];
-            ldg8(row + 8 * j8, x);
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                const float u = (s < K) ? x[k] + ((s == s0 + 8 * j8 + k) ? 1.0f : 0.0f) : 1.0f;
-                v[8 * j8 + k] = mul ? v[8 * j8 + k] * u : u;
-            }
-        }
-    };
-    // the leaf beside an internal child in two steps: raw E^T row, then the identity
-    // part (or 1 where marginalised)
-    auto leaf_load = [&](const float *Pc, int s, float *v) {
-        const float *row = Pc + (size_t)(s < K ? s : 0) * K + s0;
-#pragma unroll
-        for (int j8 = 0; j8 < 4; j8++) ldg8(row + 8 * j8, v + 8 * j8);
-    };
-    auto leaf_fix = [&](int s, float *v) {
-#pragma unroll
-        for (int j = 0; j < 32; j++) v[j] = (s < K) ? v[j] + ((s == s0 + j) ? 1.0f : 0.0f) : 1.0f;
+        for (int j = 0; j < 8; j++)
+            mma_tf32_ta(tbase + TM_D, tbase + TM_HI + 8 * j, dBhi + 128 * j, idesc, NPROD == 3 || j > 0);
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(barM) : "memory");
     };
 
-    for (int w = blockIdx.x; w < a.nwi && ok; w += gridDim.x) {
+    // a partial of the thread's two columns is v[16]: pair i of column k (states 8 i + 2 (lane % 4),
+    // + 1) at 2 i + k
+    const int c0 = 32 * (warp & 3) + 16 * (warp >> 2);      // the warp's first column (TMEM lane)
+    const uint32_t trow = tbase + ((uint32_t)c0 << 16);
+    float *stk = stack + (size_t)blockIdx.x * prune_tc_levels(a.depth) * (32 * TCP_THREADS) + 2 * tid;
+
+    // a partial into the A operand, hi and lo
+    auto stage = [&](const f2 *x) {
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            f2 h[8], l[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                float y, z;
+                upk(x[8 * q + j], y, z);
+                h[j] = pk(tf32_hi(y), tf32_hi(z));
+                l[j] = sub2(x[8 * q + j], h[j]);
+            }
+            tmem_st_rows(trow + TM_HI + 32 * q, h);
+            if (NPROD == 3) tmem_st_rows(trow + TM_LO + 32 * q, l);
+        }
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        tc_fence_before();
+        warp_arrive(barA, lane);
+    };
+    auto wait_d = [&]() {
+        if (warp == 0) {
+            if (lane == 0) contract();
+            __syncwarp();
+        }
+        if (!bad && !mbar_wait(barM, n & 1)) {
+            bad = true;
+            if (tid == 0) late_s = n & 1;       // its commit may still arrive
+        }
+        n++;
+        __syncwarp();
+        tc_fence_after();
+        if (tid == 32 && !bad) {
+            ld.done++;
+            load_next_b();      // the B operand is free again
+        }
+    };
+
+    for (int w = blockIdx.x; w < a.nwi; w += gridDim.x) {
         const WorkItem wi = a.wi[w];
         const Request rq = a.req[wi.request];
         const int md = rq.model;
         const float *Pbase = reinterpret_cast<const float *>(a.Pbuf) + (size_t)rq.pset * a.nbr * K2;
         const int ncols = wi.ncols;
-        const uint8_t *lg = a.leaves + (size_t)wi.col0 * nl;
-        __syncthreads();
-        for (int f = tid; f < TCP_M * nl; f += TCP_THREADS) {
-            int c = f / nl, l = f - c * nl;
-            lvT[lv_off(l, c)] = (c < ncols) ? lg[f] : (uint8_t)K;
-        }
-        __syncthreads();
-        // warm L1 with the leaf rows (one 128-byte line per thread and leaf) of the node
-        // after ni, while this node waits for its MMAs or its own gathers
-        auto prefetch_next = [&](int ni) {
-            if (ni + 1 >= a.n_internal) return;
-            const SchedNode nx = sched[ni + 1];
-            if (nx.lslot < 0) {
-                const int sa = lvT[lv_off(nx.lc, site)];
-                asm volatile("prefetch.global.L1 [%0];" :: "l"(Pbase + (size_t)nx.lc * K2 + (size_t)(sa < K ? sa : 0) * K + s0));
+        // the warp's leaf states (K: missing, and columns past the end)
+        {
+            const uint8_t *lg = a.leaves + ((size_t)wi.col0 + c0) * nl;
+            const int nf = max(min(ncols - c0, 16), 0) * nl;
+            __syncwarp();
+            for (int f0 = 0; f0 < 16 * nl; f0 += 32 * 16) {
+                uint8_t x[16];
+#pragma unroll
+                for (int i = 0; i < 16; i++) {
+                    const int f = f0 + 32 * i + lane;
+                    x[i] = f < nf ? __ldg(lg + f) : (uint8_t)K;
+                }
+#pragma unroll
+                for (int i = 0; i < 16; i++) {
+                    const int f = f0 + 32 * i + lane, c = f / nl;
+                    if (f < 16 * nl) lvs[lv_off(f - c * nl, c0 + c)] = x[i];
+                }
             }
-            if (nx.rslot < 0) {
-                const int sb = lvT[lv_off(nx.rc, site)];
-                asm volatile("prefetch.global.L1 [%0];" :: "l"(Pbase + (size_t)nx.rc * K2 + (size_t)(sb < K ? sb : 0) * K + s0));
+            __syncwarp();
+        }
+        // rows of a leaf's P^T (ones where it is missing) for the thread's two columns
+        auto leaf_rows = [&](int l, f2 *x) {
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                const int s = lvs[lv_off(l, c0 + 8 * k + (lane >> 2))];
+                const float *p = (s < K ? Pbase + (size_t)l * K2 + s * K : ones_row) + 8 * (lane & 3);
+                ldg4(p, x[k], x[2 + k], x[4 + k], x[6 + k]);
+                ldg4(p + 32, x[8 + k], x[10 + k], x[12 + k], x[14 + k]);
             }
         };
-        int escale = 0;     // this column's sum of rescale exponents
-        bool pend_bad = false;   // a timed-out wait seen since the last CTA-wide barrier
-        int kc = 0;         // contractions so far (index into bseq / dreg)
+        int escale[2] = {0, 0};     // the columns' sums of rescale exponents
+        int sp = 0;                 // stack entries in use
+        f2 v[16];                   // a node's partial under construction, then normalised
+        TcNode sn = sched[0];
 
-        for (int ni = 0; ni < a.n_internal && ok; ni++) {
-            const SchedNode sn = sched[ni];
-            float v[32];
-            // internal children are contracted one after the other (l before r); a
-            // leaf child beside an internal one is gathered while the MMAs run, except by
-            // warp 0, whose thread 0 issues them (all warps loading before the staging
-            // measured slower).  Every barrier also agrees on a timed-out wait (bad), so
-            // that all threads leave together.
-            const int slotL = sn.lslot, slotR = sn.rslot;
-            const int nint = (slotL >= 0) + (slotR >= 0);
-            const int lfc = (slotL < 0) ? sn.lc : sn.rc;   // the leaf child when nint == 1
-            // warp 0 (whose thread 0 issues the MMAs) loads its leaf rows before the staging
-            int ls0 = K;
-            if (nint == 1 && warp == 0) {
-                ls0 = lvT[lv_off(lfc, site)];
-                leaf_load(Pbase + (size_t)lfc * K2, ls0, v);
-            }
-            bool have = (nint == 1), bad = false;
-            int nc = 0;
-            for (int side = 0; side < 2; side++) {
-                const int s = side ? slotR : slotL;
-                if (s < 0) continue;
-                // the A operand is free again (with KEEP it is once the MMAs have completed,
-                // and the first child's D is read before the staging barrier below)
-                if (!KEEP && nc && __syncthreads_or(bad)) { ok = false; break; }
-                nc++;
-                const int r = dreg[kc++];
-                float al[KEEP ? 32 : 1];
-                stage_a(s, r >= 0, al);
-                if (tid == 0 && !wait_b()) bad = true;
-                tc_fence_before();
-                if (__syncthreads_or(bad || pend_bad)) { ok = false; break; }
-                tc_fence_after();
-                if (tid == 0) issue_mma(s, r);
-                prefetch_next(ni);      // while the MMAs run
-                if (nint == 1) {
-                    if (warp != 0) {
-                        ls0 = lvT[lv_off(lfc, site)];
-                        leaf_load(Pbase + (size_t)lfc * K2, ls0, v);
-                    }
-                    leaf_fix(ls0, v);
+#pragma unroll 1
+        for (int ni = 0; ni < a.n_internal; ni++) {
+            const int fl = sn.flags;
+            f2 x[16];
+            if (fl & TN_LEAVES) {
+                leaf_rows(sn.lc, v);
+                leaf_rows(sn.rc, x);
+                
+#pragma unroll
+                for (int j = 0; j < 16; j++) v[j] = mul2(v[j], x[j]);
+            } else {
+                // the last node's partial (in v) is contracted first
+                stage(v);
+                if (fl & TN_LEAF) {
+                    leaf_rows(sn.lc, x);
+                } else if (--sp == 0) {
+                    tmem_ld_rows(trow + TM_S, x);
+                    tmem_ld_rows(trow + TM_S + 32, x + 8);
+                } else {
+                    const f2 *e = reinterpret_cast<const f2 *>(stk + (size_t)(sp - 1) * (32 * TCP_THREADS));
+#pragma unroll
+                    for (int j = 0; j < 16; j++) x[j] = e[j * TCP_THREADS];
                 }
-                const bool done = mbar_wait(barM, ph_mma);
-                tc_fence_after();
-                if (!done) bad = true;
-                else ph_mma ^= 1u;   // after a timed-out wait the quiesce waits for this phase
-                if (tid == 0 && done) issue_next_b();     // the B operand is free again
-                child_value(s, r, al, v, have);
-                have = true;
+                
+                wait_d();
+#pragma unroll
+                for (int q = 0; q < 2; q++) {
+                    f2 d[8];
+                    tmem_ld_rows(trow + TM_D + 32 * q, d);
+#pragma unroll
+                    for (int j = 0; j < 8; j++) v[8 * q + j] = add2(v[8 * q + j], d[j]);
+                }
+                if (fl & TN_LEAF) {
+#pragma unroll
+                    for (int j = 0; j < 16; j++) v[j] = mul2(v[j], x[j]);
+                } else {
+                    // then the one from the stack
+                    stage(x);
+                    wait_d();
+#pragma unroll
+                    for (int q = 0; q < 2; q++) {
+                        f2 d[8];
+                        tmem_ld_rows(trow + TM_D + 32 * q, d);
+#pragma unroll
+                        for (int j = 0; j < 8; j++) v[8 * q + j] = mul2(v[8 * q + j], add2(x[8 * q + j], d[j]));
+                    }
+                }
             }
-            if (!ok) break;
-            if (nint == 0) {
-                leaf_value(Pbase + (size_t)sn.lc * K2, lvT[lv_off(sn.lc, site)], v, false);
-                leaf_value(Pbase + (size_t)sn.rc * K2, lvT[lv_off(sn.rc, site)], v, true);
+            sn = sched[min(ni + 1, a.n_internal - 1)];
+            // ---- rescale each column by an exact power of two
+            float mx[2];
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                float m0 = 0.0f, m1 = 0.0f;
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    float y, z;
+                    upk(v[2 * i + k], y, z);
+                    m0 = fmaxf(m0, y);
+                    m1 = fmaxf(m1, z);
+                }
+                mx[k] = fmaxf(m0, m1);
             }
-            // ---- rescale by an exact power of two and park in the output slot
-            float mx = 0.0f;
 #pragma unroll
-            for (int k = 0; k < 32; k++) mx = fmaxf(mx, v[k]);
-            float (*cm)[TCP_M] = cmax[ni & 1];          // double-buffered: no second barrier needed
-            cm[half][site] = mx;
-            // only warps w and w + 4 share these columns: a named barrier of those 64 threads
-            // (barriers 1-4; both warps walk the same schedule, so both always arrive).  A
-            // timed-out wait is carried to the next CTA-wide barrier (the next staging, or the
-            // root), which every thread reaches before any further MMA is issued.
-            asm volatile("bar.sync %0, 64;" :: "r"(1 + (warp & 3)) : "memory");
-            pend_bad |= bad;
-            mx = fmaxf(cm[0][site], cm[1][site]);
-            const int e = (mx > 0.0f) ? exp_of(mx) : 0;
-            escale += e;
-            const uint32_t tO = tbase + lane_off + 64 * sn.oslot + s0;
+            for (int o = 1; o < 4; o <<= 1) {
 #pragma unroll
-            for (int q = 0; q < 2; q++) {
-                float y[16];
+                for (int k = 0; k < 2; k++) mx[k] = fmaxf(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], o));
+            }
+            // the biased exponents: a normal maximum below 2^126 scales with one multiplication
+            const int b0 = __float_as_int(mx[0]) >> 23, b1 = __float_as_int(mx[1]) >> 23;
+            if (__all_sync(0xffffffffu, min(b0, b1) > 0 && max(b0, b1) < 253)) {
+                const float g0 = __int_as_float((253 - b0) << 23), g1 = __int_as_float((253 - b1) << 23);
+                escale[0] += b0 - 126;
+                escale[1] += b1 - 126;
+                const f2 gg[2] = {pk(g0, g0), pk(g1, g1)};
 #pragma unroll
-                for (int j = 0; j < 16; j++) y[j] = scale2(v[16 * q + j], -e);
-                tmem_st16(tO + 16 * q, y);
+                for (int j = 0; j < 16; j++) v[j] = mul2(v[j], gg[j & 1]);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+                    const int e = mx[k] > 0.0f ? exp_of(mx[k]) : 0;
+                    escale[k] += e;
+                    const float h = scale2(1.0f, -(e >> 1)), l = scale2(1.0f, -(e - (e >> 1)));
+#pragma unroll
+                    for (int i = 0; i < 8; i++) v[2 * i + k] = mul2(mul2(v[2 * i + k], pk(h, h)), pk(l, l));
+                }
+            }
+            if (fl & TN_PUSH) {
+                if (sp == 0) {
+                    tmem_st_rows(trow + TM_S, v);
+                    tmem_st_rows(trow + TM_S + 32, v + 8);
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                } else {
+                    f2 *t = reinterpret_cast<f2 *>(stk + (size_t)(sp - 1) * (32 * TCP_THREADS));
+#pragma unroll
+                    for (int k = 0; k < 16; k++) t[k * TCP_THREADS] = v[k];
+                }
+                sp++;
             }
         }
-        if (!ok) break;
-        // ---- root: z = alpha_root . prior (FP32, compensated) and the elpr term per column;
-        // log z = log m + e ln 2 with m in [0.5, 1) (logf of m is within ~4e-8 absolute,
-        // far below the tensor-core noise of these search values); FP64 only for the
-        // per-column log and the sums over the tile (this part's FP64 rate is ~1/64 of FP32)
-        // (the A operand is idle here: [2][2][128] partial sums, then the model's prior and
-        // prior * log prior in FP32)
-        float *zpart = reinterpret_cast<float *>(sm + SM_A);
-        float *prf = zpart + 4 * TCP_M, *wlf = prf + K;
-        if (__syncthreads_or(pend_bad)) { ok = false; break; }   // every warp is past its last node
+        // ---- root, two threads per column: z = alpha_root . prior (FP32, compensated) and the
+        // elpr term; log z = log m + e ln 2 with m in [0.5, 1) (logf of m is within ~4e-8
+        // absolute, far below the tensor-core noise of these search values); FP64 only for the
+        // per-column log and the sums over the tile (this part's FP64 rate is ~1/64 of FP32).
+        // The partials change threads through the idle A operand.
+        tmem_st_rows(trow + TM_HI, v);
+        tmem_st_rows(trow + TM_HI + 32, v + 8);
+        if ((lane & 3) == 0) {
+            esc[c0 + (lane >> 2)] = escale[0];
+            esc[c0 + 8 + (lane >> 2)] = escale[1];
+        }
         if (tid < K) {
             prf[tid] = (float)a.m.prior[md * K + tid];
             wlf[tid] = (float)a.m.wlog[md * K + tid];
         }
-        __syncthreads();
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        tc_fence_before();
+        bad = __syncthreads_or(bad);
+        if (bad) break;
+        tc_fence_after();
+        const int site = tid & (TCP_M - 1), half = tid >> 7, s0 = 32 * half;
+        const int es = esc[site];
         {
-            const uint32_t tR = tbase + lane_off + 64 * sched[a.n_internal - 1].oslot + s0;
+            const uint32_t t = tbase + ((uint32_t)(32 * (warp & 3)) << 16) + TM_HI + s0;
             float z = 0.0f, zc = 0.0f, wz = 0.0f;
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");   // the root's output store
 #pragma unroll
             for (int q = 0; q < 2; q++) {
-                float x[16];
-                tmem_ld16(tR + 16 * q, x);
+                float u[16];
+                tmem_ld16(t + 16 * q, u);
 #pragma unroll
                 for (int j = 0; j < 16; j++) {
-                    const float y = x[j] * prf[s0 + 16 * q + j] - zc;
-                    const float t = z + y;
-                    zc = (t - z) - y;
-                    z = t;
-                    wz = fmaf(x[j], wlf[s0 + 16 * q + j], wz);
+                    const float y = u[j] * prf[s0 + 16 * q + j] - zc;
+                    const float r = z + y;
+                    zc = (r - z) - y;
+                    z = r;
+                    wz = fmaf(u[j], wlf[s0 + 16 * q + j], wz);
                 }
             }
-            zpart[(half * 2 + 0) * TCP_M + site] = z;
-            zpart[(half * 2 + 1) * TCP_M + site] = wz;
+            zpart[half][0][site] = z;
+            zpart[half][1][site] = wz;
         }
+        tc_fence_before();
         __syncthreads();
+        tc_fence_after();
         if (half == 0) {
             double tl = 0.0, te = 0.0;
             if (site < ncols) {
-                const float z = zpart[0 * TCP_M + site] + zpart[2 * TCP_M + site];
-                const float wz = zpart[1 * TCP_M + site] + zpart[3 * TCP_M + site];
+                const float z = zpart[0][0][site] + zpart[1][0][site];
+                const float wz = zpart[0][1][site] + zpart[1][1][site];
                 if (z > 0.0f) {
                     int ez;
                     const float mz = frexpf(z, &ez);
-                    tl = (double)logf(mz) + (double)(ez + escale) * 0.69314718055994530942;
+                    tl = (double)logf(mz) + (double)(ez + es) * 0.69314718055994530942;
                     te = (double)(wz / z);
                 } else {
                     tl = -INFINITY;
@@ -497,114 +484,91 @@ __global__ void __launch_bounds__(TCP_THREADS, 2) k_prune_tc(PruneArgs a, uint32
                 tl += __shfl_down_sync(0xffffffffu, tl, o);
                 te += __shfl_down_sync(0xffffffffu, te, o);
             }
-            if ((tid & 31) == 0) { red_l[warp] = tl; red_e[warp] = te; }
-        }
-        tc_fence_before();
-        __syncthreads();
-        if (tid == 0) {
-            double sl = 0.0, se = 0.0;
-            for (int k = 0; k < TCP_M / 32; k++) { sl += red_l[k]; se += red_e[k]; }
-            a.partials[2 * (size_t)w] = sl;
-            a.partials[2 * (size_t)w + 1] = se;
-        }
-    }
-    if (!ok && tid == 0) atomicExch(err, 1);
-    // quiesce: a bulk copy may be outstanding (loads run one ahead), and after a
-    // timed-out MMA wait its commit may still arrive; both waits are bounded
-    if (tid == 0) {
-        while (b_inflight > 0) {
-            if (!mbar_wait(barB, ph_b)) { atomicExch(err, 1); break; }
-            ph_b ^= 1u;
-            b_inflight--;
+            if (lane == 0) { red_l[warp] = tl; red_e[warp] = te; }
+            asm volatile("bar.sync 6, 128;" ::: "memory");
+            if (tid == 0) {
+                double sl = 0.0, se = 0.0;
+                for (int k = 0; k < TCP_M / 32; k++) { sl += red_l[k]; se += red_e[k]; }
+                a.partials[2 * (size_t)w] = sl;
+                a.partials[2 * (size_t)w + 1] = se;
+            }
         }
     }
-    if (!ok) mbar_wait(barM, ph_mma);
-    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    // quiesce: bulk copies may be outstanding, and after a timed-out wait for a contraction its
+    // commit may still arrive; every wait is bounded
+    if (tid == 32) {
+        for (int i = ld.done; i < ld.n; i++) {
+            if (!mbar_wait(barB + 8 * (i & 1), (i >> 1) & 1)) bad = true;
+        }
+    }
+    if (tid == 0 && late_s >= 0) mbar_wait(barM, late_s);
+    if (bad && lane == 0) atomicExch(err, 1);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tbase), "r"(tmem_cols));
-}
-
-static uint32_t tmem_cols_for(int nslots)
-{
-    // at least four regions, so that most contractions find a free one for D
-    uint32_t need = (uint32_t)(64 * (nslots > 0 ? nslots : 1)), c = 256;
-    while (c < need) c <<= 1;
-    return c;
-}
-
-size_t prune_tc_smem_bytes(int nl, int nint)
-{
-    // operands, leaf states, the schedule, then per contraction the child and the D region
-    return SM_LV + (((size_t)nl * LV_STRIDE + 15) & ~(size_t)15) + (size_t)nint * (sizeof(SchedNode) + 3);
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tbase), "r"(TCP_TMEM_COLS));
 }
 
 bool prune_tc_supported(int nslots, int nl) { return nslots <= TCP_MAX_SLOTS && nl <= TCP_MAX_LEAVES; }
 
 bool prune_tc_shape_ok(int shape) { return shape >= 0 && shape < PCSF_TC_SHAPES; }
 
-template <int NPROD, bool KEEP>
+size_t prune_tc_smem_bytes(int nl, int nint) { return SM_SCHED + tc_sched_bytes(nint) + (size_t)nl * LV_STRIDE; }
+
+template <int NPROD>
 static cudaError_t set_tc_attributes(size_t smem)
 {
-    // the whole unified L1 as shared memory, so that two CTAs of ~115 KB fit
-    cudaError_t e = cudaFuncSetAttribute(k_prune_tc<NPROD, KEEP>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    // the whole unified L1 as shared memory, so that three CTAs of ~75 KB fit
+    cudaError_t e = cudaFuncSetAttribute(k_prune_tc<NPROD>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                          (int)cudaSharedmemCarveoutMaxShared);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_prune_tc<NPROD, KEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = cudaFuncSetAttribute(k_prune_tc<NPROD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     return e;
 }
 
-// CTAs per SM: the smaller of what shared memory and registers allow (from the
-// kernel's attributes and the device limits) and what tensor memory allows
-template <bool KEEP>
-static int ctas_per_sm(int nslots, int nl, int nint)
+// CTAs of dynamic shared memory smem that fit an SM: the smaller of what shared memory and
+// registers allow (from the kernel's attributes and the device limits) and what tensor memory allows
+static int ctas_that_fit(size_t smem)
 {
-    const uint32_t cols = tmem_cols_for(nslots);
-    const int by_tmem = (int)(512 / cols);
-    const size_t smem = prune_tc_smem_bytes(nl, nint);
     cudaFuncAttributes fa, fa1;
     int dev = 0, smem_sm = 0, regs_sm = 0, reserved = 0;
-    if (set_tc_attributes<3, KEEP>(smem) != cudaSuccess || set_tc_attributes<1, KEEP>(smem) != cudaSuccess ||
-        cudaFuncGetAttributes(&fa, k_prune_tc<3, KEEP>) != cudaSuccess ||
-        cudaFuncGetAttributes(&fa1, k_prune_tc<1, KEEP>) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess ||
+    if (cudaFuncGetAttributes(&fa, k_prune_tc<3>) != cudaSuccess || cudaFuncGetAttributes(&fa1, k_prune_tc<1>) != cudaSuccess ||
+        cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&regs_sm, cudaDevAttrMaxRegistersPerMultiprocessor, dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess)
         return 1;
     const size_t stat = fa.sharedSizeBytes > fa1.sharedSizeBytes ? fa.sharedSizeBytes : fa1.sharedSizeBytes;
     const int regs = fa.numRegs > fa1.numRegs ? fa.numRegs : fa1.numRegs;
-    const int by_smem = (int)((size_t)smem_sm / (stat + smem + (size_t)reserved));
-    const int by_regs = regs_sm / (regs * TCP_THREADS);
-    int n = by_tmem;
-    if (by_smem < n) n = by_smem;
-    if (by_regs < n) n = by_regs;
+    int n = (int)(512 / TCP_TMEM_COLS);
+    n = std::min(n, (int)((size_t)smem_sm / (stat + smem + (size_t)reserved)));
+    n = std::min(n, regs_sm / (regs * TCP_THREADS));
     return n > 0 ? n : 1;
 }
 
-// shapes: 0 = alpha kept in registers, 1 = alpha read back from the operands
-int prune_tc_ctas_per_sm(int nslots, int nl, int nint, int shape)
+// shapes: 0 = every CTA that fits an SM (two), 1 = one
+int prune_tc_ctas_per_sm(int nl, int nint, int shape)
 {
-    return shape == 1 ? ctas_per_sm<false>(nslots, nl, nint) : ctas_per_sm<true>(nslots, nl, nint);
+    return shape == 1 ? 1 : ctas_that_fit(prune_tc_smem_bytes(nl, nint));
 }
 
-template <int NPROD, bool KEEP>
-static cudaError_t launch_tc(const PruneArgs &a, int *err, cudaStream_t s, int grid)
+size_t prune_tc_stack_floats(int grid, int depth) { return (size_t)grid * prune_tc_levels(depth) * 32 * TCP_THREADS; }
+
+template <int NPROD>
+static cudaError_t launch_tc(const PruneArgs &a, float *stack, int *err, cudaStream_t s, int grid)
 {
     const size_t smem = prune_tc_smem_bytes(a.nl, a.n_internal);
-    cudaError_t e = set_tc_attributes<NPROD, KEEP>(smem);
+    cudaError_t e = set_tc_attributes<NPROD>(smem);
     if (e != cudaSuccess) return e;
-    k_prune_tc<NPROD, KEEP><<<grid, TCP_THREADS, smem, s>>>(a, tmem_cols_for(a.nslots), err);
+    k_prune_tc<NPROD><<<grid, TCP_THREADS, smem, s>>>(a, stack, err);
     return cudaGetLastError();
 }
 
-cudaError_t launch_prune_tc(int nprod, const PruneArgs &a, int *err, cudaStream_t s, int grid)
+cudaError_t launch_prune_tc(int nprod, const PruneArgs &a, float *stack, int *err, cudaStream_t s, int grid)
 {
     if (a.nwi <= 0) return cudaSuccess;
-    const bool keep = a.tc_shape != 1;
-    if (nprod == 3) return keep ? launch_tc<3, true>(a, err, s, grid) : launch_tc<3, false>(a, err, s, grid);
-    return keep ? launch_tc<1, true>(a, err, s, grid) : launch_tc<1, false>(a, err, s, grid);
+    return nprod == 3 ? launch_tc<3>(a, stack, err, s, grid) : launch_tc<1>(a, stack, err, s, grid);
 }
 
 }  // namespace pcsf

@@ -43,7 +43,7 @@ constexpr int PFT_TARGET = 4 * 3 * 152;   // CTAs of a launch: four waves of thr
 
 __global__ void __launch_bounds__(PFT_THREADS) k_pform_tc(const PSet *ps, const double *branch, int nbr, int nl,
                                                           DevModels m, const float *Bpf, float *Pbuf, float *Bop,
-                                                          int32_t *status_key, int *err, int per_cta)
+                                                          int32_t *status_key, int *err, int per_cta, int leaf_rows)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
     __shared__ uint32_t tbase_s;
@@ -208,8 +208,9 @@ __global__ void __launch_bounds__(PFT_THREADS) k_pform_tc(const PSet *ps, const 
                 diag = dj ? diag : s;
                 dc = dj ? dc : c;
             }
+            const float dv = leaf_rows && b < nl ? diag + 1.0f : diag;
 #pragma unroll
-            for (int j = 0; j < K; j++) row[j] = (j == i) ? diag : row[j];
+            for (int j = 0; j < K; j++) row[j] = (j == i) ? dv : row[j];
             const double rs = rowsum_minus_one(m, md, i, exs[bsel]);
             if (neg) status_min(status_key + r, b, i, PCSF_ENEGP);
             else if (fabs(rs) > m.tol) status_min(status_key + r, b, i, PCSF_EROWSUM);
@@ -219,8 +220,8 @@ __global__ void __launch_bounds__(PFT_THREADS) k_pform_tc(const PSet *ps, const 
 #pragma unroll
                 for (int q = 0; q < K / 4; q++)
                     bop_store(dst, i, q, make_float4(row[4 * q], row[4 * q + 1], row[4 * q + 2], row[4 * q + 3]));
-            } else {            // above a leaf: E^T rows for the gathers
-                float *out = Pbuf + ((size_t)r * nbr + b) * K2;
+            } else {            // above a leaf: E^T rows for the gathers, or k_prune_tc's P^T rows
+                float *out = Pbuf + ((size_t)r * nbr + b) * K2 + (leaf_rows ? leaf_pos(i) - i : 0);
 #pragma unroll
                 for (int j = 0; j < K; j++) out[(size_t)j * K + i] = row[j];
             }
@@ -239,7 +240,8 @@ __global__ void __launch_bounds__(PFT_THREADS) k_pform_tc(const PSet *ps, const 
 }
 
 cudaError_t launch_pform_tc(const PSet *ps, int nps, const double *branch, int nbr, int nl, DevModels m,
-                            const float *Bpf, float *Pbuf, float *Bop, int32_t *status_key, int *err, cudaStream_t s)
+                            const float *Bpf, float *Pbuf, float *Bop, int32_t *status_key, int *err, cudaStream_t s,
+                            bool leaf_rows)
 {
     if (nps <= 0) return cudaSuccess;
     cudaError_t e = cudaFuncSetAttribute(k_pform_tc, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -255,7 +257,8 @@ cudaError_t launch_pform_tc(const PSet *ps, int nps, const double *branch, int n
     const int want = std::min(pairs, std::max(1, (PFT_TARGET + nps - 1) / nps));
     const int per_cta = 2 * ((pairs + want - 1) / want);
     const dim3 grid(nps, (nbr + per_cta - 1) / per_cta);
-    k_pform_tc<<<grid, PFT_THREADS, PFT_SMEM, s>>>(ps, branch, nbr, nl, m, Bpf, Pbuf, Bop, status_key, err, per_cta);
+    k_pform_tc<<<grid, PFT_THREADS, PFT_SMEM, s>>>(ps, branch, nbr, nl, m, Bpf, Pbuf, Bop, status_key, err, per_cta,
+                                                       leaf_rows ? 1 : 0);
     return cudaGetLastError();
 }
 

@@ -484,7 +484,7 @@ class Engine:
                                        _p(st, ctypes.c_int32)), self.handle)
         return P, st
 
-    TC_SHAPES = {0: "alpha kept in registers", 1: "alpha read back"}
+    TC_SHAPES = {0: "every CTA that fits an SM", 1: "one CTA per SM"}
 
     def set_derivative_mode(self, mode: int) -> None:
         """Search derivative of the mle derivative rule: 1 central difference of search values
