@@ -499,7 +499,7 @@ static int setup_models(pcsf_engine *e, const double *Q[2], const double *eq[2],
     if (e->prec == PCSF_PREC_TF32X3 || e->prec == PCSF_PREC_TF32) {
         // B operand of the tensor-core P(t) formation: B[j][m] = U_jm sqrt(pi_j), TF32 hi / lo,
         // K-major core-matrix layout (element (j, m) at float (m/4)*256 + j*4 + m%4 of its part)
-        std::vector<float> bpf((size_t)2 * 2 * K2);
+        std::vector<float> bpf((size_t)6 * K2);
         for (int m = 0; m < 2; m++)
             for (int j = 0; j < K; j++)
                 for (int mm = 0; mm < K; mm++) {
@@ -513,6 +513,11 @@ static int setup_models(pcsf_engine *e, const double *Q[2], const double *eq[2],
                     bpf[o] = hi;
                     bpf[o + K2] = x - hi;
                 }
+        // then per model isq_i U_im, from which the kernel scales its A operand: [m / 4][i][m % 4]
+        for (int m = 0; m < 2; m++)
+            for (int i = 0; i < K; i++)
+                for (int mm = 0; mm < K; mm++)
+                    bpf[(size_t)(4 + m) * K2 + (mm / 4) * 256 + i * 4 + mm % 4] = (float)e->isq[m][i] * e->Uf[m][i * K + mm];
         // B operand of Q for the tangent pass: B[a][j] = Q[a][j], same layout
         std::vector<float> qop((size_t)2 * 2 * K2);
         for (int m = 0; m < 2; m++)

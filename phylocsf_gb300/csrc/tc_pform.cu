@@ -20,9 +20,18 @@
 // launch has few P sets (launch_pform_tc).  A_hi sits in tensor
 // memory (columns 64..127, lane r = row r) and only A_lo in shared memory, so a CTA
 // takes 64 KB of shared memory and 128 tensor-memory columns and three CTAs share an
-// SM (the kernel is bound by the latency of its per-pair chain).  mbarrier waits are bounded as in the pruning
-// kernel; on timeout the CTA records an error, waits (bounded) for its MMAs,
-// frees its tensor memory and stops.
+// SM.  mbarrier waits are bounded as in the pruning kernel; on timeout the CTA records an
+// error, waits (bounded) for its MMAs, frees its tensor memory and stops.
+//
+// What bounds it: the latency of its per-pair chain, 13,300 clocks beside two other CTAs
+// (19,200 before): the rows of E(t_g) from L2 while the MMAs run 3,500, A 2,700 (4,900 when
+// each lane read its own row of U: 32 lines an instruction; the host lays isq U out for
+// coalesced reads now), the row's compensated sum 2,500 (3,800 with selects in its chain
+// and a second pass to insert the diagonal), 1,600 of MMA issue, the row-sum check 850
+// (1,900 with its operands looked up for every pair), and the next pair's coefficients
+// formed in the MMAs' shadow.  Issue slots are a third used, HBM writes 30 %.  Measured, all
+// P(t) launches of a call: 384 regions on 58 leaves 13.7 -> 11.2 ms, 256 regions on 100
+// leaves 8.1 -> 7.4 ms, ORF sets 1.42 -> 1.25 ms.
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -41,15 +50,15 @@ constexpr uint32_t PFT_TMEM_COLS = 128;   // D in 0..63, A_hi in 64..127
 constexpr int PFT_MAX_BRANCHES = 320;
 constexpr int PFT_TARGET = 4 * 3 * 152;   // CTAs of a launch: four waves of three per SM
 
-__global__ void __launch_bounds__(PFT_THREADS) k_pform_tc(const PSet *ps, const double *branch, int nbr, int nl,
+__global__ void __launch_bounds__(PFT_THREADS, 3) k_pform_tc(const PSet *ps, const double *branch, int nbr, int nl,
                                                           DevModels m, const float *Bpf, float *Pbuf, float *Bop,
                                                           int32_t *status_key, int *err, int per_cta, int leaf_rows)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
     __shared__ uint32_t tbase_s;
     __shared__ __align__(8) uint64_t bar_mma, bar_b;
-    __shared__ float cfs[2][K];
-    __shared__ double exs[2][K];        // expm1(lam_m t) where w_m != 0 (row-sum check)
+    __shared__ float cfs[2][2][K];      // [pair parity][branch of the pair]
+    __shared__ double exs[2][2][K];     // expm1(lam_m t) where w_m != 0 (row-sum check)
     __shared__ int mode_g[PFT_MAX_BRANCHES];      // per branch: grid point << 2 | mode
     __shared__ float t_b[PFT_MAX_BRANCHES];       // t (FP32: the Taylor branch and expm1f only)
     __shared__ float h_b[PFT_MAX_BRANCHES];       // t - t_g, formed in FP64
@@ -62,7 +71,7 @@ __global__ void __launch_bounds__(PFT_THREADS) k_pform_tc(const PSet *ps, const 
     const uint32_t barM = smem_addr(&bar_mma), barB = smem_addr(&bar_b);
     const uint32_t sA = smem_addr(sm + PFT_A), sB = smem_addr(sm + PFT_B);
     const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
-    const float *Uf = m.Uf + (size_t)md * K2;
+    const float4 *Uq = reinterpret_cast<const float4 *>(Bpf + 4 * K2 + (size_t)md * K2);   // [m / 4][i] isq_i U_im
     const double *lam = m.lam + md * K;
     const double *wrow = m.wrow + md * K;
     const int i = tid & (K - 1), bsel = tid >> 6;      // this thread's row: branch b0 + bsel, state i
@@ -89,7 +98,6 @@ __global__ void __launch_bounds__(PFT_THREADS) k_pform_tc(const PSet *ps, const 
     const uint32_t lane_off = (uint32_t)(((tid >> 5) & 3) * 32) << 16;
     uint32_t ph = 0;
     bool pending = false;               // an MMA group was issued and its completion not seen
-    const float isq_i = (float)m.isq[md * K + i];
     // per branch: 0 t = 0, 1 below the grid (Taylor), 2 grid correction at point g
     for (int b = bb0 + tid; b < bb1; b += PFT_THREADS) {
         const double t = rq.rho * branch[b];
@@ -119,31 +127,41 @@ __global__ void __launch_bounds__(PFT_THREADS) k_pform_tc(const PSet *ps, const 
             for (int k = 0; k < WLIST; k++) listed |= (wl[k] == i);
     }
     const float ntol = -(float)m.tol, dtol = (float)(-1.0 - m.tol);
+    // the row-sum check's one term (rowsum_minus_one), where the model has just one
+    const int w0 = m.wlist[md * WLIST];
+    const bool one_w = w0 >= 0 && m.wlist[md * WLIST + 1] < 0;
+    const double wu = one_w ? m.U[(size_t)md * K2 + (size_t)i * K + w0] : 0.0, ww = one_w ? wrow[w0] : 0.0;
+    const double isq_i = m.isq[md * K + i];
 
-    for (int b0 = bb0; b0 < bb1; b0 += 2) {
+    // the coefficients cf of a pair of branches: thread (bsel, i) supplies coefficient m = i
+    auto coefficients = [&](int b0, int par) {
+        const int b = b0 + bsel;
+        const int mg = (b < bb1) ? mode_g[b] : 0;
+        float cf = 0.0f;
+        if ((mg & 3) == 2) cf = m.grid_eg[((size_t)md * m.grid_n + (mg >> 2)) * K + i] * expm1f(lam_i * h_b[b]);
+        cfs[par][bsel][i] = cf;
+        exs[par][bsel][i] = listed ? (double)expm1f(lam_i * (b < bb1 ? t_b[b] : 0.0f)) : 0.0;
+    };
+    __syncthreads();                                  // per-branch table ready
+    coefficients(bb0, 0);
+
+    for (int b0 = bb0, par = 0; b0 < bb1; b0 += 2, par ^= 1) {
         const int b = b0 + bsel;                      // this thread's branch
-        if (__syncthreads_or(!ok)) break;             // per-branch table ready / previous pair done
+        if (__syncthreads_or(!ok)) break;             // coefficients ready / previous pair done
         const int mode = (b < bb1) ? (mode_g[b] & 3) : 0, g = (b < bb1) ? (mode_g[b] >> 2) : 0;
         const float t = (b < bb1) ? t_b[b] : 0.0f;
-        {
-            float cf = 0.0f;
-            if (mode == 2) cf = m.grid_eg[((size_t)md * m.grid_n + g) * K + i] * expm1f(lam_i * h_b[b]);
-            cfs[bsel][i] = cf;      // thread (bsel, i) supplies coefficient m = i
-            exs[bsel][i] = listed ? (double)expm1f(lam_i * t) : 0.0;
-        }
-        __syncthreads();
         // ---- A operand: row tid = isq_i U_im cf_m, TF32 hi (tensor memory) / lo (shared)
         {
-            const float4 *urow = reinterpret_cast<const float4 *>(Uf + (size_t)i * K);
+            const float *cf = cfs[par][bsel];
 #pragma unroll 1
             for (int c = 0; c < 4; c++) {
                 float h[16];
 #pragma unroll
                 for (int q4 = 0; q4 < 4; q4++) {
                     const int q = 4 * c + q4;
-                    const float4 u = __ldg(urow + q);
-                    const float x0 = isq_i * u.x * cfs[bsel][4 * q], x1 = isq_i * u.y * cfs[bsel][4 * q + 1];
-                    const float x2 = isq_i * u.z * cfs[bsel][4 * q + 2], x3 = isq_i * u.w * cfs[bsel][4 * q + 3];
+                    const float4 u = __ldg(Uq + q * K + i);
+                    const float x0 = u.x * cf[4 * q], x1 = u.y * cf[4 * q + 1];
+                    const float x2 = u.z * cf[4 * q + 2], x3 = u.w * cf[4 * q + 3];
                     const float4 hv = make_float4(tf32_hi(x0), tf32_hi(x1), tf32_hi(x2), tf32_hi(x3));
                     *reinterpret_cast<float4 *>(sm + PFT_A + core_off(tid, 4 * q, 16)) =
                         make_float4(x0 - hv.x, x1 - hv.y, x2 - hv.z, x3 - hv.w);
@@ -162,7 +180,8 @@ __global__ void __launch_bounds__(PFT_THREADS) k_pform_tc(const PSet *ps, const 
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
                          :: "r"(barM) : "memory");
         }
-        // ---- epilogue inputs that do not depend on D, loaded while the MMAs run
+        // ---- epilogue inputs that do not depend on D, loaded while the MMAs run (before A is formed
+        // they cost more than they hide: A's own loads then wait behind them)
         float row[K];
         {
             const float *eg = m.gridT + ((size_t)md * m.grid_n + g) * K2;   // E(t_g)^T
@@ -175,6 +194,7 @@ __global__ void __launch_bounds__(PFT_THREADS) k_pform_tc(const PSet *ps, const 
                 else row[j] = 0.0f;
             }
         }
+        if (b0 + 2 < bb1) coefficients(b0 + 2, par ^ 1);      // the next pair's, while the MMAs run
         pending = true;
         const bool done = mbar_wait(barM, ph);
         ph ^= 1u;
@@ -192,26 +212,20 @@ __global__ void __launch_bounds__(PFT_THREADS) k_pform_tc(const PSet *ps, const 
         tc_fence_before();
         if (b < bb1 && done) {
             // branch-free in j: i differs per lane, and a branch on j == i would split the
-            // warp into single-lane paths for everything that follows
+            // warp into single-lane paths for everything that follows.  Off the diagonal:
+            // diag -= x (Kahan), the step's last two operations predicated, so that its chain
+            // is four additions; row[i] is not used any more (the diagonal is stored by itself)
             bool neg = false;
             float diag = 0.0f, dc = 0.0f;
 #pragma unroll
             for (int j = 0; j < K; j++) {
-                const bool dj = (j == i);
-                const float x0 = row[j];
-                neg |= dj ? (x0 < dtol) : (x0 < ntol);
-                const float x = fmaxf(x0, 0.0f);          // clamp an off-diagonal negative
-                row[j] = dj ? x0 : x;
-                const float y = -x - dc;                  // Kahan: diag -= x (off-diagonal only)
-                const float s = diag + y;
-                const float c = (s - diag) - y;
-                diag = dj ? diag : s;
-                dc = dj ? dc : c;
+                neg |= row[j] < (j == i ? dtol : ntol);
+                row[j] = fmaxf(row[j], 0.0f);             // clamp an off-diagonal negative
+                asm("{\n .reg .pred p;\n .reg .f32 y, s, t;\n setp.ne.s32 p, %3, %4;\n sub.rn.f32 y, %2, %1;\n"
+                    " add.rn.f32 s, %0, y;\n sub.rn.f32 t, s, %0;\n @p sub.rn.f32 %1, t, y;\n @p mov.f32 %0, s;\n}\n"
+                    : "+f"(diag), "+f"(dc) : "f"(-row[j]), "r"(i), "r"(j));
             }
-            const float dv = leaf_rows && b < nl ? diag + 1.0f : diag;
-#pragma unroll
-            for (int j = 0; j < K; j++) row[j] = (j == i) ? dv : row[j];
-            const double rs = rowsum_minus_one(m, md, i, exs[bsel]);
+            const double rs = one_w ? wu * exs[par][bsel][w0] * ww * isq_i : rowsum_minus_one(m, md, i, exs[par][bsel]);
             if (neg) status_min(status_key + r, b, i, PCSF_ENEGP);
             else if (fabs(rs) > m.tol) status_min(status_key + r, b, i, PCSF_EROWSUM);
             else if (!(diag > -1.0f)) status_min(status_key + r, b, i, PCSF_EDIAG);
@@ -220,10 +234,14 @@ __global__ void __launch_bounds__(PFT_THREADS) k_pform_tc(const PSet *ps, const 
 #pragma unroll
                 for (int q = 0; q < K / 4; q++)
                     bop_store(dst, i, q, make_float4(row[4 * q], row[4 * q + 1], row[4 * q + 2], row[4 * q + 3]));
+                dst += (i >> 2) * 256 + i * 4 + (i & 3);
+                dst[0] = tf32_hi(diag);
+                dst[K2] = diag - tf32_hi(diag);
             } else {            // above a leaf: E^T rows for the gathers, or k_prune_tc's P^T rows
                 float *out = Pbuf + ((size_t)r * nbr + b) * K2 + (leaf_rows ? leaf_pos(i) - i : 0);
 #pragma unroll
                 for (int j = 0; j < K; j++) out[(size_t)j * K + i] = row[j];
+                out[(size_t)i * K + i] = leaf_rows ? diag + 1.0f : diag;
             }
         }
         if (!done) ok = false;      // agreed on at the next pair's first barrier
@@ -252,7 +270,7 @@ cudaError_t launch_pform_tc(const PSet *ps, int nps, const double *branch, int n
     // several times over, fewer for a short list (one exon's search round asks for two to six
     // P sets): about PFT_TARGET CTAs in all, at the price of one 32 KB fetch of B per CTA.
     // Measured, P(t) of one mle call on 58 leaves: 1 region (2-6 P sets a round) 5.1 -> 0.28 ms,
-    // 384 regions (~800 P sets a round: 1.7 waves before, three CTAs per P set now) 20.0 -> 14.6 ms.
+    // 384 regions (~800 P sets a round: 1.7 waves before, three CTAs per P set now) 20.0 -> 14.6 ms (both before the steps named above).
     const int pairs = (nbr + 1) / 2;
     const int want = std::min(pairs, std::max(1, (PFT_TARGET + nps - 1) / nps));
     const int per_cta = 2 * ((pairs + want - 1) / want);
