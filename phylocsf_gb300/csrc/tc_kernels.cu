@@ -262,11 +262,13 @@ __global__ void __launch_bounds__(TCP_THREADS, 2) k_prune_tc(PruneArgs a, float 
         tc_fence_before();
         warp_arrive(barA, lane);
     };
-    auto wait_d = [&]() {
+    auto issue = [&]() {
         if (warp == 0) {
             if (lane == 0) contract();
             __syncwarp();
         }
+    };
+    auto wait_d = [&]() {
         if (!bad && !mbar_wait(barM, n & 1)) {
             bad = true;
             if (tid == 0) late_s = n & 1;       // its commit may still arrive
@@ -335,6 +337,7 @@ __global__ void __launch_bounds__(TCP_THREADS, 2) k_prune_tc(PruneArgs a, float 
                 // the last node's partial (in v) is contracted first
                 stage(v);
                 if (fl & TN_LEAF) {
+                    issue();
                     leaf_rows(sn.lc, x);
                 } else if (--sp == 0) {
                     tmem_ld_rows(trow + TM_S, x);
@@ -344,7 +347,7 @@ __global__ void __launch_bounds__(TCP_THREADS, 2) k_prune_tc(PruneArgs a, float 
 #pragma unroll
                     for (int j = 0; j < 16; j++) x[j] = e[j * TCP_THREADS];
                 }
-                
+                if (!(fl & TN_LEAF)) issue();
                 wait_d();
 #pragma unroll
                 for (int q = 0; q < 2; q++) {
@@ -359,6 +362,7 @@ __global__ void __launch_bounds__(TCP_THREADS, 2) k_prune_tc(PruneArgs a, float 
                 } else {
                     // then the one from the stack
                     stage(x);
+                    issue();
                     wait_d();
 #pragma unroll
                     for (int q = 0; q < 2; q++) {
