@@ -693,6 +693,13 @@ cudaError_t launch_d2f_rows(const double *in, float *out, size_t nmat, int nbr, 
 // rescaled by an exact power of two so its maximum lies in [0.5,1); the
 // exponents are summed per column and added back as e*ln2 in FP64 at the root.
 
+//
+// What bounds it: FP32 issue in the contractions (half of the paired FMA rate over a launch) and,
+// between them, the phases that the other CTA of the SM covers only in part: the copies of the next
+// node's operands (1,400 clocks of a node's 10,000), a leaf's factors (1,300), the rescale (1,000).
+// The diagonals' low parts come into L1 with the operands, the leaf states with eight loads in
+// flight, and the rescale multiplies once where it can: 58 leaves, 141,741 columns 2.67 -> 2.59 ms,
+// 120 leaves, 95,724 columns 4.30 -> 4.17 ms.
 constexpr int PR_THREADS = 256;
 
 // threads of a tile: 16 groups of 4 states; 4 or 2 columns per thread, or 1 in half a block (8 columns)
@@ -749,9 +756,19 @@ __global__ void __launch_bounds__(PruneThreads<TC>::N) k_prune(PruneArgs a)
         const int ncols = wi.ncols;
         const uint8_t *lg = a.leaves + (size_t)wi.col0 * nl;
         __syncthreads();   // previous work item finished with shared memory
-        for (int f = tid; f < TC * nl; f += THREADS) {
-            int c = f / nl, l = f - c * nl;
-            lvT[l * TC + c] = (c < ncols) ? lg[f] : (uint8_t)K;
+        // leaf states, eight loads in flight a thread
+        for (int f0 = tid; f0 < TC * nl; f0 += 8 * THREADS) {
+            uint8_t x[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int f = f0 + i * THREADS;
+                x[i] = f < ncols * nl ? __ldg(lg + f) : (uint8_t)K;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int f = f0 + i * THREADS, c = f / nl;
+                if (f < TC * nl) lvT[(f - c * nl) * TC + c] = x[i];
+            }
         }
         for (int f = tid; f < 2 * TC; f += THREADS) colmax[f] = 0;
         for (int f = tid; f < TC; f += THREADS) cscale[f] = 0;
@@ -761,7 +778,13 @@ __global__ void __launch_bounds__(PruneThreads<TC>::N) k_prune(PruneArgs a)
         __syncthreads();       // leaf states (and ltab) ready
         // a node's operands are copied one node ahead (issued once the previous node's contraction
         // has released the buffers)
-        stage_children<T, TC, CPT, THREADS>(Et, Pbase, sched[0], lvT, tid);
+        // and the diagonals' low parts, two lines a child, come into L1 with them
+        auto stage = [&](const SchedNode &nx) {
+            stage_children<T, TC, CPT, THREADS>(Et, Pbase, nx, lvT, tid);
+            if (dlo && tid < 4)
+                asm volatile("prefetch.global.L1 [%0];" :: "l"(dlo + (size_t)(tid < 2 ? nx.lc : nx.rc) * K + 32 * (tid & 1)));
+        };
+        stage(sched[0]);
         if (dith) {
             for (int c = tid; c < TC; c += THREADS) {
                 double sd = 0.0;
@@ -780,7 +803,7 @@ __global__ void __launch_bounds__(PruneThreads<TC>::N) k_prune(PruneArgs a)
             child_partial<T, TC, KAHAN, CPT, 7>(Et + K2, slots, sn.rslot, sn.rc, lvT, a0, c0, vr, dcol0, true,
                                         dlo ? dlo + (size_t)sn.rc * K : nullptr);
             __syncthreads();
-            if (ni + 1 < a.n_internal) stage_children<T, TC, CPT, THREADS>(Et, Pbase, sched[ni + 1], lvT, tid);   // buffers free again
+            if (ni + 1 < a.n_internal) stage(sched[ni + 1]);   // buffers free again
             MU *cm = colmax + (ni & 1) * TC;
             MU *cm_next = colmax + ((ni + 1) & 1) * TC;
             if (tid < TC) cm_next[tid] = 0;
@@ -796,12 +819,38 @@ __global__ void __launch_bounds__(PruneThreads<TC>::N) k_prune(PruneArgs a)
             }
             __syncthreads();
             T *out = slots + (size_t)sn.oslot * K * TC;
-            int ecol[CPT];
+            T mx[CPT], sc[CPT];
+            ColLoad<T, CPT>::load(reinterpret_cast<const T *>(cm) + c0, mx);
+            // sc = 2^-e as one factor where every maximum of the warp allows it, else the first of scale2's
+            // two factors goes into vl (one column a thread: the test costs what it saves)
+            bool one = false;
+            if constexpr (sizeof(T) == 4 && CPT > 1) {
+                one = true;
 #pragma unroll
-            for (int cc = 0; cc < CPT; cc++) {
-                const T mx = AtomMax<T>::get(cm + c0 + cc);
-                ecol[cc] = (mx > (T)0) ? exp_of(mx) : 0;
-                if (ty == 0) cscale[c0 + cc] += ecol[cc];
+                for (int cc = 0; cc < CPT; cc++) {
+                    const int b = __float_as_int(mx[cc]) >> 23;
+                    one &= b > 0 && b < 253;
+                }
+                one = __all_sync(0xffffffffu, one);
+                if (one) {
+#pragma unroll
+                    for (int cc = 0; cc < CPT; cc++) {
+                        const int b = __float_as_int(mx[cc]) >> 23;
+                        if (ty == 0) cscale[c0 + cc] += b - 126;
+                        sc[cc] = __int_as_float((253 - b) << 23);
+                    }
+                }
+            }
+            if (!one) {
+#pragma unroll
+                for (int cc = 0; cc < CPT; cc++) {
+                    const int e = (mx[cc] > (T)0) ? exp_of(mx[cc]) : 0, e1 = -e >> 1;
+                    if (ty == 0) cscale[c0 + cc] += e;
+                    const T first = pow2<T>(e1);
+                    sc[cc] = pow2<T>(-e - e1);
+#pragma unroll
+                    for (int i = 0; i < 4; i++) vl[i][cc] *= first;
+                }
             }
             // one vector store per state row (CPT consecutive columns): scalar stores
             // here were 4-way bank-conflicted
@@ -809,7 +858,7 @@ __global__ void __launch_bounds__(PruneThreads<TC>::N) k_prune(PruneArgs a)
             for (int i = 0; i < 4; i++) {
                 T y[CPT];
 #pragma unroll
-                for (int cc = 0; cc < CPT; cc++) y[cc] = scale2(vl[i][cc], -ecol[cc]);
+                for (int cc = 0; cc < CPT; cc++) y[cc] = vl[i][cc] * sc[cc];
                 ColStore<T, CPT>::store(out + (a0 + i) * TC + c0, y);
             }
         }

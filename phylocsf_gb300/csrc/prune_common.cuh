@@ -170,19 +170,19 @@ __device__ __forceinline__ int exp_of(double x)
     frexp(x, &e);
     return e;
 }
+// 2^e, |e| <= 126 (float) / 1022 (double)
+template <typename T> __device__ __forceinline__ T pow2(int e);
+template <> __device__ __forceinline__ float pow2<float>(int e) { return __int_as_float((e + 127) << 23); }
+template <> __device__ __forceinline__ double pow2<double>(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
 // scale2(x, e) = x * 2^e as two multiplications by exact powers of two (e split
 // in halves of equal sign, so the intermediate lies between x and the result):
 // exact, like ldexp, whenever x and the result are normal or zero; |e| <= 252
 // (float) / 2044 (double), far beyond the per-node rescales.
-__device__ __forceinline__ float scale2(float x, int e)
+template <typename T>
+__device__ __forceinline__ T scale2(T x, int e)
 {
     const int e1 = e >> 1, e2 = e - e1;
-    return x * __int_as_float((e1 + 127) << 23) * __int_as_float((e2 + 127) << 23);
-}
-__device__ __forceinline__ double scale2(double x, int e)
-{
-    const int e1 = e >> 1, e2 = e - e1;
-    return x * __longlong_as_double((long long)(e1 + 1023) << 52) * __longlong_as_double((long long)(e2 + 1023) << 52);
+    return x * pow2<T>(e1) * pow2<T>(e2);
 }
 
 // out[i][cc] = sum_j M[j][a0+i] * X[j][c0+cc] for a 64 x TC shared-memory tile
