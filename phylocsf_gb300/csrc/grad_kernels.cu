@@ -29,7 +29,7 @@
 // contracted as stored, a column's weight 2^ex / z~ is formed once ahead by one warp, all
 // eight warps share the FP64 sums of a side, and these run beside the next side's
 // contractions; each warp's sum goes to gpart, which k_reduce_grad adds up.  Measured, per
-// column: 58 leaves 173 -> 101 ns, 100 leaves with two rate parameters 955 -> 525 ns.
+// column: 58 leaves 173 -> 91 ns, 100 leaves with two rate parameters 955 -> 400 ns.
 #include <algorithm>
 #include <cmath>
 
@@ -305,6 +305,16 @@ __global__ void __launch_bounds__(GR_THREADS, sizeof(T) == 4 ? 2 : 1) k_grad(Gra
             const int p = sn.node;
             const T *Bp = B + (size_t)(p - nl) * K * TC;
             __syncthreads();   // the betas of the last node are written, X and E^T are free
+            if (ni > 0) {      // the next node's slabs, from DRAM into L2 (69,983 columns, 58 leaves: 6.61 -> 6.40 ms)
+                const SchedNode nx = sched[ni - 1];
+                constexpr int NL = K * TC * sizeof(T) / 128;
+                for (int f = tid; f < 3 * NL; f += GR_THREADS) {
+                    const int c = f < NL ? nx.lc : nx.rc;
+                    if (f < 2 * NL && RECOMP && c < nl) continue;
+                    const T *slab = f < 2 * NL ? V + vslot(c) * K * TC : B + (size_t)(nx.node - nl) * K * TC;
+                    asm volatile("prefetch.global.L2 [%0];" :: "l"(slab + (f % NL) * (128 / sizeof(T))));
+                }
+            }
             for (int side = 0; side < 2; side++, sidx++) {
                 const int c = side ? sn.rc : sn.lc;
                 const int s = side ? sn.lc : sn.rc;
