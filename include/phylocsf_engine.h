@@ -118,7 +118,7 @@ typedef struct {
     int64_t pform_launches;
     /* by pruning-kernel kind: 0 SIMT (returned values), 1 tensor core (search),
      * 2 adjoint gradient, 3 tensor-core tangent (d lpr / d rho for the search),
-     * 4 float-float SIMT (returned values of long regions, and the search
+     * 4 float-float (returned values of long regions, and the search
      * decisions of long regions that the tensor-core values cannot settle) */
     int64_t kind_launches[5];
     int64_t kind_columns[5];     /* codon-column evaluations (columns x requests)  */

@@ -40,9 +40,9 @@
 // 1,700 for its rows.  Tensor pipe and issue slots are each about half used.  Registers
 // decide: one more 32-byte array per thread spills, and spilling variants measured 10 to
 // 40 % slower, so the rows are not fetched a node ahead.
-// Measured, all search launches of a call: 384 regions on 58 leaves 46.5 -> 32.0 ms, 256
-// regions on 100 leaves 30.4 -> 21.0 ms, one region on 58 leaves (3 tiles a launch) 159 ->
-// 119 us a launch.  Before, two threads owned a column (32 states each): every child's
+// Measured, all search launches of a call: 384 regions on 58 leaves 46.5 -> 31.0 ms, 60 genes
+// (106,356 columns) on 100 leaves 30.4 -> 20.3 ms, one region on 58 leaves (3 tiles a launch)
+// 159 -> 122 us a launch.  Before, two threads owned a column (32 states each): every child's
 // partial was stored and loaded again, a lane gathered its row alone (32 lines an
 // instruction, a third of the LSU's wavefronts were leaf reads), and the maximum crossed
 // warps through shared memory.

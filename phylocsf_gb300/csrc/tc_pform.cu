@@ -30,8 +30,8 @@
 // and a second pass to insert the diagonal), 1,600 of MMA issue, the row-sum check 850
 // (1,900 with its operands looked up for every pair), and the next pair's coefficients
 // formed in the MMAs' shadow.  Issue slots are a third used, HBM writes 30 %.  Measured, all
-// P(t) launches of a call: 384 regions on 58 leaves 13.7 -> 11.2 ms, 256 regions on 100
-// leaves 8.1 -> 7.4 ms, ORF sets 1.42 -> 1.25 ms.
+// P(t) launches of a call: 384 regions on 58 leaves 13.7 -> 11.2 ms, 60 genes on 100 leaves
+// 8.1 -> 7.4 ms, ORF sets 1.42 -> 1.25 ms.
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -270,7 +270,8 @@ cudaError_t launch_pform_tc(const PSet *ps, int nps, const double *branch, int n
     // several times over, fewer for a short list (one exon's search round asks for two to six
     // P sets): about PFT_TARGET CTAs in all, at the price of one 32 KB fetch of B per CTA.
     // Measured, P(t) of one mle call on 58 leaves: 1 region (2-6 P sets a round) 5.1 -> 0.28 ms,
-    // 384 regions (~800 P sets a round: 1.7 waves before, three CTAs per P set now) 20.0 -> 14.6 ms (both before the steps named above).
+    // 384 regions (~800 P sets a round: 1.7 waves before, three CTAs per P set now) 20.0 -> 14.6 ms,
+    // both before the chain was shortened.
     const int pairs = (nbr + 1) / 2;
     const int want = std::min(pairs, std::max(1, (PFT_TARGET + nps - 1) / nps));
     const int per_cta = 2 * ((pairs + want - 1) / want);
