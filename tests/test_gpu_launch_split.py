@@ -114,3 +114,18 @@ def test_eigensystem_against_numpy():
             assert np.abs((U * lam) @ U.T - A).max() <= 1e-13 * np.abs(A).max() * 64
             assert np.abs(U.T @ U - np.eye(64)).max() <= 1e-13
             assert np.abs(np.sort(lam) - np.linalg.eigvalsh(A)).max() <= 1e-13 * np.abs(lam).max() * 64
+
+
+# the sums of a short launch's columns are formed 1,024 at a time: lengths at that edge, alone (small
+# tiles) and in a batch long enough for the long launches' tiles (64 or 32 columns)
+@pytest.mark.parametrize("name,prec", [("12flies", "fp32b"), ("12flies", "fp64"), ("120mammals", "fp32b")])
+@pytest.mark.parametrize("length", [1023, 1024, 1025, 1057, 2049])
+def test_sums_of_small_tiles(name, prec, length):
+    ps, offs, leaves = _regions(name, [length])
+    eng = P.Engine(ps.tree, ps.S_c, ps.pi_c, ps.S_n, ps.pi_n, precision=prec)
+    eng.set_exact_threshold(1 << 60)                     # the SIMT kernel for every length
+    one = eng.lpr(eng.batch(offs, leaves), 0, 1.3)
+    n = 40
+    many = eng.lpr(eng.batch(np.arange(n + 1) * length, np.tile(leaves, (n, 1))), 0, 1.3)
+    assert (one[2] == 0).all() and (many[2] == 0).all()
+    assert np.array_equal(np.repeat(one[0], n), many[0]) and np.array_equal(np.repeat(one[1], n), many[1])
