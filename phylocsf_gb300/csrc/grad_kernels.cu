@@ -555,26 +555,73 @@ cudaError_t launch_grad(int prec, int comp, const GradArgs &a, cudaStream_t s, i
 // H_x^T = (F(t) o Bdot_x)^T per (P set, branch, parameter).  F_ij = (e^{lam_i t} -
 // e^{lam_j t}) / (lam_i - lam_j), written as e^{lam_j t} (e^{d t} - 1) / d with
 // d = lam_i - lam_j and a Taylor series in d t when |d t| < 1e-2 (no cancellation).
+// F is symmetric: a CTA takes HF_BRANCHES branches of a P set, its threads the 2,016 pairs i < j
+// (1 / d and Bdot kept over the branches), F goes through shared memory and H out in rows.  The
+// quotient is corrected to the division's rounding (q = x r, q + (x - q d) r; Markstein 1990).
+// What bounds it: FP64 issue (two lanes per clock), about 14 instructions an entry where every
+// entry formed its own quotient or series and wrote with a stride of a row; 40 P sets of 198
+// branches 2.2 -> 0.75 ms.
+constexpr int HF_BRANCHES = 16, HF_LD = K + 1;
 template <typename T>
 __global__ void __launch_bounds__(256) k_hform(const PSet *ps, const double *branch, int nbr, const double *lam,
                                                const T *Bdot, T *H)
 {
-    __shared__ double el[K];
-    const int b = blockIdx.x, r = blockIdx.y, tid = threadIdx.x;
+    __shared__ double el[HF_BRANCHES][K];
+    __shared__ double F[K * HF_LD];
+    constexpr int NP = K * (K - 1) / 2, PER = (NP + 255) / 256;
+    const int b0 = blockIdx.x * HF_BRANCHES, b1 = min(nbr, b0 + HF_BRANCHES), r = blockIdx.y, tid = threadIdx.x;
     const PSet rq = ps[r];
     const int md = rq.model;
-    const double t = rq.rho * branch[b];
     const double *lm = lam + (size_t)md * K;
-    if (tid < K) el[tid] = exp(lm[tid] * t);
-    __syncthreads();
-    for (int f = tid; f < K2; f += 256) {
-        const int i = f / K, j = f % K;
-        const double d = lm[i] - lm[j], dt = d * t;
-        double F;
-        if (fabs(dt) < 1e-2) F = t * el[j] * (1.0 + dt * (0.5 + dt * (1.0 / 6.0 + dt * (1.0 / 24.0 + dt / 120.0))));
-        else F = (el[i] - el[j]) / d;
-        for (int x = 0; x < 2; x++)
-            H[(((size_t)r * nbr + b) * 2 + x) * K2 + (size_t)j * K + i] = (T)(F * (double)Bdot[((size_t)md * 2 + x) * K2 + f]);
+    for (int f = tid; f < (b1 - b0) * K; f += 256) el[f / K][f % K] = exp(lm[f % K] * (rq.rho * branch[b0 + f / K]));
+    int ij[PER];                 // the thread's pairs, row p / 64 of a 32 x 63 fold of the triangle
+    double d[PER], rd[PER];
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+        const int p = min(tid + 256 * k, NP - 1), i0 = p / (K - 1), j0 = p % (K - 1);
+        // fold: row i0 holds (i0, j) for j > i0, then row K - 1 - i0's pairs
+        const bool own = j0 >= i0;
+        const int i = own ? i0 : K - 1 - i0, j = own ? j0 + 1 : K - 1 - j0;
+        ij[k] = i << 8 | j;
+        d[k] = lm[i] - lm[j];
+        rd[k] = 1.0 / d[k];
+    }
+    double bd[2][K2 / 256];      // Bdot_x^T of the elements that the thread writes
+#pragma unroll
+    for (int k = 0; k < K2 / 256; k++)
+#pragma unroll
+        for (int x = 0; x < 2; x++) {
+            const int o = tid + 256 * k;
+            bd[x][k] = (double)Bdot[((size_t)md * 2 + x) * K2 + (o % K) * K + o / K];
+        }
+    for (int b = b0; b < b1; b++) {
+        const double t = rq.rho * branch[b];
+        const double *e = el[b - b0];
+        __syncthreads();         // el ready; the last branch's F is read
+        if (tid < K) F[tid * HF_LD + tid] = t * e[tid];
+#pragma unroll
+        for (int k = 0; k < PER; k++) {
+            const int i = ij[k] >> 8, j = ij[k] & 255;
+            const double dt = d[k] * t;
+            double v;
+            if (fabs(dt) < 1e-2) {
+                v = t * e[j] * (1.0 + dt * (0.5 + dt * (1.0 / 6.0 + dt * (1.0 / 24.0 + dt * (1.0 / 120.0)))));
+            } else {
+                const double x = e[i] - e[j], q = x * rd[k];
+                v = fma(fma(-q, d[k], x), rd[k], q);
+            }
+            F[i * HF_LD + j] = v;
+            F[j * HF_LD + i] = v;
+        }
+        __syncthreads();
+        T *out = H + ((size_t)r * nbr + b) * 2 * K2;
+#pragma unroll
+        for (int k = 0; k < K2 / 256; k++) {
+            const int o = tid + 256 * k;
+            const double v = F[(o / K) * HF_LD + o % K];
+            out[o] = (T)(v * bd[0][k]);
+            out[K2 + o] = (T)(v * bd[1][k]);
+        }
     }
 }
 
@@ -582,7 +629,7 @@ cudaError_t launch_hform(bool fp64, const PSet *ps, int nps, const double *branc
                          const void *Bdot, void *H, cudaStream_t s)
 {
     if (nps <= 0) return cudaSuccess;
-    dim3 grid(nbr, nps);
+    dim3 grid((nbr + HF_BRANCHES - 1) / HF_BRANCHES, nps);
     if (fp64) k_hform<double><<<grid, 256, 0, s>>>(ps, branch, nbr, lam, (const double *)Bdot, (double *)H);
     else k_hform<float><<<grid, 256, 0, s>>>(ps, branch, nbr, lam, (const float *)Bdot, (float *)H);
     return cudaGetLastError();
