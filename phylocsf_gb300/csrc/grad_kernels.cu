@@ -29,7 +29,7 @@
 // contracted as stored, a column's weight 2^ex / z~ is formed once ahead by one warp, all
 // eight warps share the FP64 sums of a side, and these run beside the next side's
 // contractions; each warp's sum goes to gpart, which k_reduce_grad adds up.  Measured, per
-// column: 58 leaves 173 -> 91 ns, 100 leaves with two rate parameters 955 -> 400 ns.
+// column: 58 leaves 173 -> 88 ns, 100 leaves with two rate parameters 955 -> 387 ns.
 #include <algorithm>
 #include <cmath>
 
@@ -40,6 +40,7 @@ namespace pcsf {
 
 constexpr int GR_THREADS = 256;
 constexpr int GR_WARPS = GR_THREADS / 32;
+constexpr int GR_UNROLL = 3;         // blocks of a contraction in a row (see contract_pairs)
 constexpr int GR_TC = 32;            // columns per tile
 
 template <typename T, bool RECOMP>
@@ -159,8 +160,8 @@ __global__ void __launch_bounds__(GR_THREADS, sizeof(T) == 4 ? 2 : 1) k_grad(Gra
             asm volatile("cp.async.wait_all;" ::: "memory");
             __syncthreads();
             T vl[4][CPT], vr[4][CPT];
-            child_partial<T, TC, KAHAN>(Mat, slots, sn.lslot, sn.lc, lvT, a0, c0, vl, -1, true);
-            child_partial<T, TC, KAHAN>(Mat + K2, slots, sn.rslot, sn.rc, lvT, a0, c0, vr, -1, true);
+            child_partial<T, TC, KAHAN, CPT, GR_UNROLL>(Mat, slots, sn.lslot, sn.lc, lvT, a0, c0, vl, -1, true);
+            child_partial<T, TC, KAHAN, CPT, GR_UNROLL>(Mat + K2, slots, sn.rslot, sn.rc, lvT, a0, c0, vr, -1, true);
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 if (!RECOMP || sn.lc >= nl) ColStore<T, CPT>::store(V + (vslot(sn.lc) * K + a0 + i) * TC + c0, vl[i]);
@@ -270,7 +271,7 @@ __global__ void __launch_bounds__(GR_THREADS, sizeof(T) == 4 ? 2 : 1) k_grad(Gra
                 for (int f = tid; f < K * TC; f += GR_THREADS) X[f] = sqT[f / TC];
                 __syncthreads();
                 T qv[4][CPT];
-                contract<T, TC, KAHAN>(Us, X, a0, c0, qv);
+                contract<T, TC, KAHAN, CPT, GR_UNROLL>(Us, X, a0, c0, qv);
                 if (tx == 0)
 #pragma unroll
                     for (int i = 0; i < 4; i++) wmT[a0 + i] = qv[i][0];
@@ -389,7 +390,7 @@ __global__ void __launch_bounds__(GR_THREADS, sizeof(T) == 4 ? 2 : 1) k_grad(Gra
                 T *rd = red + (size_t)buf * (1 + npar) * 16 * TC + ty * TC + c0;
                 {
                     T wq[4][CPT];
-                    contract<T, TC, KAHAN>(Qs, X, a0, c0, wq);
+                    contract<T, TC, KAHAN, CPT, GR_UNROLL>(Qs, X, a0, c0, wq);
 #pragma unroll
                     for (int cc = 0; cc < CPT; cc++) {
                         T acc = (T)0;
@@ -402,7 +403,7 @@ __global__ void __launch_bounds__(GR_THREADS, sizeof(T) == 4 ? 2 : 1) k_grad(Gra
                 MU *cm = colmax + buf * TC, *cm_next = colmax + (buf ^ 1) * TC;
                 T bt[4][CPT];
                 if (internal) {
-                    contract_rows<T, TC, KAHAN>(Er, X, a0, c0, bt);
+                    contract_rows<T, TC, KAHAN, GR_UNROLL>(Er, X, a0, c0, bt);
 #pragma unroll
                     for (int cc = 0; cc < CPT; cc++) {
                         T mx = (T)0;
@@ -418,9 +419,9 @@ __global__ void __launch_bounds__(GR_THREADS, sizeof(T) == 4 ? 2 : 1) k_grad(Gra
                 // q = U^T D^1/2 alpha_c, for a leaf one row of U (its alpha_c is one-hot)
                 T pv[4][CPT], qv[4][CPT];
                 if (npar) {
-                    contract<T, TC, KAHAN>(Us, Q1, a0, c0, pv);
+                    contract<T, TC, KAHAN, CPT, GR_UNROLL>(Us, Q1, a0, c0, pv);
                     if (internal) {
-                        contract<T, TC, KAHAN>(Us, Q2, a0, c0, qv);
+                        contract<T, TC, KAHAN, CPT, GR_UNROLL>(Us, Q2, a0, c0, qv);
                     } else {
 #pragma unroll
                         for (int cc = 0; cc < CPT; cc++) {
@@ -464,7 +465,7 @@ __global__ void __launch_bounds__(GR_THREADS, sizeof(T) == 4 ? 2 : 1) k_grad(Gra
                         if (x) asm volatile("cp.async.wait_all;" ::: "memory");
                         __syncthreads();
                         T rv[4][CPT];
-                        contract<T, TC, KAHAN>(x ? Er : Hb, Q1, a0, c0, rv);
+                        contract<T, TC, KAHAN, CPT, GR_UNROLL>(x ? Er : Hb, Q1, a0, c0, rv);
 #pragma unroll
                         for (int cc = 0; cc < CPT; cc++) {
                             T acc = (T)0;

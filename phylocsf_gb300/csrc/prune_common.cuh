@@ -276,8 +276,9 @@ __device__ inline void contract_scalar(const T *M, const T *X, int a0, int c0, T
 // 2.68 ms; what bounds it now is the mix of FP32 issue, load latency and three barriers a node.
 // entry(j, e): E's four entries of step j.
 // UNROLL: blocks of the compensated sum in a row (7: all of them).  Rolled, each block begins with
-// its loads' latency (k_prune 2.94 ms against 2.68); unrolled, a kernel with many contractions
-// outgrows the instruction cache (k_grad with rate parameters 15.6 ms against 12.8).
+// its loads' latency (k_prune 2.94 ms against 2.68 with 7); unrolled, a kernel with many contractions
+// outgrows the instruction cache (k_grad with 1 / 3 / 7: 58 leaves 6.43 / 6.19 / 6.47 ms, 100 leaves
+// with rate parameters 12.6 / 12.2 / 15.7 ms).
 template <int TC, int COMP, int CPT, int UNROLL, typename Entry>
 __device__ inline void contract_pairs(Entry entry, const float *X, int c0, float out[4][CPT])
 {
@@ -368,13 +369,13 @@ __device__ inline void contract(const T *M, const T *X, int a0, int c0, T out[4]
 // pass, which multiplies by E^T as it is stored.  Four consecutive j of a row come in one load;
 // LDN = K + 4 keeps the two row groups of a warp on different banks.
 constexpr int LDN = K + 4;
-template <typename T, int TC, int COMP>
+template <typename T, int TC, int COMP, int UNROLL = 1>
 __device__ inline void contract_rows(const T *N, const T *X, int a0, int c0, T out[4][TC / 16])
 {
     constexpr int CPT = TC / 16;
     if constexpr (sizeof(T) == 4 && CPT % 2 == 0) {
         float r[4][4];       // four steps of the thread's four rows
-        contract_pairs<TC, COMP, CPT, 1>(
+        contract_pairs<TC, COMP, CPT, UNROLL>(
             [&](int j, float e[4]) {
                 if (j % 4 == 0) {
 #pragma unroll
