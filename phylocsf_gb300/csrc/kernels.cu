@@ -388,11 +388,7 @@ __global__ void __launch_bounds__(PF_THREADS) k_pform(const PSet *ps, const doub
             else if (t < m.grid_t[0]) mode = 2;
             else {
                 mode = 3;
-                double x = log(t / m.grid_t[0]) / m.grid_lr;
-                g = (int)floor(x);
-                if (g < 0) g = 0;
-                if (g > m.grid_n - 1) g = m.grid_n - 1;
-                if (g + 1 < m.grid_n && (m.grid_t[g + 1] - t) < (t - m.grid_t[g])) g++;
+                g = grid_point(m, t);
             }
         }
         mode_s[tid] = mode;

@@ -131,6 +131,17 @@ __device__ __forceinline__ double rowsum_minus_one(const DevModels &m, int md, i
     return rs * m.isq[md * K + i];
 }
 
+// Grid point nearest to t >= grid_t[0].  FP32 places t to about a thousandth of a step, and the
+// comparison with the next point makes the choice: from a point off by one, where t is that close
+// to a grid point, it is the same one.  (The FP64 logarithm and divisions were 4,000 clocks.)
+__device__ __forceinline__ int grid_point(const DevModels &m, double t)
+{
+    int g = (int)floorf(logf((float)t / (float)m.grid_t[0]) / (float)m.grid_lr);
+    g = max(0, min(g, m.grid_n - 1));
+    if (g + 1 < m.grid_n && (m.grid_t[g + 1] - t) < (t - m.grid_t[g])) g++;
+    return g;
+}
+
 // Per-column dithering of the leaf partials (SIMT FP32 pruning): each leaf partial
 // of column col is scaled by the exact factor c = 1 + k/256, k = dither_k(col, leaf),
 // and sum_leaves log c is subtracted from the column's log-likelihood.  The values

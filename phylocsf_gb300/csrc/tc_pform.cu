@@ -30,8 +30,8 @@
 // and a second pass to insert the diagonal), 1,600 of MMA issue, the row-sum check 850
 // (1,900 with its operands looked up for every pair), and the next pair's coefficients
 // formed in the MMAs' shadow.  Issue slots are a third used, HBM writes 30 %.  Measured, all
-// P(t) launches of a call: 384 regions on 58 leaves 13.7 -> 11.2 ms, 60 genes on 100 leaves
-// 8.1 -> 7.4 ms, ORF sets 1.42 -> 1.25 ms.
+// P(t) launches of a call: 384 regions on 58 leaves 13.7 -> 11.0 ms, 60 genes on 100 leaves
+// 8.1 -> 7.3 ms, ORF sets 1.42 -> 1.13 ms.
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -49,6 +49,15 @@ constexpr uint32_t PFT_SMEM = 65536;
 constexpr uint32_t PFT_TMEM_COLS = 128;   // D in 0..63, A_hi in 64..127
 constexpr int PFT_MAX_BRANCHES = 320;
 constexpr int PFT_TARGET = 4 * 3 * 152;   // CTAs of a launch: four waves of three per SM
+
+// diag -= x by Kahan's summation except where j == i, with the low part in dc: the last two of four
+// additions are predicated, so nothing but them is on the chain
+__device__ __forceinline__ void kahan_minus(float &diag, float &dc, float x, int i, int j)
+{
+    asm("{\n .reg .pred p;\n .reg .f32 y, s, t;\n setp.ne.s32 p, %3, %4;\n sub.rn.f32 y, %2, %1;\n"
+        " add.rn.f32 s, %0, y;\n sub.rn.f32 t, s, %0;\n @p sub.rn.f32 %1, t, y;\n @p mov.f32 %0, s;\n}\n"
+        : "+f"(diag), "+f"(dc) : "f"(-x), "r"(i), "r"(j));
+}
 
 __global__ void __launch_bounds__(PFT_THREADS, 3) k_pform_tc(const PSet *ps, const double *branch, int nbr, int nl,
                                                           DevModels m, const float *Bpf, float *Pbuf, float *Bop,
@@ -106,11 +115,7 @@ __global__ void __launch_bounds__(PFT_THREADS, 3) k_pform_tc(const PSet *ps, con
         else if (t < m.grid_t[0]) mode = 1;
         else {
             mode = 2;
-            const double x = log(t / m.grid_t[0]) / m.grid_lr;
-            g = (int)floor(x);
-            if (g < 0) g = 0;
-            if (g > m.grid_n - 1) g = m.grid_n - 1;
-            if (g + 1 < m.grid_n && (m.grid_t[g + 1] - t) < (t - m.grid_t[g])) g++;
+            g = grid_point(m, t);
         }
         mode_g[b] = (g << 2) | mode;
         t_b[b] = (float)t;
@@ -221,9 +226,7 @@ __global__ void __launch_bounds__(PFT_THREADS, 3) k_pform_tc(const PSet *ps, con
             for (int j = 0; j < K; j++) {
                 neg |= row[j] < (j == i ? dtol : ntol);
                 row[j] = fmaxf(row[j], 0.0f);             // clamp an off-diagonal negative
-                asm("{\n .reg .pred p;\n .reg .f32 y, s, t;\n setp.ne.s32 p, %3, %4;\n sub.rn.f32 y, %2, %1;\n"
-                    " add.rn.f32 s, %0, y;\n sub.rn.f32 t, s, %0;\n @p sub.rn.f32 %1, t, y;\n @p mov.f32 %0, s;\n}\n"
-                    : "+f"(diag), "+f"(dc) : "f"(-row[j]), "r"(i), "r"(j));
+                kahan_minus(diag, dc, row[j], i, j);
             }
             const double rs = one_w ? wu * exs[par][bsel][w0] * ww * isq_i : rowsum_minus_one(m, md, i, exs[par][bsel]);
             if (neg) status_min(status_key + r, b, i, PCSF_ENEGP);
