@@ -205,7 +205,7 @@ __device__ __forceinline__ T scale2(T x, int e)
 // product instead of 5).
 // CPT: columns per thread (TC / 16 with 256 threads of 4 states each).
 // FP32 with two or four columns per thread works on pairs of columns (contract_pairs).
-template <typename T, int TC, int COMP, int CPT = TC / 16>
+template <typename T, int TC, int COMP, int CPT = TC / 16, int UNROLL = 1>
 __device__ inline void contract_scalar(const T *M, const T *X, int a0, int c0, T out[4][CPT])
 {
     T comp[4][CPT];
@@ -234,7 +234,7 @@ __device__ inline void contract_scalar(const T *M, const T *X, int a0, int c0, T
             }
         };
         block(0, out);
-#pragma unroll 1
+#pragma unroll UNROLL
         for (int jb = 8; jb < K; jb += 8) {
             T g[4][CPT];
             block(jb, g);
@@ -372,7 +372,7 @@ __device__ inline void contract(const T *M, const T *X, int a0, int c0, T out[4]
     if constexpr (sizeof(T) == 4 && CPT % 2 == 0)
         contract_pairs<TC, COMP, CPT, UNROLL>([&](int j, float e[4]) { Vec4<float>::load(M + j * K + a0, e); }, X, c0, out);
     else
-        contract_scalar<T, TC, COMP, CPT>(M, X, a0, c0, out);
+        contract_scalar<T, TC, COMP, CPT, UNROLL>(M, X, a0, c0, out);
 }
 
 // out[i][cc] = sum_j N[a0+i][j] * X[j][c0+cc] with row a of N at N + a * LDN: contract() of the
