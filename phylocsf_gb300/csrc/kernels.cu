@@ -719,6 +719,7 @@ template <typename T, int TC, int KAHAN>
 __global__ void __launch_bounds__(PruneThreads<TC>::N) k_prune(PruneArgs a)
 {
     constexpr int THREADS = PruneThreads<TC>::N, TXN = THREADS / 16, CPT = TC / TXN;
+    constexpr bool SMALL = TC == PRUNE_SMALL_TILE;      // a short launch
     typedef typename AtomMax<T>::U MU;
     extern __shared__ __align__(16) unsigned char ssm[];
     T *Et = reinterpret_cast<T *>(ssm);                 // [2][K][K]
@@ -801,7 +802,7 @@ __global__ void __launch_bounds__(PruneThreads<TC>::N) k_prune(PruneArgs a)
             __syncthreads();
             if (ni + 1 < a.n_internal) {
                 stage(sched[ni + 1]);       // buffers free again
-            } else if (tid < K) {           // the root's: prior and prior log prior, two doubles a copy
+            } else if (SMALL && tid < K) {  // the root's: prior and prior log prior, two doubles a copy
                 const double *src = (tid < K / 2 ? a.m.prior : a.m.wlog) + md * K + 2 * (tid % (K / 2));
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
                              :: "r"((uint32_t)__cvta_generic_to_shared(Et) + 16 * tid), "l"(src) : "memory");
@@ -864,36 +865,22 @@ __global__ void __launch_bounds__(PruneThreads<TC>::N) k_prune(PruneArgs a)
                 ColStore<T, CPT>::store(out + (a0 + i) * TC + c0, y);
             }
         }
-        asm volatile("cp.async.wait_all;" ::: "memory");
+        if (SMALL) asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
         // root: z = alpha_root . prior ; elpr term = (alpha_root . prior*log prior) / z
-        // FP32: 16 states a thread, the four parts joined in a fixed tree (one thread a column left the
-        // other sub-partitions' FP64 pipes idle: 17,000 clocks of a short launch's 63,000); FP64 in order
+        // (in order: a search's parabolic steps magnify the last bit of a value.  A short launch is one
+        // CTA's chain, so it has the prior in shared memory and eight steps' loads in flight.)
         double tl = 0.0, te = 0.0;
-        constexpr int PARTS = sizeof(T) == 4 ? 4 : 1, PW = (TC + 31) / 32;       // PW: warps across the columns
-        double2 *zp = reinterpret_cast<double2 *>(Et) + K;        // [PARTS][TC], behind prior and wlog
-        if (tid < PARTS * PW * 32) {
-            const int part = (tid >> 5) / PW, col = tid & (32 * PW - 1);
-            if (col < TC) {
-                const T *ar = slots + (size_t)sched[a.n_internal - 1].oslot * K * TC;
-                const double *pr = reinterpret_cast<const double *>(Et), *wl = pr + K;
-                double z = 0.0, wz = 0.0;
-#pragma unroll 8
-                for (int s = K / PARTS * part; s < K / PARTS * (part + 1); s++) {
-                    double x = (double)ar[s * TC + col];
-                    z += x * pr[s];
-                    wz += x * wl[s];
-                }
-                zp[part * TC + col] = make_double2(z, wz);
-            }
-        }
-        __syncthreads();
         if (tid < TC && tid < ncols) {
-            double z = zp[tid].x, wz = zp[tid].y;
-            if constexpr (PARTS == 4) {
-                const double2 p1 = zp[TC + tid], p2 = zp[2 * TC + tid], p3 = zp[3 * TC + tid];
-                z = (z + p1.x) + (p2.x + p3.x);
-                wz = (wz + p1.y) + (p2.y + p3.y);
+            const T *ar = slots + (size_t)sched[a.n_internal - 1].oslot * K * TC;
+            const double *pr = SMALL ? reinterpret_cast<const double *>(Et) : a.m.prior + md * K;
+            const double *wl = SMALL ? pr + K : a.m.wlog + md * K;
+            double z = 0.0, wz = 0.0;
+#pragma unroll (SMALL ? 8 : 4)
+            for (int s = 0; s < K; s++) {
+                double x = (double)ar[s * TC + tid];
+                z += x * pr[s];
+                wz += x * wl[s];
             }
             if (z > 0.0) {
                 tl = log(z) + (double)cscale[tid] * 0.69314718055994530942 - (dith ? dsum[tid] : 0.0);
