@@ -140,3 +140,46 @@ def test_gradient_tiles(name, prec, lengths):
         scale = np.abs(db1).max() * max(lengths)
         assert np.abs(db[r] - db1[s].sum(0)).max() <= 1e-12 * scale
         assert abs(dr[r] - dr1[s].sum()) <= 1e-12 * scale * ps.tree.branch[:ps.tree.n - 1].sum()
+
+
+def _two_inner(n, rng):
+    """A tree whose nodes have two internal children wherever they can."""
+    labels = iter(range(n))
+
+    def rec(k):
+        if k == 1:
+            return "s%d:%.6f" % (next(labels), rng.uniform(0.005, 0.4))
+        b = 1 if k < 4 else max(2, k // 3)
+        return "(%s,%s):%.6f" % (rec(k - b), rec(b), rng.uniform(0.001, 0.2))
+
+    return rec(n).rsplit(":", 1)[0]
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32b"])
+@pytest.mark.parametrize("nl", [4, 7, 40])
+def test_gradient_two_internal_children(prec, nl):
+    """Both sides of a node compute a beta, whose exponents start from that side's own: those of the other
+    side or of another column would move entries by powers of two.  64 columns, one by one and together.
+    Tolerances: FP64 as above; FP32 1e-4 relative plus 1e-5 per column (partials carry up to ~40 x 3
+    roundings of 6e-8, against terms of at most the largest |Q_aa| of about 2)."""
+    rng = np.random.default_rng(nl)
+    tree = P.Tree.from_newick(_two_inner(nl, rng))
+    lch, rch = (np.full(tree.n, -1, np.int32) for _ in range(2))
+    for i in range(tree.n - 1):
+        (lch if lch[tree.parent[i]] < 0 else rch)[tree.parent[i]] = i
+    ps = synth.load_params("12flies")
+    L = 64
+    gf = synth.gap_fractions(rng, 1, nl, 0.05, 0.4, 0.2)
+    _, leaves = synth.simulate(synth.ParamSet("t", tree, ps.S_c, ps.pi_c, ps.S_n, ps.pi_n), np.array([L]),
+                               np.ones(1, np.int32), gf, nl)
+    mc = O.OModel.from_ecm(ps.S_c, ps.pi_c)
+    ot = O.OTree(O.Tree(tree.labels, tree.parent, lch, rch, tree.branch))
+    e = P.Engine(tree, ps.S_c, ps.pi_c, ps.S_n, ps.pi_n, precision=prec)
+    for rho in (0.4, 2.0):
+        _, db, _, st = e.grad(e.batch(np.arange(L + 1), leaves), 0, rho)
+        whole = e.grad(e.batch([0, L], leaves), 0, rho)[1][0]
+        assert (st == 0).all()
+        ref = np.array([O.grad_branches(mc, ot, rho, H.u8_to_oracle(leaves[c:c + 1]))[1] for c in range(L)])
+        for got, want, cols in ((db, ref, 1), (whole, ref.sum(0), L)):
+            tol = 1e-7 * np.abs(want) + 1e-8 * cols if prec == "fp64" else 1e-4 * np.abs(want) + 1e-5 * cols
+            assert (np.abs(got - want) <= tol).all(), (rho, cols, np.abs(got - want).max())
