@@ -189,6 +189,7 @@ int pcsf_engine_exact_available(const pcsf_engine *e);
  * shapes on the same sample and keep the faster (pcsf_stats.tc_shape):
  *   0: every CTA that fits an SM (two);  1: one CTA per SM.
  * Both run the same kernel on the same tiles: the values are identical.
+ * A sample so short that the candidates run as the same launch leaves a choice as it was.
  * No reference counterpart (the reference has no device). */
 int pcsf_engine_autotune(pcsf_engine *e, pcsf_batch *b, int32_t *tile);
 

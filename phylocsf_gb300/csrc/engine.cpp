@@ -2481,7 +2481,11 @@ int pcsf_engine_autotune(pcsf_engine *e, pcsf_batch *b, int32_t *tile)
     int best = 0;
     double best_ms = 1e300;
     int rc = PCSF_OK;
+    // a sample short enough for the small tiles runs them whatever the candidate: the choice stays
+    const bool short_sample = launch_tile(e, b, reqs) == PRUNE_SMALL_TILE;
+    if (short_sample) best = simt_tile_cols(e->prec, e->nslots, e->simt_tile);
     for (int cand : {64, 32}) {
+        if (short_sample) break;
         if (prune_smem_bytes(e->prec, e->nslots, e->nl, (int)e->sched.size(), cand) > e->smem_optin) continue;
         e->simt_tile = cand;
         e->prune_grid = simt_grid(e, cand);
@@ -2505,8 +2509,10 @@ int pcsf_engine_autotune(pcsf_engine *e, pcsf_batch *b, int32_t *tile)
         e->prune_grid = saved_grid;
         return rc != PCSF_OK ? rc : e->fail(PCSF_EINVAL, "pcsf_engine_autotune: no tile fits this tree");
     }
-    e->simt_tile = best;
-    e->prune_grid = simt_grid(e, best);
+    if (!short_sample) {
+        e->simt_tile = best;
+        e->prune_grid = simt_grid(e, best);
+    }
     if (tile) *tile = best;
     // the TF32 search kernel's shape (the values do not depend on it), timed on the same
     // sample's search evaluations
@@ -2515,6 +2521,11 @@ int pcsf_engine_autotune(pcsf_engine *e, pcsf_batch *b, int32_t *tile)
         const pcsf_stats keep = e->stats;
         int best_s = -1;
         double best_s_ms = 1e300;
+        // the shapes differ in the CTAs of a launch alone: with no more tiles than one CTA per SM
+        // takes, both are the same launch, and the choice stays
+        int64_t tiles = 0;
+        for (const Request &q : reqs)
+            tiles += (b->offs[q.region + 1] - b->offs[q.region] + prune_tile_cols(e->prec) - 1) / prune_tile_cols(e->prec);
         for (int cand = 0; cand < PCSF_TC_SHAPES; cand++) {
             e->tc_shape = cand;
             e->tc_grid = e->sm_count * prune_tc_ctas_per_sm(e->nl, (int)e->sched.size(), cand);
@@ -2538,6 +2549,7 @@ int pcsf_engine_autotune(pcsf_engine *e, pcsf_batch *b, int32_t *tile)
             e->tc_grid = saved_tc_grid;
             return rc != PCSF_OK ? rc : e->fail(PCSF_EINVAL, "pcsf_engine_autotune: no tensor-core shape fits");
         }
+        if (tiles <= e->sm_count) best_s = saved_shape;
         e->tc_shape = best_s;
         e->tc_grid = e->sm_count * prune_tc_ctas_per_sm(e->nl, (int)e->sched.size(), best_s);
     }

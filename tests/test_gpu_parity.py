@@ -325,6 +325,27 @@ def test_autotune_keeps_values(name, prec):
     e.close()
 
 
+@pytest.mark.parametrize("name,prec,default", [("58mammals", "fp32b", 64), ("120mammals", "tf32x3b", 32)])
+def test_autotune_short_sample(name, prec, default):
+    """A sample too short to tell the candidates apart (both SIMT tiles run as the small one, both search
+    shapes as the same launch) leaves the choice as it was, however the timing falls."""
+    ps = synth.load_params(name)
+    offs, leaves = _synthetic(name, [40, 7, 133], seed=13)
+    for _ in range(4):
+        e = P.Engine(ps.tree, ps.S_c, ps.pi_c, ps.S_n, ps.pi_n, precision=prec)
+        shapes = (0, 1) if prec == "tf32x3b" else (None,)
+        for shape in shapes:
+            if shape is not None:
+                e.set_tc_shape(shape)
+            for _ in range(3):
+                assert e.autotune(e.batch(offs, leaves)) == default
+                assert e.stats()["simt_tile"] == default
+                if shape is not None:
+                    assert e.stats()["tc_shape"] == shape
+                    assert (e.tc_shape_times() > 0).all()
+        e.close()
+
+
 def test_batch_outlives_engine():
     """A batch destroyed after its engine (an explicit close of the engine while batches are
     still referenced): the batch's destroy reads only its own fields, and calls through a closed
