@@ -91,6 +91,9 @@ inline uint64_t splitmix64(uint64_t &s)
 inline double uniform01(uint64_t &s) { return (double)(splitmix64(s) >> 11) * (1.0 / 9007199254740992.0); }
 
 constexpr size_t ONESHOT_KEEP = size_t(64) << 20;   // most leaf bytes an engine keeps after pcsf_score_batch
+// leaf bytes up to which pcsf_score_batch reads the codes' check with its first evaluation's results
+// (waiting for the upload first would add a tenth to the smallest calls); beyond, before it scores
+constexpr size_t ONESHOT_QUEUE = size_t(1) << 20;
 
 constexpr double GOLDEN = 0.3819660;
 constexpr double SQRT_DBL_EPS = 1.4901161193847656e-08;
@@ -169,6 +172,7 @@ struct pcsf_engine {
     HostBuf<unsigned long long> hbad;
     DevBuf<double> dpart;
     std::unique_ptr<pcsf_batch> oneshot;   // pcsf_score_batch's regions; the leaf buffer stays up to ONESHOT_KEEP
+    const uint8_t *unchecked = nullptr;    // within pcsf_score_batch: its leaves, while the check of their codes is queued
     // gradient path
     DevBuf<unsigned char> gscratch;
     bool grad_recompute = false;   // adjoint: recompute leaf children's partials instead of storing them
@@ -690,6 +694,8 @@ struct Eval {
     int status;
 };
 
+static int batch_codes(pcsf_engine *e, const uint8_t *leaves);      // below: reads a queued check of leaf codes
+
 // grad (optional): d lpr / d t_c per request, [nreq][nbr], by the adjoint kernel.
 // accurate: on a tensor-core engine, use the compensated FP32 kernel instead
 // (every likelihood the engine returns comes from it; see tc_kernels.cu).
@@ -988,6 +994,10 @@ static int evaluate(pcsf_engine *e, pcsf_batch *b, const std::vector<Request> &r
     CK(cudaMemcpyAsync(e->herr.p, e->derr.p, sizeof(int), cudaMemcpyDeviceToHost, s), "D2H error flag");
     CK(cudaStreamSynchronize(s), "evaluation");
     chunk_times();
+    if (e->unchecked) {
+        const int rc = batch_codes(e, std::exchange(e->unchecked, nullptr));
+        if (rc) return rc;
+    }
     const int32_t *hstatus = reinterpret_cast<const int32_t *>(hptr(o_st));
     const double *hlpr = reinterpret_cast<const double *>(hptr(o_lpr)), *helpr = reinterpret_cast<const double *>(hptr(o_elpr));
     if (*e->herr.p) return e->fail(PCSF_ECUDA, "a tensor-core wait timed out; results of this call are invalid");
@@ -2276,7 +2286,9 @@ static int batch_upload(pcsf_engine *e, pcsf_batch *b, int32_t n_regions, const 
     if (ce == cudaSuccess) ce = launch_check_codes(b->dleaves.p, nbytes, e->dbadcode.p, e->stream);
     if (ce == cudaSuccess)
         ce = cudaMemcpyAsync(e->hbad.p, e->dbadcode.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost, e->stream);
-    return ce == cudaSuccess ? PCSF_OK : e->cuda_fail(ce, "batch upload");
+    if (ce == cudaSuccess) return PCSF_OK;
+    cudaStreamSynchronize(e->stream);      // a queued copy may still read the caller's leaves
+    return e->cuda_fail(ce, "batch upload");
 }
 
 static int batch_codes(pcsf_engine *e, const uint8_t *leaves)
@@ -2761,22 +2773,38 @@ int pcsf_score_batch(pcsf_engine *e, int32_t n_regions, const int64_t *col_offse
     if (!e) return PCSF_EINVAL;
     CK(cudaSetDevice(e->device), "cudaSetDevice");
     // the regions of a one-shot call live in the engine's own batch, whose leaf buffer is kept for
-    // the next call unless it is large; the codes' check is read after the scoring, which waits for
-    // the stream in any case, and nothing is written to out before
+    // the next call unless it is large
     if (!e->oneshot) e->oneshot.reset(new (std::nothrow) pcsf_batch());
     if (!e->oneshot) return e->fail(PCSF_ENOMEM, "out of host memory");
     pcsf_batch *b = e->oneshot.get();
+    // however the call ends: nothing reads the caller's leaves any more, and no large buffer stays
+    struct Leave {
+        pcsf_engine *e;
+        pcsf_batch *b;
+        ~Leave()
+        {
+            if (e->unchecked) cudaStreamSynchronize(e->stream);
+            e->unchecked = nullptr;
+            if (b->dleaves.n > ONESHOT_KEEP) b->dleaves.release();
+        }
+    } leave{e, b};
     int rc = batch_upload(e, b, n_regions, col_offsets, leaves);
-    if (rc == PCSF_OK) {
-        std::vector<pcsf_result> res(n_regions);
-        int rs = pcsf_score(e, b, strategy, n_regions > 0 && !out ? nullptr : res.data());
-        const std::string why = e->err;
+    if (rc) return rc;
+    // invalid codes are refused before anything is scored (large batches) or with the first
+    // evaluation's results (small ones), and in any case before another error and before out is written
+    e->unchecked = leaves;
+    auto codes = [&]() -> int {
+        if (!e->unchecked) return PCSF_OK;
         CK(cudaStreamSynchronize(e->stream), "batch upload");
-        rc = batch_codes(e, leaves);
-        if (rc == PCSF_OK && rs != PCSF_OK) rc = e->fail(rs, "%s", why.c_str());
-        if (rc == PCSF_OK && n_regions > 0) std::memcpy(out, res.data(), sizeof(pcsf_result) * n_regions);
+        return batch_codes(e, std::exchange(e->unchecked, nullptr));
+    };
+    if ((size_t)b->total_cols * e->nl > ONESHOT_QUEUE && (rc = codes())) return rc;
+    rc = pcsf_score(e, b, strategy, out);
+    if (e->unchecked) {                    // no evaluation has run
+        const std::string why = e->err;
+        if (int bad = codes()) return bad;
+        e->err = why;
     }
-    if (b->dleaves.n > ONESHOT_KEEP) b->dleaves.release();
     return rc;
 }
 

@@ -407,7 +407,8 @@ class Engine:
         return out
 
     def score_batch(self, col_offsets, leaves, strategy: int = MLE) -> np.ndarray:
-        """One-shot: host buffers in, results out (upload, score, free)."""
+        """One-shot: host buffers in, results out.  The engine keeps the leaf buffer (up to 64 MiB) for
+        the next call."""
         offs = np.ascontiguousarray(col_offsets, np.int64)
         lv = np.ascontiguousarray(leaves, np.uint8)
         out = np.zeros(len(offs) - 1, RESULT_DTYPE)
