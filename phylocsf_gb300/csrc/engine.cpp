@@ -1660,28 +1660,35 @@ static int outside_impl(pcsf_engine *e, pcsf_batch *b, int model, const double *
     const size_t scr = outside_scratch_per_cta(fp64, e->nl);
     const size_t pset_bytes = (size_t)e->nbr * K2 * es;
     const size_t cnt_bytes = counts ? (size_t)e->nbr * K2 * sizeof(double) : 0;
-    // regions per launch: P sets and counts of a chunk within ~2 GiB (a region of several parts has
-    // its parts' counts beside its own: one more per region and one per CTA at most)
+    // regions of a chunk: P sets and counts within ~2 GiB
     const int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)std::max(nreg, 1),
-                                                                (size_t(2) << 30) / (pset_bytes + 2 * cnt_bytes)));
-    // CTAs of a launch: every SM's worth, at most the tiles of the longest chunk
+                                                                (size_t(2) << 30) / (pset_bytes + cnt_bytes)));
+    // tiles of a launch: their own counts within ~2 GiB, at most the tiles of the longest chunk; and
+    // CTAs, every SM's worth
+    auto tiles_of = [&](int r) { return (b->offs[r + 1] - b->offs[r] + TC - 1) / TC; };
     int64_t most_tiles = 1;
     for (int r0 = 0; r0 < nreg; r0 += chunk) {
         int64_t t = 0;
-        for (int r = r0; r < std::min(nreg, r0 + chunk); r++) t += (b->offs[r + 1] - b->offs[r] + TC - 1) / TC;
+        for (int r = r0; r < std::min(nreg, r0 + chunk); r++) t += tiles_of(r);
         most_tiles = std::max(most_tiles, t);
     }
-    const int grid = (int)std::min<int64_t>(
-        (int64_t)e->sm_count * outside_ctas_per_sm(fp64, comp, e->nslots, e->nl, (int)e->sched.size()), most_tiles);
-    DevBuf<unsigned char> dP, dscr;
-    DevBuf<double> dcnt, dlpr, dlprp, dpost;
-    DevBuf<OutsidePart> dparts;
+    if (most_tiles > INT32_MAX) return e->fail(PCSF_ERANGE, "outside pass: more than 2^31 column tiles");
+    const size_t tile_bytes = counts ? pset_bytes : 0;
+    const int launch = (int)std::min<int64_t>(
+        most_tiles, counts ? std::max<int64_t>(1, (int64_t)((size_t(2) << 30) / tile_bytes)) : most_tiles);
+    const int grid = std::min(e->sm_count * outside_ctas_per_sm(fp64, comp, e->nslots, e->nl, (int)e->sched.size()), launch);
+    DevBuf<unsigned char> dP, dscr, dtile;
+    DevBuf<double> dcnt, dlpr, dtlpr, dpost;
     DevBuf<PSet> dps;
     DevBuf<Request> dreq;
     DevBuf<WorkItem> dwi;
     DevBuf<int32_t> dwib, dstatus, dsel;
     CK(dP.reserve((size_t)chunk * pset_bytes), "cudaMalloc P(t)");
     CK(dscr.reserve((size_t)grid * scr), "cudaMalloc outside-pass scratch");
+    if (counts) CK(dcnt.reserve((size_t)chunk * e->nbr * K2), "cudaMalloc counts");
+    CK(dtile.reserve((size_t)launch * tile_bytes), "cudaMalloc counts of the tiles");
+    CK(dtlpr.reserve(most_tiles), "cudaMalloc");
+    CK(dwi.reserve(most_tiles), "cudaMalloc");
     CK(dlpr.reserve(chunk), "cudaMalloc");
     CK(dps.reserve(chunk), "cudaMalloc");
     CK(dreq.reserve(chunk), "cudaMalloc");
@@ -1698,45 +1705,26 @@ static int outside_impl(pcsf_engine *e, pcsf_batch *b, int model, const double *
         std::vector<PSet> ps(nr);
         std::vector<Request> rq(nr);
         std::vector<WorkItem> wis;
-        std::vector<OutsidePart> parts;
-        std::vector<int32_t> pbeg(nr + 1);
-        // tiles per part: the chunk's tiles over the CTAs (a part's counts stay in its own buffer,
-        // so that shorter parts would only cost memory and the summing)
-        int64_t ntiles = 0;
-        for (int r = r0; r < r1; r++) ntiles += (b->offs[r + 1] - b->offs[r] + TC - 1) / TC;
-        const int tpp = (int)std::max<int64_t>(1, (ntiles + grid - 1) / grid);
-        int nslot = nr;
+        std::vector<int32_t> wib(nr + 1);
         for (int r = 0; r < nr; r++) {
             const int reg = r0 + r;
             if (!(rho[reg] > 0.0) || !std::isfinite(rho[reg])) return e->fail(PCSF_EINVAL, "rho[%d] = %g", reg, rho[reg]);
             ps[r] = PSet{model, 0, rho[reg]};
             rq[r] = Request{reg, model, r, (uint32_t)b->offs[reg], rho[reg]};
-            pbeg[r] = (int)parts.size();
-            const int w0 = (int)wis.size();
+            wib[r] = (int)wis.size();
             for (int64_t c = b->offs[reg]; c < b->offs[reg + 1]; c += TC)
                 wis.push_back(WorkItem{r, (int32_t)std::min<int64_t>(TC, b->offs[reg + 1] - c), c});
-            const int w1 = (int)wis.size();
-            for (int w = w0; w < w1; w += tpp)
-                parts.push_back(OutsidePart{r, w, std::min(w + tpp, w1), w1 - w0 <= tpp ? r : nslot++});
         }
-        pbeg[nr] = (int)parts.size();
-        if (counts) CK(dcnt.reserve((size_t)nslot * e->nbr * K2), "cudaMalloc counts");
-        CK(dparts.reserve(parts.size()), "cudaMalloc");
-        CK(dlprp.reserve(parts.size()), "cudaMalloc");
-        CK(dwi.reserve(std::max<size_t>(wis.size(), 1)), "cudaMalloc");
+        wib[nr] = (int)wis.size();
         CK(cudaMemcpyAsync(dps.p, ps.data(), sizeof(PSet) * nr, cudaMemcpyHostToDevice, s), "H2D");
         CK(cudaMemcpyAsync(dreq.p, rq.data(), sizeof(Request) * nr, cudaMemcpyHostToDevice, s), "H2D");
         if (!wis.empty()) CK(cudaMemcpyAsync(dwi.p, wis.data(), sizeof(WorkItem) * wis.size(), cudaMemcpyHostToDevice, s), "H2D");
-        CK(cudaMemcpyAsync(dwib.p, pbeg.data(), sizeof(int32_t) * (nr + 1), cudaMemcpyHostToDevice, s), "H2D");
-        if (!parts.empty())
-            CK(cudaMemcpyAsync(dparts.p, parts.data(), sizeof(OutsidePart) * parts.size(), cudaMemcpyHostToDevice, s), "H2D");
+        CK(cudaMemcpyAsync(dwib.p, wib.data(), sizeof(int32_t) * (nr + 1), cudaMemcpyHostToDevice, s), "H2D");
         CK(cudaMemsetAsync(dstatus.p, 0x7f, sizeof(int32_t) * nr, s), "memset");
         CK(launch_pform(fp64, dps.p, nr, e->dbranch.p, e->nbr, e->dm, dP.p, dstatus.p, s), "P(t) formation launch");
         OutsideArgs oa{};
         oa.wi = dwi.p;
-        oa.parts = dparts.p;
-        oa.nparts = (int)parts.size();
-        oa.part_begin = dwib.p;
+        oa.wi_begin = dwib.p;
         oa.nreq = nr;
         oa.req = dreq.p;
         oa.leaves = b->dleaves.p;
@@ -1749,14 +1737,21 @@ static int outside_impl(pcsf_engine *e, pcsf_batch *b, int model, const double *
         oa.m = e->dm;
         oa.scratch = dscr.p;
         oa.scratch_per_cta = scr;
-        oa.lpr = dlprp.p;
-        oa.lpr_out = dlpr.p;
+        oa.tile_lpr = dtlpr.p;
+        oa.lpr = dlpr.p;
+        oa.tile_counts = dtile.p;
         oa.counts = counts ? dcnt.p : nullptr;
         oa.sel = n_sel > 0 ? dsel.p : nullptr;
         oa.post = dpost.p;
         oa.total_cols = b->total_cols;
-        CK(launch_outside(fp64, comp, oa, s, grid), "outside-pass launch");
-        e->stats.kernel_launches += 3;
+        e->stats.kernel_launches += 1;
+        oa.wi1 = 0;
+        do {
+            oa.wi0 = oa.wi1;
+            oa.wi1 = (int)std::min<int64_t>(oa.wi0 + (int64_t)launch, (int64_t)wis.size());
+            CK(launch_outside(fp64, comp, oa, s, grid), "outside-pass launch");
+            e->stats.kernel_launches += 2;
+        } while (oa.wi1 < (int)wis.size());
         std::vector<int32_t> keys(nr);
         std::vector<double> hl(nr);
         CK(cudaMemcpyAsync(keys.data(), dstatus.p, sizeof(int32_t) * nr, cudaMemcpyDeviceToHost, s), "D2H");

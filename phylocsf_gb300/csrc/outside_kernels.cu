@@ -12,14 +12,15 @@
 // per tile a 64 x 64 x (tile columns) product, accumulated over the tiles of a region
 // and multiplied by P_c once at the end.
 //
-// One CTA owns one part of a request (region, model, rho) at a time, a run of its column
-// tiles, and walks them in order; k_counts sums a request's parts in order and multiplies
-// by P_c (no atomics; the parts depend on the number of tiles and SMs alone).  A CTA per
-// request left a call of 64 regions waiting for the longest one, 47 tiles in a row, and the
-// count products read alpha from global memory with 16 lines per load: 38.4 ms on 29 leaves
-// (27,641 columns), 3.1 ms with parts and the products' operands column by column in shared
-// memory.  What bounds it now is the chain of a side's phases at three CTAs per SM, FP64
-// conversions and sums (two lanes per clock) among them.  The inside pass is the one of k_grad and
+// One CTA owns one column tile at a time and leaves its count product in memory of the tile's own;
+// k_counts adds the tiles of a request in order in FP64 and multiplies by P_c (no atomics): the results
+// depend on the region alone, not on the launch configuration or on the call's other regions.  A CTA
+// per request, its tiles in a row, left a call of 64 regions waiting for the longest one, 47 tiles
+// (38.4 ms on 29 leaves, 27,641 columns, where the count products also read alpha from global memory
+// with 16 lines per load; now the products' operands lie column by column in shared memory).
+// Measured there: 3.1 ms.  What bounds it is the chain of a side's phases at three
+// CTAs per SM, and in k_counts FP64 conversions and sums (two lanes per clock).
+// The inside pass is the one of k_grad and
 // stores every child partial, the alpha of every internal node and the per-column
 // exponents of the power-of-two rescaling in a per-CTA scratch area; exponent
 // bookkeeping per column as in k_grad:
@@ -101,268 +102,256 @@ __global__ void __launch_bounds__(OS_THREADS) k_outside(OutsideArgs a)
 
     for (int f = tid; f < a.n_internal; f += OS_THREADS) sched[f] = a.sched[f];
 
-    for (int pt = blockIdx.x; pt < a.nparts; pt += gridDim.x) {
-        const OutsidePart part = a.parts[pt];
-        const Request rq = a.req[part.request];
+    for (int w = a.wi0 + blockIdx.x; w < a.wi1; w += gridDim.x) {
+        const WorkItem wi = a.wi[w];
+        const Request rq = a.req[wi.request];
         const int md = rq.model;
         const T *Pbase = reinterpret_cast<const T *>(a.Pbuf) + (size_t)rq.pset * a.nbr * K2;
         const double *pr = a.m.prior + md * K;
-        double *cnt = a.counts ? a.counts + (size_t)part.slot * a.nbr * K2 : nullptr;
-        double lpr = 0.0;    // thread 0: the part's log-likelihood, summed tile by tile in order
+        T *cnt = a.counts ? reinterpret_cast<T *>(a.tile_counts) + (size_t)(w - a.wi0) * a.nbr * K2 : nullptr;
+        const int ncols = wi.ncols;
+        const uint8_t *lg = a.leaves + (size_t)wi.col0 * nl;
+        __syncthreads();   // the previous tile is finished with shared memory
+        for (int f = tid; f < TC * nl; f += OS_THREADS) {
+            const int c = f / nl, l = f - c * nl;
+            lvT[l * TC + c] = (c < ncols) ? lg[f] : (uint8_t)K;
+        }
+        for (int f = tid; f < TC; f += OS_THREADS) colmax[f] = 0;
 
-        for (int w = part.wi0; w < part.wi1; w++) {
-            const WorkItem wi = a.wi[w];
-            const int ncols = wi.ncols;
-            const uint8_t *lg = a.leaves + (size_t)wi.col0 * nl;
-            __syncthreads();   // the previous tile is finished with shared memory
-            for (int f = tid; f < TC * nl; f += OS_THREADS) {
-                const int c = f / nl, l = f - c * nl;
-                lvT[l * TC + c] = (c < ncols) ? lg[f] : (uint8_t)K;
+        // ---------------- inside pass, storing the child partials and the node alphas
+        __syncthreads();   // leaf states ready
+        stage_children<T, TC, CPT, OS_THREADS>(Mat, Pbase, sched[0], lvT, tid);
+        for (int ni = 0; ni < a.n_internal; ni++) {
+            const SchedNode sn = sched[ni];
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();
+            T vl[4][CPT], vr[4][CPT];
+            child_partial<T, TC, KAHAN>(Mat, slots, sn.lslot, sn.lc, lvT, a0, c0, vl, -1, true);
+            child_partial<T, TC, KAHAN>(Mat + K2, slots, sn.rslot, sn.rc, lvT, a0, c0, vr, -1, true);
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int cc = 0; cc < CPT; cc++) {
+                    V[((size_t)sn.lc * K + a0 + i) * TC + c0 + cc] = vl[i][cc];
+                    V[((size_t)sn.rc * K + a0 + i) * TC + c0 + cc] = vr[i][cc];
+                }
+            __syncthreads();   // Mat and slot reads done
+            if (ni + 1 < a.n_internal) stage_children<T, TC, CPT, OS_THREADS>(Mat, Pbase, sched[ni + 1], lvT, tid);
+#pragma unroll
+            for (int cc = 0; cc < CPT; cc++) {
+                T mx = (T)0;
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    vl[i][cc] *= vr[i][cc];
+                    mx = vl[i][cc] > mx ? vl[i][cc] : mx;
+                }
+                AtomMax<T>::upd(colmax + c0 + cc, mx);
             }
+            __syncthreads();
+            T *out = slots + (size_t)sn.oslot * K * TC;
+            T *Ai = A + (size_t)(sn.node - nl) * K * TC;
+#pragma unroll
+            for (int cc = 0; cc < CPT; cc++) {
+                const T mx = AtomMax<T>::get(colmax + c0 + cc);
+                const int e = (mx > (T)0) ? exp_of(mx) : 0;
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const T y = scale2(vl[i][cc], -e);
+                    out[(a0 + i) * TC + c0 + cc] = y;
+                    Ai[(size_t)(a0 + i) * TC + c0 + cc] = y;
+                }
+                if (ty == 0) {
+                    const int col = c0 + cc;
+                    eS[(size_t)sn.node * TC + col] = e_of(sn.lc, col) + e_of(sn.rc, col) + e;
+                }
+            }
+            __syncthreads();   // colmax reads done
             for (int f = tid; f < TC; f += OS_THREADS) colmax[f] = 0;
-
-            // ---------------- inside pass, storing the child partials and the node alphas
-            __syncthreads();   // leaf states ready
-            stage_children<T, TC, CPT, OS_THREADS>(Mat, Pbase, sched[0], lvT, tid);
-            for (int ni = 0; ni < a.n_internal; ni++) {
-                const SchedNode sn = sched[ni];
-                asm volatile("cp.async.wait_all;" ::: "memory");
-                __syncthreads();
-                T vl[4][CPT], vr[4][CPT];
-                child_partial<T, TC, KAHAN>(Mat, slots, sn.lslot, sn.lc, lvT, a0, c0, vl, -1, true);
-                child_partial<T, TC, KAHAN>(Mat + K2, slots, sn.rslot, sn.rc, lvT, a0, c0, vr, -1, true);
+        }
+        __syncthreads();
+        // ---------------- root: z~ and the column log-likelihoods
+        double tl = 0.0;
+        if (tid < TC) {
+            const T *ar = A + (size_t)(root - nl) * K * TC;
+            double z = 0.0;
+            for (int s = 0; s < K; s++) z += (double)ar[s * TC + tid] * pr[s];
+            zt[tid] = z;
+            eroot[tid] = eS[(size_t)root * TC + tid];
+            if (tid < ncols) tl = (z > 0.0) ? log(z) + (double)eroot[tid] * 0.69314718055994530942 : -INFINITY;
+        }
 #pragma unroll
-                for (int i = 0; i < 4; i++)
-#pragma unroll
-                    for (int cc = 0; cc < CPT; cc++) {
-                        V[((size_t)sn.lc * K + a0 + i) * TC + c0 + cc] = vl[i][cc];
-                        V[((size_t)sn.rc * K + a0 + i) * TC + c0 + cc] = vr[i][cc];
-                    }
-                __syncthreads();   // Mat and slot reads done
-                if (ni + 1 < a.n_internal) stage_children<T, TC, CPT, OS_THREADS>(Mat, Pbase, sched[ni + 1], lvT, tid);
-#pragma unroll
-                for (int cc = 0; cc < CPT; cc++) {
-                    T mx = (T)0;
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        vl[i][cc] *= vr[i][cc];
-                        mx = vl[i][cc] > mx ? vl[i][cc] : mx;
-                    }
-                    AtomMax<T>::upd(colmax + c0 + cc, mx);
-                }
-                __syncthreads();
-                T *out = slots + (size_t)sn.oslot * K * TC;
-                T *Ai = A + (size_t)(sn.node - nl) * K * TC;
-#pragma unroll
-                for (int cc = 0; cc < CPT; cc++) {
-                    const T mx = AtomMax<T>::get(colmax + c0 + cc);
-                    const int e = (mx > (T)0) ? exp_of(mx) : 0;
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        const T y = scale2(vl[i][cc], -e);
-                        out[(a0 + i) * TC + c0 + cc] = y;
-                        Ai[(size_t)(a0 + i) * TC + c0 + cc] = y;
-                    }
-                    if (ty == 0) {
-                        const int col = c0 + cc;
-                        eS[(size_t)sn.node * TC + col] = e_of(sn.lc, col) + e_of(sn.rc, col) + e;
-                    }
-                }
-                __syncthreads();   // colmax reads done
-                for (int f = tid; f < TC; f += OS_THREADS) colmax[f] = 0;
-            }
-            __syncthreads();
-            // ---------------- root: z~ and the column log-likelihoods
-            double tl = 0.0;
-            if (tid < TC) {
+        for (int o = 16; o > 0; o >>= 1) tl += __shfl_down_sync(0xffffffffu, tl, o);
+        if ((tid & 31) == 0) wsum[tid >> 5] = tl;
+        {   // beta~_root = prior, f(root) = 0
+            T *Br = B + (size_t)(root - nl) * K * TC;
+            for (int f = tid; f < K * TC; f += OS_THREADS) Br[f] = (T)pr[f / TC];
+            for (int f = tid; f < TC; f += OS_THREADS) fS[(size_t)root * TC + f] = 0;
+        }
+        __syncthreads();
+        if (tid == 0) {
+            double lpr = 0.0;
+            for (int k = 0; k < (TC + 31) / 32; k++) lpr += wsum[k];
+            a.tile_lpr[w] = lpr;
+        }
+        // posteriors of the selected root and leaves (node_posterior: zeros where z = 0)
+        if (a.sel) {
+            const int kr = a.sel[root];
+            if (kr >= 0) {
                 const T *ar = A + (size_t)(root - nl) * K * TC;
-                double z = 0.0;
-                for (int s = 0; s < K; s++) z += (double)ar[s * TC + tid] * pr[s];
-                zt[tid] = z;
-                eroot[tid] = eS[(size_t)root * TC + tid];
-                if (tid < ncols) tl = (z > 0.0) ? log(z) + (double)eroot[tid] * 0.69314718055994530942 : -INFINITY;
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) tl += __shfl_down_sync(0xffffffffu, tl, o);
-            if ((tid & 31) == 0) wsum[tid >> 5] = tl;
-            {   // beta~_root = prior, f(root) = 0
-                T *Br = B + (size_t)(root - nl) * K * TC;
-                for (int f = tid; f < K * TC; f += OS_THREADS) Br[f] = (T)pr[f / TC];
-                for (int f = tid; f < TC; f += OS_THREADS) fS[(size_t)root * TC + f] = 0;
-            }
-            __syncthreads();
-            if (tid == 0)
-                for (int k = 0; k < (TC + 31) / 32; k++) lpr += wsum[k];
-            // posteriors of the selected root and leaves (node_posterior: zeros where z = 0)
-            if (a.sel) {
-                const int kr = a.sel[root];
-                if (kr >= 0) {
-                    const T *ar = A + (size_t)(root - nl) * K * TC;
-                    for (int f = tid; f < K * TC; f += OS_THREADS) {
-                        const int x = f / TC, col = f % TC;
-                        if (col >= ncols) continue;
-                        const double z = zt[col];
-                        a.post[((size_t)kr * a.total_cols + wi.col0 + col) * K + x] =
-                            (z > 0.0) ? (double)ar[x * TC + col] * pr[x] / z : 0.0;
-                    }
-                }
-                for (int l = 0; l < nl; l++) {
-                    const int kl = a.sel[l];
-                    if (kl < 0) continue;
-                    for (int f = tid; f < K * TC; f += OS_THREADS) {
-                        const int x = f / TC, col = f % TC;
-                        if (col >= ncols) continue;
-                        const int s = lvT[l * TC + col];
-                        a.post[((size_t)kl * a.total_cols + wi.col0 + col) * K + x] =
-                            (zt[col] > 0.0) ? ((s >= K || s == x) ? 1.0 : 0.0) : 0.0;
-                    }
+                for (int f = tid; f < K * TC; f += OS_THREADS) {
+                    const int x = f / TC, col = f % TC;
+                    if (col >= ncols) continue;
+                    const double z = zt[col];
+                    a.post[((size_t)kr * a.total_cols + wi.col0 + col) * K + x] =
+                        (z > 0.0) ? (double)ar[x * TC + col] * pr[x] / z : 0.0;
                 }
             }
-
-            // ---------------- outside pass, parents before children
-            for (int ni = a.n_internal - 1; ni >= 0; ni--) {
-                const SchedNode sn = sched[ni];
-                const int p = sn.node;
-                const T *Bp = B + (size_t)(p - nl) * K * TC;
-                for (int side = 0; side < 2; side++) {
-                    const int c = side ? sn.rc : sn.lc;
-                    const int s = side ? sn.lc : sn.rc;
-                    const bool internal = c >= nl;
-                    __syncthreads();   // the previous side is finished with X, Mat[0], colmax, wcol
-                    if (internal) stage_rows<T, OS_THREADS>(Ert, Pbase + (size_t)c * K2, tid);
-                    for (int f = tid; f < TC; f += OS_THREADS) colmax[f] = 0;
-                    const T *Vs = V + (size_t)s * K * TC;
-                    for (int f = tid; f < K * TC; f += OS_THREADS) X[f] = Bp[f] * Vs[f];    // inter~
-                    if (tid < TC) {   // weight of column tid in the counts: 2^{f(p) + e(s) + e(c) - e(root)} / z~
-                        const double z = zt[tid];
-                        wcol[tid] = (tid < ncols && z > 0.0)
-                                        ? ldexp(1.0, fS[(size_t)p * TC + tid] + e_of(s, tid) + e_of(c, tid) - eroot[tid]) / z
-                                        : 0.0;
-                    }
-                    asm volatile("cp.async.wait_all;" ::: "memory");
-                    __syncthreads();
-                    if (internal) {
-                        // beta~_c = P_c^T inter~ = inter~ + E_c^T inter~, rescaled per column
-                        T bt[4][CPT];
-                        contract_rows<T, TC, KAHAN>(Ert, X, a0, c0, bt);
-#pragma unroll
-                        for (int cc = 0; cc < CPT; cc++) {
-                            T mx = (T)0;
-#pragma unroll
-                            for (int i = 0; i < 4; i++) {
-                                bt[i][cc] += X[(a0 + i) * TC + c0 + cc];
-                                mx = bt[i][cc] > mx ? bt[i][cc] : mx;
-                            }
-                            AtomMax<T>::upd(colmax + c0 + cc, mx);
-                        }
-                        __syncthreads();
-                        T *Bc = B + (size_t)(c - nl) * K * TC;
-                        const T *Ac = A + (size_t)(c - nl) * K * TC;
-                        const int kc = a.sel ? a.sel[c] : -1;
-#pragma unroll
-                        for (int cc = 0; cc < CPT; cc++) {
-                            const int col = c0 + cc;
-                            const T mx = AtomMax<T>::get(colmax + col);
-                            const int e = (mx > (T)0) ? exp_of(mx) : 0;
-                            const int fc = fS[(size_t)p * TC + col] + e_of(s, col) + e;
-#pragma unroll
-                            for (int i = 0; i < 4; i++) {
-                                const T y = scale2(bt[i][cc], -e);
-                                Bc[(size_t)(a0 + i) * TC + col] = y;
-                                if (kc >= 0 && col < ncols) {
-                                    const double z = zt[col];
-                                    a.post[((size_t)kc * a.total_cols + wi.col0 + col) * K + a0 + i] =
-                                        (z > 0.0) ? ldexp((double)Ac[(size_t)(a0 + i) * TC + col] * (double)y,
-                                                          e_of(c, col) + fc - eroot[col]) / z
-                                                  : 0.0;
-                                }
-                            }
-                            if (ty == 0) fS[(size_t)c * TC + col] = fc;
-                        }
-                    }
-                    if (cnt) {
-                        // inter~ w and alpha~_c, column by column (from here a column's 64 states
-                        // are contiguous: one vector load for each of a thread's two sides)
-                        const T *Ac = A + (size_t)(internal ? c - nl : 0) * K * TC;
-                        for (int f = tid; f < K * TC; f += OS_THREADS) {
-                            XT[(f % TC) * LDN + f / TC] = (T)((double)X[f] * wcol[f % TC]);
-                            if (internal) YT[(f % TC) * LDN + f / TC] = Ac[f];
-                        }
-                        __syncthreads();
-                        // M_c[a][b] += sum_col inter~[a] w alpha~_c[b] for this thread's 4 x 4 block
-                        T acc[4][4];
-#pragma unroll
-                        for (int i = 0; i < 4; i++)
-#pragma unroll
-                            for (int j = 0; j < 4; j++) acc[i][j] = (T)0;
-                        if (internal) {
-#pragma unroll 4
-                            for (int col = 0; col < TC; col++) {
-                                T xa[4], yb[4];
-                                Vec4<T>::load(XT + col * LDN + a0, xa);
-                                Vec4<T>::load(YT + col * LDN + b0, yb);
-#pragma unroll
-                                for (int i = 0; i < 4; i++)
-#pragma unroll
-                                    for (int j = 0; j < 4; j++) acc[i][j] += xa[i] * yb[j];
-                            }
-                        } else {
-#pragma unroll 4
-                            for (int col = 0; col < TC; col++) {
-                                const int sl = lvT[c * TC + col];
-                                T xa[4];
-                                Vec4<T>::load(XT + col * LDN + a0, xa);
-#pragma unroll
-                                for (int j = 0; j < 4; j++) {
-                                    const bool hit = sl >= K || sl == b0 + j;
-#pragma unroll
-                                    for (int i = 0; i < 4; i++) acc[i][j] = hit ? acc[i][j] + xa[i] : acc[i][j];
-                                }
-                            }
-                        }
-                        double *cc4 = cnt + (size_t)c * K2;
-                        const bool first = w == part.wi0;
-#pragma unroll
-                        for (int i = 0; i < 4; i++) {
-                            double2 *q = reinterpret_cast<double2 *>(cc4 + (a0 + i) * K + b0);
-                            double2 u = first ? make_double2(0.0, 0.0) : q[0], v = first ? make_double2(0.0, 0.0) : q[1];
-                            u.x += (double)acc[i][0];
-                            u.y += (double)acc[i][1];
-                            v.x += (double)acc[i][2];
-                            v.y += (double)acc[i][3];
-                            q[0] = u;
-                            q[1] = v;
-                        }
-                    }
+            for (int l = 0; l < nl; l++) {
+                const int kl = a.sel[l];
+                if (kl < 0) continue;
+                for (int f = tid; f < K * TC; f += OS_THREADS) {
+                    const int x = f / TC, col = f % TC;
+                    if (col >= ncols) continue;
+                    const int s = lvT[l * TC + col];
+                    a.post[((size_t)kl * a.total_cols + wi.col0 + col) * K + x] =
+                        (zt[col] > 0.0) ? ((s >= K || s == x) ? 1.0 : 0.0) : 0.0;
                 }
             }
         }
-        if (tid == 0) a.lpr[pt] = lpr;
-        __syncthreads();
+
+        // ---------------- outside pass, parents before children
+        for (int ni = a.n_internal - 1; ni >= 0; ni--) {
+            const SchedNode sn = sched[ni];
+            const int p = sn.node;
+            const T *Bp = B + (size_t)(p - nl) * K * TC;
+            for (int side = 0; side < 2; side++) {
+                const int c = side ? sn.rc : sn.lc;
+                const int s = side ? sn.lc : sn.rc;
+                const bool internal = c >= nl;
+                __syncthreads();   // the previous side is finished with X, Mat[0], colmax, wcol
+                if (internal) stage_rows<T, OS_THREADS>(Ert, Pbase + (size_t)c * K2, tid);
+                for (int f = tid; f < TC; f += OS_THREADS) colmax[f] = 0;
+                const T *Vs = V + (size_t)s * K * TC;
+                for (int f = tid; f < K * TC; f += OS_THREADS) X[f] = Bp[f] * Vs[f];    // inter~
+                if (tid < TC) {   // weight of column tid in the counts: 2^{f(p) + e(s) + e(c) - e(root)} / z~
+                    const double z = zt[tid];
+                    wcol[tid] = (tid < ncols && z > 0.0)
+                                    ? ldexp(1.0, fS[(size_t)p * TC + tid] + e_of(s, tid) + e_of(c, tid) - eroot[tid]) / z
+                                    : 0.0;
+                }
+                asm volatile("cp.async.wait_all;" ::: "memory");
+                __syncthreads();
+                if (internal) {
+                    // beta~_c = P_c^T inter~ = inter~ + E_c^T inter~, rescaled per column
+                    T bt[4][CPT];
+                    contract_rows<T, TC, KAHAN>(Ert, X, a0, c0, bt);
+#pragma unroll
+                    for (int cc = 0; cc < CPT; cc++) {
+                        T mx = (T)0;
+#pragma unroll
+                        for (int i = 0; i < 4; i++) {
+                            bt[i][cc] += X[(a0 + i) * TC + c0 + cc];
+                            mx = bt[i][cc] > mx ? bt[i][cc] : mx;
+                        }
+                        AtomMax<T>::upd(colmax + c0 + cc, mx);
+                    }
+                    __syncthreads();
+                    T *Bc = B + (size_t)(c - nl) * K * TC;
+                    const T *Ac = A + (size_t)(c - nl) * K * TC;
+                    const int kc = a.sel ? a.sel[c] : -1;
+#pragma unroll
+                    for (int cc = 0; cc < CPT; cc++) {
+                        const int col = c0 + cc;
+                        const T mx = AtomMax<T>::get(colmax + col);
+                        const int e = (mx > (T)0) ? exp_of(mx) : 0;
+                        const int fc = fS[(size_t)p * TC + col] + e_of(s, col) + e;
+#pragma unroll
+                        for (int i = 0; i < 4; i++) {
+                            const T y = scale2(bt[i][cc], -e);
+                            Bc[(size_t)(a0 + i) * TC + col] = y;
+                            if (kc >= 0 && col < ncols) {
+                                const double z = zt[col];
+                                a.post[((size_t)kc * a.total_cols + wi.col0 + col) * K + a0 + i] =
+                                    (z > 0.0) ? ldexp((double)Ac[(size_t)(a0 + i) * TC + col] * (double)y,
+                                                      e_of(c, col) + fc - eroot[col]) / z
+                                              : 0.0;
+                            }
+                        }
+                        if (ty == 0) fS[(size_t)c * TC + col] = fc;
+                    }
+                }
+                if (cnt) {
+                    // inter~ w and alpha~_c, column by column (from here a column's 64 states
+                    // are contiguous: one vector load for each of a thread's two sides)
+                    const T *Ac = A + (size_t)(internal ? c - nl : 0) * K * TC;
+                    for (int f = tid; f < K * TC; f += OS_THREADS) {
+                        XT[(f % TC) * LDN + f / TC] = (T)((double)X[f] * wcol[f % TC]);
+                        if (internal) YT[(f % TC) * LDN + f / TC] = Ac[f];
+                    }
+                    __syncthreads();
+                    // M_c[a][b] += sum_col inter~[a] w alpha~_c[b] for this thread's 4 x 4 block
+                    T acc[4][4];
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+#pragma unroll
+                        for (int j = 0; j < 4; j++) acc[i][j] = (T)0;
+                    if (internal) {
+#pragma unroll 4
+                        for (int col = 0; col < TC; col++) {
+                            T xa[4], yb[4];
+                            Vec4<T>::load(XT + col * LDN + a0, xa);
+                            Vec4<T>::load(YT + col * LDN + b0, yb);
+#pragma unroll
+                            for (int i = 0; i < 4; i++)
+#pragma unroll
+                                for (int j = 0; j < 4; j++) acc[i][j] += xa[i] * yb[j];
+                        }
+                    } else {
+#pragma unroll 4
+                        for (int col = 0; col < TC; col++) {
+                            const int sl = lvT[c * TC + col];
+                            T xa[4];
+                            Vec4<T>::load(XT + col * LDN + a0, xa);
+#pragma unroll
+                            for (int j = 0; j < 4; j++) {
+                                const bool hit = sl >= K || sl == b0 + j;
+#pragma unroll
+                                for (int i = 0; i < 4; i++) acc[i][j] = hit ? acc[i][j] + xa[i] : acc[i][j];
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; i++) ColStore<T, 4>::store(cnt + (size_t)c * K2 + (a0 + i) * K + b0, acc[i]);
+                }
+            }
+        }
     }
 }
 
-// Request r's parts in order: counts = P_c o sum M_c, and the log-likelihood.  A request of one
-// part has accumulated in its own counts already (slot r); the others' parts hold slots from
-// nreq on.  One CTA per (branch, request).
+// Request r's tiles of this launch, in order, onto the sums of those before: the log-likelihood and
+// sum M_c, which the request's last tile makes counts = P_c o sum M_c.  One CTA per (branch, request).
 template <typename T>
 __global__ void __launch_bounds__(OS_THREADS) k_counts(OutsideArgs a)
 {
     const int c = blockIdx.y, r = blockIdx.x, tid = threadIdx.x;
-    const int p0 = a.part_begin[r], p1 = a.part_begin[r + 1];
+    const int b0 = a.wi_begin[r], b1 = a.wi_begin[r + 1], w0 = max(b0, a.wi0), w1 = min(b1, a.wi1);
+    // nothing of this request in this launch (an empty one has its zeros from the first)
+    if (w0 >= w1 && (b0 < b1 || a.wi0 > 0)) return;
+    const bool first = b0 >= a.wi0, last = b1 <= a.wi1;
     if (c == 0 && tid == 0) {
-        double lpr = 0.0;
-        for (int p = p0; p < p1; p++) lpr += a.lpr[p];
-        a.lpr_out[r] = lpr;
+        double lpr = first ? 0.0 : a.lpr[r];
+        for (int w = w0; w < w1; w++) lpr += a.tile_lpr[w];
+        a.lpr[r] = lpr;
     }
     if (!a.counts) return;
     const T *Et = reinterpret_cast<const T *>(a.Pbuf) + ((size_t)a.req[r].pset * a.nbr + c) * K2;
+    const T *tc = reinterpret_cast<const T *>(a.tile_counts) + (size_t)c * K2;
     double *out = a.counts + ((size_t)r * a.nbr + c) * K2;
     for (int f = tid; f < K2; f += OS_THREADS) {
         const int aa = f / K, bb = f % K;
-        double m = 0.0;
-        for (int p = p0; p < p1; p++) m += a.counts[((size_t)a.parts[p].slot * a.nbr + c) * K2 + f];
-        out[f] = m * ((double)Et[bb * K + aa] + (aa == bb ? 1.0 : 0.0));
+        double m = first ? 0.0 : out[f];
+        for (int w = w0; w < w1; w++) m += (double)tc[(size_t)(w - a.wi0) * a.nbr * K2 + f];
+        out[f] = last ? m * ((double)Et[bb * K + aa] + (aa == bb ? 1.0 : 0.0)) : m;
     }
 }
 
@@ -372,7 +361,7 @@ cudaError_t launch_outside_t(const OutsideArgs &a, cudaStream_t s, int grid)
     const size_t smem = OutLayout<T>::smem(a.nslots, a.nl, a.n_internal);
     cudaError_t e = cudaFuncSetAttribute(k_outside<T, KAHAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    if (a.nparts > 0) k_outside<T, KAHAN><<<std::min(grid, a.nparts), OS_THREADS, smem, s>>>(a);
+    if (a.wi1 > a.wi0) k_outside<T, KAHAN><<<std::min(grid, a.wi1 - a.wi0), OS_THREADS, smem, s>>>(a);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     k_counts<T><<<dim3(a.nreq, a.counts ? a.nbr : 1), OS_THREADS, 0, s>>>(a);

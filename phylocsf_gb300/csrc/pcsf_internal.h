@@ -225,31 +225,27 @@ size_t ff_stack_floats(int grid, int depth);
 size_t prune_ff_smem_bytes(int nl, int nint);
 
 // Outside-pass products (outside_kernels.cu): per request the log-likelihood, optionally the
-// expected substitution counts of every branch and the posteriors of selected nodes.  A part is
-// a run of one request's work items (tiles of outside_tile_cols() columns, in order), worked by
-// one CTA at a time; parts of one request are contiguous.
-struct OutsidePart {
-    int32_t request;             // the request's index
-    int32_t wi0, wi1;            // its work items
-    int32_t slot;                // where its counts accumulate: the request, or nreq + k if it has several parts
-};
+// expected substitution counts of every branch and the posteriors of selected nodes.  A launch takes
+// the work items (tiles of outside_tile_cols() columns) [wi0, wi1) of those that wi holds; the sums
+// over a request's tiles go on from one launch to the next, so that they do not depend on where the
+// launches end.
 struct OutsideArgs {
-    const WorkItem *wi;
-    const OutsidePart *parts;
-    int nparts;
-    const int32_t *part_begin;   // [nreq + 1]
+    const WorkItem *wi;          // work items, contiguous per request
+    const int32_t *wi_begin;     // [nreq + 1]
+    int wi0, wi1;
     int nreq;
     const Request *req;          // Request.pset indexes Pbuf
     const uint8_t *leaves;       // [total_cols][nl]
-    const void *Pbuf;            // per P set [nbr][K][K] E^T, FP64 or FP32
+    const void *Pbuf;            // E^T sets [nps][nbr][K2] (float or double)
     const SchedNode *sched;
     int n_internal, nl, nbr, nslots;
     DevModels m;
     void *scratch;               // gridDim.x * scratch_per_cta bytes
     size_t scratch_per_cta;
-    double *lpr;                 // [nparts]
-    double *lpr_out;             // [nreq]
-    double *counts;              // [nreq + parts of split requests][nbr][K][K]; null: none
+    double *tile_lpr;            // [work items]
+    double *lpr;                 // [nreq]
+    void *tile_counts;           // [wi1 - wi0][nbr][K][K] (float or double), one launch's
+    double *counts;              // [nreq][nbr][K][K]; null: none
     const int32_t *sel;          // [n] output row of each node, -1 if not selected; null: no posteriors
     double *post;                // [n_selected][total_cols][K]
     int64_t total_cols;

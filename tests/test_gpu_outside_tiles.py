@@ -1,0 +1,50 @@
+"""Expected counts, their log-likelihoods and node posteriors depend on the region alone: the same bits
+whatever else the call holds and wherever its launches end."""
+import numpy as np
+import pytest
+
+import phylocsf_gb300 as P
+from phylocsf_gb300 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _region(name, length, seed=5):
+    ps = synth.load_params(name)
+    gf = synth.gap_fractions(np.random.default_rng(seed), 1, ps.tree.nl, 0.05, 0.4, 0.2)
+    _, leaves = synth.simulate(ps, np.array([length]), np.zeros(1, np.int32), gf, seed)
+    return ps, leaves
+
+
+# copies of one region of 10 or 96 tiles (32 columns): alone; a few; enough for several waves of CTAs;
+# and past the tiles of one launch (2 GiB of their counts: 5,957 tiles of 12 leaves in FP32, 2,978 in
+# FP64), so that a launch ends inside a copy
+@pytest.mark.parametrize("prec,length,copies", [("fp32b", 32 * 9 + 5, (1, 5, 121, 500)), ("fp32b", 3050, (1, 65)),
+                                                ("fp64", 32 * 9 + 5, (1, 4, 40)), ("fp64", 3050, (1, 33))])
+def test_same_bits_in_any_call(prec, length, copies):
+    ps, leaves = _region("12flies", length)
+    eng = P.Engine(ps.tree, ps.S_c, ps.pi_c, ps.S_n, ps.pi_n, precision=prec)
+    nodes = [0, ps.tree.nl, ps.tree.n - 1]
+    one = None
+    for n in copies:
+        # empty regions at both ends and in the middle
+        offs = np.concatenate([[0, 0], np.arange(1, n + 1) * length, [n * length]])
+        offs = np.insert(offs, 2, length if n > 1 else 0)
+        b = eng.batch(offs, np.tile(leaves, (n, 1)))
+        full = np.flatnonzero(np.diff(offs))
+        counts, lpr, st = eng.branch_counts(b, 0, 0.7)
+        assert (st == 0).all() and len(full) == n
+        for r in np.flatnonzero(np.diff(offs) == 0):
+            assert not counts[r].any() and lpr[r] == 0
+        if one is None:
+            one = counts[full[0]], lpr[full[0]]
+            # every branch's counts add up to the columns: FP64 sums of terms that carry FP32 rounding
+            tol = 1e-9 if prec == "fp64" else 2e-5
+            assert np.abs(one[0].sum((1, 2)) - length).max() <= tol * length
+        for r in full:
+            assert np.array_equal(counts[r], one[0]) and lpr[r] == one[1], (n, r)
+        if n <= 5:
+            post, _ = eng.node_posteriors(b, 0, 0.7, nodes)
+            alone, _ = eng.node_posteriors(eng.batch([0, length], leaves), 0, 0.7, nodes)
+            assert np.array_equal(post, np.tile(alone, (1, n, 1)))
+    eng.close()
