@@ -1639,6 +1639,8 @@ static int score_impl(pcsf_engine *e, pcsf_batch *b, int strategy, pcsf_result *
 // Outside-pass products: expected branch counts and node posteriors
 // (PhyloLik.ml:96-174, PhyloEM.ml:14-20), one FP64 or FP32 P set per region.
 
+constexpr size_t OUTSIDE_BYTES = size_t(2) << 30;   // most workspace of a launch: CTAs' scratch and tiles' counts
+
 static int outside_impl(pcsf_engine *e, pcsf_batch *b, int model, const double *rho, double *counts, int n_sel,
                         const int32_t *nodes, double *post, double *lpr, int32_t *status)
 {
@@ -1663,8 +1665,6 @@ static int outside_impl(pcsf_engine *e, pcsf_batch *b, int model, const double *
     // regions of a chunk: P sets and counts within ~2 GiB
     const int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)std::max(nreg, 1),
                                                                 (size_t(2) << 30) / (pset_bytes + cnt_bytes)));
-    // tiles of a launch: their own counts within ~2 GiB, at most the tiles of the longest chunk; and
-    // CTAs, every SM's worth
     auto tiles_of = [&](int r) { return (b->offs[r + 1] - b->offs[r] + TC - 1) / TC; };
     int64_t most_tiles = 1;
     for (int r0 = 0; r0 < nreg; r0 += chunk) {
@@ -1673,10 +1673,6 @@ static int outside_impl(pcsf_engine *e, pcsf_batch *b, int model, const double *
         most_tiles = std::max(most_tiles, t);
     }
     if (most_tiles > INT32_MAX) return e->fail(PCSF_ERANGE, "outside pass: more than 2^31 column tiles");
-    const size_t tile_bytes = counts ? pset_bytes : 0;
-    const int launch = (int)std::min<int64_t>(
-        most_tiles, counts ? std::max<int64_t>(1, (int64_t)((size_t(2) << 30) / tile_bytes)) : most_tiles);
-    const int grid = std::min(e->sm_count * outside_ctas_per_sm(fp64, comp, e->nslots, e->nl, (int)e->sched.size()), launch);
     DevBuf<unsigned char> dP, dscr, dtile;
     DevBuf<double> dcnt, dlpr, dtlpr, dpost;
     DevBuf<PSet> dps;
@@ -1684,8 +1680,19 @@ static int outside_impl(pcsf_engine *e, pcsf_batch *b, int model, const double *
     DevBuf<WorkItem> dwi;
     DevBuf<int32_t> dwib, dstatus, dsel;
     CK(dP.reserve((size_t)chunk * pset_bytes), "cudaMalloc P(t)");
-    CK(dscr.reserve((size_t)grid * scr), "cudaMalloc outside-pass scratch");
     if (counts) CK(dcnt.reserve((size_t)chunk * e->nbr * K2), "cudaMalloc counts");
+    if (n_sel > 0) CK(dpost.reserve((size_t)n_sel * std::max<int64_t>(b->total_cols, 1) * K), "cudaMalloc posteriors");
+    // a launch: CTAs (every SM's worth) with their scratch, and tiles with their own counts, together
+    // within OUTSIDE_BYTES and half of the free memory; at most the tiles of the longest chunk, at least one
+    const size_t tile_bytes = counts ? pset_bytes : 0;
+    size_t freeb = 0, totalb = 0;
+    CK(cudaMemGetInfo(&freeb, &totalb), "cudaMemGetInfo");
+    const size_t budget = std::min(OUTSIDE_BYTES, freeb / 2);
+    const size_t ctas = (size_t)e->sm_count * outside_ctas_per_sm(fp64, comp, e->nslots, e->nl, (int)e->sched.size());
+    const int grid = (int)std::max<size_t>(1, std::min({ctas, budget / (scr + tile_bytes), (size_t)most_tiles}));
+    const size_t rest = budget > grid * scr ? budget - grid * scr : 0;
+    const int launch = (int)std::min<int64_t>(most_tiles, counts ? std::max<int64_t>(grid, rest / tile_bytes) : most_tiles);
+    CK(dscr.reserve((size_t)grid * scr), "cudaMalloc outside-pass scratch");
     CK(dtile.reserve((size_t)launch * tile_bytes), "cudaMalloc counts of the tiles");
     CK(dtlpr.reserve(most_tiles), "cudaMalloc");
     CK(dwi.reserve(most_tiles), "cudaMalloc");
@@ -1697,7 +1704,6 @@ static int outside_impl(pcsf_engine *e, pcsf_batch *b, int model, const double *
     cudaStream_t s = e->stream;
     if (n_sel > 0) {
         CK(dsel.reserve(e->n), "cudaMalloc");
-        CK(dpost.reserve((size_t)n_sel * std::max<int64_t>(b->total_cols, 1) * K), "cudaMalloc posteriors");
         CK(cudaMemcpyAsync(dsel.p, sel.data(), sizeof(int32_t) * e->n, cudaMemcpyHostToDevice, s), "H2D");
     }
     for (int r0 = 0; r0 < nreg; r0 += chunk) {

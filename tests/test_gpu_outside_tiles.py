@@ -17,8 +17,8 @@ def _region(name, length, seed=5):
 
 
 # copies of one region of 10 or 96 tiles (32 columns): alone; a few; enough for several waves of CTAs;
-# and past the tiles of one launch (2 GiB of their counts: 5,957 tiles of 12 leaves in FP32, 2,978 in
-# FP64), so that a launch ends inside a copy
+# and past the tiles of one launch (at most 2 GiB of their counts: 5,957 tiles of 12 leaves in FP32, 2,978
+# in FP64), so that a launch ends inside a copy
 @pytest.mark.parametrize("prec,length,copies", [("fp32b", 32 * 9 + 5, (1, 5, 121, 500)), ("fp32b", 3050, (1, 65)),
                                                 ("fp64", 32 * 9 + 5, (1, 4, 40)), ("fp64", 3050, (1, 33))])
 def test_same_bits_in_any_call(prec, length, copies):
@@ -47,4 +47,36 @@ def test_same_bits_in_any_call(prec, length, copies):
             post, _ = eng.node_posteriors(b, 0, 0.7, nodes)
             alone, _ = eng.node_posteriors(eng.batch([0, length], leaves), 0, 0.7, nodes)
             assert np.array_equal(post, np.tile(alone, (1, n, 1)))
+    eng.close()
+
+
+@pytest.mark.parametrize("name,prec,length", [("120mammals", "fp32b", 15000), ("58mammals", "fp64", 20000)])
+def test_workspace_bound(name, prec, length):
+    """One long region on a large tree: P(t) and the counts of one region, and for CTAs and tiles 2 GiB at
+    most (64 MiB beside them for the small arrays and the allocator's granularity)."""
+    import threading
+    import torch
+
+    ps, leaves = _region(name, length)
+    eng = P.Engine(ps.tree, ps.S_c, ps.pi_c, ps.S_n, ps.pi_n, precision=prec)
+    b = eng.batch([0, length], leaves)
+    short = eng.batch([0, 40], leaves[:40])
+    eng.branch_counts(short, 0, 0.7)
+    free = torch.cuda.mem_get_info()[0]
+    low, done = [free], threading.Event()
+
+    def watch():
+        while not done.is_set():
+            low[0] = min(low[0], torch.cuda.mem_get_info()[0])
+
+    t = threading.Thread(target=watch)
+    t.start()
+    try:
+        _, _, st = eng.branch_counts(b, 0, 0.7)
+    finally:
+        done.set()
+        t.join()
+    assert (st == 0).all()
+    matrices = (ps.tree.n - 1) * 4096 * (8 + (8 if prec == "fp64" else 4))
+    assert 0 < free - low[0] <= (2 << 30) + matrices + (64 << 20)
     eng.close()
