@@ -840,7 +840,7 @@ static int evaluate(pcsf_engine *e, pcsf_batch *b, const std::vector<Request> &r
     if (grad) {
         gscr = grad_scratch_per_cta(e->prec, e->nl, npar, e->grad_recompute);
         CK(e->gscratch.reserve(gscr * (size_t)e->grad_grid[npar ? 1 : 0]), "cudaMalloc gradient scratch");
-        CK(e->dgpart.reserve(grad_part_doubles(std::max(nwi, 1), gstride)), "cudaMalloc");
+        CK(e->dgpart.reserve((size_t)std::max(nwi, 1) * gstride), "cudaMalloc");
         CK(e->dgrad.reserve((size_t)nreq * gstride), "cudaMalloc");
         CK(e->hgrad.reserve((size_t)nreq * gstride), "cudaMallocHost");
         if (npar)
@@ -936,7 +936,7 @@ static int evaluate(pcsf_engine *e, pcsf_batch *b, const std::vector<Request> &r
             ga.scratch_per_cta = gscr;
             ga.recompute_leaves = e->grad_recompute ? 1 : 0;
             ga.partials = pa.partials;
-            ga.gpart = e->dgpart.p + grad_part_doubles(wib[r0], gstride);
+            ga.gpart = e->dgpart.p + (size_t)wib[r0] * gstride;
             int grid = std::min(e->grad_grid[npar ? 1 : 0], std::max(pa.nwi, 1));
             const bool tce = tc_prec(e->prec);
             CK(launch_grad(e->prec == PCSF_PREC_FP64 ? PCSF_PREC_FP64 : PCSF_PREC_FP32,

@@ -28,8 +28,10 @@
 // a division on two of the eight warps (an SM issues two FP64 lanes per clock).  Now E^T is
 // contracted as stored, a column's weight 2^ex / z~ is formed once ahead by one warp, all
 // eight warps share the FP64 sums of a side, and these run beside the next side's
-// contractions; each warp's sum goes to gpart, which k_reduce_grad adds up.  Measured, per
-// column: 58 leaves 173 -> 88 ns, 100 leaves with two rate parameters 955 -> 387 ns.
+// contractions; the warps' sums meet in shared memory one side later, so that a tile leaves one
+// row of sums (a row per warp took eight times the memory, and k_reduce_grad eight times as many
+// dependent additions).  Measured, per column: 58 leaves 173 -> 88 ns, 100 leaves with two rate
+// parameters 955 -> 387 ns.
 #include <algorithm>
 #include <cmath>
 
@@ -64,7 +66,7 @@ struct GradLayout {
     static size_t smem(int nslots, int nl, int nint, int npar)
     {
         size_t b = sizeof(T) * ((size_t)K2 + (npar ? (size_t)K2 + 3 * K : 0) + region(nslots, npar) + reds(npar));
-        b += sizeof(double) * 3 * TC;
+        b += sizeof(double) * (3 * TC + 2 * (1 + npar) * GR_WARPS);
         b += sizeof(typename AtomMax<T>::U) * 2 * TC + sizeof(int) * (5 * TC + (size_t)nslots * TC);
         b += sizeof(SchedNode) * nint;
         b = (b + 15) & ~size_t(15);
@@ -103,7 +105,8 @@ __global__ void __launch_bounds__(GR_THREADS, sizeof(T) == 4 ? 2 : 1) k_grad(Gra
     double *zp = reinterpret_cast<double *>(red);                   // root: [2][GR_WARPS][TC]
     double *zt = reinterpret_cast<double *>(red + Layout::reds(npar));   // [TC] 1 / z~ (0: no gradient)
     double *wcol = zt + TC;                                         // [2][TC] column weights 2^ex / z~
-    MU *colmax = reinterpret_cast<MU *>(wcol + 2 * TC);             // [2][TC]
+    double *wsum = wcol + 2 * TC;                                   // [2][1 + npar][GR_WARPS] a side's sums of each warp
+    MU *colmax = reinterpret_cast<MU *>(wsum + 2 * (1 + npar) * GR_WARPS);    // [2][TC]
     int *eroot = reinterpret_cast<int *>(colmax + 2 * TC);          // [TC]
     int *ebase = eroot + TC;                                        // [2][TC] f(p) + e(s), by side: one side's is read
                                                                     //   (by half a warp) while the next side's is written
@@ -145,7 +148,7 @@ __global__ void __launch_bounds__(GR_THREADS, sizeof(T) == 4 ? 2 : 1) k_grad(Gra
         const T *Pbase = reinterpret_cast<const T *>(a.Pbuf) + (size_t)rq.pset * a.nbr * K2;
         const int ncols = wi.ncols;
         const uint8_t *lg = a.leaves + (size_t)wi.col0 * nl;
-        double *gout = a.gpart + ((size_t)w * GR_WARPS + warp) * gstride;    // this warp's sums
+        double *gout = a.gpart + (size_t)w * gstride;
         __syncthreads();   // previous work item finished with shared memory
         for (int f = tid; f < TC * nl; f += GR_THREADS) {
             int c = f / nl, l = f - c * nl;
@@ -280,11 +283,23 @@ __global__ void __launch_bounds__(GR_THREADS, sizeof(T) == 4 ? 2 : 1) k_grad(Gra
         }
 
         // ---------------- outside pass, parents before children
-        // a side's column sums (FP32, 16 per column) are weighted and added over the columns in
-        // FP64 one side later: pc = the branch that waits in buffer pb
-        int pc = -1, pb = 0;
-        double pacc[2] = {0.0, 0.0};      // this warp's parameter derivatives (lane 0)
+        // a side's column sums (FP32, 16 per column) are weighted and added over a warp's columns in
+        // FP64 one side later, and over the warps two sides later: pc, qc = the branches that wait in
+        // buffers pb, qb.  Warp x adds value x (0 the branch's, 1 and 2 the parameters').
+        int pc = -1, pb = 0, qc = -1, qb = 0;
+        double pacc = 0.0;                // parameter warp - 1's derivative (lane 0 of warps 1 and 2)
         auto flush = [&]() {
+            if (qc >= 0 && warp <= npar) {
+                double g = lane < GR_WARPS ? wsum[(qb * (1 + npar) + warp) * GR_WARPS + lane] : 0.0;
+#pragma unroll
+                for (int o = GR_WARPS / 2; o > 0; o >>= 1) g += __shfl_down_sync(0xffffffffu, g, o);
+                if (lane == 0) {
+                    if (warp == 0) gout[qc] = g;
+                    else pacc += g;
+                }
+            }
+            qc = pc;
+            qb = pb;
             if (pc < 0) return;
             const double wv = wcol[pb * TC + lane];
             const int we = wexp[pb * TC + lane];
@@ -294,10 +309,7 @@ __global__ void __launch_bounds__(GR_THREADS, sizeof(T) == 4 ? 2 : 1) k_grad(Gra
                 g = (we ? ldexp(g, we) : g) * wv;
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) g += __shfl_down_sync(0xffffffffu, g, o);
-                if (lane == 0) {
-                    if (x == 0) gout[pc] = g;
-                    else pacc[x - 1] += g;
-                }
+                if (lane == 0) wsum[(pb * (1 + npar) + x) * GR_WARPS + warp] = g;
             }
             pc = -1;
         };
@@ -480,10 +492,11 @@ __global__ void __launch_bounds__(GR_THREADS, sizeof(T) == 4 ? 2 : 1) k_grad(Gra
                 pb = buf;
             }
         }
-        __syncthreads();
-        flush();
-        if (npar && lane == 0)
-            for (int x = 0; x < npar; x++) gout[a.nbr + x] = pacc[x];
+        for (int k = 0; k < 2; k++) {      // the last two sides'
+            __syncthreads();
+            flush();
+        }
+        if (lane == 0 && warp >= 1 && warp <= npar) gout[a.nbr + warp - 1] = pacc;
     }
 }
 
@@ -501,7 +514,6 @@ size_t grad_smem_bytes(int prec, int nslots, int nl, int nint, int npar)
 }
 
 int grad_tile_cols() { return GR_TC; }
-size_t grad_part_doubles(int nwi, int gstride) { return (size_t)nwi * GR_WARPS * gstride; }
 
 template <typename T, int KAHAN, bool RECOMP>
 static int ctas_per_sm_r(int nslots, int nl, int nint, int npar)
@@ -637,14 +649,14 @@ cudaError_t launch_hform(bool fp64, const PSet *ps, int nps, const double *branc
     return cudaGetLastError();
 }
 
-// grad[r][c] = sum of gpart ([work item][warp][branch]) over request r's work items (fixed order)
+// grad[r][c] = sum of gpart over request r's work items (fixed order)
 __global__ void k_reduce_grad(const double *gpart, const int32_t *wi_begin, int nreq, int nbr, double *grad)
 {
     int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= nreq * nbr) return;
     int r = idx / nbr, c = idx % nbr;
     double g = 0.0;
-    for (size_t w = (size_t)wi_begin[r] * GR_WARPS; w < (size_t)wi_begin[r + 1] * GR_WARPS; w++) g += gpart[w * nbr + c];
+    for (size_t w = wi_begin[r]; w < (size_t)wi_begin[r + 1]; w++) g += gpart[w * nbr + c];
     grad[idx] = g;
 }
 

@@ -144,7 +144,7 @@ struct GradArgs {
     void *scratch;           // gridDim.x * scratch_per_cta bytes
     size_t scratch_per_cta;
     double *partials;        // [nwi][2]
-    double *gpart;           // [nwi][warps][nbr + npar]: grad_part_doubles(nwi, nbr + npar)
+    double *gpart;           // [nwi][nbr + npar]
     // rate-matrix parameter derivatives (OmegaModel kappa, omega): d lpr / d x =
     // sum_c sum_col inter_c^T (dP_c / dx) alpha_c / z, with dP/dx = D^-1/2 U (F o Bdot_x) U^T D^1/2
     int npar;                // 0 or 2
@@ -156,7 +156,6 @@ cudaError_t launch_grad(int prec, int comp, const GradArgs &a, cudaStream_t s, i
 size_t grad_scratch_per_cta(int prec, int nl, int npar, bool recompute_leaves);
 size_t grad_smem_bytes(int prec, int nslots, int nl, int nint, int npar);   // the limit on trees
 int grad_tile_cols();
-size_t grad_part_doubles(int nwi, int gstride);
 int grad_ctas_per_sm(int prec, int nslots, int nl, int nint, int npar);
 // H_x = (F(t) o Bdot_x)^T for every (P set, branch, parameter): F_ij = (e^{lam_i t} - e^{lam_j t}) /
 // (lam_i - lam_j), t e^{lam_i t} on the diagonal (Frechet derivative of exp in the eigenbasis)

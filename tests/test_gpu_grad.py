@@ -183,3 +183,24 @@ def test_gradient_two_internal_children(prec, nl):
         for got, want, cols in ((db, ref, 1), (whole, ref.sum(0), L)):
             tol = 1e-7 * np.abs(want) + 1e-8 * cols if prec == "fp64" else 1e-4 * np.abs(want) + 1e-5 * cols
             assert (np.abs(got - want) <= tol).all(), (rho, cols, np.abs(got - want).max())
+
+
+def test_gradient_memory():
+    """The sums that the adjoint keeps for a call: one row of doubles per branch and tile of 32 columns
+    (22 MB here; with the work list and the allocator's granularity 48 MiB at most), and the same gradient as the region's copies alone
+    give (FP64 sums of n terms: 1e-12)."""
+    import torch
+
+    e = engine("12flies", "fp32b")
+    offs, leaves = _data("12flies", [4000], seed=6)
+    one, short = e.batch(offs, leaves), e.batch([0, 40], leaves[:40])
+    n = 1000
+    b = e.batch([0, 4000 * n], np.tile(leaves, (n, 1)))
+    _, g1, _, _ = e.grad(one, 0, 0.9)
+    e.grad(short, 0, 0.9)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    _, g, _, st = e.grad(b, 0, 0.9)
+    assert (st == 0).all()
+    assert free - torch.cuda.mem_get_info()[0] <= 48 << 20
+    assert np.abs(g[0] - n * g1[0]).max() <= 1e-12 * n * np.abs(g1).max()
