@@ -193,6 +193,7 @@ struct pcsf_engine {
     // engines only (the FP64 engine is exact already)
     int64_t exact_min_units = 150000;
     int sm_count = 0;
+    int jac_cluster = 1;           // the eigensolver's largest cluster on this device
     DevBuf<int> derr;     // set by a kernel whose bounded wait timed out
     DevBuf<unsigned long long> dbadcode;   // first invalid leaf code of an uploaded batch
     DevBuf<float> Dlo;    // [chunk P sets][nbr][K] low parts of diag(E) (SIMT FP32 evaluations)
@@ -447,7 +448,7 @@ static int setup_models(pcsf_engine *e, const double *Q[2], const double *eq[2],
     CK(dl.reserve(2 * K), "cudaMalloc");
     CK(dst.reserve(2), "cudaMalloc");
     CK(cudaMemcpyAsync(dA.p, A.data(), sizeof(double) * 2 * K2, cudaMemcpyHostToDevice, e->stream), "H2D Q");
-    CK(launch_jacobi(dA.p, dUtmp.p, dl.p, dst.p, 2, e->stream), "eigensolver launch");
+    CK(launch_jacobi(dA.p, dUtmp.p, dl.p, dst.p, 2, jacobi_cluster(2, e->sm_count, e->jac_cluster), e->stream), "eigensolver launch");
     e->stats.kernel_launches += 1;
     int hst[2];
     CK(cudaMemcpyAsync(e->U, dUtmp.p, sizeof(double) * 2 * K2, cudaMemcpyDeviceToHost, e->stream), "D2H U");
@@ -634,6 +635,7 @@ static int engine_init_common(pcsf_engine *e, const pcsf_tree *tree, int32_t fla
         e->depth = std::max(e->depth, (int)waiting);
     }
     e->sm_count = prop.multiProcessorCount;
+    e->jac_cluster = jacobi_max_cluster();
     e->smem_optin = prop.sharedMemPerBlockOptin;
     CK(e->derr.reserve(1), "cudaMalloc");
     CK(cudaMemsetAsync(e->derr.p, 0, sizeof(int), e->stream), "memset");
@@ -1974,7 +1976,8 @@ static int dyn_prepare(pcsf_engine *e, DynModels &dmod, const std::vector<OmegaK
         }
         double *dA = dmod.deig.p, *dUo = dA + nA, *dlo = dUo + nA;
         CK(cudaMemcpyAsync(dA, A, sizeof(double) * nA, cudaMemcpyHostToDevice, e->stream), "H2D");
-        CK(launch_jacobi(dA, dUo, dlo, reinterpret_cast<int *>(dlo + (size_t)nf * K), nf, e->stream), "eigensolver launch");
+        CK(launch_jacobi(dA, dUo, dlo, reinterpret_cast<int *>(dlo + (size_t)nf * K), nf,
+                         jacobi_cluster(nf, e->sm_count, e->jac_cluster), e->stream), "eigensolver launch");
         e->stats.kernel_launches += 1;
         CK(cudaMemcpyAsync(Uh, dUo, sizeof(double) * (nA + (size_t)nf * K + nst), cudaMemcpyDeviceToHost, e->stream), "D2H");
         CK(cudaStreamSynchronize(e->stream), "eigensolver");

@@ -277,36 +277,56 @@ __global__ void __launch_bounds__(JAC_THREADS) k_jacobi(const double *A_in, doub
 }
 
 template <int C>
-static cudaError_t launch_jacobi_c(const double *A, double *U, double *lam, int *status, int nmat, cudaStream_t s)
+static cudaError_t config_jacobi_c(cudaLaunchConfig_t &cfg, cudaLaunchAttribute &attr, int nmat, cudaStream_t s)
 {
     const size_t smem = sizeof(double) * (3 * (K / C) * JAC_LD + JAC_THREADS + 128) + sizeof(int) * 128;
     cudaError_t err = cudaFuncSetAttribute(k_jacobi<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err == cudaSuccess && C > 8)
         err = cudaFuncSetAttribute(k_jacobi<C>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (err != cudaSuccess) return err;
-    cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(nmat * C);
     cfg.blockDim = dim3(JAC_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.x = C;
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = C > 1 ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, k_jacobi<C>, A, U, lam, status);
+    return cudaSuccess;
 }
 
-cudaError_t launch_jacobi(const double *A, double *U, double *lam, int *status, int nmat, cudaStream_t s)
+template <int C>
+static cudaError_t launch_jacobi_c(const double *A, double *U, double *lam, int *status, int nmat, cudaStream_t s)
+{
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr{};
+    const cudaError_t err = config_jacobi_c<C>(cfg, attr, nmat, s);
+    return err == cudaSuccess ? cudaLaunchKernelEx(&cfg, k_jacobi<C>, A, U, lam, status) : err;
+}
+
+int jacobi_max_cluster()
+{
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr{};
+    int n = 0;
+    if (config_jacobi_c<16>(cfg, attr, 1, nullptr) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&n, k_jacobi<16>, &cfg) == cudaSuccess && n > 0)
+        return 16;
+    cudaGetLastError();
+    return 8;
+}
+
+cudaError_t launch_jacobi(const double *A, double *U, double *lam, int *status, int nmat, int cluster, cudaStream_t s)
 {
     if (nmat <= 0) return cudaSuccess;
-    // the largest cluster whose CTAs still have an SM each
-    if (nmat <= 8) return launch_jacobi_c<16>(A, U, lam, status, nmat, s);
-    if (nmat <= 18) return launch_jacobi_c<8>(A, U, lam, status, nmat, s);
-    if (nmat <= 38) return launch_jacobi_c<4>(A, U, lam, status, nmat, s);
-    if (nmat <= 76) return launch_jacobi_c<2>(A, U, lam, status, nmat, s);
-    return launch_jacobi_c<1>(A, U, lam, status, nmat, s);
+    switch (cluster) {
+    case 16: return launch_jacobi_c<16>(A, U, lam, status, nmat, s);
+    case 8: return launch_jacobi_c<8>(A, U, lam, status, nmat, s);
+    case 4: return launch_jacobi_c<4>(A, U, lam, status, nmat, s);
+    case 2: return launch_jacobi_c<2>(A, U, lam, status, nmat, s);
+    default: return launch_jacobi_c<1>(A, U, lam, status, nmat, s);
+    }
 }
 
 // ---------------------------------------------------------------------------

@@ -78,7 +78,20 @@ struct LaunchStats {
 
 // ---- kernels (kernels.cu) -------------------------------------------------
 // Jacobi eigensolver: A [nmat][K][K] symmetric -> U [nmat][K][K], lam [nmat][K].
-cudaError_t launch_jacobi(const double *A, double *U, double *lam, int *status, int nmat, cudaStream_t s);
+// cluster = jacobi_cluster(nmat, SMs, jacobi_max_cluster())
+cudaError_t launch_jacobi(const double *A, double *U, double *lam, int *status, int nmat, int cluster, cudaStream_t s);
+// the largest cluster (of 16, 8) of the eigensolver's CTAs that the current device can place: 16 is
+// beyond the portable 8, and whether it fits depends on the SMs left in each processing cluster
+int jacobi_max_cluster();
+// CTAs per matrix: the largest cluster whose CTAs still have an SM each (the processing clusters' odd
+// SMs take one cluster of 8 or 16 off what the SM count alone would allow: on 152 SMs up to 8, 18, 38
+// and 76 matrices for 16, 8, 4 and 2)
+inline int jacobi_cluster(int nmat, int sm_count, int most)
+{
+    for (int c = most; c > 1; c /= 2)
+        if (nmat <= sm_count / c - (c >= 8 ? 1 : 0)) return c;
+    return 1;
+}
 
 // P(t) formation for P sets [nps]: writes E^T = (P - I)^T per branch into
 // Pbuf ([nps][nbr][K][K], element (j,i) = E[i][j]) in FP64 or FP32.
