@@ -315,7 +315,8 @@ __global__ void __launch_bounds__(FF_THREADS, 1) k_prune_ff(PruneArgs a, size_t 
     const uint32_t tbase = tbase_s;
     const int nbseq = nbseq_s;
     const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
-    uint32_t ph_d = 0, ph_b = 0;        // parities: both D halves complete once per contraction
+    ContractionPhase ph_d;              // both D halves complete once per contraction
+    uint32_t ph_b = 0;
     int ld_w = blockIdx.x, ld_k = 0, ld_n = 0;   // next B load: work item, index into bseq, loads issued
     int b_inflight = 0;
     int cn = 0;                          // contractions so far (parity: the row-scale buffer)
@@ -465,7 +466,7 @@ __global__ void __launch_bounds__(FF_THREADS, 1) k_prune_ff(PruneArgs a, size_t 
                 const float *sc = reinterpret_cast<const float *>(sm + FS_SC) + (cn & 1) * 3 * K + s0;
 #pragma unroll
                 for (int hf = 0; hf < 2; hf++) {
-                    if (!mbar_wait(hf ? bar1 : bar0, ph_d)) bad = true;
+                    if (!mbar_wait(hf ? bar1 : bar0, ph_d.wait())) bad = true;
                     tc_fence_after();
                     if (hf == 1 && tid == 0 && !bad) issue_next_b();     // every MMA of B has completed
 #pragma unroll
@@ -502,7 +503,7 @@ __global__ void __launch_bounds__(FF_THREADS, 1) k_prune_ff(PruneArgs a, size_t 
                         }
                     }
                 }
-                ph_d ^= 1u;
+                ph_d.next();
                 cn++;
                 have = true;
             }
@@ -602,8 +603,8 @@ __global__ void __launch_bounds__(FF_THREADS, 1) k_prune_ff(PruneArgs a, size_t 
     // wait, MMAs; both waits are bounded
     if (tid == 0 && b_inflight > 0 && !mbar_wait(barB, ph_b)) atomicExch(err, 1);
     if (!ok) {
-        mbar_wait(bar0, ph_d);
-        mbar_wait(bar1, ph_d);
+        mbar_wait(bar0, ph_d.last());
+        mbar_wait(bar1, ph_d.last());
     }
     tc_fence_before();
     __syncthreads();

@@ -174,6 +174,18 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity)
     return done != 0;
 }
 
+// Parities of an mbarrier that completes once per contraction, in order.  wait() is the parity of the
+// contraction now waited for; after next(), last() is that of the contraction that was: what a kernel
+// that leaves has to wait for again, as the wait may have run out before the commit arrived (a wait for
+// wait() itself, a phase that has not begun, returns at once).  Before the first contraction last()
+// returns at once, as it should.
+struct ContractionPhase {
+    uint32_t p = 0;
+    __host__ __device__ uint32_t wait() const { return p; }
+    __host__ __device__ void next() { p ^= 1u; }
+    __host__ __device__ uint32_t last() const { return p ^ 1u; }
+};
+
 // hi part of the TF32 split x = hi + lo: x rounded to the nearest TF32 value (ties away
 // from zero), so lo = x - hi (exact in FP32) takes either sign and the bits of lo the
 // MMA drops (it reads 10 mantissa bits) cancel on average instead of always shrinking |x|

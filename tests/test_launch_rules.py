@@ -1,4 +1,5 @@
-"""Rules that choose a launch's shape, compiled from the library's own header and run on the host."""
+"""Rules of the kernels and their launches that need no GPU, compiled from the library's own headers and
+run on the host."""
 import os
 import shutil
 import subprocess
@@ -9,14 +10,18 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 
 
-def _run(tmp_path, body):
-    cc = shutil.which("g++") or shutil.which("c++")
-    if cc is None or not os.path.exists(os.path.join(CUDA, "include", "cuda_runtime.h")):
-        pytest.skip("no C++ compiler or CUDA headers")
-    src = tmp_path / "rule.cpp"
-    src.write_text('#include <cstdio>\n#include "pcsf_internal.h"\nusing namespace pcsf;\nint main()\n{\n%s\n}\n' % body)
+def _run(tmp_path, body, headers=("pcsf_internal.h",), decl=""):
+    """Output rows of a main() with this body: g++ for the host header, nvcc where device headers are in it."""
+    cuh = any(h.endswith(".cuh") for h in headers)
+    cc = (shutil.which("nvcc") or os.path.join(CUDA, "bin", "nvcc")) if cuh else shutil.which("g++")
+    if cc is None or not os.path.exists(cc) or not os.path.exists(os.path.join(CUDA, "include", "cuda_runtime.h")):
+        pytest.skip("no compiler or CUDA headers")
+    src = tmp_path / ("rule.cu" if cuh else "rule.cpp")
+    src.write_text("#include <cstdio>\n" + "".join('#include "%s"\n' % h for h in headers) +
+                   "using namespace pcsf;\n%s\nint main()\n{\n%s\n}\n" % (decl, body))
     exe = tmp_path / "rule"
-    subprocess.run([cc, "-std=c++17", "-I", os.path.join(ROOT, "phylocsf_gb300", "csrc"), "-I",
+    flags = ["-gencode", "arch=compute_103a,code=sm_103a"] if cuh else []
+    subprocess.run([cc, "-std=c++17"] + flags + ["-I", os.path.join(ROOT, "phylocsf_gb300", "csrc"), "-I",
                     os.path.join(CUDA, "include"), str(src), "-o", str(exe)], check=True)
     out = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout
     return [tuple(int(x) for x in line.split()) for line in out.splitlines()]
@@ -37,3 +42,28 @@ def test_eigensolver_clusters(tmp_path):
     at = {(most, n): c for sms, most, n, c in rows if sms == 152}
     for n, c in ((1, 16), (8, 16), (9, 8), (18, 8), (19, 4), (38, 4), (39, 2), (76, 2), (77, 1)):
         assert at[16, n] == c and at[8, n] == min(c, 8)
+
+
+def test_wait_for_the_last_contraction(tmp_path):
+    """The parity that a leaving kernel waits for, against an mbarrier restated on the host (a wait for a
+    parity returns at once unless the phase of that parity is the one in progress): it blocks exactly
+    while the last contraction's commit is outstanding."""
+    rows = _run(tmp_path, """
+    for (int done = 0; done < 6; done++)               // contractions seen to complete
+        for (int late = 0; late < 2; late++) {         // one more issued, its wait ran out
+            ContractionPhase ph;
+            uint32_t phase = 0;                        // the mbarrier's phase in progress
+            for (int k = 0; k < done; k++) {
+                phase++;                               // the commit arrives
+                if ((phase & 1) == (ph.wait() & 1)) return 1;      // the wait would not return
+                ph.next();
+            }
+            if (late) ph.next();
+            std::printf("%d %d %d %d\\n", done, late, (phase & 1) == ph.last(), ((phase + 1) & 1) == ph.last());
+        }
+""", headers=("pcsf_internal.h", "prune_common.cuh", "tc_common.cuh"))
+    assert len(rows) == 12
+    for done, late, blocks, blocks_after in rows:
+        assert blocks == late                          # waits while the commit is outstanding
+        if late:
+            assert not blocks_after                    # and no longer once it has arrived
