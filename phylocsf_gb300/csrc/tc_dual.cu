@@ -420,6 +420,7 @@ __global__ void __launch_bounds__(TD_THREADS, 1) k_prune_tc_dual(PruneArgs a, co
     }
     if (!ok && tid == 0) atomicExch(err, 1);
     if (tid == 0) {
+        if (bad) mbar_wait(barQ, 0);     // Q's fetch may still be on its way
         while (b_inflight > 0) {
             if (!mbar_wait(barB, ph_b)) { atomicExch(err, 1); break; }
             ph_b ^= 1u;
