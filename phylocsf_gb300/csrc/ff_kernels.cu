@@ -638,7 +638,7 @@ cudaError_t launch_prune_ff(const PruneArgs &a, float *stack, int *err, cudaStre
 {
     if (a.nwi <= 0) return cudaSuccess;
     const size_t smem = ff_smem(a.nl, a.n_internal);
-    cudaError_t e = cudaFuncSetAttribute(k_prune_ff, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem<k_prune_ff>();
     if (e != cudaSuccess) return e;
     k_prune_ff<<<grid, FF_THREADS, smem, s>>>(a, ff_pset_bytes(a.nl, a.nbr), stack, err);
     return cudaGetLastError();

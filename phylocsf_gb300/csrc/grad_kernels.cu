@@ -520,7 +520,7 @@ static int ctas_per_sm_r(int nslots, int nl, int nint, int npar)
 {
     const size_t smem = GradLayout<T, RECOMP>::smem(nslots, nl, nint, npar);
     int n = 0;
-    if (cudaFuncSetAttribute(k_grad<T, KAHAN, RECOMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+    if (allow_smem<k_grad<T, KAHAN, RECOMP>>() != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_grad<T, KAHAN, RECOMP>, GR_THREADS, smem) != cudaSuccess) {
         cudaGetLastError();
         return 1;
@@ -545,7 +545,7 @@ template <typename T, int KAHAN, bool RECOMP>
 static cudaError_t launch_grad_r(const GradArgs &a, cudaStream_t s, int grid)
 {
     size_t smem = GradLayout<T, RECOMP>::smem(a.nslots, a.nl, a.n_internal, a.npar);
-    cudaError_t e = cudaFuncSetAttribute(k_grad<T, KAHAN, RECOMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem<k_grad<T, KAHAN, RECOMP>>();
     if (e != cudaSuccess) return e;
     k_grad<T, KAHAN, RECOMP><<<grid, GR_THREADS, smem, s>>>(a);
     return cudaGetLastError();
@@ -783,8 +783,8 @@ cudaError_t launch_omega_deriv(bool fp64, const double *keys, const double *U, c
     if (nmodels <= 0) return cudaSuccess;
     const size_t smem = sizeof(double) * 3 * K2;
     const dim3 grid(nmodels, 2);
-    cudaError_t e = fp64 ? cudaFuncSetAttribute(k_omega_deriv<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                         : cudaFuncSetAttribute(k_omega_deriv<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = fp64 ? allow_smem<k_omega_deriv<double>>()
+                         : allow_smem<k_omega_deriv<float>>();
     if (e != cudaSuccess) return e;
     if (fp64) k_omega_deriv<double><<<grid, OD_THREADS, smem, s>>>(keys, U, sq, isq, (double *)Q, (double *)Bdot);
     else k_omega_deriv<float><<<grid, OD_THREADS, smem, s>>>(keys, U, sq, isq, (float *)Q, (float *)Bdot);

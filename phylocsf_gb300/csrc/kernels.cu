@@ -280,7 +280,7 @@ template <int C>
 static cudaError_t config_jacobi_c(cudaLaunchConfig_t &cfg, cudaLaunchAttribute &attr, int nmat, cudaStream_t s)
 {
     const size_t smem = sizeof(double) * (3 * (K / C) * JAC_LD + JAC_THREADS + 128) + sizeof(int) * 128;
-    cudaError_t err = cudaFuncSetAttribute(k_jacobi<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t err = allow_smem<k_jacobi<C>>();
     if (err == cudaSuccess && C > 8)
         err = cudaFuncSetAttribute(k_jacobi<C>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (err != cudaSuccess) return err;
@@ -593,13 +593,13 @@ cudaError_t launch_pform(bool fp64, const PSet *req, int nreq, const double *bra
     dim3 grid((nbr + per_cta - 1) / per_cta, nreq);
     if (fp64) {
         const size_t smem = pform_smem<double>(per_cta);
-        cudaError_t e = cudaFuncSetAttribute(k_pform<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_smem<k_pform<double>>();
         if (e != cudaSuccess) return e;
         k_pform<double><<<grid, PF_THREADS, smem, s>>>(req, branch, nbr, m, (double *)Pbuf, status_key, raw ? 1 : 0,
                                                        nullptr, 0, nullptr, per_cta);
     } else {
         const size_t smem = pform_smem<float>(per_cta);
-        cudaError_t e = cudaFuncSetAttribute(k_pform<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_smem<k_pform<float>>();
         if (e != cudaSuccess) return e;
         k_pform<float><<<grid, PF_THREADS, smem, s>>>(req, branch, nbr, m, (float *)Pbuf, status_key, raw ? 1 : 0,
                                                       bop, bop_nl, raw ? nullptr : dlo, per_cta);
@@ -965,7 +965,7 @@ template <typename T, int TC, int KAHAN>
 static cudaError_t launch_prune_t(const PruneArgs &a, cudaStream_t s, int grid)
 {
     size_t smem = PruneSmem<T, TC>::bytes(a.nslots, a.nl, a.n_internal);
-    cudaError_t e = cudaFuncSetAttribute(k_prune<T, TC, KAHAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem<k_prune<T, TC, KAHAN>>();
     if (e != cudaSuccess) return e;
     k_prune<T, TC, KAHAN><<<grid, PruneThreads<TC>::N, smem, s>>>(a);
     return cudaGetLastError();

@@ -359,7 +359,7 @@ template <typename T, int KAHAN>
 cudaError_t launch_outside_t(const OutsideArgs &a, cudaStream_t s, int grid)
 {
     const size_t smem = OutLayout<T>::smem(a.nslots, a.nl, a.n_internal);
-    cudaError_t e = cudaFuncSetAttribute(k_outside<T, KAHAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem<k_outside<T, KAHAN>>();
     if (e != cudaSuccess) return e;
     if (a.wi1 > a.wi0) k_outside<T, KAHAN><<<std::min(grid, a.wi1 - a.wi0), OS_THREADS, smem, s>>>(a);
     e = cudaGetLastError();
@@ -373,7 +373,7 @@ int ctas_per_sm_t(int nslots, int nl, int nint)
 {
     const size_t smem = OutLayout<T>::smem(nslots, nl, nint);
     int n = 0;
-    if (cudaFuncSetAttribute(k_outside<T, KAHAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+    if (allow_smem<k_outside<T, KAHAN>>() != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_outside<T, KAHAN>, OS_THREADS, smem) != cudaSuccess) {
         cudaGetLastError();
         return 1;

@@ -1,5 +1,6 @@
 // Internal declarations shared by the host runtime and the CUDA kernels.
 #pragma once
+#include <atomic>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -67,6 +68,25 @@ struct DevModels {
     const float *Qf;        // [2][K][K]  Q (row-major)
     const float *Q2f;       // [2][K][K]  Q^2
 };
+
+// Lets Kernel be launched with any dynamic shared memory that fits beside its static share.  The limit
+// belongs to the kernel, not to a launch, and engines on different threads launch one kernel with
+// different sizes (trees, branches per CTA): with a launch's own size here, another thread could lower
+// the limit before the launch.  Every thread sets the same value.
+constexpr int SMEM_OPTIN = 232448;      // sm_103a: shared memory of a block, at most
+template <auto Kernel> inline cudaError_t allow_smem()
+{
+    static std::atomic<int> limit{0};   // the kernel's, once known
+    int n = limit.load(std::memory_order_relaxed);
+    if (n == 0) {
+        cudaFuncAttributes fa;
+        const cudaError_t e = cudaFuncGetAttributes(&fa, Kernel);
+        if (e != cudaSuccess) return e;
+        n = SMEM_OPTIN - (int)fa.sharedSizeBytes;
+        limit.store(n, std::memory_order_relaxed);
+    }
+    return cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, n);
+}
 
 // Status keys: ((branch*K + row) << 4) | code, min-reduced so the first error
 // in the reference's (branch, row) order wins.  INT32_MAX = no error.

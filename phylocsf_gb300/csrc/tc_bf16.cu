@@ -386,7 +386,7 @@ cudaError_t set_bf16_attributes(size_t smem)
 {
     cudaError_t e = cudaFuncSetAttribute(k_prune_bf16, cudaFuncAttributePreferredSharedMemoryCarveout,
                                          (int)cudaSharedmemCarveoutMaxShared);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_prune_bf16, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = allow_smem<k_prune_bf16>();
     return e;
 }
 

@@ -449,7 +449,7 @@ cudaError_t launch_prune_tc_dual(const PruneArgs &a, const float *Qop, const dou
     const size_t smem = prune_tc_dual_smem_bytes(a.nl, a.n_internal);
     cudaError_t e = cudaFuncSetAttribute(k_prune_tc_dual, cudaFuncAttributePreferredSharedMemoryCarveout,
                                          (int)cudaSharedmemCarveoutMaxShared);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_prune_tc_dual, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = allow_smem<k_prune_tc_dual>();
     if (e != cudaSuccess) return e;
     k_prune_tc_dual<<<grid, TD_THREADS, smem, s>>>(a, Qop, branch, dpart, err);
     return cudaGetLastError();

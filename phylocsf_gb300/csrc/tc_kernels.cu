@@ -527,7 +527,7 @@ static cudaError_t set_tc_attributes(size_t smem)
     cudaError_t e = cudaFuncSetAttribute(k_prune_tc<NPROD>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                          (int)cudaSharedmemCarveoutMaxShared);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_prune_tc<NPROD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = allow_smem<k_prune_tc<NPROD>>();
     return e;
 }
 

@@ -269,7 +269,7 @@ cudaError_t launch_pform_tc(const PSet *ps, int nps, const double *branch, int n
     if (nps <= 0) return cudaSuccess;
     cudaError_t e = cudaFuncSetAttribute(k_pform_tc, cudaFuncAttributePreferredSharedMemoryCarveout,
                                          (int)cudaSharedmemCarveoutMaxShared);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_pform_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PFT_SMEM);
+    if (e == cudaSuccess) e = allow_smem<k_pform_tc>();
     if (e != cudaSuccess) return e;
     // Branch pairs per CTA: all of a P set's when there are enough P sets to fill the GPU
     // several times over, fewer for a short list (one exon's search round asks for two to six
