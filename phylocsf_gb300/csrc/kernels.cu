@@ -13,6 +13,7 @@
 
 #include <cooperative_groups.h>
 
+#include "jacobi_rotation.cuh"
 #include "pcsf_internal.h"
 #include "prune_common.cuh"
 
@@ -47,78 +48,6 @@ __device__ inline void jac_pair(int r, int i, int &p, int &q)
     else { a = (r + i) % (K - 1); b = (r - i + (K - 1)) % (K - 1); }
     p = a < b ? a : b;
     q = a < b ? b : a;
-}
-
-// Reciprocal and reciprocal square root of a normal d > 0 (exponent well inside the range) to about
-// 2^-44: the leading 24 bits by the FP32 approximation, the rest by one Newton step on two floats,
-// put together as integers.  FP64 instructions take 69 clocks each in a chain on this part, FP32 and
-// integer ones four.
-__device__ __forceinline__ double seed_bits(float y0, float y1, int e)
-{
-    // (double)y0 + y1 for y0 in [0.5, 1], |y1| < 2^-22, times 2^-e
-    const int k = __float_as_int(fmaf(y1, 0x1p44f, 12582912.0f)) - 0x4B400000;             // y1 in units of 2^-44
-    return __longlong_as_double(((long long)__float_as_int(y0) << 29) + ((long long)(896 - e) << 52) + ((long long)k << 9));
-}
-__device__ __forceinline__ double recip_seed(double d)
-{
-    const long long b = __double_as_longlong(d);
-    const float mh = __int_as_float(0x3F800000 | ((int)(b >> 29) & 0x7FFFFF));              // mantissa in [1, 2): 24 bits
-    const float ml = (__int_as_float(0x4B000000 | ((int)(b >> 6) & 0x7FFFFF)) - 8388608.0f) * 0x1p-46f;
-    float y0;
-    asm("rcp.approx.f32 %0, %1;" : "=f"(y0) : "f"(mh));
-    const float r = fmaf(-ml, y0, fmaf(-mh, y0, 1.0f));
-    return seed_bits(y0, y0 * r, (int)(b >> 52) - 1023);
-}
-__device__ __forceinline__ double rsqrt_seed(double d)
-{
-    const long long b = __double_as_longlong(d);
-    const int e = (int)(b >> 52) - 1023, odd = e & 1;
-    const float mh = __int_as_float((0x3F800000 + (odd << 23)) | ((int)(b >> 29) & 0x7FFFFF));   // [1, 4)
-    const float ml = (__int_as_float(0x4B000000 | ((int)(b >> 6) & 0x7FFFFF)) - 8388608.0f) * (odd ? 0x1p-45f : 0x1p-46f);
-    float y0;
-    asm("rsqrt.approx.f32 %0, %1;" : "=f"(y0) : "f"(mh));
-    const float p = y0 * y0, pl = fmaf(y0, y0, -p);
-    const float r = fmaf(-ml, p, fmaf(-mh, pl, fmaf(-mh, p, 1.0f)));
-    return seed_bits(y0, 0.5f * y0 * r, (e - odd) / 2);
-}
-
-// The rotation (c, s) that annihilates apq != 0: theta = (aqq - app) / (2 apq), t = sign(theta) /
-// (|theta| + sqrt(theta^2 + 1)), c = 1 / sqrt(t^2 + 1), s = t c, each operation rounded to nearest.
-// Quotients and roots are seeds (above) with one residual correction in FP64 (Markstein, IBM J. Res.
-// Dev. 34 (1990) 111): an error of ~2^-88 before the final rounding, so that they round as the
-// library's do (it would take about 2^35 operations to meet one that does not), in 5 x 69 + 90
-// clocks for a root and its reciprocal instead of 705 + 459.  Operands far from 1, and |theta|
-// beyond 2^300, take the library's operations.
-__device__ __forceinline__ void jac_rotation(double app, double aqq, double apq, double &c, double &s)
-{
-    const double num = aqq - app, den = 2.0 * apq, ad = fabs(den);
-    const int en = (__double2hiint(num) >> 20) & 0x7FF, ed = __double2hiint(ad) >> 20;
-    double theta;
-    if ((num == 0.0 || (en > 223 && en < 1823)) && ed > 223 && ed < 1823) {
-        const double y = recip_seed(ad), q = num * y;
-        theta = __fma_rn(__fma_rn(-q, ad, num), y, q);
-        if (den < 0.0) theta = -theta;
-    } else {
-        theta = num / den;
-    }
-    double t;
-    if (fabs(theta) < 0x1p300) {
-        const double x = __fma_rn(theta, theta, 1.0);
-        double y = rsqrt_seed(x);
-        const double g = x * y;
-        const double d = fabs(theta) + __fma_rn(__fma_rn(-g, g, x), 0.5 * y, g);
-        y = recip_seed(d);
-        t = __fma_rn(y, __fma_rn(-d, y, 1.0), y);
-        if (!(theta >= 0.0)) t = -t;
-    } else {
-        t = (fabs(theta) > 1e150) ? 0.5 / theta
-            : (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(__fma_rn(theta, theta, 1.0)));
-    }
-    const double u = __fma_rn(t, t, 1.0);          // in [1, 2]
-    const double y = rsqrt_seed(u), g = u * y;
-    const double v = __fma_rn(__fma_rn(-g, g, u), 0.5 * y, g);
-    c = __fma_rn(y, __fma_rn(-v, y, 1.0), y);
-    s = t * c;
 }
 
 template <int C>

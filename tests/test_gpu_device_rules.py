@@ -1,0 +1,78 @@
+"""Arithmetic of the kernels that has a rule of its own, run on the device from the library's own headers
+and compared there, value for value, with the plain expression that it stands for."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+
+def _run(tmp_path, headers, decl, body):
+    """Whole numbers, by line, that a main() with this body prints."""
+    nvcc = shutil.which("nvcc") or os.path.join(CUDA, "bin", "nvcc")
+    src, exe = tmp_path / "rule.cu", tmp_path / "rule"
+    src.write_text("#include <cmath>\n#include <cstdio>\n#include <vector>\n" + "".join('#include "%s"\n' % h for h in headers) +
+                   "using namespace pcsf;\n%s\nint main()\n{\n%s\n}\n" % (decl, body))
+    subprocess.run([nvcc, "-O2", "-std=c++17", "-gencode", "arch=compute_103a,code=sm_103a", "-I",
+                    os.path.join(ROOT, "phylocsf_gb300", "csrc"), str(src), "-o", str(exe)], check=True)
+    out = subprocess.run([str(exe)], check=True, capture_output=True, text=True, timeout=120).stdout
+    return [[int(x) for x in line.split()] for line in out.splitlines()]
+
+
+# Spans of the operands' exponents: what a search meets, and far beyond.
+# No tolerance: each corrected operation is off by ~2^-88 before its rounding, so that one of ~2^35 rounds
+# otherwise than the correctly rounded one, and 2^22 rotations have 2^24 operations.
+@pytest.mark.parametrize("span", [3, 60, 290, 460])
+def test_rotation(tmp_path, span):
+    rows = _run(tmp_path, ["jacobi_rotation.cuh"], """
+constexpr int N = 1 << 22;
+__device__ unsigned long long mix(unsigned long long z)
+{
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+    return z ^ (z >> 31);
+}
+// +-m 2^e, m in [1, 2), |e| <= span; now and then a power of two
+__device__ double draw(unsigned long long i, int span)
+{
+    const unsigned long long x = mix(i * 0x9E3779B97F4A7C15ull + span), y = mix(x);
+    const double m = 1.0 + ((y & 15) ? (double)(x >> 12) * 0x1p-52 : 0.0);
+    return ldexp((y >> 8) & 1 ? -m : m, (int)((y >> 16) % (2 * span + 1)) - span);
+}
+__global__ void check(int span, int *counts, double *first)
+{
+    const unsigned long long i = blockIdx.x * 256ull + threadIdx.x;
+    double app = draw(3 * i, span), aqq = draw(3 * i + 1, span), apq = draw(3 * i + 2, span);
+    if (i % 64 == 1) aqq = app;                     // a rotation by 45 degrees
+    if (i % 64 == 2) app = 0.0;
+    double c, s;
+    jac_rotation(app, aqq, apq, c, s);
+    const double theta = __ddiv_rn(aqq - app, 2.0 * apq);
+    const double t = fabs(theta) > 1e150 ? 0.5 / theta
+                     : __ddiv_rn(theta >= 0.0 ? 1.0 : -1.0, fabs(theta) + __dsqrt_rn(__fma_rn(theta, theta, 1.0)));
+    const double rc = __ddiv_rn(1.0, __dsqrt_rn(__fma_rn(t, t, 1.0))), rs = t * rc;
+    if (!isfinite(theta)) atomicAdd(counts + 1, 1);
+    if (fabs(theta) < 0x1p300) atomicAdd(counts + 2, 1);
+    if (!(c == rc && s == rs) && atomicAdd(counts, 1) == 0) {
+        first[0] = app; first[1] = aqq; first[2] = apq; first[3] = c; first[4] = s; first[5] = rc; first[6] = rs;
+    }
+}
+""", """
+    int *counts;
+    double *first;
+    if (cudaMallocManaged(&counts, 3 * sizeof(int)) != cudaSuccess) return 1;
+    if (cudaMallocManaged(&first, 7 * sizeof(double)) != cudaSuccess) return 1;
+    for (int k = 0; k < 3; k++) counts[k] = 0;
+    check<<<N / 256, 256>>>(SPAN, counts, first);
+    if (cudaDeviceSynchronize() != cudaSuccess) return 2;
+    if (counts[0]) for (int k = 0; k < 7; k++) std::fprintf(stderr, "%a\\n", first[k]);
+    std::printf("%d %d %d\\n", counts[0], counts[1], counts[2]);
+""".replace("SPAN", str(span)))
+    wrong, infinite, common = rows[0]
+    assert wrong == 0
+    assert common > 0 and infinite == 0
