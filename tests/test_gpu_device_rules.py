@@ -24,10 +24,10 @@ def _run(tmp_path, headers, decl, body):
     return [[int(x) for x in line.split()] for line in out.splitlines()]
 
 
-# Spans of the operands' exponents: what a search meets, and far beyond.
+# Spans of the operands' exponents: what a search meets, and up to where a quotient overflows or vanishes.
 # No tolerance: each corrected operation is off by ~2^-88 before its rounding, so that one of ~2^35 rounds
 # otherwise than the correctly rounded one, and 2^22 rotations have 2^24 operations.
-@pytest.mark.parametrize("span", [3, 60, 290, 460])
+@pytest.mark.parametrize("span", [3, 60, 290, 460, 790, 1000])
 def test_rotation(tmp_path, span):
     rows = _run(tmp_path, ["jacobi_rotation.cuh"], """
 constexpr int N = 1 << 22;
@@ -75,4 +75,4 @@ __global__ void check(int span, int *counts, double *first)
 """.replace("SPAN", str(span)))
     wrong, infinite, common = rows[0]
     assert wrong == 0
-    assert common > 0 and infinite == 0
+    assert common > 0 and (infinite > 0) == (span >= 790)
