@@ -76,3 +76,49 @@ __global__ void check(int span, int *counts, double *first)
     wrong, infinite, common = rows[0]
     assert wrong == 0
     assert common > 0 and (infinite > 0) == (span >= 790)
+
+
+def test_grid_point(tmp_path):
+    """The grid point nearest to t, against the same rule with t's place found in FP64, at and around every
+    grid point and midpoint, below the second point, beyond the last one and past the range of FP32."""
+    rows = _run(tmp_path, ["pcsf_internal.h", "prune_common.cuh"], """
+__global__ void check(DevModels m, const double *t, int n, int *counts)
+{
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= n || t[i] < m.grid_t[0]) return;
+    const double x = floor(log(t[i] / m.grid_t[0]) / m.grid_lr);
+    int g = x < 0.0 ? 0 : x > m.grid_n - 1 ? m.grid_n - 1 : (int)x;
+    if (g + 1 < m.grid_n && (m.grid_t[g + 1] - t[i]) < (t[i] - m.grid_t[g])) g++;
+    atomicAdd(counts, 1);
+    if (grid_point(m, t[i]) != g) atomicAdd(counts + 1, 1);
+}
+""", """
+    const int G = 6500;
+    const double lr = std::log(1.002), rel[] = {0, 1e-16, 1e-13, 1e-10, 1e-8, 1e-7, 1e-6, 1e-5, 3e-4};
+    std::vector<double> grid(G), ts = {1e-3, 1.0, 1e30, 1e38, 1e39, 1e200, 1e308};
+    for (int g = 0; g < G; g++) grid[g] = 1e-5 * std::exp(lr * g);
+    for (int g = 0; g < G; g++)
+        for (double r : rel)
+            for (double sign : {1.0, -1.0}) {
+                ts.push_back(grid[g] * (1.0 + sign * r));
+                if (g) ts.push_back(0.5 * (grid[g] + grid[g - 1]) * (1.0 + sign * r));
+            }
+    const int n = (int)ts.size();
+    DevModels m{};
+    double *dg, *dt;
+    int *counts;
+    if (cudaMallocManaged(&dg, G * sizeof(double)) != cudaSuccess) return 1;
+    if (cudaMallocManaged(&dt, n * sizeof(double)) != cudaSuccess) return 1;
+    if (cudaMallocManaged(&counts, 2 * sizeof(int)) != cudaSuccess) return 1;
+    for (int k = 0; k < G; k++) dg[k] = grid[k];
+    for (int k = 0; k < n; k++) dt[k] = ts[k];
+    counts[0] = counts[1] = 0;
+    m.grid_t = dg;
+    m.grid_n = G;
+    m.grid_lr = lr;
+    check<<<(n + 255) / 256, 256>>>(m, dt, n, counts);
+    if (cudaDeviceSynchronize() != cudaSuccess) return 2;
+    std::printf("%d %d\\n", counts[0], counts[1]);
+""")
+    compared, wrong = rows[0]
+    assert compared > 200_000 and wrong == 0
