@@ -575,23 +575,18 @@ static int simt_grid(const pcsf_engine *e, int tile)
     return e->sm_count * std::min(per_sm, 8);
 }
 
-// Column tile of a SIMT pruning launch over these requests: small tiles while all of them are
-// resident at once (FP32, four per SM), or are few enough that an uneven last wave would show
-// (FP64: bound by its two lanes per clock and SM at any tile, so that only the balance counts;
-// 212 tiles of 32 left 92 SMs with one and 60 with two), the engine's tile beyond.  A launch of a few hundred columns is
-// as long as one CTA's walk down the tree, which takes a third to a half of the time with a
-// column per thread.  Measured with 64 (FP64: 32) against 8 columns: 58 leaves FP32 300 columns
-// 254 / 129 us, 4,800 columns 258 / 159, 9,600 columns 261 / 354; 12 leaves FP32 300 columns 66 /
-// 39; 12 leaves FP64 1,200 columns 404 / 135, 4,800 columns 404 / 301, 9,600 columns 783 / 799.
+// Column tile of a SIMT pruning launch over these requests: small tiles in short launches
+// (small_tiles), the engine's tile beyond.
 static int launch_tile(const pcsf_engine *e, const pcsf_batch *b, const std::vector<Request> &reqs)
 {
-    const int64_t most = (e->prec == PCSF_PREC_FP64 ? 16 : 4) * (int64_t)e->sm_count;
+    const bool fp64 = e->prec == PCSF_PREC_FP64;
+    const int64_t most = small_tiles_most(fp64, e->sm_count);
     int64_t tiles = 0;
     for (const Request &q : reqs) {
         tiles += (b->offs[q.region + 1] - b->offs[q.region] + PRUNE_SMALL_TILE - 1) / PRUNE_SMALL_TILE;
-        if (tiles > most) return simt_tile_cols(e->prec, e->nslots, e->simt_tile);
+        if (tiles > most) break;
     }
-    return PRUNE_SMALL_TILE;
+    return small_tiles(fp64, tiles, e->sm_count) ? PRUNE_SMALL_TILE : simt_tile_cols(e->prec, e->nslots, e->simt_tile);
 }
 
 static int engine_init_common(pcsf_engine *e, const pcsf_tree *tree, int32_t flags)

@@ -155,6 +155,24 @@ struct PruneArgs {
 // comp: 0 plain FP32 sums, 1 Kahan, 2 blocked Kahan (see prune_common.cuh)
 cudaError_t launch_prune(int prec, int comp, const PruneArgs &a, cudaStream_t s, int grid);
 constexpr int PRUNE_SMALL_TILE = 8;   // the SIMT kernel's column tile in a short launch
+// Whether a launch of this many small tiles is short.  FP32: while all of them are resident at once, four
+// per SM; such a launch is as long as one CTA's walk down the tree, which takes a third to a half of the
+// time with a column per thread (64 against 8 columns: 58 leaves, 300 columns 212 / 105 us, 4,800 columns
+// 214 / 167; 12 leaves 56 / 33 and 57 / 52; 120 leaves, 32 against 8 columns, 302 / 193 and 302 / 322).  FP64 is bound by its two
+// lanes per clock and SM at any tile, so that only the balance counts, up to four long tiles (32 columns)
+// an SM: small ones unless the last wave of long ones is more than three quarters full.  The third is no
+// exception to them: where two CTAs share an SM, it does not spread evenly.  Measured with 32 and 8
+// columns, ms at 2,424 / 4,856 / 7,288 / 9,720 / 12,152 / 14,584 / 17,016 / 19,448 columns: 12 leaves 0.41,
+// 0.41, 0.79, 0.79, 1.17, 1.56, 1.57, 1.57 and 0.21, 0.50, 0.60, 0.89, 1.09, 1.19, 1.48, 1.68; 58 leaves
+// 2.17, 2.16, 4.32, 4.32, 6.48, 6.48, 8.64, 8.63 and 1.09, 2.17, 3.25, 4.33, 5.41, 6.49, 7.57, 8.65.
+inline int64_t small_tiles_most(bool fp64, int sm_count) { return (fp64 ? 16 : 4) * (int64_t)sm_count; }
+inline bool small_tiles(bool fp64, int64_t tiles, int sm_count)
+{
+    if (tiles > small_tiles_most(fp64, sm_count)) return false;
+    if (!fp64 || tiles == 0) return true;
+    const int64_t wave = 4 * (int64_t)sm_count, waves = (tiles + wave - 1) / wave;
+    return waves == 3 || 4 * (tiles - (waves - 1) * wave) <= 3 * wave;
+}
 int prune_tile_cols(int prec);
 int simt_tile_cols(int prec, int nslots, int tile = 0);   // the SIMT kernel's column tile (k_prune)
 size_t prune_smem_bytes(int prec, int nslots, int nl, int nint, int tile = 0);

@@ -67,3 +67,17 @@ def test_wait_for_the_last_contraction(tmp_path):
         assert blocks == late                          # waits while the commit is outstanding
         if late:
             assert not blocks_after                    # and no longer once it has arrived
+
+
+def test_small_tiles(tmp_path):
+    """FP32: up to four small tiles an SM.  FP64, in waves of long tiles (four small ones): while the last
+    wave is at most three quarters full, in the third wave always, and up to four waves."""
+    rows = _run(tmp_path, """
+    for (int sms : {1, 7, 148, 152})
+        for (int n = 0; n <= 17 * sms; n++) std::printf("%d %d %d %d\\n", sms, n, small_tiles(false, n, sms), small_tiles(true, n, sms));
+""")
+    assert len(rows) == 17 * (1 + 7 + 148 + 152) + 4
+    for sms, n, fp32, fp64 in rows:
+        assert fp32 == (n <= 4 * sms)
+        quarters = -(-n // sms)               # of waves, the last one's begun
+        assert fp64 == (quarters <= 16 and quarters not in (4, 8, 16))
