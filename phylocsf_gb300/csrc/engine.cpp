@@ -733,7 +733,7 @@ static int evaluate(pcsf_engine *e, pcsf_batch *b, const std::vector<Request> &r
                                                                                               : e->comp_mode();
 
     const int kind = drho ? 3 : grad ? 2 : tc ? 1 : ff ? 4 : 0;
-    // a float-float P set (8-12 B per entry) and its FP64 staging take at most five times an FP32 one
+    // a float-float P set (8-14 B per entry) and its FP64 staging take at most five times an FP32 one
     const size_t chunk_psets = ff ? std::max<size_t>(1, e->pbuf_psets / 5) : e->pbuf_psets;
     int64_t kind_cols = 0;
     // work items, P-set dedup and chunking (at most pbuf_psets distinct P sets per chunk)

@@ -11,18 +11,18 @@
 //   - E = P - I comes from the FP64 P(t) formation (the FP64 engine's own matrices, row
 //     rule of Q.ml:226-247 applied in FP64).  Once per P set (k_split_ff) each row of a
 //     branch above an internal node is written as its diagonal in hi / lo floats and its
-//     off-diagonal entries as 2^ea sum_l e_l 2^(-8-9l), six signed 9-bit digits (an error
-//     below 2^-54 of the largest of them, the order of the FP64 formation's own), and each
-//     branch above a leaf as P in hi / lo floats;
-//   - a partial alpha, normalised per column to [0.5, 1), becomes sum_k A_k 2^(-8-9k), six
-//     signed 9-bit digits (an error below 2^-54 of the column's largest entry);
+//     off-diagonal entries as 2^ea sum_l e_l 2^(-8-9l), seven signed 9-bit digits (an error
+//     below 2^-63 of the largest of them), and each branch above a leaf as P in hi / lo floats;
+//   - a partial alpha, normalised per column to [0.5, 1), becomes sum_k A_k 2^(-8-9k), seven
+//     signed 9-bit digits (an error below 2^-60 of the column's largest entry);
 //   - sum_{j != a} E[a][j] alpha[j] = 2^(ea-16) sum_g 2^(-9g) G_g with G_g = sum_{k+l=g} sum_j
-//     e_l[a][j] A_k[j], kept for g <= 6 (26 of the 36 digit products; the rest are below
-//     2^-58).  Digits are FP16 operands of tcgen05.mma kind::f16 (at most 9 bits + sign of
+//     e_l[a][j] A_k[j], kept for g <= 7 (34 of the 49 digit products; the rest are below
+//     2^-63).  Digits are FP16 operands of tcgen05.mma kind::f16 (at most 9 bits + sign of
 //     FP16's 11); the products of a group share one FP32 accumulator in tensor memory and
 //     are integers whose sums stay below 2^24 for g <= 3 (64 x 2^16 x 4 pairs) and, in any
-//     case, round by 2^-52 or less beyond, so the accumulation is exact: it does not
-//     matter in which order or with which rounding the tensor cores add;
+//     case, round by 2^-52 or less beyond, where the digits' signs keep them far below 2^24:
+//     so the accumulation is exact, and it does not matter in which order or with which
+//     rounding the tensor cores add;
 //   - the groups are summed, and alpha and the diagonal's term added (v = alpha + E alpha,
 //     PhyloLik.ml:89-92), with error-free transforms; a leaf child's partial is a gathered row of P
 //     (PhyloLik.ml:87-88 with a one-hot leaf);
@@ -35,24 +35,29 @@
 // scalar FP32 at half the issue slots), which the compiler never contracts.
 //
 // Shape: one CTA of 512 threads per SM and 128-column tile; thread t owns column t % 128
-// (its TMEM lane) and states 16 (t / 128) .. + 15.  A_k (6 x 16 KB) and the e_l of one
-// branch (48 KB, one bulk copy, fetched while the previous contraction is combined) sit in
+// (its TMEM lane) and states 16 (t / 128) .. + 15.  A_k (7 x 16 KB) and the e_l of one
+// branch (56 KB, one bulk copy, fetched while the previous contraction is combined) sit in
 // shared memory.  B's rows are ordered [digit l][state], so one MMA of A_k against the
 // first digits of B adds into consecutive groups: D column 32 g + state for half of the
 // states at a time, so the first half is combined while the second half's MMAs run.
 // The node evaluated just before its parent is handed over in registers; the other
 // internal child (a first child whose sibling is internal) waits on a per-thread stack in
 // global memory (L2).
-// What bounds it: the chain of a contraction's phases, 13,900 clocks on 120 leaves: digits
-// 1,900, staging barrier 1,100, first half's MMAs 2,700 (with the sibling leaf's gather), its
-// combination beside the second half's MMAs 2,300, the second half's 2,000, the maximum and
-// rescale 500, and per node 3,200 of leaf gathers and stack traffic; a third of the issue slots
-// are used.  The MMAs need 3,400 clocks, and a float-float dot product on the FP32 units (64 x
-// 12 instructions per state and column instead of about 75) took 75,000.  Measured per column
-// and evaluation: 120 leaves 238 -> 43 ns, 100 leaves 210 -> 39, 58 leaves (launches of a few
-// regions, which leave SMs idle) 133 -> 43.  Against the FP64 engine on the same P(t), lpr is
-// within 6e-16 relative at rho >= 1 and 5e-14 at rho = 0.01, where two independent FP64
-// evaluations differ by 2e-12.
+// What bounds it: the chain of a contraction's phases, 14,700 clocks on 120 leaves (13,700 with
+// six digits, of which: digits 1,900, staging barrier 1,100, first half's MMAs 2,700 (with the
+// sibling leaf's gather), its combination beside the second half's MMAs 2,300, the second half's
+// 2,000, the maximum and rescale 500, and per node 3,200 of leaf gathers and stack traffic); a
+// third of the issue slots are used.  The MMAs need 4,450 clocks, and a float-float dot product
+// on the FP32 units (64 x 12 instructions per state and column instead of about 65) took 75,000.
+// Measured per column and evaluation: 120 leaves 238 -> 48 ns, 100 leaves 210 -> 39, 58 leaves 133
+// -> 25 (23 in launches that fill the GPU).
+// Why seven digits: they are counted from a row's and a column's largest entries.  In a column
+// whose two halves of the tree hold codons three substitutions apart, the entries that matter
+// lie 2^-20 and more below those.  Against the FP64 engine on the same P(t), the lpr of such a
+// column on 58 leaves is off by 1e-14, 3e-14 and 2e-13 at rho = 1, 0.1 and 0.01 (with six digits
+// 1e-12, 1e-11 and 1e-10), a thousandth and less of what the FP64 formation of P(t) leaves there.
+// The lpr of regions is within 6e-16 relative at rho >= 1 and 5e-14 at rho = 0.01, where two
+// independent FP64 evaluations differ by 2e-12.
 #include <algorithm>
 
 #include <cuda_fp16.h>
@@ -67,30 +72,33 @@ namespace {
 
 constexpr int FF_THREADS = 512;
 constexpr int FF_TC = 128;           // columns per tile
-constexpr int FF_DIG = 6;            // 9-bit digits per operand
-constexpr int FF_GRP = 7;            // digit groups k + l = 0 .. 6
+constexpr int FF_DIG = 7;            // 9-bit digits per operand
+constexpr int FF_GRP = 8;            // digit groups k + l = 0 .. 7
+constexpr int FF_BROWS = 32 * FF_DIG;   // rows of B: [digit][32 states]
 constexpr int FF_SPT = 16;           // states per thread
 constexpr size_t FF_LEAF_BYTES = 2 * K2 * sizeof(float);            // P of a leaf branch, [s][hi 64 | lo 64]
-constexpr uint32_t FF_HALF_BYTES = FF_DIG * 32 * K * 2;             // e_l of 32 states: 192 rows x 64, FP16
+constexpr uint32_t FF_HALF_BYTES = FF_BROWS * K * 2;                // e_l of 32 states: 224 rows x 64, FP16
 constexpr size_t FF_INNER_BYTES = 2 * FF_HALF_BYTES;
 constexpr uint32_t FF_ROW_BYTES = 3 * K * 4;                        // per row: scale 2^(ea - 16), E_aa hi, E_aa lo
 
 // dynamic shared memory (bytes)
 constexpr uint32_t FS_A = 0;                                        // [digit][128 x 64] FP16
 constexpr uint32_t FS_ADIG = 128 * K * 2;
-constexpr uint32_t FS_B = FS_A + FF_DIG * FS_ADIG;                  // [half][192 x 64] FP16
+constexpr uint32_t FS_B = FS_A + FF_DIG * FS_ADIG;                  // [half][224 x 64] FP16
 constexpr uint32_t FS_SC = FS_B + 2 * FF_HALF_BYTES;                // [2][3][64] row scales and diagonals
 constexpr uint32_t FS_CM = FS_SC + 2 * FF_ROW_BYTES;                       // [2][4][128] column maxima
-constexpr uint32_t FS_LV = FS_CM + 2 * 4 * FF_TC * 4;               // [nl][128] leaf states, schedule, order
+constexpr uint32_t FS_LV = FS_CM + 2 * 4 * FF_TC * 4;               // [nl][128] leaf states (if they fit), schedule, order
 
 // byte offset of (leaf l, site c): words XOR-swizzled per leaf, so that the fill (consecutive
 // threads on consecutive leaves) and the reads (on consecutive sites) are free of conflicts
 __device__ __forceinline__ int ff_lv(int l, int c) { return l * FF_TC + (c ^ ((l & 31) << 2)); }
 
-size_t ff_smem(int nl, int nint)
+size_t ff_smem(int nl, int nint, bool lv)
 {
-    return FS_LV + (((size_t)nl * FF_TC + 15) & ~size_t(15)) + (size_t)nint * (sizeof(SchedNode) + 2) + 16;
+    return FS_LV + (lv ? (size_t)nl * FF_TC : 0) + (size_t)nint * (sizeof(SchedNode) + 2) + 16;
 }
+// a tile's leaf states are kept in shared memory where the tree leaves them room (up to 362 leaves)
+bool ff_lv_fits(int nl, int nint) { return ff_smem(nl, nint, true) + 4096 <= (size_t)SMEM_OPTIN; }
 
 // s + e = a + b exactly (Knuth)
 __device__ __forceinline__ void two_sum2(f2 a, f2 b, f2 &s, f2 &e)
@@ -104,6 +112,14 @@ __device__ __forceinline__ void fast_two_sum2(f2 a, f2 b, f2 &s, f2 &e)
 {
     s = add2(a, b);
     e = sub2(b, sub2(s, a));
+}
+// s + e = a + G c exactly, for a group's sum G (an integer below 2^24) with weight c and the sum a of the
+// groups before, a multiple of 512 c: if |s| < 2^24 c, s is not rounded; beyond, a - s is a multiple of
+// s's last place and at most 2^24 c, a float either way, and what G c has left over it one too
+__device__ __forceinline__ void add_group(f2 a, f2 G, f2 c, f2 &s, f2 &e)
+{
+    s = fma2(G, c, a);
+    e = fma2(G, c, sub2(a, s));
 }
 // two FP16 values from a pair of floats that hold small integers (exact)
 __device__ __forceinline__ uint32_t half2_of(f2 a)
@@ -125,10 +141,11 @@ __device__ __forceinline__ void ff_mul2(f2 ah, f2 al, f2 bh, f2 bl, f2 &h, f2 &l
     fast_two_sum2(p, lo, h, l);
 }
 
-// Six signed 9-bit digits of a pair x = h + l in [0, 1): x = sum_k d_k 2^(-8-9k).  Rounding to
+// Seven signed 9-bit digits of a pair x = h + l in [0, 1): x = sum_k d_k 2^(-8-9k).  Rounding to
 // an integer by adding 1.5 x 2^23; the residual r is kept negated, so that each digit comes out
-// as magic - t without a sign flip.  l joins before digit 2 (error-free: its sum's error e joins
-// the residual of digit 3).
+// as magic - t without a sign flip.  l joins before digit 2 (error-free: r is 0 or a multiple of h's
+// last place, at least twice l, so that r - s is exact; the sum's error e joins
+// the residual of digit 3: rounded there by at most 2^-61).
 __device__ __forceinline__ void ff_digits(f2 h, f2 l, uint32_t d[FF_DIG])
 {
     const f2 M = pk(12582912.0f, 12582912.0f), S = pk(512.0f, 512.0f);
@@ -139,8 +156,7 @@ __device__ __forceinline__ void ff_digits(f2 h, f2 l, uint32_t d[FF_DIG])
     nd = sub2(M, fma2(r, S, M));
     d[1] = half2_of(nd);
     r = fma2(r, S, nd);
-    f2 s, e;
-    two_sum2(r, mul2(l, pk(-131072.0f, -131072.0f)), s, e);      // units 2^-17
+    const f2 ml = pk(-131072.0f, -131072.0f), s = fma2(l, ml, r), e = fma2(l, ml, sub2(r, s));      // units 2^-17
     nd = sub2(M, fma2(s, S, M));
     d[2] = half2_of(nd);
     r = fma2(s, S, nd);
@@ -151,7 +167,10 @@ __device__ __forceinline__ void ff_digits(f2 h, f2 l, uint32_t d[FF_DIG])
     nd = sub2(M, fma2(r, S, M));
     d[4] = half2_of(nd);
     r = fma2(r, S, nd);
-    d[5] = half2_of(sub2(M, fma2(r, S, M)));
+    nd = sub2(M, fma2(r, S, M));
+    d[5] = half2_of(nd);
+    r = fma2(r, S, nd);
+    d[6] = half2_of(sub2(M, fma2(r, S, M)));
 }
 
 __device__ __forceinline__ void mma_f16(uint32_t dt, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t acc)
@@ -161,23 +180,25 @@ __device__ __forceinline__ void mma_f16(uint32_t dt, uint64_t ad, uint64_t bd, u
                  :: "r"(dt), "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
 }
 
-// four columns of each of the seven groups (32 columns apart), and the wait, in one asm block
+// four columns of each of the eight groups (32 columns apart), and the wait, in one asm block
 __device__ __forceinline__ void tmem_ld_groups(uint32_t ta, float g[FF_GRP][4])
 {
     uint32_t r[FF_GRP * 4];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%28];\n"
-                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%4,%5,%6,%7}, [%29];\n"
-                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%8,%9,%10,%11}, [%30];\n"
-                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%12,%13,%14,%15}, [%31];\n"
-                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%16,%17,%18,%19}, [%32];\n"
-                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%20,%21,%22,%23}, [%33];\n"
-                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%24,%25,%26,%27}, [%34];\n"
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%32];\n"
+                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%4,%5,%6,%7}, [%33];\n"
+                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%8,%9,%10,%11}, [%34];\n"
+                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%12,%13,%14,%15}, [%35];\n"
+                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%16,%17,%18,%19}, [%36];\n"
+                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%20,%21,%22,%23}, [%37];\n"
+                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%24,%25,%26,%27}, [%38];\n"
+                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%28,%29,%30,%31}, [%39];\n"
                  "tcgen05.wait::ld.sync.aligned;"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
                    "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
                    "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-                   "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27])
-                 : "r"(ta), "r"(ta + 32), "r"(ta + 64), "r"(ta + 96), "r"(ta + 128), "r"(ta + 160), "r"(ta + 192)
+                   "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+                 : "r"(ta), "r"(ta + 32), "r"(ta + 64), "r"(ta + 96), "r"(ta + 128), "r"(ta + 160), "r"(ta + 192),
+                   "r"(ta + 224)
                  : "memory");
 #pragma unroll
     for (int k = 0; k < FF_GRP; k++)
@@ -229,7 +250,7 @@ __global__ void __launch_bounds__(256) k_split_ff(const double *in, unsigned cha
     __syncthreads();
     hi = max(max(emax[0][a], emax[1][a]), max(emax[2][a], emax[3][a]));
     const int ea = max((hi >> 20) - 1022, -110);
-    const double up = __hiloint2double((1023 + 53 - ea) << 20, 0);
+    const double up = __hiloint2double((1023 + 9 * FF_DIG - 1 - ea) << 20, 0);
     const int half = (a >> 3) & 1, n0 = (a >> 4) * 8 + (a & 7);         // state 16 q + 8 half + i -> row 8 q + i
     unsigned char *dst = base + (size_t)nl * FF_LEAF_BYTES + (size_t)(b - nl) * FF_INNER_BYTES + half * FF_HALF_BYTES;
 #pragma unroll
@@ -255,14 +276,14 @@ __global__ void __launch_bounds__(256) k_split_ff(const double *in, unsigned cha
 #pragma unroll
         for (int l = 0; l < FF_DIG; l++) {
             const int n = 32 * l + n0;
-            *reinterpret_cast<uint4 *>(dst + (((2 * qd + c) * 24 + (n >> 3)) << 7) + ((n & 7) << 4)) =
+            *reinterpret_cast<uint4 *>(dst + (((2 * qd + c) * (FF_BROWS / 8) + (n >> 3)) << 7) + ((n & 7) << 4)) =
                 make_uint4(w[l][0], w[l][1], w[l][2], w[l][3]);
         }
     }
     if (qd == 0) row[a] = __int_as_float((127 + ea - 16) << 23);
 }
 
-__global__ void __launch_bounds__(FF_THREADS, 1) k_prune_ff(PruneArgs a, size_t pset_bytes, float *stack, int *err)
+__global__ void __launch_bounds__(FF_THREADS, 1) k_prune_ff(PruneArgs a, size_t pset_bytes, float *stack, int *err, int lv_smem)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
     __shared__ uint32_t tbase_s;
@@ -276,7 +297,7 @@ __global__ void __launch_bounds__(FF_THREADS, 1) k_prune_ff(PruneArgs a, size_t 
     const int h = tid >> 7, s0 = FF_SPT * h;      // states s0 .. s0 + 15
     const int nl = a.nl, nin = a.n_internal;
     uint8_t *lvT = sm + FS_LV;
-    SchedNode *sched = reinterpret_cast<SchedNode *>(sm + FS_LV + ((nl * FF_TC + 15) & ~15));
+    SchedNode *sched = reinterpret_cast<SchedNode *>(sm + FS_LV + (lv_smem ? nl * FF_TC : 0));
     int16_t *bseq = reinterpret_cast<int16_t *>(sched + nin);        // internal child of each contraction, in order
     const uint32_t bar0 = smem_addr(&bar_h0), bar1 = smem_addr(&bar_h1), barB = smem_addr(&bar_b);
     const uint32_t sA = smem_addr(sm + FS_A), sB = smem_addr(sm + FS_B);
@@ -345,25 +366,25 @@ __global__ void __launch_bounds__(FF_THREADS, 1) k_prune_ff(PruneArgs a, size_t 
 
     // thread 0, after the staging barrier: the digit products of one contraction.  Operand
     // layouts: K-major core matrices (8 rows x 16 bytes); A_k 128 rows: 2048 B between core
-    // matrices along K, B 192 rows: 3072 B; a K step (16 values) is two of them.
+    // matrices along K, B 224 rows: 3584 B; a K step (16 values) is two of them.
     auto issue_mma = [&]() {
-        const uint64_t dA = sdesc(sA, 2048, 128), dB = sdesc(sB, 3072, 128);
+        const uint64_t dA = sdesc(sA, 2048, 128), dB = sdesc(sB, FF_BROWS * 16, 128);
         const uint32_t id0 = (1u << 4) | ((128u >> 4) << 24);     // f32 += f16 x f16, M = 128
 #pragma unroll 1
         for (int hf = 0; hf < 2; hf++) {
-            const uint32_t dt = tbase + 224 * hf;
+            const uint32_t dt = tbase + 32 * FF_GRP * hf;
             const uint64_t dBh = dB + (FF_HALF_BYTES >> 4) * hf;
-            // the first K step starts every group: groups 1-6 by A_1 x e_0..5, group 0 by A_0 x e_0
-            mma_f16(dt + 32, dA + (FS_ADIG >> 4), dBh, id0 | ((192u >> 3) << 17), 0);
+            // the first K step starts every group: groups 1-7 by A_1 x e_0..6, group 0 by A_0 x e_0
+            mma_f16(dt + 32, dA + (FS_ADIG >> 4), dBh, id0 | ((uint32_t)(FF_BROWS >> 3) << 17), 0);
             mma_f16(dt, dA, dBh, id0 | ((32u >> 3) << 17), 0);
-            mma_f16(dt + 32, dA, dBh + (32 * 16 >> 4), id0 | ((160u >> 3) << 17), 1);
+            mma_f16(dt + 32, dA, dBh + (32 * 16 >> 4), id0 | ((uint32_t)((FF_BROWS - 32) >> 3) << 17), 1);
 #pragma unroll
             for (int ks = 0; ks < 4; ks++) {
 #pragma unroll
                 for (int k = 0; k < FF_DIG; k++) {
                     if (ks == 0 && k < 2) continue;
-                    const uint32_t n = 32u * (k == 0 ? 6 : 7 - k);
-                    mma_f16(dt + 32 * k, dA + (FS_ADIG >> 4) * k + 256 * ks, dBh + 384 * ks, id0 | ((n >> 3) << 17), 1);
+                    const uint32_t n = 32u * (k == 0 ? FF_DIG : FF_GRP - k);
+                    mma_f16(dt + 32 * k, dA + (FS_ADIG >> 4) * k + 256 * ks, dBh + (FF_BROWS * 2) * ks, id0 | ((n >> 3) << 17), 1);
                 }
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
@@ -392,10 +413,15 @@ __global__ void __launch_bounds__(FF_THREADS, 1) k_prune_ff(PruneArgs a, size_t 
         const int ncols = wi.ncols;
         const uint8_t *lg = a.leaves + (size_t)wi.col0 * nl;
         __syncthreads();
-        for (int f = tid; f < FF_TC * nl; f += FF_THREADS) {
-            const int c = f / nl, l = f - c * nl;
-            lvT[ff_lv(l, c)] = (c < ncols) ? lg[f] : (uint8_t)K;
-        }
+        if (lv_smem)
+            for (int f = tid; f < FF_TC * nl; f += FF_THREADS) {
+                const int c = f / nl, l = f - c * nl;
+                lvT[ff_lv(l, c)] = (c < ncols) ? lg[f] : (uint8_t)K;
+            }
+        auto leaf_state = [&](int l) -> int {
+            if (lv_smem) return lvT[ff_lv(l, site)];
+            return site < ncols ? lg[(size_t)site * nl + l] : K;
+        };
         if (tid < K) {
             prd[tid] = a.m.prior[md * K + tid];
             wld[tid] = a.m.wlog[md * K + tid];
@@ -413,8 +439,8 @@ __global__ void __launch_bounds__(FF_THREADS, 1) k_prune_ff(PruneArgs a, size_t 
             bool have = false;
             if (nint == 0) {
                 float xh[FF_SPT], xl[FF_SPT], yh[FF_SPT], yl[FF_SPT];
-                leaf_rows(Pbase + (size_t)sn.lc * FF_LEAF_BYTES, lvT[ff_lv(sn.lc, site)], xh, xl);
-                leaf_rows(Pbase + (size_t)sn.rc * FF_LEAF_BYTES, lvT[ff_lv(sn.rc, site)], yh, yl);
+                leaf_rows(Pbase + (size_t)sn.lc * FF_LEAF_BYTES, leaf_state(sn.lc), xh, xl);
+                leaf_rows(Pbase + (size_t)sn.rc * FF_LEAF_BYTES, leaf_state(sn.rc), yh, yl);
 #pragma unroll
                 for (int i = 0; i < FF_SPT / 2; i++)
                     ff_mul2(pk(xh[2 * i], xh[2 * i + 1]), pk(xl[2 * i], xl[2 * i + 1]), pk(yh[2 * i], yh[2 * i + 1]),
@@ -454,7 +480,7 @@ __global__ void __launch_bounds__(FF_THREADS, 1) k_prune_ff(PruneArgs a, size_t 
                 if (nint == 1) {                // the leaf beside it, gathered while the MMAs run
                     const int lc = (sn.lslot < 0) ? sn.lc : sn.rc;
                     float xh[FF_SPT], xl[FF_SPT];
-                    leaf_rows(Pbase + (size_t)lc * FF_LEAF_BYTES, lvT[ff_lv(lc, site)], xh, xl);
+                    leaf_rows(Pbase + (size_t)lc * FF_LEAF_BYTES, leaf_state(lc), xh, xl);
 #pragma unroll
                     for (int i = 0; i < FF_SPT / 2; i++) {
                         vh[i] = pk(xh[2 * i], xh[2 * i + 1]);
@@ -472,7 +498,7 @@ __global__ void __launch_bounds__(FF_THREADS, 1) k_prune_ff(PruneArgs a, size_t 
 #pragma unroll
                     for (int q = 0; q < 2; q++) {
                         float g[FF_GRP][4];
-                        tmem_ld_groups(tbase + lane_off + 224 * hf + 8 * h + 4 * q, g);
+                        tmem_ld_groups(tbase + lane_off + 32 * FF_GRP * hf + 8 * h + 4 * q, g);
 #pragma unroll
                         for (int i = 0; i < 2; i++) {
                             const int x = 4 * hf + 2 * q + i;            // pair of states s0 + 2 x, s0 + 2 x + 1
@@ -480,12 +506,13 @@ __global__ void __launch_bounds__(FF_THREADS, 1) k_prune_ff(PruneArgs a, size_t 
 #pragma unroll
                             for (int k = 0; k < FF_GRP; k++) G[k] = pk(g[k][2 * i], g[k][2 * i + 1]);
                             const f2 c9 = pk(0x1p-9f, 0x1p-9f);
-                            f2 s1, e1, s2, e2, s3, e3;
-                            two_sum2(G[0], mul2(G[1], c9), s1, e1);
-                            two_sum2(s1, mul2(G[2], pk(0x1p-18f, 0x1p-18f)), s2, e2);
-                            two_sum2(s2, mul2(G[3], pk(0x1p-27f, 0x1p-27f)), s3, e3);
-                            const f2 L = fma2(fma2(G[6], c9, G[5]), c9, G[4]);
-                            const f2 lo = add2(add2(e1, e2), fma2(L, pk(0x1p-36f, 0x1p-36f), e3));
+                            f2 s1, e1, s2, e2, s3, e3, s4, e4;
+                            add_group(G[0], G[1], c9, s1, e1);
+                            add_group(s1, G[2], pk(0x1p-18f, 0x1p-18f), s2, e2);
+                            add_group(s2, G[3], pk(0x1p-27f, 0x1p-27f), s3, e3);
+                            add_group(s3, G[4], pk(0x1p-36f, 0x1p-36f), s4, e4);
+                            const f2 L = fma2(fma2(G[7], c9, G[6]), c9, G[5]);
+                            const f2 lo = add2(add2(e1, e2), add2(e3, fma2(L, pk(0x1p-45f, 0x1p-45f), e4)));
                             const f2 scale = *reinterpret_cast<const f2 *>(sc + 2 * x);
                             // + (alpha + E_aa alpha), the largest terms: three float-float numbers
                             const f2 dh = *reinterpret_cast<const f2 *>(sc + K + 2 * x);
@@ -495,8 +522,8 @@ __global__ void __launch_bounds__(FF_THREADS, 1) k_prune_ff(PruneArgs a, size_t 
                             pl = fma2(dh, al[x], pl);
                             pl = fma2(dl, ah[x], pl);
                             f2 t, e, u, f, uh, ul;
-                            two_sum2(ah[x], p, t, e);
-                            two_sum2(t, mul2(s3, scale), u, f);
+                            fast_two_sum2(ah[x], p, t, e);      // |E_aa| < 1
+                            two_sum2(t, mul2(s4, scale), u, f);
                             fast_two_sum2(u, add2(add2(al[x], pl), add2(e, fma2(lo, scale, f))), uh, ul);
                             if (have) ff_mul2(vh[x], vl[x], uh, ul, vh[x], vl[x]);
                             else { vh[x] = uh; vl[x] = ul; }
@@ -632,15 +659,16 @@ cudaError_t launch_split_ff(const double *in, void *out, int nps, int nbr, int n
     return cudaGetLastError();
 }
 
-size_t prune_ff_smem_bytes(int nl, int nint) { return ff_smem(nl, nint); }
+size_t prune_ff_smem_bytes(int nl, int nint) { return ff_smem(nl, nint, ff_lv_fits(nl, nint)); }
 
 cudaError_t launch_prune_ff(const PruneArgs &a, float *stack, int *err, cudaStream_t s, int grid)
 {
     if (a.nwi <= 0) return cudaSuccess;
-    const size_t smem = ff_smem(a.nl, a.n_internal);
+    const bool lv = ff_lv_fits(a.nl, a.n_internal);
+    const size_t smem = ff_smem(a.nl, a.n_internal, lv);
     cudaError_t e = allow_smem<k_prune_ff>();
     if (e != cudaSuccess) return e;
-    k_prune_ff<<<grid, FF_THREADS, smem, s>>>(a, ff_pset_bytes(a.nl, a.nbr), stack, err);
+    k_prune_ff<<<grid, FF_THREADS, smem, s>>>(a, ff_pset_bytes(a.nl, a.nbr), stack, err, lv);
     return cudaGetLastError();
 }
 
