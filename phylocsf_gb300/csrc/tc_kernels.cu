@@ -91,7 +91,6 @@ struct TcNode {
 };
 constexpr int TN_LEAVES = 1, TN_LEAF = 2;    // two leaves; one leaf (lc)
 constexpr int TN_PUSH = 4;                   // the next node does not take the partial: it waits on the stack
-constexpr int TN_PAIR = 8;                   // the next node has two leaves
 static __host__ __device__ size_t tc_sched_bytes(int nint) { return ((size_t)nint * (sizeof(TcNode) + 2) + 15) & ~(size_t)15; }
 
 __device__ const __align__(32) float ones_row[K] = {
@@ -159,10 +158,7 @@ __global__ void __launch_bounds__(TCP_THREADS, 2) k_prune_tc(PruneArgs a, float 
         t.lc = ll || !rl ? sn.lc : sn.rc;
         t.rc = ll || !rl ? sn.rc : sn.lc;
         t.flags = (ll && rl ? TN_LEAVES : ll || rl ? TN_LEAF : 0);
-        if (f + 1 < a.n_internal) {
-            if (nx.lc != sn.node && nx.rc != sn.node) t.flags |= TN_PUSH;
-            if (nx.lslot < 0 && nx.rslot < 0) t.flags |= TN_PAIR;
-        }
+        if (f + 1 < a.n_internal && nx.lc != sn.node && nx.rc != sn.node) t.flags |= TN_PUSH;
         sched[f] = t;
     }
     if (tid == 0) {
@@ -330,7 +326,6 @@ __global__ void __launch_bounds__(TCP_THREADS, 2) k_prune_tc(PruneArgs a, float 
             if (fl & TN_LEAVES) {
                 leaf_rows(sn.lc, v);
                 leaf_rows(sn.rc, x);
-                
 #pragma unroll
                 for (int j = 0; j < 16; j++) v[j] = mul2(v[j], x[j]);
             } else {
@@ -521,9 +516,9 @@ bool prune_tc_shape_ok(int shape) { return shape >= 0 && shape < PCSF_TC_SHAPES;
 size_t prune_tc_smem_bytes(int nl, int nint) { return SM_SCHED + tc_sched_bytes(nint) + (size_t)nl * LV_STRIDE; }
 
 template <int NPROD>
-static cudaError_t set_tc_attributes(size_t smem)
+static cudaError_t set_tc_attributes()
 {
-    // the whole unified L1 as shared memory, so that three CTAs of ~75 KB fit
+    // the whole unified L1 as shared memory, so that the two CTAs that tensor memory allows fit on every tree
     cudaError_t e = cudaFuncSetAttribute(k_prune_tc<NPROD>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                          (int)cudaSharedmemCarveoutMaxShared);
     if (e == cudaSuccess)
@@ -563,7 +558,7 @@ template <int NPROD>
 static cudaError_t launch_tc(const PruneArgs &a, float *stack, int *err, cudaStream_t s, int grid)
 {
     const size_t smem = prune_tc_smem_bytes(a.nl, a.n_internal);
-    cudaError_t e = set_tc_attributes<NPROD>(smem);
+    cudaError_t e = set_tc_attributes<NPROD>();
     if (e != cudaSuccess) return e;
     k_prune_tc<NPROD><<<grid, TCP_THREADS, smem, s>>>(a, stack, err);
     return cudaGetLastError();
