@@ -629,7 +629,7 @@ static int engine_init_common(pcsf_engine *e, const pcsf_tree *tree, int32_t fla
         if (k + 1 < e->sched.size() && e->sched[k + 1].lc != sn.node && e->sched[k + 1].rc != sn.node) waiting++;
         e->depth = std::max(e->depth, (int)waiting);
     }
-    e->sm_count = prop.multiProcessorCount;
+    e->sm_count = e->dm.sm_count = prop.multiProcessorCount;
     e->jac_cluster = jacobi_max_cluster();
     e->smem_optin = prop.sharedMemPerBlockOptin;
     CK(e->derr.reserve(1), "cudaMalloc");
@@ -2032,6 +2032,7 @@ static int dyn_prepare(pcsf_engine *e, DynModels &dmod, const std::vector<OmegaK
     dmod.dm.wlog = dd(o_wl);
     dmod.dm.tol = e->tol;
     dmod.dm.grid_n = 0;
+    dmod.dm.sm_count = e->sm_count;
     return PCSF_OK;
 }
 

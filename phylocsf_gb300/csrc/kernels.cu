@@ -272,7 +272,7 @@ cudaError_t launch_jacobi(const double *A, double *U, double *lam, int *status, 
 
 constexpr int PF_THREADS = 256;
 constexpr int PF_BRANCHES = 2;   // most branches per CTA (the eigenvectors are staged once)
-constexpr int PF_SPREAD = 2 * 4 * 152;   // FP32 matrices of a launch up to which each gets its own CTA
+constexpr int PF_SPREAD = 2 * 4;         // FP32 matrices of a launch, per SM, up to which each gets its own CTA
 
 // shared memory (dynamic): U^T, with FP64 U^T times the coefficients, per branch E^T and the coefficients
 template <typename T> __host__ __device__ constexpr size_t pform_smem(int per_cta)
@@ -518,7 +518,7 @@ cudaError_t launch_pform(bool fp64, const PSet *req, int nreq, const double *bra
     // for short FP32 launches, which more would leave on a part of the SMs.  Measured: FP64,
     // 24 P sets of 29 leaves 0.95 -> 0.69 ms, six of 12 leaves 0.36 -> 0.13 ms; FP32, two P
     // sets of 12 leaves 39 -> 17 us.
-    const int per_cta = (fp64 || (int64_t)nreq * nbr <= PF_SPREAD) ? 1 : PF_BRANCHES;
+    const int per_cta = (fp64 || (int64_t)nreq * nbr <= (int64_t)PF_SPREAD * m.sm_count) ? 1 : PF_BRANCHES;
     dim3 grid((nbr + per_cta - 1) / per_cta, nreq);
     if (fp64) {
         const size_t smem = pform_smem<double>(per_cta);

@@ -67,6 +67,7 @@ struct DevModels {
     double grid_lr;         // log of the grid ratio
     const float *Qf;        // [2][K][K]  Q (row-major)
     const float *Q2f;       // [2][K][K]  Q^2
+    int sm_count;           // the device's, for the split of a P(t) launch
 };
 
 // Lets Kernel be launched with any dynamic shared memory that fits beside its static share.  The limit

@@ -48,7 +48,7 @@ constexpr uint32_t PFT_A = 32768;      // [128 x 64]  A_lo, 32 KB
 constexpr uint32_t PFT_SMEM = 65536;
 constexpr uint32_t PFT_TMEM_COLS = 128;   // D in 0..63, A_hi in 64..127
 constexpr int PFT_MAX_BRANCHES = 320;
-constexpr int PFT_TARGET = 4 * 3 * 152;   // CTAs of a launch: four waves of three per SM
+constexpr int PFT_TARGET = 4 * 3;      // CTAs of a launch per SM: four waves of three
 
 // diag -= x by Kahan's summation except where j == i, with the low part in dc: the last two of four
 // additions are predicated, so nothing but them is on the chain
@@ -273,12 +273,12 @@ cudaError_t launch_pform_tc(const PSet *ps, int nps, const double *branch, int n
     if (e != cudaSuccess) return e;
     // Branch pairs per CTA: all of a P set's when there are enough P sets to fill the GPU
     // several times over, fewer for a short list (one exon's search round asks for two to six
-    // P sets): about PFT_TARGET CTAs in all, at the price of one 32 KB fetch of B per CTA.
+    // P sets): about PFT_TARGET CTAs per SM in all, at the price of one 32 KB fetch of B per CTA.
     // Measured, P(t) of one mle call on 58 leaves: 1 region (2-6 P sets a round) 5.1 -> 0.28 ms,
     // 384 regions (~800 P sets a round: 1.7 waves before, three CTAs per P set now) 20.0 -> 14.6 ms,
     // both before the chain was shortened.
     const int pairs = (nbr + 1) / 2;
-    const int want = std::min(pairs, std::max(1, (PFT_TARGET + nps - 1) / nps));
+    const int want = std::min(pairs, std::max(1, (PFT_TARGET * m.sm_count + nps - 1) / nps));
     const int per_cta = 2 * ((pairs + want - 1) / want);
     const dim3 grid(nps, (nbr + per_cta - 1) / per_cta);
     k_pform_tc<<<grid, PFT_THREADS, PFT_SMEM, s>>>(ps, branch, nbr, nl, m, Bpf, Pbuf, Bop, status_key, err, per_cta,
