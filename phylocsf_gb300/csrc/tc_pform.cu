@@ -251,9 +251,11 @@ __global__ void __launch_bounds__(PFT_THREADS, 3) k_pform_tc(const PSet *ps, con
         tc_fence_after();
     }
     if (__syncthreads_or(!ok)) ok = false;
-    if (!ok && tid == 0) atomicExch(err, 1);
     // bounded again: the first fetch and the last MMAs may still be on their way after a wait that ran out
-    if (tid == 0) mbar_wait(barB, 0);
+    if (!ok && tid == 0) {
+        atomicExch(err, 1);
+        mbar_wait(barB, 0);
+    }
     if (pending) mbar_wait(barM, ph ^ 1u);
     tc_fence_before();
     __syncthreads();
