@@ -257,8 +257,11 @@ void pcsf_batch_destroy(pcsf_batch *b);
  * lockstep rounds on the device).  out: [n_regions]. */
 int pcsf_score(pcsf_engine *e, pcsf_batch *b, int32_t strategy, pcsf_result *out);
 
-/* One-shot scoring from host buffers: upload, score, free.  This is the call
- * a batching ForkMaybe.map would make over its region list (PhyloCSF.ml:317). */
+/* One-shot scoring from host buffers: upload and score; the engine keeps a leaf
+ * buffer of up to 64 MiB for the next call.  An invalid leaf code is refused
+ * before any search, with pcsf_batch_create's error, and out is not written.
+ * This is the call a batching ForkMaybe.map would make over its region list
+ * (PhyloCSF.ml:317). */
 int pcsf_score_batch(pcsf_engine *e, int32_t n_regions, const int64_t *col_offsets, const uint8_t *leaves,
                      int32_t strategy, pcsf_result *out);
 
@@ -290,7 +293,8 @@ int pcsf_grad(pcsf_engine *e, pcsf_batch *b, int32_t model, const double *rho, d
  * the columns as PhyloEM.collect_sufficient_statistics does (lib/CamlPaml/PhyloEM.ml:14-20).
  * Each branch's counts sum to the number of columns with z > 0.  counts:
  * [n_regions][2*n_leaves-2][64][64]; lpr and status ([n_regions]) may be NULL.
- * Computed in FP64 on the FP64 engine, in FP32 with compensated sums otherwise. */
+ * Computed in FP64 on the FP64 engine, in FP32 with compensated sums otherwise; a region's
+ * results do not depend on the call's other regions. */
 int pcsf_branch_counts(pcsf_engine *e, pcsf_batch *b, int32_t model, const double *rho, double *counts, double *lpr,
                        int32_t *status);
 

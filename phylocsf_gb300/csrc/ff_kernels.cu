@@ -55,7 +55,7 @@
 // whose two halves of the tree hold codons three substitutions apart, the entries that matter
 // lie 2^-20 and more below those.  Against the FP64 engine on the same P(t), the lpr of such a
 // column on 58 leaves is off by 1e-14, 3e-14 and 2e-13 at rho = 1, 0.1 and 0.01 (with six digits
-// 1e-12, 1e-11 and 1e-10), a thousandth and less of what the FP64 formation of P(t) leaves there.
+// 1e-12, 1e-11 and 1e-10); the FP64 formation of P(t) itself leaves 8e-12, 7e-11 and 7e-10 there.
 // The lpr of regions is within 6e-16 relative at rho >= 1 and 5e-14 at rho = 0.01, where two
 // independent FP64 evaluations differ by 2e-12.
 #include <algorithm>
