@@ -259,7 +259,8 @@ int pcsf_score(pcsf_engine *e, pcsf_batch *b, int32_t strategy, pcsf_result *out
 
 /* One-shot scoring from host buffers: upload and score; the engine keeps a leaf
  * buffer of up to 64 MiB for the next call.  An invalid leaf code is refused
- * before any search, with pcsf_batch_create's error, and out is not written.
+ * with pcsf_batch_create's error, after the first evaluation at the latest, and
+ * out is not written.
  * This is the call a batching ForkMaybe.map would make over its region list
  * (PhyloCSF.ml:317). */
 int pcsf_score_batch(pcsf_engine *e, int32_t n_regions, const int64_t *col_offsets, const uint8_t *leaves,

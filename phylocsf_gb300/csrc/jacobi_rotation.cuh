@@ -61,8 +61,9 @@ __device__ __forceinline__ double sqrt_rn(double x, double y)
 // Quotients and roots are seeds (above) with one residual correction in FP64 (Markstein, IBM J. Res.
 // Dev. 34 (1990) 111): an error of ~2^-88 before the final rounding, so that, with the ties that
 // recip_rn and sqrt_rn settle, they round as the library's do (it would take about 2^35 operations to
-// meet one that does not), in 5 x 69 + 90 clocks for a root and its reciprocal instead of 705 + 459.  Operands far from 1, a theta that may
-// overflow (its correction would make a NaN of it) and |theta| beyond 2^300 take the library's operations.
+// meet one that does not), in 5 x 69 + 90 clocks for a root and its reciprocal instead of 705 + 459
+// (the ties cost the omega test of six alignments 2 %).  Operands far from 1, a theta that may overflow
+// (its correction would make a NaN of it) and |theta| beyond 2^300 take the library's operations.
 __device__ __forceinline__ void jac_rotation(double app, double aqq, double apq, double &c, double &s)
 {
     const double num = aqq - app, den = 2.0 * apq, ad = fabs(den);
