@@ -67,7 +67,7 @@ struct GradLayout {
     {
         size_t b = sizeof(T) * ((size_t)K2 + (npar ? (size_t)K2 + 3 * K : 0) + region(nslots, npar) + reds(npar));
         b += sizeof(double) * (3 * TC + 2 * (1 + npar) * GR_WARPS);
-        b += sizeof(typename AtomMax<T>::U) * 2 * TC + sizeof(int) * (5 * TC + (size_t)nslots * TC);
+        b += sizeof(typename AtomMax<T>::U) * 2 * TC + sizeof(int) * ((npar ? 4 : 5) * TC + (size_t)nslots * TC);
         b += sizeof(SchedNode) * nint;
         b = (b + 15) & ~size_t(15);
         b += (size_t)nl * TC;
@@ -110,7 +110,8 @@ __global__ void __launch_bounds__(GR_THREADS, sizeof(T) == 4 ? 2 : 1) k_grad(Gra
     int *eroot = reinterpret_cast<int *>(colmax + 2 * TC);          // [TC]
     int *ebase = eroot + TC;                                        // [2][TC] f(p) + e(s), by side: one side's is read
                                                                     //   (by half a warp) while the next side's is written
-    int *wexp = ebase + 2 * TC;                                     // [2][TC] the weight's exponent where 2^ex / z~ may not be normal, else 0
+                                                                    //   (npar: a barrier apart, [TC] for both)
+    int *wexp = ebase + (npar ? 1 : 2) * TC;                        // [2][TC] the weight's exponent where 2^ex / z~ may not be normal, else 0
     int *slexp = wexp + 2 * TC;                                        // [nslots][TC] exponents of the slots' partials
     SchedNode *sched = reinterpret_cast<SchedNode *>(slexp + a.nslots * TC);   // [n_internal]
     size_t off = (reinterpret_cast<unsigned char *>(sched + a.n_internal) - gsm + 15) & ~size_t(15);
@@ -334,6 +335,7 @@ __global__ void __launch_bounds__(GR_THREADS, sizeof(T) == 4 ? 2 : 1) k_grad(Gra
                 const int s = side ? sn.lc : sn.rc;
                 const bool internal = c >= nl;
                 const int buf = sidx & 1;
+                int *eb_side = ebase + (npar ? 0 : buf * TC);
                 if (side && npar) __syncthreads();     // the last side is finished with X, E^T and H
                 if (internal) stage_rows<T, GR_THREADS>(Er, Pbase + (size_t)c * K2, tid);
                 const T *Hg = reinterpret_cast<const T *>(a.Hmat) + ((size_t)rq.pset * a.nbr + c) * npar * K2;
@@ -380,7 +382,7 @@ __global__ void __launch_bounds__(GR_THREADS, sizeof(T) == 4 ? 2 : 1) k_grad(Gra
                 }
                 if (tid < TC) {
                     const int eb = fS[(size_t)p * TC + tid] + e_of(s, tid);
-                    ebase[buf * TC + tid] = eb;
+                    eb_side[tid] = eb;
                     const int ex = eb + e_of(c, tid) - eroot[tid];
                     const bool far = ex <= -900 || ex >= 900;
                     wcol[buf * TC + tid] = far ? zt[tid] : zt[tid] * __hiloint2double((ex + 1023) << 20, 0);
@@ -455,7 +457,7 @@ __global__ void __launch_bounds__(GR_THREADS, sizeof(T) == 4 ? 2 : 1) k_grad(Gra
                     for (int cc = 0; cc < CPT; cc++) {
                         const T mx = AtomMax<T>::get(cm + c0 + cc);
                         ecol[cc] = (mx > (T)0) ? exp_of(mx) : 0;
-                        if (ty == 0) fS[(size_t)c * TC + c0 + cc] = ebase[buf * TC + c0 + cc] + ecol[cc];
+                        if (ty == 0) fS[(size_t)c * TC + c0 + cc] = eb_side[c0 + cc] + ecol[cc];
                     }
 #pragma unroll
                     for (int i = 0; i < 4; i++) {

@@ -220,3 +220,28 @@ def test_gradient_map_100vertebrates_beside_brent_and_omega_mle():
     long = np.diff(wl.col_offsets) >= 1500
     assert np.all(np.abs(np.log(fo["omega"][long] / wl.omega[long])) <= np.log(1.35)), (fo["omega"], wl.omega)
     e.close()
+
+
+def test_omega_grad_largest_tree():
+    """The FP64 adjoint with rate parameters on 512 leaves and three partial slots, the tree that asks for
+    most shared memory: central differences as above, their evaluation noise (1e-12 of lpr over h)
+    counted from lpr, and the chain rule between branches and tree scale."""
+    rng = np.random.default_rng(512)
+    t = "((((s0:.05,s1:.07):.01,(s2:.04,s3:.02):.02):.01,((s4:.03,s5:.06):.01,(s6:.05,s7:.02):.02):.01):.02,s8:.05)"
+    for k in range(9, 512):
+        t = "(%s:%.4f,s%d:%.4f)" % (t, rng.uniform(0.0, 0.01), k, rng.uniform(0.005, 0.1))
+    tree = P.Tree.from_newick(t)
+    ps = synth.load_params("12flies")
+    par = synth.ParamSet("t", tree, ps.S_c, ps.pi_c, ps.S_n, ps.pi_n)
+    offs, leaves = synth.simulate(par, np.array([7]), np.zeros(1, np.int32), None, 5)
+    e = P.Engine.for_tree(tree, precision="fp64")
+    b = e.batch(offs, leaves)
+    kappa, omega, rho, sigma, h = 2.5, 0.3, 0.8, 1.0, 1e-5
+    g = e.omega_grad(b, kappa, omega, rho, sigma)
+    assert (g["status"] == 0).all()
+    for k, v in enumerate(("d_kappa", "d_omega", "d_rho")):
+        lp, lm = (e.omega_grad(b, kappa + s * (k == 0), omega + s * (k == 1), rho + s * (k == 2), sigma,
+                               branches=False)["lpr"] for s in (h, -h))
+        fd = (lp - lm) / (2 * h)
+        assert np.all(np.abs(g[v] - fd) <= 1e-5 * np.abs(fd) + 1e-12 * np.abs(g["lpr"]) / h), (v, g[v], fd)
+    assert np.allclose(g["d_branch"] @ tree.branch[: tree.n - 1], g["d_rho"], rtol=1e-12, atol=1e-12)
