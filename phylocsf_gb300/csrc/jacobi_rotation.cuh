@@ -40,8 +40,11 @@ __device__ __forceinline__ double rsqrt_seed(double d)
 // off by ~2^-36 of the last place before its rounding.  That does not tell the side of a tie where the
 // operand lies few last places from a power of two or four, as 1 + theta^2 does for every theta below
 // 2^-21.  There the value is known: 1 / (1 - k 2^-53) = 1 + k 2^-53 + k^2 2^-106, for odd k just above the
-// tie, sqrt(1 + k 2^-52) = 1 + k 2^-53 - k^2 2^-107 and sqrt(1 - k 2^-53) = 1 - k 2^-54 - k^2 2^-109 just
-// below: half of k, rounded up or down, in the bits of the result (b: the operand's, less those of 1.0).
+// tie, and half of k, rounded up, in the bits of the result (b: the operand's, less those of 1.0).
+// sqrt(1 + k 2^-52) = 1 + k 2^-53 - k^2 2^-107 and sqrt(1 - k 2^-53) = 1 - k 2^-54 - k^2 2^-109 lie for odd k
+// just below the tie, so that they round as the root of the operand with its last bit cleared, whose own
+// value is next to a double: settle_root clears it.  (After the correction, the same choice between two
+// results lengthened a round of the eigensolver by about 60 clocks instead of 25.)
 constexpr long long ONE_BITS = 1023ll << 52, NEAR_BITS = 1ll << 20;
 __device__ __forceinline__ double recip_rn(double d, double y)
 {
@@ -49,20 +52,26 @@ __device__ __forceinline__ double recip_rn(double d, double y)
     const double v = __fma_rn(y, __fma_rn(-d, y, 1.0), y);
     return k < NEAR_BITS ? __longlong_as_double(ONE_BITS - (b + k) + ((k + 1) >> 1)) : v;
 }
+__device__ __forceinline__ double settle_root(double x)
+{
+    // the exponent's lowest bit, as an even power's, and the 31 bits after it all zeros or all ones
+    const int hi = __double2hiint(x), lo = __double2loint(x);
+    const bool near = __funnelshift_l(lo, hi - (int)(ONE_BITS >> 32), 11) + 1u <= 1u;
+    return __hiloint2double(hi, near ? lo & ~1 : lo);
+}
 __device__ __forceinline__ double sqrt_rn(double x, double y)
 {
-    const long long b = __double_as_longlong(x) - ONE_BITS;
-    const double g = x * y, v = __fma_rn(__fma_rn(-g, g, x), 0.5 * y, g);
-    return ((b + NEAR_BITS) & ((1ll << 53) - 1)) < 2 * NEAR_BITS ? __longlong_as_double(ONE_BITS + (b >> 1)) : v;
+    const double g = x * y;
+    return __fma_rn(__fma_rn(-g, g, x), 0.5 * y, g);
 }
 
 // The rotation (c, s) that annihilates apq != 0: theta = (aqq - app) / (2 apq), t = sign(theta) /
 // (|theta| + sqrt(theta^2 + 1)), c = 1 / sqrt(t^2 + 1), s = t c, each operation rounded to nearest.
 // Quotients and roots are seeds (above) with one residual correction in FP64 (Markstein, IBM J. Res.
 // Dev. 34 (1990) 111): an error of ~2^-88 before the final rounding, so that, with the ties that
-// recip_rn and sqrt_rn settle, they round as the library's do (it would take about 2^35 operations to
+// recip_rn and settle_root settle, they round as the library's do (it would take about 2^35 operations to
 // meet one that does not), in 5 x 69 + 90 clocks for a root and its reciprocal instead of 705 + 459
-// (the ties cost the omega test of six alignments 2 %).  Operands far from 1, a theta that may overflow
+// (the ties cost the omega test of six alignments 1 %).  Operands far from 1, a theta that may overflow
 // (its correction would make a NaN of it) and |theta| beyond 2^300 take the library's operations.
 __device__ __forceinline__ void jac_rotation(double app, double aqq, double apq, double &c, double &s)
 {
@@ -78,7 +87,7 @@ __device__ __forceinline__ void jac_rotation(double app, double aqq, double apq,
     }
     double t;
     if (fabs(theta) < 0x1p300) {
-        const double x = __fma_rn(theta, theta, 1.0);
+        const double x = settle_root(__fma_rn(theta, theta, 1.0));
         const double d = fabs(theta) + sqrt_rn(x, rsqrt_seed(x));
         t = recip_rn(d, recip_seed(d));
         if (!(theta >= 0.0)) t = -t;
@@ -86,7 +95,7 @@ __device__ __forceinline__ void jac_rotation(double app, double aqq, double apq,
         t = (fabs(theta) > 1e150) ? 0.5 / theta
             : (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(__fma_rn(theta, theta, 1.0)));
     }
-    const double u = __fma_rn(t, t, 1.0);          // in [1, 2]
+    const double u = settle_root(__fma_rn(t, t, 1.0));      // in [1, 2]
     const double y = rsqrt_seed(u), v = sqrt_rn(u, y);
     c = __fma_rn(y, __fma_rn(-v, y, 1.0), y);
     s = t * c;
